@@ -465,7 +465,7 @@ def run_chunked_prefill(args):
                        "shared_prefix_tokens": prefix, "copy_on_write_tail_pages": cow_copies},
             "roofline": {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                          "peak_kind": f"of {kind} (sustained bf16)",
-                         "kernel": "tq4_attention_prefill_exact_kernel (register MMAs, value + residual operands, 128-row CTAs)", "traffic": None,
+                         "kernel": "attention_prefill_pair_kernel (tcgen05 over CTA pairs, value + residual operands, 256-row tiles)", "traffic": None,
                          "attention_ms_rank0": attn_ms},
             "append_tokens_per_s": n_tok / (app_ms * 1e-3) if app_ms > 0 else None,
             "prefill_tokens_per_s": tot_tok / (ms * 1e-3), "gpu_launches": 2 * len(evs),

@@ -208,7 +208,8 @@ int warp34_fused_k_rmsnorm_rope_kv_cache_write_f16(
  * selects the fp32 kernel, which stays below a seventh of the bound on all of these.
  * WARP34_B200_EXEC_FLAG_FAST_ATTENTION trades the residual operands for speed.  Kernels: decode and verify batches
  * (up to 24 query rows per request and kv head) stream split-KV work items of 8 rows; larger
- * chunks take a 128-row prefill kernel (register MMAs; tcgen05 + TMEM with the fast flag).
+ * chunks, of TQ4 and of 8-bit layers, take a tcgen05 kernel of two CTAs and 256 rows (TQ4 with the fast flag: one
+ * CTA, 128 rows, single operands).
  * 8-bit boundary layers (Q8_0, FP8 E4M3) in the canonical packing stream the same way on a
  * tensor-core kernel whose operands are exact (codes convert exactly to fp16); other packings of
  * them, callers without scratch and WARP34_B200_EXEC_FLAG_PRECISE_ATTENTION take an fp32 kernel.
@@ -233,8 +234,8 @@ int warp34_paged_attention_scalar_f16(const warp34_exec* ex, const warp34_kv_lay
  * Test-only kernel selector.  Replaces warp34_paged_attention_f16_force_kernel_for_test
  * (op_paged_attn.cu:1451-1458), against which the reference's variant-equality tests link
  * (crates/warp34-host/src/cuda/tests.rs:111-576).  use_64q: 0 = the reference's 16-row kernel,
- * here the 8-row split-KV items; 1 = its 64-row prefill kernel, here the 128-row register-MMA
- * prefill kernel; 2 = its 128-row prefill kernel, here the 128-row tcgen05 kernel.  The
+ * here the 8-row split-KV items; 1 = its 64-row prefill kernel, here the two-CTA, 256-row
+ * value + residual kernel; 2 = its 128-row prefill kernel, here the 128-row tcgen05 kernel.  The
  * reference's three variants share their arithmetic and are compared at 0 ULP; these do not:
  * selectors 0 and 1 meet 2e-3 + 1e-2 |b| against dequant-then-attend on every element,
  * selector 2 computes with single fp16 operands (see WARP34_B200_EXEC_FLAG_FAST_ATTENTION).
@@ -254,7 +255,8 @@ int warp34_paged_attention_f16_force_kernel_for_test(const warp34_exec* ex, cons
  * attention output through HBM.  gate and out are fp16 [total_tokens, num_q_heads, 256]; out may
  * not alias q_in.  Rounding follows the two-kernel sequence (attention output to fp16, gated value
  * to fp16 before the Hadamard); masked rows of out are left untouched.  TQ4 layers apply the
- * epilogue inside the merge / prefill kernels, 8-bit layers in a second launch in place.
+ * epilogue inside the merge / prefill kernels, as do chunks of 8-bit layers; decode batches of those run it as a
+ * second launch in place.
  */
 int warp34_paged_attention_gated_f16(const warp34_exec* ex, const warp34_kv_layer_layout* layout,
                                      const warp34_attention_batch* batch,

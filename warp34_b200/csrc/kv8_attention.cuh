@@ -322,24 +322,6 @@ __device__ __forceinline__ uint2 lds64_dep(uint32_t addr, uint32_t token) {
     asm("ld.shared.v2.u32 {%0,%1}, [%2+0];  // dep %3" : "=r"(v.x), "=r"(v.y) : "r"(addr), "r"(token));
     return v;
 }
-// Four 8-bit codes -> two fp16 pairs (bytes 0,1 and bytes 2,3), exactly.
-template <int FMT>
-__device__ __forceinline__ void kv8x4_to_f16x4(uint32_t w, uint32_t& lo, uint32_t& hi) {
-    if (FMT == WARP34_KV_FORMAT_FP8_E4M3) {
-        asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tcvt.rn.f16x2.e4m3x2 %0, l;\n\tcvt.rn.f16x2.e4m3x2 %1, h;\n\t}"
-            : "=r"(lo), "=r"(hi) : "r"(w));
-    } else {
-        const uint32_t x = w ^ 0x80808080u;                               // q + 128 as an unsigned byte
-        const uint32_t l = __byte_perm(x, 0x64646464u, 0x4140);           // halves 1024 + (q + 128)
-        const uint32_t h = __byte_perm(x, 0x64646464u, 0x4342);
-        const __half2 bias = __half2half2(__ushort_as_half((unsigned short)0x6480));   // 1152
-        const __half2 lh = __hsub2(*reinterpret_cast<const __half2*>(&l), bias);
-        const __half2 hh = __hsub2(*reinterpret_cast<const __half2*>(&h), bias);
-        lo = *reinterpret_cast<const uint32_t*>(&lh);
-        hi = *reinterpret_cast<const uint32_t*>(&hh);
-    }
-}
-
 // SPARSE: the query-sparse lists of warp34_qsa_sparse_paged_attn_f16 (see the TQ4 stream kernel): request r
 // is token r, a unit is four entries of its selected list, lanes 0-3 copy their entry's four rows and leave
 // its first position in 16 bytes behind the stage.
@@ -822,10 +804,10 @@ static bool kv8_attention_layout_ok(const warp34_kv_layer_layout* l) {
            l->k_transform == WARP34_KV_TRANSFORM_IDENTITY && l->v_transform == WARP34_KV_TRANSFORM_IDENTITY;
 }
 
-// The tensor-core path serves K and V of one 8-bit format in the canonical packing with 16-byte-aligned
-// runs, an 8-byte-aligned query and a workspace that holds the plan and at least one CTA's partial slots.
-static bool kv8_stream_ok(const warp34_exec* ex, const warp34_kv_layer_layout* l, const warp34_attention_batch* b,
-                          const void* q_in, int io_bf16) {
+// The tensor-core paths serve K and V of one 8-bit format in the canonical packing with 16-byte-aligned
+// runs; the stream kernel also needs an 8-byte-aligned query and a workspace that holds the plan and at least
+// one CTA's partial slots.
+static bool kv8_canonical(const warp34_kv_layer_layout* l) {
     if (l->k_format != l->v_format) return false;
     const uint64_t row = l->k_format == WARP34_KV_FORMAT_FP8_E4M3 ? (uint64_t)Kv8Stage<WARP34_KV_FORMAT_FP8_E4M3>::kRow
                                                                   : (uint64_t)Kv8Stage<WARP34_KV_FORMAT_Q8_0>::kRow;
@@ -834,6 +816,11 @@ static bool kv8_stream_ok(const warp34_exec* ex, const warp34_kv_layer_layout* l
          l->v_head_stride_bytes) & 15u) {
         return false;
     }
+    return true;
+}
+static bool kv8_stream_ok(const warp34_exec* ex, const warp34_kv_layer_layout* l, const warp34_attention_batch* b,
+                          const void* q_in, int io_bf16) {
+    if (!kv8_canonical(l)) return false;
     if (!io_bf16 && ((uintptr_t)q_in & 7u) != 0) return false;
     if (b->block_tables == nullptr || b->max_blocks_per_req <= 0) return false;
     return ex->scratch_ptr != 0 && (ex->scratch_ptr & 15u) == 0;

@@ -1,0 +1,713 @@
+// Chunked-prefill attention on the 5th-generation tensor cores at the accuracy of fp32 dequant-then-attend:
+// every operand is fed to tcgen05.mma as fp16 value + fp16 rounding residual.  Included by tq4_attention.cu
+// (shares the PTX wrappers, the geometry helpers and the epilogue).
+//
+// Replaces paged_attention_prefill_mma_f16_kernel<64 / 128> (crates/warp34-kernels/csrc/ops/
+// op_paged_attn.cu:594-1128) for head_dim 256, 16-token pages, canonical packing of TQ4, FP8 E4M3 or Q8_0 rows.
+//
+// A cluster of two CTAs (cta_group::2, one SM each) owns 256 query rows (256 / gqa tokens x gqa heads of one kv
+// head), 128 rows per CTA, and walks the keys its rows can see in blocks of 64.  The two SMs share every K and V
+// tile: each CTA dequantises half of it (K: 32 of the 64 keys; V: 128 of the 256 channels) and the MMA reads both
+// halves, so a code is dequantised once per 256 query rows.
+//
+//   warps 0-3   consumers: thread = query row = TMEM lane: scores from TMEM, online softmax with a lazily moved
+//               reference maximum, P written over its scores as fp16 value (columns 0-31) and residual (32-63)
+//   warps 4-7   K producers, warps 8-11 V producers: lane = key, warp = 32 of the stage's 128 channels
+//   warp 12     (CTA 0) issues every MMA; the scores of block j + 1 ahead of the output product of block j
+//   warp 13     bulk-copies the raw (page, head) runs
+//
+//   S[256 x 64]   = Q'hi Khi^T + Q'lo Khi^T + Q'hi Klo^T      A in TMEM (Q'hi) or shared memory (Q'lo)
+//   O[256 x 256] += Phi Vhi + Plo Vhi + Phi Vlo               A in TMEM
+//
+// K and V elements are row scale x centroid (or code): hi = fp16(d c), lo = fp16(d c - hi), about 22 bits together.
+// What bounds it: the tensor pipe under the power cap.  Six (TQ4) or five (8-bit) products per visible pair instead of
+// two; 8 x 2048 tokens after 8192 (16 / 4 heads) take 5.6 ms = 440 TFLOP/s of attention = 1320 TFLOP/s issued, against
+// 21.6 ms for register MMAs (mma.sync) over the same operands.  A pair rather than one CTA because dequantising once per
+// 128 rows would cost as many shared-memory cycles as the MMAs take.  The MMAs are issued by one elected thread
+// (elect.sync; with `lane == 0` as the condition each issue took about 45 cycles and the kernel 6.4 ms), and cross-CTA
+// arrivals use the default semantics (cluster-scope release / acquire put a memory barrier in front of each).
+// For 8-bit layers the query is neither rotated nor scaled: it is the fp16 operand as it arrives and has no residual.
+#pragma once
+
+namespace w34 {
+
+constexpr int kPpRows = 256;                         // query rows of a pair
+constexpr int kPpCtaRows = 128;
+constexpr int kPpKeys = 64;                          // keys of a block = 4 pages
+constexpr int kPpWarps = 14;
+constexpr int kPpThreads = kPpWarps * 32;
+constexpr int kPpStages = 3;                         // half-block stages of K and of V
+constexpr uint32_t kPpPart = 2u * 32u * 128u;        // 8192: [2 blocks of 64 channels][32 keys][128 B], value or residual
+constexpr uint32_t kPpStage = 2u * kPpPart;          // value + residual
+constexpr uint32_t kPpQLoBytes = 4u * kPpCtaRows * 128u;   // 65536: [4 blocks of 64 channels][128 rows][128 B]
+constexpr uint32_t kPpLutBytes = 256u * 128u;        // byte -> (value pair, residual pair), 16 lane copies of 8 bytes
+constexpr int kPpRawStages = 2;
+// Table factor: close to the fp16 grid (see kLutScale), and small enough that scale x centroid stays finite for every
+// fp16 scale.
+constexpr float kPpLutScale = 0.25f * kLutScale;
+constexpr float kPpRescaleThreshold = 8.0f;          // log2 units: the reference maximum may lag by this much
+constexpr float kPpShift = 6.0f;                     // P is carried times 2^6: at most 2^14, subnormal only below 2^-20
+constexpr uint32_t kPpColO = 0, kPpColS = 256, kPpColQ = 384;
+constexpr int kPpOutStride = 257;                    // floats per row of the epilogue staging
+
+template <int FMT> struct PpFormat;
+template <> struct PpFormat<WARP34_KV_FORMAT_TQ4> {
+    static constexpr uint32_t kRow = kTq4RowBytes;
+    static constexpr bool kRotated = true;
+};
+template <> struct PpFormat<WARP34_KV_FORMAT_FP8_E4M3> {
+    static constexpr uint32_t kRow = kHeadDim + 8;
+    static constexpr bool kRotated = false;
+};
+template <> struct PpFormat<WARP34_KV_FORMAT_Q8_0> {
+    static constexpr uint32_t kRow = 4 * 68;
+    static constexpr bool kRotated = false;
+};
+
+template <int FMT> struct PpSmem {
+    static constexpr uint32_t kRun = kPageTokens * PpFormat<FMT>::kRow;      // one (page, head) run
+    static constexpr uint32_t kRawK = 2u * kRun, kRawV = 4u * kRun;
+    static constexpr uint32_t kRaw = kRawK + kRawV;
+    static constexpr uint32_t kOffK = 0;
+    static constexpr uint32_t kOffV = kOffK + kPpStages * kPpStage;
+    static constexpr uint32_t kOffQLo = kOffV + kPpStages * kPpStage;
+    static constexpr uint32_t kOffRaw = kOffQLo + (PpFormat<FMT>::kRotated ? kPpQLoBytes : 0u);
+    static constexpr uint32_t kOffLut = (kOffRaw + kPpRawStages * kRaw + 127u) & ~127u;
+    static constexpr uint32_t kOffBars = kOffLut + (PpFormat<FMT>::kRotated ? kPpLutBytes : 0u);
+    static constexpr uint32_t kBytes = kOffBars + 256u;
+    static_assert(kPpCtaRows * kPpOutStride * 4 <= (int)kOffLut, "epilogue staging must end before the table");
+    static_assert(kPpCtaRows * 512 <= (int)kOffQLo, "Q' staging fits the tile stages");
+    static_assert(kBytes <= 227u * 1024u, "shared memory");
+};
+
+// barrier slots (8 bytes each).  Full / PReady: waited for by the MMA warp of CTA 0, arrivals from both CTAs.
+// Empty, S, Pv: one arrival per CTA from the MMA warp's commits.  Raw*: within a CTA.
+enum { kPpFullK = 0, kPpFullV = kPpFullK + kPpStages, kPpEmptyK = kPpFullV + kPpStages, kPpEmptyV = kPpEmptyK + kPpStages,
+       kPpS = kPpEmptyV + kPpStages, kPpPReady = kPpS + 2, kPpPv = kPpPReady + 2, kPpDrain, kPpRawKFull,
+       kPpRawKFree = kPpRawKFull + kPpRawStages, kPpRawVFull = kPpRawKFree + kPpRawStages,
+       kPpRawVFree = kPpRawVFull + kPpRawStages, kPpBarCount = kPpRawVFree + kPpRawStages };
+static_assert(kPpBarCount * 8 <= 240, "barrier slots end before the TMEM address and abort words");
+
+// ---- CTA-pair wrappers ------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t saddr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// One lane of a converged warp, chosen by the hardware: the compiler then knows that the branch runs in one thread.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+    return ok != 0;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tc2_alloc(uint32_t smem_dst, uint32_t ncols) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void tc2_relinquish() {
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tc2_dealloc(uint32_t taddr, uint32_t ncols) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void tc2_mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tc2_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+// One arrival on this barrier slot of both CTAs when every MMA issued so far by this thread has completed.
+__device__ __forceinline__ void tc2_commit_both(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void tc_ld16(uint32_t (&r)[16], uint32_t taddr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+                 :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+
+struct PrefillPairParams {
+    warp34_kv_layer_layout layout;
+    warp34_attention_batch batch;
+    const void* q_in;
+    void* attn_out;
+    int io_bf16;
+    int num_q_heads;
+    int gqa;
+    int tok_per_tile;      // 256 / gqa
+    float q_scale;         // TQ4: sm_scale * log2(e) / kPpLutScale, folded into Q'; 8-bit: sm_scale * log2(e), applied to the scores
+    int32_t* status;       // may be null; bit 0: a wait gave up, bit 1: shared-memory window misaligned
+    OutputGate og;
+};
+
+template <int FMT>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) attention_prefill_pair_kernel(const PrefillPairParams p) {
+    using S = PpSmem<FMT>;
+    constexpr bool ROT = PpFormat<FMT>::kRotated;
+    constexpr uint32_t ROW = PpFormat<FMT>::kRow;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const uint32_t rank = cluster_rank();
+    const uint32_t base = smem_u32(smem_raw);
+    uint8_t* gen = smem_raw;
+
+    // ---- which (request, token tile) is this pair?  Both CTAs agree on every exit here. -------------
+    const int tpt = p.tok_per_tile;
+    const int kv_head = blockIdx.y;
+    int req = -1, tile_in_req = 0;
+    {
+        int t = (int)(blockIdx.x >> 1);
+        for (int r = 0; r < p.batch.num_reqs; ++r) {
+            const int ql = p.batch.query_start_loc[r + 1] - p.batch.query_start_loc[r];
+            const int nt = (ql + tpt - 1) / tpt;
+            if (t < nt) { req = r; tile_in_req = nt - 1 - t; break; }    // the tiles with the most keys first
+            t -= nt;
+        }
+    }
+    if (req < 0) return;
+    const ReqGeom g = load_req(p.batch, req);
+    if (!g.valid) return;
+    if ((base & 1023u) != 0u) {      // the swizzled tiles need a 1024-byte-aligned window (the kernel has no static shared memory)
+        if (tid == 0 && p.status != nullptr) atomicOr(p.status, 2);
+        return;
+    }
+    const int tok0 = tile_in_req * tpt;
+    const int ntok = min(tpt, g.q_len - tok0);
+    const int rows_used = ntok * p.gqa;
+    const int row0 = (int)rank * kPpCtaRows;      // first row of this CTA in the tile
+    // keys any row of the pair can see (both limits grow with the token)
+    const int kv_lo = row_min_kv(p.batch, g, tok0);
+    const int kv_hi = row_max_kv(p.batch, g, tok0 + ntok - 1);
+    const bool any_keys = kv_hi >= kv_lo;
+    const int kb_lo = any_keys ? (kv_lo >> 6) : 0;
+    const int nblocks = any_keys ? ((kv_hi >> 6) - kb_lo + 1) : 0;
+    const int pg_lo = any_keys ? (kv_lo >> 4) : 0, pg_hi = any_keys ? (kv_hi >> 4) : -1;
+
+    const uint32_t k_t = base + S::kOffK, v_t = base + S::kOffV, qlo_t = base + S::kOffQLo;
+    const uint32_t raw = base + S::kOffRaw, lut = base + S::kOffLut, bars = base + S::kOffBars;
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + S::kOffBars + 240);
+    volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(gen + S::kOffBars + 244);
+    auto bar = [&](int which) { return bars + 8u * (uint32_t)which; };
+    // Waits and abort checks are warp-uniform: no lane leaves a loop alone.
+    auto wait_all = [&](uint32_t b, uint32_t parity) {
+        const bool ok = mbar_wait(b, parity);
+        return __all_sync(0xffffffffu, ok) != 0;
+    };
+    auto aborted_any = [&]() { return __any_sync(0xffffffffu, *abort_flag != 0u) != 0; };
+
+    // ---- one-time setup -------------------------------------------------------------------------
+    if (ROT) {
+        for (int i = tid; i < 256 * 16; i += kPpThreads) {
+            const int byte = i >> 4, copy = i & 15;
+            const float c0 = kPpLutScale * tq4_centroid(byte & 15), c1 = kPpLutScale * tq4_centroid(byte >> 4);
+            const uint32_t hi = pack_half2(c0, c1);
+            const float2 hf = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+            sts32(lut + (uint32_t)(byte * 128 + copy * 8), hi);
+            sts32(lut + (uint32_t)(byte * 128 + copy * 8 + 4), pack_half2(c0 - hf.x, c1 - hf.y));
+        }
+    }
+    if (tid == 0) {
+        for (int s = 0; s < kPpStages; ++s) {
+            mbar_init(bar(kPpFullK + s), 8u);      // four producer warps of each CTA
+            mbar_init(bar(kPpFullV + s), 8u);
+            mbar_init(bar(kPpEmptyK + s), 1u);
+            mbar_init(bar(kPpEmptyV + s), 1u);
+        }
+        mbar_init(bar(kPpS), 1u);
+        mbar_init(bar(kPpS + 1), 1u);
+        mbar_init(bar(kPpPv), 1u);
+        mbar_init(bar(kPpPReady), 8u);             // four consumer warps of each CTA
+        mbar_init(bar(kPpPReady + 1), 8u);
+        mbar_init(bar(kPpDrain), 1u);
+        for (int s = 0; s < kPpRawStages; ++s) {
+            mbar_init(bar(kPpRawKFull + s), 1u);
+            mbar_init(bar(kPpRawKFree + s), 4u);
+            mbar_init(bar(kPpRawVFull + s), 1u);
+            mbar_init(bar(kPpRawVFree + s), 4u);
+        }
+        *abort_flag = 0u;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    if (wid == 0) {
+        tc2_alloc(base + S::kOffBars + 240, 512);
+        tc2_relinquish();
+    }
+
+    // ---- Q rows of this CTA: one warp per row.  TQ4: rotated, scaled, split into value (staging) and
+    //      residual (swizzled A tile); 8-bit: the fp16 row as it is ------------------------------------
+    const uint32_t q_stage = k_t;     // 128 rows x 512 B over the tile stages
+    for (int row = wid; row < kPpCtaRows; row += kPpWarps) {
+        const int trow = row0 + row;
+        const int q_off = tok0 + trow / p.gqa;
+        const int q_head = kv_head * p.gqa + trow % p.gqa;
+        const bool ok = trow < rows_used &&
+                        (p.batch.valid_token_mask == nullptr || p.batch.valid_token_mask[g.q_start + q_off] != 0);
+        float tv[8];
+        const size_t q_base = ((size_t)(g.q_start + q_off) * p.num_q_heads + q_head) * kHeadDim;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) tv[j] = ok ? load_act(p.q_in, q_base + lane + 32 * j, p.io_bf16) : 0.0f;
+        if (ROT) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) tv[j] = apply_sign(tv[j], lane + 32 * j);
+            wht256_lanes(tv, lane);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int c = lane + 32 * j;
+            const float f = ROT ? tv[j] * p.q_scale : tv[j];
+            const __half h = __float2half_rn(f);
+            // staging row = 512 B; its 16-byte chunks are XOR-swizzled by the row (the reads below are thread-per-row)
+            sts16(q_stage + (uint32_t)row * 512u + (uint32_t)((((c >> 3) ^ (row & 31)) << 4) + ((c & 7) << 1)),
+                  (uint32_t)__half_as_ushort(h));
+            if (ROT) {
+                const uint32_t addr = qlo_t + (uint32_t)(c >> 6) * (kPpCtaRows * 128u) + (uint32_t)row * 128u +
+                                      (uint32_t)(((((c & 63) >> 3) ^ (row & 7)) << 4) + ((c & 7) << 1));
+                sts16(addr, (uint32_t)__half_as_ushort(__float2half_rn(f - __half2float(h))));
+            }
+        }
+    }
+    if (ROT) fence_proxy_async();     // the residual tile is read by the tensor core
+    tc_fence_before();
+    cluster_sync_all();               // barriers of both CTAs exist, TMEM of both is allocated, staging is written
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    if (wid < 4) {
+        const uint32_t t_q = tmem + ((uint32_t)(32 * wid) << 16) + kPpColQ;
+#pragma unroll 1
+        for (int c4 = 0; c4 < 4; ++c4) {
+            uint32_t r[32];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const uint32_t chunk = (uint32_t)(8 * c4 + c);
+                const uint32_t addr = q_stage + (uint32_t)tid * 512u + ((chunk ^ (uint32_t)(tid & 31)) << 4);
+                asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(r[4 * c]), "=r"(r[4 * c + 1]), "=r"(r[4 * c + 2]), "=r"(r[4 * c + 3]) : "r"(addr));
+            }
+            tc_st32(t_q + 32u * c4, r);
+        }
+        tc_wait_st();
+    }
+    tc_fence_before();
+    cluster_sync_all();               // Q' of both CTAs is in place, the staging area becomes the tile stages
+    tc_fence_after();
+
+    const int32_t* blocks = p.batch.block_tables + (size_t)req * p.batch.max_blocks_per_req;
+    float l_run = 0.0f;
+
+    if (wid == 12) {
+        // ======================= MMA issue: lane 0 of CTA 0 feeds both tensor cores ====================
+        // Order in the pipe: QK(0), QK(1), PV(0), QK(2), PV(1), ...  QK(j) overwrites the buffer of P(j - 2),
+        // which PV(j - 2), issued before it, has read.
+        if (rank == 0 && elect_one()) {
+            constexpr uint32_t kIdescQk = tc_idesc(kPpRows, kPpKeys, 0);
+            constexpr uint32_t kIdescPv = tc_idesc(kPpRows, kHeadDim, 1);
+            const uint64_t desc_k = tc_smem_desc(k_t, 16u, 1024u);
+            const uint64_t desc_v = tc_smem_desc(v_t, 4096u, 1024u);
+            const uint64_t desc_q = tc_smem_desc(qlo_t, 16u, 1024u);
+            uint32_t kst = 0, kph = 0, vst = 0, vph = 0;
+            bool ok = true;
+#pragma unroll 1
+            for (int j = 0; j <= nblocks && ok && *abort_flag == 0u; ++j) {
+                if (j < nblocks) {
+                    const uint32_t d = tmem + kPpColS + 64u * (uint32_t)(j & 1);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        ok = ok && mbar_wait(bar(kPpFullK + (int)kst), kph);
+                        if (!ok) break;
+                        tc_fence_after();
+                        const uint64_t b0 = desc_k + (uint64_t)(kst * (kPpStage / 16));
+#pragma unroll
+                        for (int ks = 0; ks < 8; ++ks) {
+                            const uint64_t b = b0 + (uint64_t)((ks >> 2) * (4096 / 16) + 2 * (ks & 3));
+                            const uint32_t a = tmem + kPpColQ + 64u * (uint32_t)h + 8u * (uint32_t)ks;
+                            tc2_mma_f16_ts(d, a, b, kIdescQk, (h || ks) ? 1u : 0u);
+                            tc2_mma_f16_ts(d, a, b + kPpPart / 16, kIdescQk, 1u);
+                            if (ROT) {
+                                tc2_mma_f16(d, desc_q + (uint64_t)((2 * h + (ks >> 2)) * (kPpCtaRows * 128 / 16) + 2 * (ks & 3)), b,
+                                            kIdescQk, 1u);
+                            }
+                        }
+                        tc2_commit_both(bar(kPpEmptyK + (int)kst));
+                        if (h == 1) tc2_commit_both(bar(kPpS + (j & 1)));
+                        if (++kst == kPpStages) { kst = 0; kph ^= 1u; }
+                    }
+                }
+                if (j > 0 && ok) {
+                    const int i = j - 1;
+                    ok = mbar_wait(bar(kPpPReady + (i & 1)), (uint32_t)((i >> 1) & 1));
+                    const uint32_t a0 = tmem + kPpColS + 64u * (uint32_t)(i & 1);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        ok = ok && mbar_wait(bar(kPpFullV + (int)vst), vph);
+                        if (!ok) break;
+                        tc_fence_after();
+                        const uint64_t b0 = desc_v + (uint64_t)(vst * (kPpStage / 16));
+#pragma unroll
+                        for (int ks = 0; ks < 2; ++ks) {
+                            const uint64_t b = b0 + (uint64_t)((2048 / 16) * ks);
+                            const uint32_t a = a0 + 8u * (uint32_t)(2 * h + ks);
+                            tc2_mma_f16_ts(tmem + kPpColO, a, b, kIdescPv, (i > 0 || h > 0 || ks > 0) ? 1u : 0u);
+                            tc2_mma_f16_ts(tmem + kPpColO, a + 32u, b, kIdescPv, 1u);
+                            tc2_mma_f16_ts(tmem + kPpColO, a, b + kPpPart / 16, kIdescPv, 1u);
+                        }
+                        tc2_commit_both(bar(kPpEmptyV + (int)vst));
+                        if (h == 1) tc2_commit_both(bar(kPpPv));
+                        if (++vst == kPpStages) { vst = 0; vph ^= 1u; }
+                    }
+                }
+            }
+            if (!ok) *abort_flag = 1u;
+            // nothing may be in flight when the CTAs leave (after an abort as well)
+            tc2_commit_both(bar(kPpDrain));
+        }
+        __syncwarp();
+        if (!wait_all(bar(kPpDrain), 0u)) *abort_flag = 1u;
+    } else if (wid == 13) {
+        // ======================= copy issue: raw (page, head) runs of a block ===========================
+        const uint8_t* k_head_base = (const uint8_t*)(uintptr_t)p.layout.k_base + (size_t)kv_head * p.layout.k_head_stride_bytes;
+        const uint8_t* v_head_base = (const uint8_t*)(uintptr_t)p.layout.v_base + (size_t)kv_head * p.layout.v_head_stride_bytes;
+        auto page_id = [&](int j) -> int32_t {      // lane pp < 4: page pp of block j, -1 outside the visible range
+            const int pg = 4 * (kb_lo + j) + (lane & 3);
+            return (j < nblocks && pg >= pg_lo && pg <= pg_hi) ? block_table_page(blocks, pg, p.batch.max_blocks_per_req, ROT ? kInPrefillExact : kInKv8) : -1;
+        };
+        int32_t id = page_id(0);
+        int issued = 0;
+#pragma unroll 1
+        for (int j = 0; j < nblocks; ++j) {
+            if (aborted_any()) break;
+            const int s = j % kPpRawStages;
+            const int32_t next_id = page_id(j + 1);
+            const uint32_t mask = __ballot_sync(0xffffffffu, id >= 0) & 15u;
+            const uint32_t kmask = (mask >> (2 * rank)) & 3u;
+            if (j >= kPpRawStages && !wait_all(bar(kPpRawKFree + s), (uint32_t)((j / kPpRawStages - 1) & 1))) { *abort_flag = 1u; break; }
+            const uint32_t rk = raw + (uint32_t)s * S::kRaw, rv = rk + S::kRawK;
+            if (lane == 0) mbar_expect_tx(bar(kPpRawKFull + s), (uint32_t)__popc(kmask) * S::kRun);
+            __syncwarp();
+            if (lane < 4 && (lane >> 1) == (int)rank && id >= 0) {
+                bulk_g2s(rk + (uint32_t)(lane & 1) * S::kRun, k_head_base + (size_t)id * p.layout.k_page_stride_bytes, S::kRun, bar(kPpRawKFull + s));
+            }
+            issued = 2 * j + 1;
+            if (j >= kPpRawStages && !wait_all(bar(kPpRawVFree + s), (uint32_t)((j / kPpRawStages - 1) & 1))) { *abort_flag = 1u; break; }
+            if (lane == 0) mbar_expect_tx(bar(kPpRawVFull + s), (uint32_t)__popc(mask) * S::kRun);
+            __syncwarp();
+            if (lane < 4 && id >= 0) {
+                bulk_g2s(rv + (uint32_t)lane * S::kRun, v_head_base + (size_t)id * p.layout.v_page_stride_bytes, S::kRun, bar(kPpRawVFull + s));
+            }
+            issued = 2 * j + 2;
+            id = next_id;
+        }
+        // copies in flight must land before the CTA leaves
+        const int kn = (issued + 1) / 2, vn = issued / 2;
+        for (int j = max(0, kn - kPpRawStages); j < kn; ++j) (void)wait_all(bar(kPpRawKFull + j % kPpRawStages), (uint32_t)((j / kPpRawStages) & 1));
+        for (int j = max(0, vn - kPpRawStages); j < vn; ++j) (void)wait_all(bar(kPpRawVFull + j % kPpRawStages), (uint32_t)((j / kPpRawStages) & 1));
+    } else if (wid >= 4) {
+        // ======================= producers: lane = key, this warp's 32 channels of the stage's 128 ========
+        const bool is_v = wid >= 8;
+        const int quarter = wid & 3;
+        const int raw_full = is_v ? kPpRawVFull : kPpRawKFull, raw_free = is_v ? kPpRawVFree : kPpRawKFree;
+        const int full = is_v ? kPpFullV : kPpFullK, empty = is_v ? kPpEmptyV : kPpEmptyK;
+        const uint32_t tiles = is_v ? v_t : k_t;
+        // chunk c (8 channels) of key `lane`: [block of 64 channels][key][16-byte chunk XOR (key & 7)]
+        const uint32_t dst0 = (uint32_t)(quarter >> 1) * 4096u + (uint32_t)lane * 128u;
+        const uint32_t lut_lane = lut + 8u * (uint32_t)(lane & 15);
+        const uint32_t leader_full = map_to_rank(bar(full), 0u);
+        uint32_t st = 0, ph = 1;      // parity 1: the first pass over the ring does not wait
+#pragma unroll 1
+        for (int j = 0; j < nblocks; ++j) {
+            if (aborted_any()) break;
+            const int rs = j % kPpRawStages;
+            if (!wait_all(bar(raw_full + rs), (uint32_t)((j / kPpRawStages) & 1))) { *abort_flag = 1u; break; }
+            const uint32_t run = raw + (uint32_t)rs * S::kRaw + (is_v ? S::kRawK : 0u);
+            bool ok = true;
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+                // K: channels [128 h, + 128) of this CTA's 32 keys.  V: channels [128 rank, + 128) of keys 32 h + lane.
+                const int key = is_v ? 32 * h + lane : lane;
+                const int half = is_v ? (int)rank : h;
+                const int pos = ((kb_lo + j) << 6) + (is_v ? key : 32 * (int)rank + lane);
+                const bool key_ok = pos >= kv_lo && pos <= kv_hi;     // others may hold never-written bytes
+                const uint32_t rowp = run + (uint32_t)key * ROW;
+                uint32_t w[FMT == WARP34_KV_FORMAT_TQ4 ? 4 : 8];
+                float d = 0.0f;
+                uint32_t dbits = 0;
+                if (FMT == WARP34_KV_FORMAT_TQ4) {
+                    if (half == 0) {       // codes of half 0 start at byte 2
+                        uint32_t x[5];
+#pragma unroll
+                        for (int i = 0; i < 5; ++i) x[i] = lds32(rowp + 16u * quarter + 4u * i);
+                        dbits = lds_u16(rowp);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) w[i] = __funnelshift_r(x[i], x[i + 1], 16);
+                    } else {
+                        dbits = lds_u16(rowp + 66u);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) w[i] = lds32(rowp + 68u + 16u * quarter + 4u * i);
+                    }
+                    if (!key_ok) dbits = 0u;
+                } else if (FMT == WARP34_KV_FORMAT_FP8_E4M3) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) w[i] = lds32(rowp + 128u * half + 32u * quarter + 4u * i);
+                    d = __uint_as_float(lds32(rowp + kHeadDim + 4u * half));
+                } else {
+                    const uint32_t blk = rowp + 68u * (uint32_t)(2 * half + (quarter >> 1));
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) w[i] = lds32(blk + 4u + 32u * (quarter & 1) + 4u * i);
+                    d = __uint_as_float(lds32(blk));
+                }
+                if (FMT != WARP34_KV_FORMAT_TQ4 && !key_ok) {
+                    d = 0.0f;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) w[i] = 0u;      // e4m3 codes of unwritten rows can be NaN patterns
+                }
+                __syncwarp();
+                if (h == 1 && lane == 0) mbar_arrive(bar(raw_free + rs));     // the runs are in registers
+                ok = wait_all(bar(empty + (int)st), ph);
+                if (!ok) break;
+                const uint32_t dst = tiles + st * kPpStage + dst0;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    uint32_t hi[4], lo[4];
+                    if (FMT == WARP34_KV_FORMAT_TQ4) {
+                        const __half2 d2 = __half2half2(__ushort_as_half((unsigned short)dbits));
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const uint32_t off = (k == 0 ? (w[c] << 7) : (w[c] >> (8 * k - 7))) & 0x7f80u;
+                            const uint2 e = lds64_lut(lut_lane + off);
+                            const __half2 ch = *reinterpret_cast<const __half2*>(&e.x), cl = *reinterpret_cast<const __half2*>(&e.y);
+                            const __half2 vh = __hmul2(d2, ch);
+                            const __half2 vl = __hfma2(d2, cl, __hfma2(d2, ch, __hneg2(vh)));     // the inner fma is exact
+                            hi[k] = *reinterpret_cast<const uint32_t*>(&vh);
+                            lo[k] = *reinterpret_cast<const uint32_t*>(&vl);
+                        }
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) {
+                            uint32_t c01, c23;
+                            kv8x4_to_f16x4<FMT>(w[2 * c + k], c01, c23);
+#pragma unroll
+                            for (int x = 0; x < 2; ++x) {
+                                const uint32_t cc = x ? c23 : c01;
+                                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&cc));
+                                const __half2 vh = __floats2half2_rn(d * f.x, d * f.y);
+                                const float2 hf = __half22float2(vh);
+                                const __half2 vl = __floats2half2_rn(__fmaf_rn(d, f.x, -hf.x), __fmaf_rn(d, f.y, -hf.y));
+                                hi[2 * k + x] = *reinterpret_cast<const uint32_t*>(&vh);
+                                lo[2 * k + x] = *reinterpret_cast<const uint32_t*>(&vl);
+                            }
+                        }
+                    }
+                    const uint32_t a = dst + (uint32_t)(((4 * (quarter & 1) + c) ^ (lane & 7)) << 4);
+                    sts128(a, hi[0], hi[1], hi[2], hi[3]);
+                    sts128(a + kPpPart, lo[0], lo[1], lo[2], lo[3]);
+                }
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(leader_full + 8u * st);
+                if (++st == kPpStages) { st = 0; ph ^= 1u; }
+            }
+            if (!ok) { *abort_flag = 1u; break; }
+        }
+    } else {
+        // ======================= consumers: softmax, P, rescale =========================================
+        const int trow = row0 + tid;
+        const int q_off = tok0 + trow / p.gqa;
+        const bool row_ok = trow < rows_used &&
+                            (p.batch.valid_token_mask == nullptr || p.batch.valid_token_mask[g.q_start + q_off] != 0);
+        const int rmax = row_ok ? row_max_kv(p.batch, g, q_off) : -1;
+        const int rmin = row_ok ? row_min_kv(p.batch, g, q_off) : 0x7fffffff;
+        const uint32_t lane_base = (uint32_t)(32 * wid) << 16;
+        const uint32_t t_o = tmem + lane_base + kPpColO, t_s = tmem + lane_base + kPpColS;
+        const uint32_t leader_pready = map_to_rank(bar(kPpPReady), 0u);
+        float m_ref = -1e30f;
+#pragma unroll 1
+        for (int j = 0; j < nblocks; ++j) {
+            if (aborted_any()) break;
+            if (!wait_all(bar(kPpS + (j & 1)), (uint32_t)((j >> 1) & 1))) { *abort_flag = 1u; break; }
+            tc_fence_after();
+            // PV(j - 2) precedes QK(j) in the pipe; waiting for every phase of kPpPv keeps its parity unambiguous
+            if (j >= 2 && !wait_all(bar(kPpPv), (uint32_t)(j & 1))) { *abort_flag = 1u; break; }
+            const uint32_t t_sj = t_s + 64u * (uint32_t)(j & 1);
+            float sv[64];
+            {
+                uint32_t r0[32], r1[32];
+                tc_ld32(r0, t_sj);
+                tc_ld32(r1, t_sj + 32u);
+                tc_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 32; ++i) { sv[i] = __uint_as_float(r0[i]); sv[32 + i] = __uint_as_float(r1[i]); }
+            }
+            if (!ROT) {
+#pragma unroll
+                for (int i = 0; i < 64; ++i) sv[i] *= p.q_scale;
+            }
+            const int kbase = (kb_lo + j) << 6;
+            if (!(kbase >= rmin && kbase + 63 <= rmax)) {
+#pragma unroll
+                for (int i = 0; i < 64; ++i) {
+                    const int pos = kbase + i;
+                    if (!(pos >= rmin && pos <= rmax)) sv[i] = -1e30f;
+                }
+            }
+            float mx4[4] = {sv[0], sv[1], sv[2], sv[3]};     // four independent chains
+#pragma unroll
+            for (int i = 4; i < 64; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], sv[i]);
+            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+            // the reference maximum moves only when the true maximum ran ahead by more than the threshold
+            const bool need = mx > m_ref + kPpRescaleThreshold;
+            float alpha = 1.0f;
+            if (need) {
+                alpha = ex2(m_ref - mx);      // 0 when nothing was visible before
+                m_ref = mx;
+            }
+            if (j > 0 && __any_sync(0xffffffffu, need)) {
+                // O is at rest once the previous output product has completed (the next one waits for this block's P)
+                if (!wait_all(bar(kPpPv), (uint32_t)((j - 1) & 1))) { *abort_flag = 1u; break; }
+                tc_fence_after();
+#pragma unroll 1
+                for (int c = 0; c < 16; ++c) {
+                    uint32_t o[16];
+                    tc_ld16(o, t_o + 16u * c);
+                    tc_wait_ld();
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                    tc_st16(t_o + 16u * c, o);
+                }
+            }
+            float ls4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            const float m_use = ((m_ref < -1e29f) ? 0.0f : m_ref) - kPpShift;     // nothing visible yet: every P is 0
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                uint32_t hi[16], lo[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    // masked scores are -1e30: ex2 gives exactly 0 against any finite reference
+                    const float pa = ex2(sv[32 * c + 2 * i] - m_use), pb = ex2(sv[32 * c + 2 * i + 1] - m_use);
+                    ls4[i & 3] += pa + pb;
+                    const __half2 h = __floats2half2_rn(pa, pb);
+                    const float2 hf = __half22float2(h);
+                    hi[i] = *reinterpret_cast<const uint32_t*>(&h);
+                    lo[i] = pack_half2(pa - hf.x, pb - hf.y);
+                }
+                tc_st16(t_sj + 16u * c, hi);
+                tc_st16(t_sj + 32u + 16u * c, lo);
+            }
+            tc_wait_st();
+            l_run = l_run * alpha + ((ls4[0] + ls4[1]) + (ls4[2] + ls4[3]));
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(leader_pready + 8u * (uint32_t)(j & 1));
+        }
+        // the last output product
+        if (nblocks > 0 && !aborted_any()) {
+            if (nblocks > 1 && !wait_all(bar(kPpPv), (uint32_t)(nblocks & 1))) *abort_flag = 1u;
+            if (!wait_all(bar(kPpPv), (uint32_t)((nblocks - 1) & 1))) *abort_flag = 1u;
+        }
+        tc_fence_after();
+    }
+
+    // ---- epilogue: O / l -> staging -> inverse rotation -> global ---------------------------------
+    // (staging aliases the tiles: every MMA of the pair that read them has completed, see kPpDrain)
+    __syncthreads();
+    const bool aborted = *abort_flag != 0u;
+    float* stage = reinterpret_cast<float*>(gen);
+    if (wid < 4 && nblocks > 0 && !aborted) {
+        const uint32_t t_o = tmem + ((uint32_t)(32 * wid) << 16) + kPpColO;
+        const float inv = (l_run > 0.0f) ? (1.0f / (ROT ? l_run * kPpLutScale : l_run)) : 0.0f;
+#pragma unroll 1
+        for (int c = 0; c < 8; ++c) {
+            uint32_t o[32];
+            tc_ld32(o, t_o + 32u * c);
+            tc_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) stage[tid * kPpOutStride + 32 * c + i] = __uint_as_float(o[i]) * inv;
+        }
+        stage[tid * kPpOutStride + 256] = l_run;
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (!aborted) {
+        for (int row = wid; row < kPpCtaRows; row += kPpWarps) {
+            const int trow = row0 + row;
+            if (trow >= rows_used) break;
+            const int q_off = tok0 + trow / p.gqa;
+            const int q_head = kv_head * p.gqa + trow % p.gqa;
+            if (p.batch.valid_token_mask != nullptr && p.batch.valid_token_mask[g.q_start + q_off] == 0) continue;
+            float tv[8];
+            const bool has = nblocks > 0 && stage[row * kPpOutStride + 256] > 0.0f;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) tv[j] = has ? stage[row * kPpOutStride + lane + 32 * j] : 0.0f;
+            const size_t out_base = ((size_t)(g.q_start + q_off) * p.num_q_heads + q_head) * kHeadDim;
+            if (ROT) {
+                wht256_lanes(tv, lane);
+                store_output_row(p.attn_out, out_base, tv, lane, p.io_bf16, p.og);
+            } else {
+                apply_output_gate(tv, p.og, out_base, lane, p.io_bf16);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) store_act(p.attn_out, out_base + lane + 32 * j, tv[j], p.io_bf16);
+            }
+        }
+    } else if (tid == 0 && p.status != nullptr) {
+        atomicOr(p.status, 1);
+    }
+    // neither CTA leaves (or frees tensor memory) while the other may still signal it
+    cluster_sync_all();
+    if (wid == 0) {
+        tc_fence_after();
+        tc2_dealloc(tmem, 512);
+    }
+}
+
+}  // namespace w34
+
+namespace w34 {
+// The pair kernel for one layer's chunk: no workspace beyond the status word.
+template <int FMT>
+static int launch_prefill_pair(const warp34_exec* ex, const warp34_kv_layer_layout* layout, const warp34_attention_batch* batch,
+                               const void* q_in, void* attn_out, int num_q_heads, int io_bf16, int32_t* status, const OutputGate& og) {
+    if (layout->local_kv_heads > 65535) return (int)cudaErrorInvalidValue;
+    PrefillPairParams pp;
+    pp.layout = *layout;
+    pp.batch = *batch;
+    pp.q_in = q_in;
+    pp.attn_out = attn_out;
+    pp.io_bf16 = io_bf16;
+    pp.num_q_heads = num_q_heads;
+    pp.gqa = num_q_heads / layout->local_kv_heads;
+    pp.tok_per_tile = kPpRows / pp.gqa;
+    pp.q_scale = batch->sm_scale * 1.4426950408889634f;
+    if (PpFormat<FMT>::kRotated) pp.q_scale /= kPpLutScale;
+    pp.status = status;
+    pp.og = og;
+    const long long tiles = (long long)batch->total_tokens / pp.tok_per_tile + batch->num_reqs;
+    if (tiles > 0x3fffffffll) return (int)cudaErrorInvalidValue;
+    const dim3 grid(2u * (unsigned)tiles, (unsigned)layout->local_kv_heads);
+    attention_prefill_pair_kernel<FMT><<<grid, kPpThreads, PpSmem<FMT>::kBytes, (cudaStream_t)ex->stream>>>(pp);
+    return (int)cudaGetLastError();
+}
+}  // namespace w34

@@ -704,6 +704,24 @@ __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
+// Four 8-bit codes -> two fp16 pairs (bytes 0,1 and bytes 2,3), exactly.
+template <int FMT>
+__device__ __forceinline__ void kv8x4_to_f16x4(uint32_t w, uint32_t& lo, uint32_t& hi) {
+    if (FMT == WARP34_KV_FORMAT_FP8_E4M3) {
+        asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tcvt.rn.f16x2.e4m3x2 %0, l;\n\tcvt.rn.f16x2.e4m3x2 %1, h;\n\t}"
+            : "=r"(lo), "=r"(hi) : "r"(w));
+    } else {
+        const uint32_t x = w ^ 0x80808080u;                               // q + 128 as an unsigned byte
+        const uint32_t l = __byte_perm(x, 0x64646464u, 0x4140);           // halves 1024 + (q + 128)
+        const uint32_t h = __byte_perm(x, 0x64646464u, 0x4342);
+        const __half2 bias = __half2half2(__ushort_as_half((unsigned short)0x6480));   // 1152
+        const __half2 lh = __hsub2(*reinterpret_cast<const __half2*>(&l), bias);
+        const __half2 hh = __hsub2(*reinterpret_cast<const __half2*>(&h), bias);
+        lo = *reinterpret_cast<const uint32_t*>(&lh);
+        hi = *reinterpret_cast<const uint32_t*>(&hh);
+    }
+}
+
 // A 132-byte row is 33 aligned words W0..W32.  Codes of the first 128-half sit at bytes 2..65,
 // i.e. shifted by half a word.  "Virtual word" vw (0..15) of half 0 is W[vw] for vw >= 1 and the
 // splice {bytes 2,3 | bytes 64,65} = (W0 >> 16) | (W16 << 16) for vw = 0; of half 1 it is
@@ -747,17 +765,11 @@ constexpr int kExactWarps = 8, kExactStages = 4;
 // below a quarter of the mass moves the output by less than a quarter of that.  (Gating the residual
 // of P x d_v the same way, at 1/16 of the mass, measured no faster than carrying it on every page.)
 constexpr float kPeakedWeight = 0.25f;
-// The prefill kernel (tensor-bound) also gates the residual of P x d_v, at this fraction of the mass.
-constexpr float kPResidualWeight = 1.0f / 64.0f;
-// The prefill kernel takes the V-centroid residual pass from an eighth of the mass (its pages serve 16 rows
-// per warp, and the pass costs it little).
-constexpr float kPxPeakedWeight = 0.125f;
 // Rounding residuals are 2^-12 of their values.  Those of the table's centroids (values 0.12 .. 2.6
 // after the common factor; residuals at most 1e-3, at least a few hundred fp16 subnormal steps) are
 // stored in this kernel's table times 2^11, as normal fp16 numbers, and their products scaled back in
-// fp32: the MMA takes subnormal operands as they are (the prefill kernel's table holds the residuals
-// unscaled and adds their product straight to the scores), but this kernel measured 1.4 % faster with
-// the scaled table.  The residual of Q' is kept as one byte per element in units of a step of its own
+// fp32: the MMA takes subnormal operands as they are, but this kernel measured 1.4 % faster with the scaled
+// table.  The residual of Q' is kept as one byte per element in units of a step of its own
 // row (see the query-fragment block).
 constexpr float kResidualScale = 2048.0f;
 
@@ -1905,7 +1917,7 @@ W34_BOUNDS_HOST_HOOKS(attention)
 
 }  // namespace w34
 #include "tq4_prefill_tc.cuh"
-#include "tq4_prefill_exact.cuh"
+#include "prefill_pair.cuh"
 namespace w34 {
 
 // Row triple written when the caller merges across page shards itself: 256 un-normalised
@@ -2211,12 +2223,6 @@ static size_t stream_smem_min_bytes() {
     return kLutBytes + (fast > exact ? fast : exact);
 }
 
-// Exact prefill kernel: table, eight fragment areas, the page ring and its barriers.
-static size_t prefill_exact_smem_min_bytes() {
-    return kLutBytes + (size_t)kPxWarps * (kPxQHiBytes + kPxQLoBytes) + (size_t)kPxStages * kStageStride + 128 +
-           2 * kPxStages * 8 + 16 * kPxWarps;
-}
-
 struct DeviceInfo {
     int sm_count;
     int smem_optin;
@@ -2255,15 +2261,14 @@ static DeviceInfo* device_info(int* rc) {
         *rc = (int)cudaFuncSetAttribute(tq4_attention_team_kernel<3>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
         if (*rc != 0) return nullptr;
-        if ((size_t)optin < prefill_exact_smem_min_bytes()) { *rc = (int)cudaErrorNotSupported; return nullptr; }
-        *rc = (int)cudaFuncSetAttribute(tq4_attention_prefill_exact_kernel<kPxWarps>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+        *rc = (int)cudaFuncSetAttribute(attention_prefill_pair_kernel<WARP34_KV_FORMAT_TQ4>,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PpSmem<WARP34_KV_FORMAT_TQ4>::kBytes);
         if (*rc != 0) return nullptr;
-        *rc = (int)cudaFuncSetAttribute(tq4_attention_prefill_exact_kernel<kPxWarps / 2>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+        *rc = (int)cudaFuncSetAttribute(attention_prefill_pair_kernel<WARP34_KV_FORMAT_FP8_E4M3>,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PpSmem<WARP34_KV_FORMAT_FP8_E4M3>::kBytes);
         if (*rc != 0) return nullptr;
-        *rc = (int)cudaFuncSetAttribute(tq4_attention_prefill_exact_kernel<kPxWarps / 4>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+        *rc = (int)cudaFuncSetAttribute(attention_prefill_pair_kernel<WARP34_KV_FORMAT_Q8_0>,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PpSmem<WARP34_KV_FORMAT_Q8_0>::kBytes);
         if (*rc != 0) return nullptr;
         *rc = (int)cudaFuncSetAttribute(tq4_attention_prefill_tc_kernel,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmemBytes);
@@ -2474,13 +2479,30 @@ static bool takes_prefill_path(uint64_t flags, const warp34_kv_layer_layout* l,
                                const warp34_attention_batch* b, int gqa) {
     const bool want_tc = (flags & WARP34_B200_EXEC_FLAG_TCGEN05_VERIFY) != 0 && (long long)b->max_q_len * gqa > 8;
     return (flags & WARP34_B200_EXEC_FLAG_PRECISE_ATTENTION) == 0 && stream_layout_ok(l) &&
-           b->max_blocks_per_req > 0 && gqa <= kPxRows && ((long long)b->max_q_len * gqa > 24 || want_tc);
+           b->max_blocks_per_req > 0 && gqa <= kPpCtaRows && ((long long)b->max_q_len * gqa > 24 || want_tc);
+}
+
+static bool takes_kv8_chunk_path(uint64_t flags, const warp34_kv_layer_layout* l, const warp34_attention_batch* b, int num_q_heads) {
+    if ((flags & WARP34_B200_EXEC_FLAG_PRECISE_ATTENTION) != 0 || !kv8_canonical(l) || l->k_base == 0 || l->v_base == 0 ||
+        l->local_kv_heads <= 0 || num_q_heads % l->local_kv_heads != 0 || b->num_reqs <= 0 || b->block_tables == nullptr ||
+        b->max_blocks_per_req <= 0) {
+        return false;
+    }
+    const int gqa = num_q_heads / l->local_kv_heads;
+    return gqa <= kPpCtaRows && (long long)b->max_q_len * gqa > 24;
+}
+
+// The chunk kernels report through the first word of the workspace, when there is one.
+static int chunk_status_word(const warp34_exec* ex, int32_t** status) {
+    if (ex->scratch_ptr == 0 || (ex->scratch_ptr & 3u) != 0 || ex->scratch_size < sizeof(PlanHeader)) return 0;
+    *status = reinterpret_cast<int32_t*>((uintptr_t)ex->scratch_ptr);   // PlanHeader::status
+    return (int)cudaMemsetAsync(*status, 0, sizeof(int32_t), (cudaStream_t)ex->stream);
 }
 
 // Shared body of the attention entry points.  triple_out != nullptr: stop after the split-KV
 // merge and write per-row (acc, m, l) instead of attn_out (streaming path only).
 // force: -1 = dispatch by batch geometry and flags; otherwise the kernel family the reference's
-// test selector names: 0 = the row-group kernels (8 query rows per item), 1 = the register-MMA
+// test selector names: 0 = the row-group kernels (8 query rows per item), 1 = the CTA-pair
 // prefill kernel, 2 = the tcgen05 prefill kernel.
 static int launch_attention(const warp34_exec* ex, const warp34_kv_layer_layout* layout,
                             const warp34_attention_batch* batch, const void* q_in, void* attn_out,
@@ -2495,8 +2517,18 @@ static int launch_attention(const warp34_exec* ex, const warp34_kv_layer_layout*
         return (int)cudaErrorInvalidValue;
     }
     if (batch->total_tokens <= 0 || num_q_heads <= 0) return 0;
-    if (kv8_attention_layout_ok(layout)) {   // unrotated 8-bit boundary layers: the epilogue is a second launch, in place
+    if (kv8_attention_layout_ok(layout)) {   // unrotated 8-bit boundary layers; a decode batch's epilogue is a second launch, in place
         if (triple_out != nullptr) return (int)cudaErrorNotSupported;
+        if (force <= 0 && takes_kv8_chunk_path(ex->flags, layout, batch, num_q_heads)) {
+            int rc = 0;
+            if (device_info(&rc) == nullptr) return rc;
+            int32_t* status = nullptr;
+            rc = chunk_status_word(ex, &status);
+            if (rc != 0) return rc;
+            return layout->k_format == WARP34_KV_FORMAT_FP8_E4M3
+                       ? launch_prefill_pair<WARP34_KV_FORMAT_FP8_E4M3>(ex, layout, batch, q_in, attn_out, num_q_heads, io_bf16, status, og)
+                       : launch_prefill_pair<WARP34_KV_FORMAT_Q8_0>(ex, layout, batch, q_in, attn_out, num_q_heads, io_bf16, status, og);
+        }
         const int rc8 = launch_kv8_attention(ex, layout, batch, q_in, attn_out, num_q_heads, io_bf16,
                                              (ex->flags & WARP34_B200_EXEC_FLAG_PRECISE_ATTENTION) == 0 && force <= 0);
         if (rc8 != 0 || og.mode == 0) return rc8;
@@ -2512,21 +2544,18 @@ static int launch_attention(const warp34_exec* ex, const warp34_kv_layer_layout*
 
     const int gqa = num_q_heads / layout->local_kv_heads;
     // Prefill chunks: 128-row CTAs, no scratch.  Not for the partial-output mode, which is a
-    // decode-time feature.  Default: register MMAs with value + residual operands; with the fast
+    // decode-time feature.  Default: the CTA-pair tcgen05 kernel with value + residual operands; with the fast
     // flag (or the tcgen05-verify flag) tcgen05 + TMEM with single fp16 operands.
-    const bool chunk_geometry_ok = stream_layout_ok(layout) && batch->max_blocks_per_req > 0 && gqa <= kPxRows;
+    const bool chunk_geometry_ok = stream_layout_ok(layout) && batch->max_blocks_per_req > 0 && gqa <= kPpCtaRows;
     if (force >= 1 && (!chunk_geometry_ok || triple_out != nullptr)) return (int)cudaErrorNotSupported;
     if (force >= 1 || (force < 0 && triple_out == nullptr && takes_prefill_path(ex->flags, layout, batch, gqa))) {
         int32_t* status = nullptr;
-        if (ex->scratch_ptr != 0 && (ex->scratch_ptr & 3u) == 0 && ex->scratch_size >= sizeof(PlanHeader)) {
-            status = reinterpret_cast<int32_t*>((uintptr_t)ex->scratch_ptr);   // PlanHeader::status
-            rc = (int)cudaMemsetAsync(status, 0, sizeof(int32_t), (cudaStream_t)ex->stream);
-            if (rc != 0) return rc;
-        }
+        rc = chunk_status_word(ex, &status);
+        if (rc != 0) return rc;
         const bool tc = force == 2 || (force < 0 && (ex->flags & (WARP34_B200_EXEC_FLAG_FAST_ATTENTION |
                                                                   WARP34_B200_EXEC_FLAG_TCGEN05_VERIFY)) != 0);
-        if (layout->local_kv_heads > 65535) return (int)cudaErrorInvalidValue;
         if (tc) {
+            if (layout->local_kv_heads > 65535) return (int)cudaErrorInvalidValue;
             if ((size_t)dev->smem_optin < kTcSmemBytes) return (int)cudaErrorNotSupported;
             PrefillTcParams tp;
             tp.layout = *layout;
@@ -2546,43 +2575,7 @@ static int launch_attention(const warp34_exec* ex, const warp34_kv_layer_layout*
             tq4_attention_prefill_tc_kernel<<<grid, kTcThreads, kTcSmemBytes, (cudaStream_t)ex->stream>>>(tp);
             return (int)cudaGetLastError();
         }
-        PrefillExactParams pp;
-        pp.layout = *layout;
-        pp.batch = *batch;
-        pp.q_in = q_in;
-        pp.attn_out = attn_out;
-        pp.io_bf16 = io_bf16;
-        pp.num_q_heads = num_q_heads;
-        pp.gqa = gqa;
-        pp.q_scale = batch->sm_scale * 1.4426950408889634f / kLutScale;
-        pp.status = status;
-        pp.smem_bytes = (uint32_t)dev->smem_optin;
-        pp.og = og;
-        // 128-row CTAs, or 64- / 32-row CTAs when that is faster for this call (a short chunk whose 128-row tiles
-        // would leave SMs without a CTA).  One CTA fits an SM; a CTA of 4 (2) warps takes about 0.69 (0.55) of the
-        // time of one of 8 warps over the same keys (measured: fewer warps share the SM's tensor pipe), so the
-        // estimate is waves x that factor.
-        int warps = kPxWarps;
-        long long tiles = 0;
-        {
-            const float factor[3] = {1.0f, 0.69f, 0.55f};
-            float best = 0.0f;
-            for (int k = 0, w = kPxWarps; k < 3 && gqa <= 16 * w; ++k, w /= 2) {
-                const int tpt = (16 * w) / gqa;
-                const long long t = (long long)batch->total_tokens / tpt + batch->num_reqs;
-                const long long waves = (t * layout->local_kv_heads + dev->sm_count - 1) / dev->sm_count;
-                const float est = (float)waves * factor[k];
-                if (k == 0 || est < best) { best = est; warps = w; tiles = t; pp.tok_per_tile = tpt; }
-            }
-        }
-        if (tiles > 0x7fffffffll) return (int)cudaErrorInvalidValue;
-        const dim3 grid((unsigned)tiles, (unsigned)layout->local_kv_heads);
-        const size_t smem_px = (size_t)dev->smem_optin;
-        cudaStream_t st_px = (cudaStream_t)ex->stream;
-        if (warps == kPxWarps) tq4_attention_prefill_exact_kernel<kPxWarps><<<grid, kPxWarps * 32, smem_px, st_px>>>(pp);
-        else if (warps == kPxWarps / 2) tq4_attention_prefill_exact_kernel<kPxWarps / 2><<<grid, (kPxWarps / 2) * 32, smem_px, st_px>>>(pp);
-        else tq4_attention_prefill_exact_kernel<kPxWarps / 4><<<grid, (kPxWarps / 4) * 32, smem_px, st_px>>>(pp);
-        return (int)cudaGetLastError();
+        return launch_prefill_pair<WARP34_KV_FORMAT_TQ4>(ex, layout, batch, q_in, attn_out, num_q_heads, io_bf16, status, og);
     }
 
     // Streaming path: canonical layout, scratch that holds the plan plus at least one partial
@@ -2868,7 +2861,7 @@ extern "C" int warp34_paged_attention_f16(const warp34_exec* ex, const warp34_kv
 }
 
 // Test-only selector of the reference (op_paged_attn.cu:1451-1458): 0 = its 16-row kernel, 1 = its
-// 64-row, 2 = its 128-row prefill kernel.  Here: 0 = the row-group kernels, 1 = the register-MMA
+// 64-row, 2 = its 128-row prefill kernel.  Here: 0 = the row-group kernels, 1 = the CTA-pair
 // prefill kernel (value + residual operands), 2 = the tcgen05 prefill kernel.
 extern "C" int warp34_paged_attention_f16_force_kernel_for_test(const warp34_exec* ex, const warp34_kv_layer_layout* layout,
                                                                 const warp34_attention_batch* batch, const void* q_in,
