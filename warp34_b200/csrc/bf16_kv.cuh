@@ -81,6 +81,8 @@ __global__ void __launch_bounds__(128) kv_cache_write_bf16_kernel(const warp34_k
 }
 
 __global__ void __launch_bounds__(kBfWarps * 32, 1) bf16kv_attention_stream_kernel(const StreamParams p) {
+    grid_dependency_wait();
+    grid_launch_dependents();
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr int PARTIAL = kBfRows * kHeadDim + 2 * kBfRows;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -449,13 +451,8 @@ extern "C" int warp34_paged_attention_bf16(const warp34_exec* ex, const warp34_k
     p.q_groups_max = 0;
     p.smem_bytes = (uint32_t)(w34::kBfWarps * w34::kBfStages * w34::kBfStageBytes);
     cudaStream_t st = (cudaStream_t)ex->stream;
-    w34::tq4_attention_plan_kernel<<<1, 32, 0, st>>>(p);
-    w34::bf16kv_attention_stream_kernel<<<grid, w34::kBfWarps * 32, p.smem_bytes, st>>>(p);
-    const long long rows = (long long)batch->total_tokens * num_q_heads;
-    if (rows * 4 < (long long)grid * w34::kBfWarps / 8) {
-        w34::tq4_attention_merge_kernel<false, 32><<<(unsigned)rows, 1024, 0, st>>>(p);
-    } else {
-        w34::tq4_attention_merge_kernel<false, 4><<<(unsigned)rows, 128, 0, st>>>(p);
-    }
-    return (int)cudaGetLastError();
+    rc = w34::launch_behind(w34::tq4_attention_plan_kernel, 1u, 32, 0, st, p);
+    if (rc == 0) rc = w34::launch_behind(w34::bf16kv_attention_stream_kernel, (unsigned)grid, w34::kBfWarps * 32, p.smem_bytes, st, p);
+    if (rc != 0) return rc;
+    return w34::launch_merge<false>(p, (long long)batch->total_tokens * num_q_heads, st);
 }

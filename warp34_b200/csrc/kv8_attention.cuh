@@ -343,6 +343,8 @@ __global__ void __launch_bounds__(kKv8StreamWarps * 32, 1) kv8_attention_stream_
         for (int s = 0; s < STAGES; ++s) mbar_init(bars + 8u * s, 1u);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    grid_dependency_wait();      // nothing above touches global memory
+    grid_launch_dependents();
     __syncthreads();
 
     const int R = p.batch.num_reqs;
@@ -375,15 +377,7 @@ __global__ void __launch_bounds__(kKv8StreamWarps * 32, 1) kv8_attention_stream_
     uint32_t phase_bits = 0, pending = 0;
     bool failed = false;
 
-    int r;
-    {
-        int lo = 0, hi = R;
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (unit_prefix[mid] <= u) lo = mid; else hi = mid;
-        }
-        r = lo;
-    }
+    int r = last_not_above(unit_prefix, R, u);
 
     while (u < u_end && !failed) {
         while (unit_prefix[r + 1] <= u) ++r;
@@ -906,18 +900,16 @@ static int launch_kv8_stream(const warp34_exec* ex, const warp34_kv_layer_layout
         p.q_groups_max = 0;
         p.rows_from_first_token = in_parts ? 1 : 0;
         p.keep_status = r0 > 0 ? 1 : 0;
-        tq4_attention_plan_kernel<<<1, 32, 0, st>>>(p);
+        rc = launch_behind(tq4_attention_plan_kernel, 1u, 32, 0, st, p);
+        if (rc != 0) return rc;
         if (fp8) {
-            kv8_attention_stream_kernel<WARP34_KV_FORMAT_FP8_E4M3, kKv8StreamStages><<<grid, kKv8StreamWarps * 32, smem, st>>>(p);
+            rc = launch_behind(kv8_attention_stream_kernel<WARP34_KV_FORMAT_FP8_E4M3, kKv8StreamStages>, (unsigned)grid, kKv8StreamWarps * 32, smem, st, p);
         } else {
-            kv8_attention_stream_kernel<WARP34_KV_FORMAT_Q8_0, kKv8StreamStages><<<grid, kKv8StreamWarps * 32, smem, st>>>(p);
+            rc = launch_behind(kv8_attention_stream_kernel<WARP34_KV_FORMAT_Q8_0, kKv8StreamStages>, (unsigned)grid, kKv8StreamWarps * 32, smem, st, p);
         }
         const long long rows = (long long)p.batch.total_tokens * num_q_heads;
-        if (rows * 4 < (long long)grid * kKv8StreamWarps / 8) {
-            tq4_attention_merge_kernel<false, 32><<<(unsigned)rows, 1024, 0, st>>>(p);
-        } else {
-            tq4_attention_merge_kernel<false, 4><<<(unsigned)rows, 128, 0, st>>>(p);
-        }
+        if (rc == 0) rc = launch_merge<false>(p, rows, st);
+        if (rc != 0) return rc;
         rc = (int)cudaGetLastError();
         if (rc != 0) return rc;
     }

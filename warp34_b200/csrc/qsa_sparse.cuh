@@ -14,7 +14,7 @@
 //   * the sigmoid gate multiplies the fp32 result (no rounding before it); the Hadamard-64 variant then
 //     rounds to fp16 and rotates every 64 columns.
 // Two paths.  With a workspace (ex->scratch_ptr) and the canonical packing the lists run on the
-// tensor-core stream kernels (tq4_attention_stream_kernel<.., sparse> for TQ4 rows,
+// tensor-core stream kernels (tq4_attention_stream_exact_kernel<sparse> for TQ4 rows,
 // kv8_attention_stream_kernel<.., sparse> for 8-bit rows: launch_qsa_stream in tq4_attention.cu).
 // Otherwise (no workspace, other strides, WARP34_B200_EXEC_FLAG_PRECISE_ATTENTION) the fp32
 // dequant-then-attend kernel of this file: one block of four warps per (token, group of G query heads

@@ -214,6 +214,8 @@ constexpr int kProducerBlocksPerSm = 4;   // with the K producer in front: 128 r
 // PRODUCER: K rows go through k_producer() first (fp16 activations only).
 template <bool IN_BF16, bool PRODUCER>
 __global__ void __launch_bounds__(128, PRODUCER ? kProducerBlocksPerSm : kAppendBlocksPerSm) tq4_append_kernel(const AppendParams p) {
+    // an attention kernel launched behind this one may set itself up meanwhile (it waits for this grid's end before it reads)
+    asm volatile("griddepcontrol.launch_dependents;");
     __shared__ float s_centroid[16];
     __shared__ float s_w1[PRODUCER ? kHeadDim : 1];
     __shared__ float s_inv_freq[PRODUCER ? kHeadDim / 2 : 1];

@@ -301,6 +301,77 @@ __global__ void __launch_bounds__(128) attn_output_gate_kernel(const void* __res
     }
 }
 
+__device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
+    const __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// ---- rows held as 8 consecutive columns per lane ------------------------------------------------------------
+// 16-byte accesses when the matrix starts on a 16-byte boundary (rows are 512 bytes apart).
+__device__ __forceinline__ void load8(const void* base, size_t row_base, int lane, int bf16, float (&v)[8]) {
+    const uint16_t* src = static_cast<const uint16_t*>(base) + row_base + 8 * lane;
+    uint32_t w[4];
+    if (((uintptr_t)base & 15u) == 0u) {
+        const uint4 q = *reinterpret_cast<const uint4*>(src);
+        w[0] = q.x; w[1] = q.y; w[2] = q.z; w[3] = q.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[i] = (uint32_t)src[2 * i] | ((uint32_t)src[2 * i + 1] << 16);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 f = bf16 ? make_float2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u))
+                              : __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+        v[2 * i] = f.x;
+        v[2 * i + 1] = f.y;
+    }
+}
+__device__ __forceinline__ void store8(void* base, size_t row_base, int lane, int bf16, const float (&v)[8]) {
+    uint16_t* dst = static_cast<uint16_t*>(base) + row_base + 8 * lane;
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (bf16) {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+            w[i] = *reinterpret_cast<const uint32_t*>(&h);
+        } else {
+            w[i] = pack_half2(v[2 * i], v[2 * i + 1]);
+        }
+    }
+    if (((uintptr_t)base & 15u) == 0u) {
+        *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { dst[2 * i] = (uint16_t)w[i]; dst[2 * i + 1] = (uint16_t)(w[i] >> 16); }
+    }
+}
+// Butterfly over column bits [3, 3 + LEVELS): lanes.  Upper lane o - x, lower x + o, one rounding either way.
+template <int LEVELS>
+__device__ __forceinline__ void butterfly8(float (&v)[8], int lane) {
+#pragma unroll
+    for (int d = 1; d < 8; d <<= 1) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if ((i & d) == 0) {
+                const float a = v[i], b = v[i | d];
+                v[i] = a + b;
+                v[i | d] = a - b;
+            }
+        }
+    }
+#pragma unroll
+    for (int d = 1; d < (1 << LEVELS); d <<= 1) {
+        const float dir = (lane & d) ? -1.0f : 1.0f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = __fmaf_rn(dir, v[i], __shfl_xor_sync(0xffffffffu, v[i], d));
+    }
+}
+__device__ __forceinline__ void sign8(float (&v)[8], int lane) {
+    const uint32_t bits = c_sign_mask[lane >> 2] >> (8 * (lane & 3));
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(__float_as_uint(v[i]) ^ ((bits >> i) << 31));
+}
+
 // ---------------------------------------------------------------------------------------
 // Scalar dequant-then-attend: one block of four warps per (token, q head), fp32, any strides.
 // ---------------------------------------------------------------------------------------
@@ -433,7 +504,7 @@ constexpr int kRowsPerGroup = 8;            // N of the MMA: query rows per work
 constexpr int kLutBytes = 256 * 256;         // byte-pair table: 256-byte entry stride, 32 lane copies each
 constexpr int kPartialFloats = kRowsPerGroup * kHeadDim + 2 * kRowsPerGroup;
 constexpr long long kWaitCycleLimit = 1ll << 31;  // about one second of SM clocks
-constexpr int kMinUnitsPerWarp = 4;   // 8, 16 and 32 measured equal or slower on small batches
+constexpr int kMinUnitsPerWarp = 2;   // one two-page step of the exact kernel; 4 and more measured slower on small batches
 // The lookup table holds fp16(kLutScale * centroid).  fp16 rounding of the 8 centroid
 // magnitudes is a systematic error of up to 3.7e-4 relative; with this common factor every one
 // of them lands within 9.5e-5 of an fp16 grid point (found by exhaustive search over
@@ -510,19 +581,43 @@ __device__ __forceinline__ int32_t* plan_array(uint8_t* scratch, int which, int 
 // Words per lane of one work item's query fragments: 16 k-steps x 2 B-fragment words of fp16(Q'),
 // then 16 words holding the residual of Q' as bytes (four per k-step): Q' = hi + lo with hi the fp16
 // value just below Q' (rounded towards minus infinity), so that 0 <= lo < 1 ulp; lo divided by the
-// row's own step (largest lo of the row / 255) and rounded is an integer 0..255, which as the low
-// byte of an fp16 word is the subnormal number integer x 2^-24: exact, and no arithmetic to widen it;
-// then the steps of the lane's two rows (2 tig, 2 tig + 1), times 2^24, as floats.
-constexpr int kQFragWords = 50;
+// row's own step (largest lo of the row / 255) and rounded is an integer 0..255; then the step of the
+// lane's row (gid) as a float.
+constexpr int kQFragWords = 49;
 __host__ __device__ inline size_t qfrag_item_bytes() { return (size_t)kQFragWords * 32 * sizeof(uint32_t); }
 __device__ void qprep_block(const StreamParams& p, int idx);
 constexpr int kPlanThreads = 32 * kRowsPerGroup;  // the query-fragment blocks use one warp per query row
+
+// ---- dependent launches ---------------------------------------------------------------------------
+// The kernels of one attention call are launched behind each other with programmatic stream serialization: a kernel may
+// begin while the last blocks of the one before it finish, which hides the launch latency (about 2 us each on a stream).
+// Every kernel therefore waits for its predecessor's end before it touches global memory, and lets its successor start
+// being scheduled once its own blocks run.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
+
+template <class Params>
+static int launch_behind(void (*kernel)(const Params), unsigned grid, unsigned threads, size_t smem, cudaStream_t st, const Params& p) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return (int)cudaLaunchKernelEx(&cfg, kernel, p);
+}
 
 // Block 0 plans the split.  Blocks 1.. (one-warp items only) each rotate and scale the query rows
 // of one (request, kv head, row group) and store them as the B fragments of S^T = K Q'^T, so that
 // the stream kernel's warps (several per item, and again for every further item a warp reaches)
 // only load them.  The fragments are indexed without the plan, so both run side by side.
 __global__ void __launch_bounds__(kPlanThreads) tq4_attention_plan_kernel(const StreamParams p) {
+    grid_dependency_wait();
+    grid_launch_dependents();
     if (blockIdx.x > 0) {
         qprep_block(p, (int)blockIdx.x - 1);
         return;
@@ -606,6 +701,9 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 }
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
@@ -699,10 +797,6 @@ __device__ __forceinline__ float ex2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
-    const __half2 h = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<const uint32_t*>(&h);
-}
 
 // Four 8-bit codes -> two fp16 pairs (bytes 0,1 and bytes 2,3), exactly.
 template <int FMT>
@@ -747,14 +841,12 @@ __device__ __forceinline__ uint32_t token_offset(int t) {  // byte offset of tok
     return (uint32_t)((t >> 3) * kHalfStride + (t & 7) * kTq4RowBytes);
 }
 
-// The streaming kernel comes in two builds.
-//  * exact (default): every fp16 tensor-core operand that carries a rounding error of its own is
-//    fed as value + residual: Q' (residual kept as one byte per element, widened in registers), the K
-//    centroids (the lookup returns value pair and residual pair at once) and, on pages where some
-//    weight is large enough to matter, P x d_v.  Three score MMAs per k-step instead of one.  With
-//    fp16 operands alone a softmax weight is off by a few 1e-4 relative, which a x20 outlier channel
-//    of V turns into several 1e-3 absolute where its large terms cancel.
-//  * fast (WARP34_B200_EXEC_FLAG_FAST_ATTENTION): single fp16 operands, as the reference's own
+// The streaming kernel comes in two forms.
+//  * exact (default, tq4_stream_exact.cuh): every fp16 tensor-core operand that carries a rounding error of its own is
+//    fed as value + residual: Q', the K centroids, P x d_v and, on pages where some weight is large enough to matter,
+//    the V centroids.  With fp16 operands alone a softmax weight is off by a few 1e-4 relative, which a x20 outlier
+//    channel of V turns into several 1e-3 absolute where its large terms cancel.
+//  * fast (WARP34_B200_EXEC_FLAG_FAST_ATTENTION, below): single fp16 operands, as the reference's own
 //    tensor-core kernel computes (op_paged_attn.cu:357, :47-50, :470).
 constexpr int kFastWarps = 12, kFastStages = 3;
 constexpr int kExactWarps = 8, kExactStages = 4;
@@ -773,74 +865,24 @@ constexpr float kPeakedWeight = 0.25f;
 // row (see the query-fragment block).
 constexpr float kResidualScale = 2048.0f;
 
-// Eight warps: the query fragments of item idx = (request * kv heads + kv head) * q_groups_max + group.
-// Warp w rotates and scales query row w of the group into shared memory (fp32 [8 rows][256 rotated
-// columns], times q_scale); after the barrier it builds the fragment words of step w.
-__device__ void qprep_block(const StreamParams& p, int idx) {
-    __shared__ float q_stage[kRowsPerGroup * kHeadDim];
-    __shared__ float q_step[kRowsPerGroup];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int gid = lane >> 2, tig = lane & 3;
-    const int hkv = p.layout.local_kv_heads;
-    const int group = idx % p.q_groups_max;
-    const int kv_head = (idx / p.q_groups_max) % hkv;
-    const int r = idx / (p.q_groups_max * hkv);
-    if (r >= p.batch.num_reqs || p.qfrag == nullptr) return;  // block-uniform
-    const ReqGeom g = stream_req(p, r);
-    const int rows_in_req = g.q_len * p.gqa;
-    if (!g.valid || group * kRowsPerGroup >= rows_in_req) return;  // block-uniform
-    {
-        const int row8 = wid;
-        const int row = group * kRowsPerGroup + row8;
-        const int q_off = row / p.gqa;
-        const int q_head = kv_head * p.gqa + (row - q_off * p.gqa);
-        const bool ok = row < rows_in_req &&
-                        (p.batch.valid_token_mask == nullptr || p.batch.valid_token_mask[g.q_start + q_off] != 0);
-        float t[8];
-        if (ok) {
-            const size_t q_base = ((size_t)(g.q_start + q_off) * p.num_q_heads + q_head) * kHeadDim;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) t[j] = apply_sign(load_act(p.q_in, q_base + lane + 32 * j, p.io_bf16), lane + 32 * j);
-            wht256_lanes(t, lane);
-        } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) t[j] = 0.0f;
-        }
-        float rmax = 0.0f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const float f = t[j] * p.q_scale;
-            q_stage[row8 * kHeadDim + lane + 32 * j] = f;
-            if (p.q_floor) rmax = fmaxf(rmax, f - __half2float(__float2half_rd(f)));
-        }
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, d));
-        if (lane == 0) q_step[row8] = rmax * (1.0f / 255.0f);
-    }
-    __syncthreads();
-    // B fragments of Q'^T: step s (0..7) covers half s >> 2, virtual word 4 tig + (s & 3);
-    // k-step 2 s uses elements 0..3 of the word, k-step 2 s + 1 elements 4..7.
-    // Q' = hi + lo: hi is fp16 (rounded down), lo >= 0 is kept as 4 bytes per k-step, integers in units
-    // of the row's step, and widened to fp16 pairs (subnormals) by two PRMTs right before its MMA.
-    const int s = wid;
+// Words of step s (0..7) of one item's B fragments of Q'^T, for this lane: half s >> 2, virtual word 4 tig + (s & 3); k-step
+// 2 s uses elements 0..3 of the word, k-step 2 s + 1 elements 4..7.  `value(c)` is rotated column c of the lane's row
+// (gid), `step` the step of that row's residuals.
+template <class Value>
+__device__ __forceinline__ void query_fragments(int s, int lane, float step, Value value, uint32_t* dst, bool floor) {
+    const int tig = lane & 3;
     const int half = s >> 2, vw = 4 * tig + (s & 3);
-    uint32_t* dst = p.qfrag + (size_t)idx * (kQFragWords * 32) + lane;
-    const float step = q_step[gid];
     const float inv_step = step > 0.0f ? 1.0f / step : 0.0f;
-    if (s == 0) {   // the steps of the rows whose scores this lane holds in the stream kernel
-        dst[48 * 32] = __float_as_uint(q_step[2 * tig] * 16777216.0f);
-        dst[49 * 32] = __float_as_uint(q_step[2 * tig + 1] * 16777216.0f);
-    }
+    if (s == 0) dst[48 * 32] = __float_as_uint(step);
 #pragma unroll
     for (int hk = 0; hk < 2; ++hk) {
         uint32_t lo_bytes = 0;
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
             const int e = 4 * hk + 2 * x;
-            const float f0 = q_stage[gid * kHeadDim + vword_col(half, vw, e)];
-            const float f1 = q_stage[gid * kHeadDim + vword_col(half, vw, e + 1)];
-            const __half h0 = p.q_floor ? __float2half_rd(f0) : __float2half_rn(f0);
-            const __half h1 = p.q_floor ? __float2half_rd(f1) : __float2half_rn(f1);
+            const float f0 = value(vword_col(half, vw, e)), f1 = value(vword_col(half, vw, e + 1));
+            const __half h0 = floor ? __float2half_rd(f0) : __float2half_rn(f0);
+            const __half h1 = floor ? __float2half_rd(f1) : __float2half_rn(f1);
             dst[(2 * (2 * s + hk) + x) * 32] = (uint32_t)__half_as_ushort(h0) | ((uint32_t)__half_as_ushort(h1) << 16);
             // residuals in units of the row's step: integers 0..255
             const uint32_t b0 = (uint32_t)max(min(__float2int_rn((f0 - __half2float(h0)) * inv_step), 255), 0);
@@ -851,7 +893,55 @@ __device__ void qprep_block(const StreamParams& p, int idx) {
     }
 }
 
-template <int STAGES, int WARPS, bool EXACT, bool SPARSE = false>
+// Row stride of the rotated rows in shared memory: with a word of padding per 32 columns the fragment reads (8 rows x 4
+// words 32 columns apart) hit 32 distinct banks.
+constexpr int kQStageStride = 268;
+
+// Eight warps: the query fragments of item idx = (request * kv heads + kv head) * q_groups_max + group.
+// Warp w rotates and scales query row w of the group into shared memory (fp32, rotated, times q_scale); after the barrier it builds the fragment words of step w.
+__device__ void qprep_block(const StreamParams& p, int idx) {
+    __shared__ float q_stage[kRowsPerGroup * kQStageStride];
+    __shared__ float q_step[kRowsPerGroup];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int gid = lane >> 2;
+    const int hkv = p.layout.local_kv_heads;
+    const int group = idx % p.q_groups_max;
+    const int kv_head = (idx / p.q_groups_max) % hkv;
+    const int r = idx / (p.q_groups_max * hkv);
+    if (r >= p.batch.num_reqs || p.qfrag == nullptr) return;  // block-uniform
+    const ReqGeom g = stream_req(p, r);
+    const int rows_in_req = g.q_len * p.gqa;
+    if (!g.valid || group * kRowsPerGroup >= rows_in_req) return;  // block-uniform
+    {
+        const int row = group * kRowsPerGroup + wid;
+        const int q_off = row / p.gqa;
+        const int q_head = kv_head * p.gqa + (row - q_off * p.gqa);
+        const bool ok = row < rows_in_req &&
+                        (p.batch.valid_token_mask == nullptr || p.batch.valid_token_mask[g.q_start + q_off] != 0);
+        float t[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};     // columns [8 lane, + 8)
+        if (ok) {
+            load8(p.q_in, ((size_t)(g.q_start + q_off) * p.num_q_heads + q_head) * kHeadDim, lane, p.io_bf16, t);
+            sign8(t, lane);
+            butterfly8<5>(t, lane);
+        }
+        float rmax = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float f = t[i] * (p.q_scale * 0.0625f);
+            q_stage[wid * kQStageStride + 8 * lane + (lane >> 2) + i] = f;     // one word of padding per 32 columns
+            if (p.q_floor) rmax = fmaxf(rmax, f - __half2float(__float2half_rd(f)));
+        }
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, d));
+        if (lane == 0) q_step[wid] = rmax * (1.0f / 255.0f);
+    }
+    __syncthreads();
+    const float step = q_step[gid];
+    query_fragments(wid, lane, step, [&](int c) { return q_stage[gid * kQStageStride + c + (c >> 5)]; }, p.qfrag + (size_t)idx * (kQFragWords * 32) + lane,
+                    p.q_floor != 0);
+}
+
+template <int STAGES, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 1) tq4_attention_stream_kernel(const StreamParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];
     // The lookup table sits at the first 64 KB-aligned SHARED address inside the dynamic window,
@@ -881,20 +971,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) tq4_attention_stream_kernel(con
     for (int i = threadIdx.x; i < 256 * 32; i += blockDim.x) {
         const int byte = i >> 5, ln = i & 31;
         const float c0 = kLutScale * tq4_centroid(byte & 15), c1 = kLutScale * tq4_centroid(byte >> 4);
-        if (EXACT) {
-            // K table: (value pair, residual pair) in 16 copies of 8 bytes; V table: value pair in
-            // 32 copies of 4 bytes, in the upper half of the same 256-byte entry
-            const uint32_t hi = pack_half2(c0, c1);
-            const float2 hf = __half22float2(*reinterpret_cast<const __half2*>(&hi));
-            if (ln < 16) {
-                sts32(lut_addr + (uint32_t)(byte * 256 + ln * 8), hi);
-                sts32(lut_addr + (uint32_t)(byte * 256 + ln * 8 + 4),
-                      pack_half2((c0 - hf.x) * kResidualScale, (c1 - hf.y) * kResidualScale));
-            }
-            sts32(lut_addr + (uint32_t)(byte * 256 + 128 + ln * 4), hi);
-        } else {
-            sts32(lut_addr + (uint32_t)(byte * 256 + ln * 4), pack_half2(c0, c1));
-        }
+        sts32(lut_addr + (uint32_t)(byte * 256 + ln * 4), pack_half2(c0, c1));
     }
     if (lane == 0) {
         for (int s = 0; s < STAGES; ++s) mbar_init(bars + 8u * s, 1u);
@@ -926,8 +1003,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) tq4_attention_stream_kernel(con
     // In the PV product thread tig owns tokens kv0 + {0, 1, 4, 5} (k positions 2tig, 2tig+1, +8, +9).
     const int kv0 = 2 * (tig & 1) + 8 * (tig >> 1);
     // byte 1 of these is zero: the code byte goes there
-    const uint32_t lut_lane = EXACT ? lut_addr + 128u + 4u * lane : lut_addr + 4u * lane;   // V (and K) values
-    const uint32_t lutk_lane = lut_addr + 8u * (lane & 15);                                      // K value + residual
+    const uint32_t lut_lane = lut_addr + 4u * lane;
     uint32_t phase_bits = 0;   // bit s = parity to wait for on stage s
     uint32_t pending = 0;      // bit s = a copy into stage s has been issued and not yet awaited
     bool failed = false;
@@ -981,8 +1057,6 @@ __global__ void __launch_bounds__(WARPS * 32, 1) tq4_attention_stream_kernel(con
 
         // ---- Q' fragments of this item, prepared by the plan launch ---------------------------
         uint32_t qb[16][2];
-        uint32_t qlo[16];
-        float q_step[2] = {0.0f, 0.0f};
         {
             const uint32_t* qf = p.qfrag + ((size_t)(r * p.layout.local_kv_heads + kv_head) * p.q_groups_max + group) *
                                                (kQFragWords * 32) + lane;
@@ -990,11 +1064,6 @@ __global__ void __launch_bounds__(WARPS * 32, 1) tq4_attention_stream_kernel(con
             for (int i = 0; i < 16; ++i) {
                 qb[i][0] = __ldg(qf + (2 * i) * 32);
                 qb[i][1] = __ldg(qf + (2 * i + 1) * 32);
-                qlo[i] = EXACT ? __ldg(qf + (32 + i) * 32) : 0u;
-            }
-            if (EXACT) {
-                q_step[0] = __uint_as_float(__ldg(qf + 48 * 32));
-                q_step[1] = __uint_as_float(__ldg(qf + 49 * 32));
             }
         }
         // ---- accumulators ----------------------------------------------------------------
@@ -1008,50 +1077,10 @@ __global__ void __launch_bounds__(WARPS * 32, 1) tq4_attention_stream_kernel(con
         const int32_t* blocks = p.batch.block_tables + (size_t)r * p.batch.max_blocks_per_req;
         const uint8_t* k_head_base = (const uint8_t*)(uintptr_t)p.layout.k_base + (size_t)kv_head * p.layout.k_head_stride_bytes;
         const uint8_t* v_head_base = (const uint8_t*)(uintptr_t)p.layout.v_base + (size_t)kv_head * p.layout.v_head_stride_bytes;
-        int32_t my_page = 0, next_page = 0;
-        if (!SPARSE) {
-            my_page = (lane < n_here) ? block_table_page(blocks, pg0 + lane, p.batch.max_blocks_per_req, kInStream) : 0;  // page ids of units [0, 32)
-            next_page = (32 + lane < n_here) ? block_table_page(blocks, pg0 + 32 + lane, p.batch.max_blocks_per_req, kInStream) : 0;
-        }
-        // query-sparse: the token's selected list, its length and its position
-        const int32_t* sel_phys = SPARSE ? p.sel_phys + (size_t)r * p.select_k : nullptr;
-        const int32_t* sel_logical = SPARSE ? p.sel_logical + (size_t)r * p.select_k : nullptr;
-        const int n_sel = SPARSE ? min(p.num_selected[r], p.select_k) : 0;
-
+        int32_t my_page = (lane < n_here) ? block_table_page(blocks, pg0 + lane, p.batch.max_blocks_per_req, kInStream) : 0;  // page ids of units [0, 32)
+        int32_t next_page = (32 + lane < n_here) ? block_table_page(blocks, pg0 + 32 + lane, p.batch.max_blocks_per_req, kInStream) : 0;
         fence_proxy_async();  // the staging writes above precede async-proxy writes to the ring
         auto issue = [&](int idx) {  // called by all lanes; lane 0 issues the four copies
-            if (SPARSE) {
-                // Unit idx = entries 4 (pg0 + idx) .. + 3 of the list.  Lane j < 4 takes entry j: a group of
-                // four rows (528 bytes of K, 528 of V) lands at rows 4 j .. 4 j + 3 of the stage; a skipped
-                // entry (negative id, past the list's end, or wholly after the token's position) copies
-                // nothing and is masked below through the position word kept in the stage's padding.
-                const int s = idx % STAGES;
-                const uint32_t bar = bars + 8u * s;
-                const uint32_t dst = ring + (uint32_t)s * kStageStride;
-                const int gi = 4 * (pg0 + idx) + lane;
-                int ph = -1, first_pos = 0x3fffffff;
-                if (lane < 4 && gi < n_sel) {
-                    ph = sel_phys[gi];
-                    const int lg = sel_logical[gi];
-                    if (ph >= 0 && 4 * lg <= g.ctx_before) first_pos = 4 * lg; else ph = -1;
-                }
-                const int n_valid = __popc(__ballot_sync(0xffffffffu, ph >= 0));
-                pending |= 1u << s;
-                if (lane == 0) mbar_expect_tx(bar, (uint32_t)n_valid * 8u * kTq4RowBytes);
-                __syncwarp();
-                if (lane < 4) {
-                    sts32(dst + kHalfBytes + 4u * lane, (uint32_t)first_pos);
-                    if (ph >= 0) {
-                        const int page = pool_page(ph >> 2, kInStream);
-                        const uint32_t row_off = (uint32_t)(ph & 3) * 4u * kTq4RowBytes;
-                        bulk_g2s(dst + token_offset(4 * lane), k_head_base + (size_t)page * p.layout.k_page_stride_bytes + row_off,
-                                 4u * kTq4RowBytes, bar);
-                        bulk_g2s(dst + kRunStride + token_offset(4 * lane),
-                                 v_head_base + (size_t)page * p.layout.v_page_stride_bytes + row_off, 4u * kTq4RowBytes, bar);
-                    }
-                }
-                return;
-            }
             const int32_t page = __shfl_sync(0xffffffffu, (idx & 32) ? next_page : my_page, idx & 31);
             pending |= 1u << (idx % STAGES);
             if (lane == 0) {
@@ -1070,12 +1099,11 @@ __global__ void __launch_bounds__(WARPS * 32, 1) tq4_attention_stream_kernel(con
         // `my_page` holds ids for units [64 c, 64 c + 32), `next_page` for [64 c + 32, 64 c + 64).
 #pragma unroll 1
         for (int i = 0; i < STAGES - 1 && i < n_here; ++i) issue(i);
-        if (SPARSE) __syncwarp();   // the position words written by lanes 0-3 are read by all lanes
 
 #pragma unroll 1
         for (int i = 0; i < n_here; ++i) {
             // refill page-id registers every 32 units, one window ahead
-            if (!SPARSE && (i & 31) == 0 && i > 0) {
+            if ((i & 31) == 0 && i > 0) {
                 const int base = i + 32;  // ids for [i+32, i+64) replace the window just consumed
                 const int32_t fresh = (base + lane < n_here) ? block_table_page(blocks, pg0 + base + lane, p.batch.max_blocks_per_req, kInStream) : 0;
                 if (i & 32) my_page = fresh; else next_page = fresh;
@@ -1092,30 +1120,13 @@ __global__ void __launch_bounds__(WARPS * 32, 1) tq4_attention_stream_kernel(con
             const uint32_t kst = ring + (uint32_t)s * kStageStride;
             const uint32_t vst = kst + kRunStride;
             const int kv_base = (pg0 + i) << 4;
-            bool full = (kv_base >= safe_lo) && (kv_base + 15 <= safe_hi);
+            const bool full = (kv_base >= safe_lo) && (kv_base + 15 <= safe_hi);
             const uint32_t ptok = page_token(i);
-            // query-sparse: position of the first row of the two groups this lane's keys sit in
-            int pos_a_sparse = 0, pos_b_sparse = 0;
-            if (SPARSE) {
-                const uint32_t pw = kst + kHalfBytes;
-                const int f0 = (int)lds32_dep(pw, ptok), f1 = (int)lds32_dep(pw + 4, ptok);
-                const int f2 = (int)lds32_dep(pw + 8, ptok), f3 = (int)lds32_dep(pw + 12, ptok);
-                full = max(max(f0, f1), max(f2, f3)) + 3 <= safe_hi;
-                pos_a_sparse = ((key_a >> 3) ? f2 : f0) + (key_a & 3);
-                pos_b_sparse = ((key_a >> 3) ? f3 : f1) + (key_a & 3);
-            }
 #define W34_LDS(addr) lds32_dep(addr, ptok)
 #define W34_LUT(word, k) lds32_lut(__byte_perm((word), lut_lane, 0x7604 + ((k) << 4)))
-#define W34_LUTK(word, k) lds64_lut(__byte_perm((word), lutk_lane, 0x7604 + ((k) << 4)))
 
             // ---- S^T = K Q'^T, one accumulator per 128-half ------------------------------
-            float sa[2][4], sl[2][4], sk[2][4];  // value, query-residual and key-residual chains are independent
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                sa[h][0] = sa[h][1] = sa[h][2] = sa[h][3] = 0.0f;
-                sl[h][0] = sl[h][1] = sl[h][2] = sl[h][3] = 0.0f;
-                sk[h][0] = sk[h][1] = sk[h][2] = sk[h][3] = 0.0f;
-            }
+            float sa[2][4];
             const uint32_t krow_a = kst + token_offset(key_a);
             const uint32_t krow_b = krow_a + 4u * kTq4RowBytes;
             const uint32_t ka0 = W34_LDS(krow_a), ka16 = W34_LDS(krow_a + 64);
@@ -1139,26 +1150,14 @@ __global__ void __launch_bounds__(WARPS * 32, 1) tq4_attention_stream_kernel(con
                 }
 #pragma unroll
                 for (int hk = 0; hk < 2; ++hk) {
-                    uint32_t a0, a1, a2, a3;
-                    if (EXACT) {
-                        const uint2 e0 = W34_LUTK(wa, 2 * hk), e1 = W34_LUTK(wb, 2 * hk);
-                        const uint2 e2 = W34_LUTK(wa, 2 * hk + 1), e3 = W34_LUTK(wb, 2 * hk + 1);
-                        a0 = e0.x; a1 = e1.x; a2 = e2.x; a3 = e3.x;
-                        mma16816(sk[half], e0.y, e1.y, e2.y, e3.y, qb[2 * s8 + hk][0], qb[2 * s8 + hk][1]);
-                    } else {
-                        a0 = W34_LUT(wa, 2 * hk);
-                        a1 = W34_LUT(wb, 2 * hk);
-                        a2 = W34_LUT(wa, 2 * hk + 1);
-                        a3 = W34_LUT(wb, 2 * hk + 1);
-                    }
-                    const uint32_t ql = qlo[2 * s8 + hk];
+                    const uint32_t a0 = W34_LUT(wa, 2 * hk);
+                    const uint32_t a1 = W34_LUT(wb, 2 * hk);
+                    const uint32_t a2 = W34_LUT(wa, 2 * hk + 1);
+                    const uint32_t a3 = W34_LUT(wb, 2 * hk + 1);
                     if ((s8 & 3) == 0 && hk == 0) {
                         mma16816_zero(sa[half], a0, a1, a2, a3, qb[2 * s8 + hk][0], qb[2 * s8 + hk][1]);
                     } else {
                         mma16816(sa[half], a0, a1, a2, a3, qb[2 * s8 + hk][0], qb[2 * s8 + hk][1]);
-                    }
-                    if (EXACT) {   // residual bytes -> fp16 pairs: byte b becomes the half 0x00bb = b x 2^-24
-                        mma16816(sl[half], a0, a1, a2, a3, __byte_perm(ql, 0, 0x4140), __byte_perm(ql, 0, 0x4342));
                     }
                 }
             }
@@ -1168,13 +1167,6 @@ __global__ void __launch_bounds__(WARPS * 32, 1) tq4_attention_stream_kernel(con
             const float dkb0 = __half2float(__ushort_as_half((unsigned short)(kb0 & 0xffffu)));
             const float dkb1 = __half2float(__ushort_as_half((unsigned short)(kb16 >> 16)));
             // sc[0],sc[1]: token key_a, rows 2tig, 2tig+1;  sc[2],sc[3]: token key_a + 4
-            if (EXACT) {
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-#pragma unroll
-                    for (int x = 0; x < 4; ++x) sa[h][x] += sl[h][x] * q_step[x & 1] + sk[h][x] * (1.0f / kResidualScale);
-                }
-            }
             float sc[4];
             sc[0] = dka0 * sa[0][0] + dka1 * sa[1][0];
             sc[1] = dka0 * sa[0][1] + dka1 * sa[1][1];
@@ -1191,7 +1183,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) tq4_attention_stream_kernel(con
 
             bool msk[4] = {false, false, false, false};
             if (!full) {
-                const int pos_a = SPARSE ? pos_a_sparse : kv_base + key_a, pos_b = SPARSE ? pos_b_sparse : pos_a + 4;
+                const int pos_a = kv_base + key_a, pos_b = pos_a + 4;
                 msk[0] = !(pos_a >= rmin[0] && pos_a <= rmax[0]);
                 msk[1] = !(pos_a >= rmin[1] && pos_a <= rmax[1]);
                 msk[2] = !(pos_b >= rmin[0] && pos_b <= rmax[0]);
@@ -1231,28 +1223,10 @@ __global__ void __launch_bounds__(WARPS * 32, 1) tq4_attention_stream_kernel(con
                 if (msk[0] && msk[1]) { dva0 = 0.0f; dva1 = 0.0f; }
                 if (msk[2] && msk[3]) { dvb0 = 0.0f; dvb1 = 0.0f; }
             }
-            bool peaked = false;
-            if (EXACT) {
-                // the exact build keeps the row totals (every lane of a row holds the same l) for the test
-                float ps0 = pr[0] + pr[2], ps1 = pr[1] + pr[3];
-#pragma unroll
-                for (int d = 4; d < 32; d <<= 1) {
-                    ps0 += __shfl_xor_sync(0xffffffffu, ps0, d);
-                    ps1 += __shfl_xor_sync(0xffffffffu, ps1, d);
-                }
-                l_run[0] += ps0;
-                l_run[1] += ps1;
-                // (rows that do not exist score 0 against their zero query; they must not count as peaks)
-                const bool pk0 = rvalid[0] && fmaxf(pr[0], pr[2]) > kPeakedWeight * l_run[0];
-                const bool pk1 = rvalid[1] && fmaxf(pr[1], pr[3]) > kPeakedWeight * l_run[1];
-                peaked = __any_sync(0xffffffffu, pk0 || pk1);
-            } else {
-                l_run[0] += pr[0] + pr[2];
-                l_run[1] += pr[1] + pr[3];
-            }
-            // P * d_v per half as B fragments (k = key, n = query row); the exact build adds the fp16
-            // rounding residual of P * d_v as a second fragment.
-            uint32_t pb[2][2], pl[2][2] = {{0u, 0u}, {0u, 0u}};
+            l_run[0] += pr[0] + pr[2];
+            l_run[1] += pr[1] + pr[3];
+            // P * d_v per half as B fragments (k = key, n = query row)
+            uint32_t pb[2][2];
             const float pd[2][4] = {{pr[0] * dva0, pr[1] * dva0, pr[2] * dvb0, pr[3] * dvb0},
                                     {pr[0] * dva1, pr[1] * dva1, pr[2] * dvb1, pr[3] * dvb1}};
 #pragma unroll
@@ -1261,11 +1235,6 @@ __global__ void __launch_bounds__(WARPS * 32, 1) tq4_attention_stream_kernel(con
                 for (int x = 0; x < 2; ++x) {
                     const __half2 hi = __floats2half2_rn(pd[h][2 * x], pd[h][2 * x + 1]);
                     pb[h][x] = movmatrix_trans(*reinterpret_cast<const uint32_t*>(&hi));
-                    if (EXACT) {
-                        const float2 hf = __half22float2(hi);
-                        const __half2 lo = __floats2half2_rn(pd[h][2 * x] - hf.x, pd[h][2 * x + 1] - hf.y);
-                        pl[h][x] = movmatrix_trans(*reinterpret_cast<const uint32_t*>(&lo));
-                    }
                 }
             }
 
@@ -1274,10 +1243,6 @@ __global__ void __launch_bounds__(WARPS * 32, 1) tq4_attention_stream_kernel(con
             // tokens kv0 + {0, 1, 4, 5}
             const uint32_t vr = vst + token_offset(kv0);
             const uint32_t vwb = 4u * (uint32_t)(gid >> 1) + (uint32_t)(gid & 1);
-            // Every page: V P + V P_residual.  A peaked page then adds V_residual P in a second pass over
-            // its V codes (the K table holds the residuals).
-            // The second pass is a branch of its own so that the common pass stays one basic block
-            // with the softmax above it, whose latencies its loads and look-ups fill.
 #pragma unroll
             for (int i4 = 0; i4 < 4; ++i4) {
                 const int half = i4 >> 1;
@@ -1305,53 +1270,9 @@ __global__ void __launch_bounds__(WARPS * 32, 1) tq4_attention_stream_kernel(con
                     const uint32_t a2 = W34_LUT(lo_cd, t);
                     const uint32_t a3 = W34_LUT(hi_cd, t);
                     mma16816(o[4 * i4 + t], a0, a1, a2, a3, pb[half][0], pb[half][1]);
-                    if (EXACT) mma16816(o[4 * i4 + t], a0, a1, a2, a3, pl[half][0], pl[half][1]);
                 }
-            }
-            if (peaked) {
-                // P * d_v / kResidualScale, the partner of the scaled centroid residuals
-                uint32_t ps[2][2];
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-#pragma unroll
-                    for (int x = 0; x < 2; ++x) {
-                        const __half2 sc2 = __floats2half2_rn(pd[h][2 * x] * (1.0f / kResidualScale),
-                                                              pd[h][2 * x + 1] * (1.0f / kResidualScale));
-                        ps[h][x] = movmatrix_trans(*reinterpret_cast<const uint32_t*>(&sc2));
-                    }
-                }
-                auto pv_fix = [&]() {
-#pragma unroll
-                    for (int i4 = 0; i4 < 4; ++i4) {
-                        const int half = i4 >> 1;
-                        uint32_t w[4];
-                        const uint32_t off = 4u * ((half ? 17u : 0u) + vwb + 2u * (i4 & 1));
-                        w[0] = W34_LDS(vr + off);
-                        w[1] = W34_LDS(vr + kTq4RowBytes + off);
-                        w[2] = W34_LDS(vr + 4u * kTq4RowBytes + off);
-                        w[3] = W34_LDS(vr + 5u * kTq4RowBytes + off);
-                        if (i4 == 0 && gid == 0) {
-                            w[0] = (w[0] >> 16) | (W34_LDS(vr + 64) << 16);
-                            w[1] = (w[1] >> 16) | (W34_LDS(vr + kTq4RowBytes + 64) << 16);
-                            w[2] = (w[2] >> 16) | (W34_LDS(vr + 4u * kTq4RowBytes + 64) << 16);
-                            w[3] = (w[3] >> 16) | (W34_LDS(vr + 5u * kTq4RowBytes + 64) << 16);
-                        }
-                        const uint32_t lo_ab = (w[0] & 0x0f0f0f0fu) | ((w[1] << 4) & 0xf0f0f0f0u);
-                        const uint32_t hi_ab = ((w[0] >> 4) & 0x0f0f0f0fu) | (w[1] & 0xf0f0f0f0u);
-                        const uint32_t lo_cd = (w[2] & 0x0f0f0f0fu) | ((w[3] << 4) & 0xf0f0f0f0u);
-                        const uint32_t hi_cd = ((w[2] >> 4) & 0x0f0f0f0fu) | (w[3] & 0xf0f0f0f0u);
-#pragma unroll
-                        for (int t = 0; t < 4; ++t) {
-                            const uint2 e0 = W34_LUTK(lo_ab, t), e1 = W34_LUTK(hi_ab, t);
-                            const uint2 e2 = W34_LUTK(lo_cd, t), e3 = W34_LUTK(hi_cd, t);
-                            mma16816(o[4 * i4 + t], e0.y, e1.y, e2.y, e3.y, ps[half][0], ps[half][1]);
-                        }
-                    }
-                };
-                pv_fix();
             }
 #undef W34_LUT
-#undef W34_LUTK
 #undef W34_LDS
             __syncwarp();  // every lane is done with stage s before it is refilled
         }
@@ -1368,13 +1289,11 @@ __global__ void __launch_bounds__(WARPS * 32, 1) tq4_attention_stream_kernel(con
         }
 
         // ---- write the partial: natural column order, through the idle ring ------------------
-        // l: add the 8 lanes (gid) that share a query row (the exact build already holds row totals)
-        if (!EXACT) {
+        // l: add the 8 lanes (gid) that share a query row
 #pragma unroll
-            for (int d = 4; d < 32; d <<= 1) {
-                l_run[0] += __shfl_xor_sync(0xffffffffu, l_run[0], d);
-                l_run[1] += __shfl_xor_sync(0xffffffffu, l_run[1], d);
-            }
+        for (int d = 4; d < 32; d <<= 1) {
+            l_run[0] += __shfl_xor_sync(0xffffffffu, l_run[0], d);
+            l_run[1] += __shfl_xor_sync(0xffffffffu, l_run[1], d);
         }
         float* stage_o = reinterpret_cast<float*>(ring_gen);  // [8 rows][256]
 #pragma unroll
@@ -1916,6 +1835,7 @@ __device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, ui
 W34_BOUNDS_HOST_HOOKS(attention)
 
 }  // namespace w34
+#include "tq4_stream_exact.cuh"
 #include "tq4_prefill_tc.cuh"
 #include "prefill_pair.cuh"
 namespace w34 {
@@ -1934,6 +1854,8 @@ template <bool PARTIAL_OUT, int MW>
 __global__ void __launch_bounds__(MW * 32) tq4_attention_merge_kernel(const StreamParams p) {
     __shared__ float s_acc[MW][kHeadDim];
     __shared__ float s_m[MW], s_l[MW];
+    grid_dependency_wait();
+    grid_launch_dependents();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const long long row_ll = blockIdx.x;
     int tok = (int)(row_ll / p.num_q_heads);
@@ -1958,8 +1880,11 @@ __global__ void __launch_bounds__(MW * 32) tq4_attention_merge_kernel(const Stre
     };
     if (p.batch.valid_token_mask != nullptr && p.batch.valid_token_mask[tok] == 0) { skip_row(); return; }
     const int R = p.batch.num_reqs;
-    const int r = p.sel_phys != nullptr ? tok : find_request(p.batch.query_start_loc, R, tok);
-    if (r < 0) { skip_row(); return; }
+    int r = tok;
+    if (p.sel_phys == nullptr) {
+        if (tok < p.batch.query_start_loc[0] || tok >= p.batch.query_start_loc[R]) { skip_row(); return; }
+        r = last_not_above(p.batch.query_start_loc, R, tok);
+    }
     if (p.batch.valid_req_mask != nullptr && p.batch.valid_req_mask[r] == 0) { skip_row(); return; }
 
     const PlanHeader* hdr = reinterpret_cast<const PlanHeader*>(p.scratch);
@@ -1987,15 +1912,18 @@ __global__ void __launch_bounds__(MW * 32) tq4_attention_merge_kernel(const Stre
         const int w_first = us / per, w_last = (us + npages - 1) / per;
         const float* base = partials + (size_t)(w_first + item_prefix[r] + item) * part_floats;
         const int nparts = w_last - w_first + 1;
-        // this warp's partials: wid, wid + MW, ...; lanes fetch up to 32 (m, l) pairs at once so
-        // that the accumulation runs over independent loads
-        for (int c0 = wid; c0 < nparts; c0 += 32 * MW) {
-            const int mine = c0 + MW * lane;
+        // Slots go to the warps by groups of eight workers (what the workers of one CTA hold of an item usually sits in the
+        // first of their slots, the others are empty).  A warp looks at four of its groups at once, a lane per slot, and
+        // then reads the slots that hold anything, four at a time.
+        const int groups = ((w_first & 7) + nparts + 7) >> 3;
+        for (int g0 = wid; g0 < groups; g0 += 4 * MW) {
+            const int mine = (g0 + MW * (lane >> 3)) * 8 - (w_first & 7) + (lane & 7);
             float m_s = -1e30f, l_s = 0.0f;
-            if (mine < nparts) {
+            if (mine >= 0 && mine < nparts) {
                 const float* ps = base + (size_t)mine * part_floats + rpg * kHeadDim;
                 l_s = ps[rpg + row8];
-                m_s = (l_s > 0.0f) ? ps[row8] : -1e30f;
+                m_s = ps[row8];
+                if (!(l_s > 0.0f)) { l_s = 0.0f; m_s = -1e30f; }
             }
             float m_chunk = m_s;
 #pragma unroll
@@ -2011,13 +1939,24 @@ __global__ void __launch_bounds__(MW * 32) tq4_attention_merge_kernel(const Stre
 #pragma unroll
             for (int d = 16; d > 0; d >>= 1) lw += __shfl_xor_sync(0xffffffffu, lw, d);
             l_tot += lw;
-            const int n_here = min(32, (nparts - c0 + MW - 1) / MW);
-#pragma unroll 4
-            for (int sidx = 0; sidx < n_here; ++sidx) {
-                const float wgt = __shfl_sync(0xffffffffu, w_s, sidx);
-                const float* pa = base + (size_t)(c0 + MW * sidx) * part_floats + row8 * kHeadDim;
+            uint32_t full = __ballot_sync(0xffffffffu, w_s > 0.0f);
+            while (full != 0u) {
+                float wgt[4], v[4][8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) acc[j] += pa[lane + 32 * j] * wgt;
+                for (int k = 0; k < 4; ++k) {
+                    const int src = full != 0u ? __ffs((int)full) - 1 : 0;
+                    wgt[k] = full != 0u ? __shfl_sync(0xffffffffu, w_s, src) : 0.0f;
+                    const int slot = __shfl_sync(0xffffffffu, mine, src);
+                    const float* pa = base + (size_t)slot * part_floats + row8 * kHeadDim;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) v[k][j] = full != 0u ? pa[lane + 32 * j] : 0.0f;
+                    full &= full - 1u;
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) acc[j] += v[k][j] * wgt[k];
+                }
             }
         }
     }
@@ -2213,8 +2152,6 @@ __global__ void __launch_bounds__(128) kv_page_copy_kernel(const warp34_kv_layer
 }
 
 // ---- host side ---------------------------------------------------------------------------
-constexpr int kWarpsPerCta = kFastWarps > kExactWarps ? kFastWarps : kExactWarps;   // scratch is sized for the larger build
-
 // LUT + rings + mbarriers, plus up to 64 KB - 1 of alignment slack in front of the table; the
 // kernel is given the whole opt-in maximum and checks the carve-up itself.
 static size_t stream_smem_min_bytes() {
@@ -2246,13 +2183,13 @@ static DeviceInfo* device_info(int* rc) {
         *rc = (int)cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         if (*rc != 0) return nullptr;
         if ((size_t)optin < stream_smem_min_bytes()) { *rc = (int)cudaErrorNotSupported; return nullptr; }
-        *rc = (int)cudaFuncSetAttribute(tq4_attention_stream_kernel<kExactStages, kExactWarps, true>,
+        *rc = (int)cudaFuncSetAttribute(tq4_attention_stream_exact_kernel<false>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
         if (*rc != 0) return nullptr;
-        *rc = (int)cudaFuncSetAttribute(tq4_attention_stream_kernel<kFastStages, kFastWarps, false>,
+        *rc = (int)cudaFuncSetAttribute(tq4_attention_stream_kernel<kFastStages, kFastWarps>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
         if (*rc != 0) return nullptr;
-        *rc = (int)cudaFuncSetAttribute(tq4_attention_stream_kernel<kExactStages, kExactWarps, true, true>,
+        *rc = (int)cudaFuncSetAttribute(tq4_attention_stream_exact_kernel<true>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
         if (*rc != 0) return nullptr;
         *rc = (int)cudaFuncSetAttribute(tq4_attention_team_kernel<2>,
@@ -2378,6 +2315,15 @@ static warp34_attention_batch batch_part(const warp34_attention_batch* batch, in
     b.num_reqs = reqs;
     b.total_tokens = (int)part_tokens(batch, reqs);
     return b;
+}
+
+// The merge behind a streaming kernel.  Few rows with hundreds of partials each (one long sequence): 32 warps per row
+// instead of 4.
+template <bool PARTIAL_OUT>
+static int launch_merge(const StreamParams& p, long long rows, cudaStream_t st) {
+    const bool wide = rows * 4 < (long long)p.num_warps / 8;
+    return wide ? launch_behind(tq4_attention_merge_kernel<PARTIAL_OUT, 32>, (unsigned)rows, 1024, 0, st, p)
+                : launch_behind(tq4_attention_merge_kernel<PARTIAL_OUT, 4>, (unsigned)rows, 128, 0, st, p);
 }
 
 }  // namespace w34
@@ -2653,10 +2599,11 @@ static int launch_attention(const warp34_exec* ex, const warp34_kv_layer_layout*
         p.qfrag = (nt == 1) ? reinterpret_cast<uint32_t*>(p.scratch + plan + (size_t)p.max_slots * slot_bytes) : nullptr;
         p.smem_bytes = (uint32_t)smem;
         p.q_groups_max = (nt == 1) ? (int)(q_items / ((long long)reqs * layout->local_kv_heads)) : 0;
-        tq4_attention_plan_kernel<<<1 + (unsigned)q_items, q_items > 0 ? kPlanThreads : 32, 0, st>>>(p);
+        rc = launch_behind(tq4_attention_plan_kernel, 1 + (unsigned)q_items, q_items > 0 ? kPlanThreads : 32, 0, st, p);
+        if (rc != 0) return rc;
         if (nt == 1) {
-            if (fast) tq4_attention_stream_kernel<kFastStages, kFastWarps, false><<<grid, kFastWarps * 32, smem, st>>>(p);
-            else tq4_attention_stream_kernel<kExactStages, kExactWarps, true><<<grid, kExactWarps * 32, smem, st>>>(p);
+            if (fast) tq4_attention_stream_kernel<kFastStages, kFastWarps><<<grid, kFastWarps * 32, smem, st>>>(p);
+            else rc = launch_behind(tq4_attention_stream_exact_kernel<false>, (unsigned)grid, kXThreads, smem, st, p);
         } else if (nt == 2) {
             tq4_attention_team_kernel<2><<<grid, kTeams * kTeamWarps * 32, smem, st>>>(p);
         } else {
@@ -2665,15 +2612,8 @@ static int launch_attention(const warp34_exec* ex, const warp34_kv_layer_layout*
         // rows of the merge: every token of the batch, or (a part) as many as the part can hold, counted
         // from its first token
         const long long rows = (long long)p.batch.total_tokens * num_q_heads;
-        // Few rows with hundreds of partials each (one long sequence): 32 warps per row instead of 4.
-        const bool wide = rows * 4 < (long long)grid * workers_per_cta / 8;
-        if (triple_out != nullptr) {
-            if (wide) tq4_attention_merge_kernel<true, 32><<<(unsigned)rows, 1024, 0, st>>>(p);
-            else tq4_attention_merge_kernel<true, 4><<<(unsigned)rows, 128, 0, st>>>(p);
-        } else {
-            if (wide) tq4_attention_merge_kernel<false, 32><<<(unsigned)rows, 1024, 0, st>>>(p);
-            else tq4_attention_merge_kernel<false, 4><<<(unsigned)rows, 128, 0, st>>>(p);
-        }
+        if (rc == 0) rc = triple_out != nullptr ? launch_merge<true>(p, rows, st) : launch_merge<false>(p, rows, st);
+        if (rc != 0) return rc;
         rc = (int)cudaGetLastError();
         if (rc != 0) return rc;
     }
@@ -2763,20 +2703,17 @@ static int launch_qsa_stream_kv8(const warp34_exec* ex, const QsaParams& q, bool
     p.seq_pos = q.seq_pos;
     p.select_k = q.select_k;
     cudaStream_t st = (cudaStream_t)ex->stream;
-    tq4_attention_plan_kernel<<<1, 32, 0, st>>>(p);
+    rc = launch_behind(tq4_attention_plan_kernel, 1u, 32, 0, st, p);
+    if (rc != 0) return rc;
     if (fp8) {
-        kv8_attention_stream_kernel<WARP34_KV_FORMAT_FP8_E4M3, kKv8StreamStages, true><<<grid, kKv8StreamWarps * 32, smem, st>>>(p);
+        rc = launch_behind(kv8_attention_stream_kernel<WARP34_KV_FORMAT_FP8_E4M3, kKv8StreamStages, true>, (unsigned)grid, kKv8StreamWarps * 32, smem, st, p);
     } else {
-        kv8_attention_stream_kernel<WARP34_KV_FORMAT_Q8_0, kKv8StreamStages, true><<<grid, kKv8StreamWarps * 32, smem, st>>>(p);
+        rc = launch_behind(kv8_attention_stream_kernel<WARP34_KV_FORMAT_Q8_0, kKv8StreamStages, true>, (unsigned)grid, kKv8StreamWarps * 32, smem, st, p);
     }
     const long long rows = (long long)q.num_tokens * q.num_q_heads;
-    if (rows * 4 < (long long)grid * kKv8StreamWarps / 8) {
-        tq4_attention_merge_kernel<false, 32><<<(unsigned)rows, 1024, 0, st>>>(p);
-    } else {
-        tq4_attention_merge_kernel<false, 4><<<(unsigned)rows, 128, 0, st>>>(p);
-    }
+    if (rc != 0) return rc;
     *taken = true;
-    return (int)cudaGetLastError();
+    return launch_merge<false>(p, rows, st);
 }
 
 static int launch_qsa_stream(const warp34_exec* ex, const QsaParams& q, bool* taken) {
@@ -2839,16 +2776,13 @@ static int launch_qsa_stream(const warp34_exec* ex, const QsaParams& q, bool* ta
     p.seq_pos = q.seq_pos;
     p.select_k = q.select_k;
     cudaStream_t st = (cudaStream_t)ex->stream;
-    tq4_attention_plan_kernel<<<1 + (unsigned)items, kPlanThreads, 0, st>>>(p);
-    tq4_attention_stream_kernel<kExactStages, kExactWarps, true, true><<<grid, kExactWarps * 32, p.smem_bytes, st>>>(p);
+    rc = launch_behind(tq4_attention_plan_kernel, 1 + (unsigned)items, kPlanThreads, 0, st, p);
+    if (rc != 0) return rc;
+    rc = launch_behind(tq4_attention_stream_exact_kernel<true>, (unsigned)grid, kXThreads, p.smem_bytes, st, p);
     const long long rows = (long long)q.num_tokens * q.num_q_heads;
-    if (rows * 4 < (long long)grid * kExactWarps / 8) {
-        tq4_attention_merge_kernel<false, 32><<<(unsigned)rows, 1024, 0, st>>>(p);
-    } else {
-        tq4_attention_merge_kernel<false, 4><<<(unsigned)rows, 128, 0, st>>>(p);
-    }
+    if (rc != 0) return rc;
     *taken = true;
-    return (int)cudaGetLastError();
+    return launch_merge<false>(p, rows, st);
 }
 
 }  // namespace w34

@@ -79,6 +79,22 @@ __device__ __forceinline__ int find_request(const int32_t* __restrict__ qsl, int
     return lo;
 }
 
+// The largest r in [0, n) with prefix[r] <= v, for prefix[0] <= v, by one warp: every lane counts its share of the entries
+// (one round trip to memory; a binary search makes log2(n)).  Long arrays are searched.
+__device__ __forceinline__ int last_not_above(const int32_t* __restrict__ prefix, int n, int v) {
+    if (n > 1024) {
+        int lo = 0, hi = n;
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (prefix[mid] <= v) lo = mid; else hi = mid;
+        }
+        return lo;
+    }
+    int count = 0;
+    for (int i = 1 + (int)(threadIdx.x & 31); i < n; i += 32) count += prefix[i] <= v ? 1 : 0;
+    return (int)__reduce_add_sync(0xffffffffu, (unsigned)count);
+}
+
 // ---- bounds-checked build (-DW34_BOUNDS) ----------------------------------------------------------
 // Every index into a block table, every page id read from one and every write slot is range-checked
 // before an address is formed from it.  The first violation is recorded in a device word (what, the
