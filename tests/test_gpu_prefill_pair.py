@@ -59,3 +59,44 @@ def test_chunks_at_tile_edges_match_dequant_then_attend(env, fmt, hq, hkv, ctx, 
     assert ok, msg
     if drop is not None:
         assert (out[drop] == -7.0).all() and (out[n - new[-1]:] == -7.0).all()
+
+
+@pytest.mark.parametrize("fmt", ["TQ4", "FP8_E4M3", "Q8_0"])
+@pytest.mark.parametrize("hq,hkv,ctx,new,gate", [
+    (4, 1, [2000], [7], 0),                            # more ranges than tiles, one row in 32 in use
+    (24, 4, [700, 64, 1500], [40, 33, 50], 2),         # requests whose last ranges are empty
+    (6, 2, [3000], [129], 1),
+])
+def test_split_chunks_equal_the_unsplit_ones(env, fmt, hq, hkv, ctx, new, gate):
+    """Few tiles after a long context: the keys are cut into ranges whose states are merged.  Without a workspace there is one
+    range; both meet the bound, with the output epilogue applied to the merged rows."""
+    ffi, kv, synth = env["ffi"], env["kv"], env["synth"]
+    f = getattr(ffi, "KV_FORMAT_" + fmt)
+    tr = ffi.KV_TRANSFORM_RADEMACHER_WHT256 if fmt == "TQ4" else ffi.KV_TRANSFORM_IDENTITY
+    wl = synth.PagedWorkload(ctx, new, hkv, seed=3, fill=0x7F, formats=(f, f, tr, tr))
+    wl.fill_context(env["ex"], 3)
+    n = sum(new)
+    k, v = synth.make_kv(n, hkv, 4, device="cuda")
+    q, g = synth.make_q(n, hq, 4, device="cuda"), synth.make_q(n, hq, 5, device="cuda")
+    vtm = np.ones(n, np.uint8)
+    vtm[1] = 0
+    b = wl.step(valid_token_mask=vtm)
+    kv.kv_cache_write(env["ex"], wl.layer, wl.step(), k, v)
+    outs = []
+    for ex in (env["ex"], kv.Executor(256)):
+        out = torch.full((n, hq, 256), -7.0, dtype=torch.float16, device="cuda")
+        if gate:
+            kv.paged_attention_gated(ex, wl.layer, b, q, g, out, hq, hadamard64=gate == 2)
+        else:
+            kv.paged_attention(ex, wl.layer, b, q, out, hq)
+        torch.cuda.synchronize()
+        assert (out[1] == -7.0).all()
+        outs.append(out.float().cpu().numpy())
+    ok, msg = plain_parity(outs[0], outs[1])
+    assert ok, msg
+    if not gate:
+        want = torch.full((n, hq, 256), -7.0, dtype=torch.float16, device="cuda")
+        kv.paged_attention(env["ex"], wl.layer, b, q, want, hq, scalar=True)
+        torch.cuda.synchronize()
+        ok, msg = plain_parity(outs[0], want.float().cpu().numpy())
+        assert ok, msg

@@ -11,7 +11,7 @@
 // halves, so a code is dequantised once per 256 query rows.
 //
 //   warps 0-3   consumers: thread = query row = TMEM lane: scores from TMEM, online softmax with a lazily moved
-//               reference maximum, P written over its scores as fp16 value (columns 0-31) and residual (32-63)
+//               reference maximum, P written over the scores it came from as fp16 value and residual (16 columns each per 32 keys)
 //   warps 4-7   K producers, warps 8-11 V producers: lane = key, warp = 32 of the stage's 128 channels
 //   warp 12     (CTA 0) issues every MMA; the scores of block j + 1 ahead of the output product of block j
 //   warp 13     bulk-copies the raw (page, head) runs
@@ -48,7 +48,8 @@ constexpr float kPpLutScale = 0.25f * kLutScale;
 constexpr float kPpRescaleThreshold = 8.0f;          // log2 units: the reference maximum may lag by this much
 constexpr float kPpShift = 6.0f;                     // P is carried times 2^6: at most 2^14, subnormal only below 2^-20
 constexpr uint32_t kPpColO = 0, kPpColS = 256, kPpColQ = 384;
-constexpr int kPpOutStride = 257;                    // floats per row of the epilogue staging
+constexpr int kPpOutStride = 260;                    // floats per row of the epilogue staging: 256 columns, l, m
+constexpr int kPpMaxSplits = 24;                     // at most 32: a lane per split in the merge
 
 template <int FMT> struct PpFormat;
 template <> struct PpFormat<WARP34_KV_FORMAT_TQ4> {
@@ -163,7 +164,62 @@ struct PrefillPairParams {
     float q_scale;         // TQ4: sm_scale * log2(e) / kPpLutScale, folded into Q'; 8-bit: sm_scale * log2(e), applied to the scores
     int32_t* status;       // may be null; bit 0: a wait gave up, bit 1: shared-memory window misaligned
     OutputGate og;
+    // A chunk of few tiles after a long context: blockIdx.z takes one of `splits` equal ranges of a tile's key blocks and
+    // leaves [split][token][q head][256] un-normalised rows and [split][token][q head]{m, l}; prefill_merge_kernel finishes.
+    int splits;
+    float* parts;
+    float2* parts_ml;
 };
+
+// Accumulator of one row (columns [8 lane, + 8)) and its mass -> output row.
+template <bool ROT>
+__device__ __forceinline__ void prefill_finish_row(const PrefillPairParams& p, float (&v)[8], float l, size_t row_base, int lane) {
+    const float inv = (l > 0.0f) ? 1.0f / (ROT ? l * (kPpLutScale * 16.0f) : l) : 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] *= inv;
+    if (ROT) {
+        butterfly8<5>(v, lane);
+        sign8(v, lane);
+    }
+    apply_output_gate8(v, p.og, row_base, lane, p.io_bf16);
+    store8(p.attn_out, row_base, lane, p.io_bf16, v);
+}
+
+// Combines the splits of every row that takes part: one warp per (token, q head).
+template <bool ROT>
+__global__ void __launch_bounds__(128) prefill_merge_kernel(const PrefillPairParams p) {
+    grid_dependency_wait();
+    grid_launch_dependents();
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const long long rows = (long long)p.batch.total_tokens * p.num_q_heads, row = (long long)blockIdx.x * 4 + wid;
+    if (row >= rows) return;
+    const int tok = (int)(row / p.num_q_heads);
+    // the same exits as the attention kernel: rows it skipped have no parts
+    if (p.batch.valid_token_mask != nullptr && p.batch.valid_token_mask[tok] == 0) return;
+    const int R = p.batch.num_reqs;
+    if (tok < p.batch.query_start_loc[0] || tok >= p.batch.query_start_loc[R]) return;
+    const int r = last_not_above(p.batch.query_start_loc, R, tok);
+    if (p.batch.valid_req_mask != nullptr && p.batch.valid_req_mask[r] == 0) return;
+    float2 ml = make_float2(-1e30f, 0.0f);
+    if (lane < p.splits) ml = p.parts_ml[(size_t)lane * rows + row];
+    float m_tot = ml.y > 0.0f ? ml.x : -1e30f;
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) m_tot = fmaxf(m_tot, __shfl_xor_sync(0xffffffffu, m_tot, d));
+    const float w = ml.y > 0.0f ? ex2(ml.x - m_tot) : 0.0f;
+    float l_tot = ml.y * w;
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) l_tot += __shfl_xor_sync(0xffffffffu, l_tot, d);
+    float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int s = 0; s < p.splits; ++s) {
+        const float ws = __shfl_sync(0xffffffffu, w, s);
+        const float4* src = reinterpret_cast<const float4*>(p.parts + ((size_t)s * rows + row) * kHeadDim + 8 * lane);
+        const float4 a = src[0], b = src[1];
+        v[0] += ws * a.x; v[1] += ws * a.y; v[2] += ws * a.z; v[3] += ws * a.w;
+        v[4] += ws * b.x; v[5] += ws * b.y; v[6] += ws * b.z; v[7] += ws * b.w;
+    }
+    prefill_finish_row<ROT>(p, v, l_tot, (size_t)row * kHeadDim, lane);
+}
 
 template <int FMT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) attention_prefill_pair_kernel(const PrefillPairParams p) {
@@ -175,38 +231,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
     const uint32_t rank = cluster_rank();
     const uint32_t base = smem_u32(smem_raw);
     uint8_t* gen = smem_raw;
-
-    // ---- which (request, token tile) is this pair?  Both CTAs agree on every exit here. -------------
-    const int tpt = p.tok_per_tile;
-    const int kv_head = blockIdx.y;
-    int req = -1, tile_in_req = 0;
-    {
-        int t = (int)(blockIdx.x >> 1);
-        for (int r = 0; r < p.batch.num_reqs; ++r) {
-            const int ql = p.batch.query_start_loc[r + 1] - p.batch.query_start_loc[r];
-            const int nt = (ql + tpt - 1) / tpt;
-            if (t < nt) { req = r; tile_in_req = nt - 1 - t; break; }    // the tiles with the most keys first
-            t -= nt;
-        }
-    }
-    if (req < 0) return;
-    const ReqGeom g = load_req(p.batch, req);
-    if (!g.valid) return;
-    if ((base & 1023u) != 0u) {      // the swizzled tiles need a 1024-byte-aligned window (the kernel has no static shared memory)
-        if (tid == 0 && p.status != nullptr) atomicOr(p.status, 2);
-        return;
-    }
-    const int tok0 = tile_in_req * tpt;
-    const int ntok = min(tpt, g.q_len - tok0);
-    const int rows_used = ntok * p.gqa;
-    const int row0 = (int)rank * kPpCtaRows;      // first row of this CTA in the tile
-    // keys any row of the pair can see (both limits grow with the token)
-    const int kv_lo = row_min_kv(p.batch, g, tok0);
-    const int kv_hi = row_max_kv(p.batch, g, tok0 + ntok - 1);
-    const bool any_keys = kv_hi >= kv_lo;
-    const int kb_lo = any_keys ? (kv_lo >> 6) : 0;
-    const int nblocks = any_keys ? ((kv_hi >> 6) - kb_lo + 1) : 0;
-    const int pg_lo = any_keys ? (kv_lo >> 4) : 0, pg_hi = any_keys ? (kv_hi >> 4) : -1;
 
     const uint32_t k_t = base + S::kOffK, v_t = base + S::kOffV, qlo_t = base + S::kOffQLo;
     const uint32_t raw = base + S::kOffRaw, lut = base + S::kOffLut, bars = base + S::kOffBars;
@@ -220,6 +244,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
     };
     auto aborted_any = [&]() { return __any_sync(0xffffffffu, *abort_flag != 0u) != 0; };
 
+    if ((base & 1023u) != 0u) {      // the swizzled tiles need a 1024-byte-aligned window (the kernel has no static shared memory)
+        grid_dependency_wait();
+        if (tid == 0 && p.status != nullptr) *p.status = 2;
+        return;
+    }
     // ---- one-time setup -------------------------------------------------------------------------
     if (ROT) {
         for (int i = tid; i < 256 * 16; i += kPpThreads) {
@@ -227,8 +256,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
             const float c0 = kPpLutScale * tq4_centroid(byte & 15), c1 = kPpLutScale * tq4_centroid(byte >> 4);
             const uint32_t hi = pack_half2(c0, c1);
             const float2 hf = __half22float2(*reinterpret_cast<const __half2*>(&hi));
-            sts32(lut + (uint32_t)(byte * 128 + copy * 8), hi);
-            sts32(lut + (uint32_t)(byte * 128 + copy * 8 + 4), pack_half2(c0 - hf.x, c1 - hf.y));
+            asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(lut + (uint32_t)(byte * 128 + copy * 8)), "r"(hi),
+                         "r"(pack_half2(c0 - hf.x, c1 - hf.y)) : "memory");
         }
     }
     if (tid == 0) {
@@ -253,48 +282,129 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
         *abort_flag = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    grid_dependency_wait();          // nothing above touches global memory
+    grid_launch_dependents();
+    if (tid == 0 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0 && p.status != nullptr) *p.status = 0;
+
+    // ---- which (request, token tile) is this pair?  Both CTAs agree on every exit here. -------------
+    const int tpt = p.tok_per_tile;
+    const int kv_head = blockIdx.y;
+    int req = -1, tile_in_req = 0;
+    {
+        int t = (int)(blockIdx.x >> 1);
+        for (int r = 0; r < p.batch.num_reqs; ++r) {
+            const int ql = p.batch.query_start_loc[r + 1] - p.batch.query_start_loc[r];
+            const int nt = (ql + tpt - 1) / tpt;
+            if (t < nt) { req = r; tile_in_req = nt - 1 - t; break; }    // the tiles with the most keys first
+            t -= nt;
+        }
+    }
+    if (req < 0) return;
+    const ReqGeom g = load_req(p.batch, req);
+    if (!g.valid) return;
+    const int tok0 = tile_in_req * tpt;
+    const int ntok = min(tpt, g.q_len - tok0);
+    const int rows_used = ntok * p.gqa;
+    const int row0 = (int)rank * kPpCtaRows;      // first row of this CTA in the tile
+    // keys any row of the pair can see (both limits grow with the token)
+    const int kv_lo = row_min_kv(p.batch, g, tok0);
+    const int kv_hi = row_max_kv(p.batch, g, tok0 + ntok - 1);
+    const bool any_keys = kv_hi >= kv_lo;
+    const int all_lo = any_keys ? (kv_lo >> 6) : 0, all = any_keys ? ((kv_hi >> 6) - all_lo + 1) : 0;
+    const int kb_lo = all_lo + (int)((long long)all * blockIdx.z / p.splits);     // this split's key blocks
+    const int nblocks = all_lo + (int)((long long)all * (blockIdx.z + 1) / p.splits) - kb_lo;
+    const int pg_lo = any_keys ? (kv_lo >> 4) : 0, pg_hi = any_keys ? (kv_hi >> 4) : -1;
+
     __syncwarp();
     if (wid == 0) {
         tc2_alloc(base + S::kOffBars + 240, 512);
         tc2_relinquish();
     }
+    __syncthreads();                 // this CTA's barriers exist
+
+    // ---- raw (page, head) runs of a block; the first blocks are on their way before the query is prepared ----------
+    const int32_t* blocks = p.batch.block_tables + (size_t)req * p.batch.max_blocks_per_req;
+    const uint8_t* k_head_base = (const uint8_t*)(uintptr_t)p.layout.k_base + (size_t)kv_head * p.layout.k_head_stride_bytes;
+    const uint8_t* v_head_base = (const uint8_t*)(uintptr_t)p.layout.v_base + (size_t)kv_head * p.layout.v_head_stride_bytes;
+    auto page_id = [&](int j) -> int32_t {      // lane pp < 4: page pp of block j, -1 outside the visible range
+        const int pg = 4 * (kb_lo + j) + (lane & 3);
+        return (j < nblocks && pg >= pg_lo && pg <= pg_hi)
+                   ? block_table_page(blocks, pg, p.batch.max_blocks_per_req, ROT ? kInPrefillExact : kInKv8) : -1;
+    };
+    auto copy_k = [&](int j, int32_t id) {      // this CTA's two pages
+        const int s = j % kPpRawStages;
+        const uint32_t mask = (__ballot_sync(0xffffffffu, id >= 0) >> (2 * rank)) & 3u;
+        if (lane == 0) mbar_expect_tx(bar(kPpRawKFull + s), (uint32_t)__popc(mask) * S::kRun);
+        __syncwarp();
+        if (lane < 4 && (lane >> 1) == (int)rank && id >= 0) {
+            bulk_g2s(raw + (uint32_t)s * S::kRaw + (uint32_t)(lane & 1) * S::kRun, k_head_base + (size_t)id * p.layout.k_page_stride_bytes,
+                     S::kRun, bar(kPpRawKFull + s));
+        }
+    };
+    auto copy_v = [&](int j, int32_t id) {      // all four
+        const int s = j % kPpRawStages;
+        const uint32_t mask = __ballot_sync(0xffffffffu, id >= 0) & 15u;
+        if (lane == 0) mbar_expect_tx(bar(kPpRawVFull + s), (uint32_t)__popc(mask) * S::kRun);
+        __syncwarp();
+        if (lane < 4 && id >= 0) {
+            bulk_g2s(raw + (uint32_t)s * S::kRaw + S::kRawK + (uint32_t)lane * S::kRun, v_head_base + (size_t)id * p.layout.v_page_stride_bytes,
+                     S::kRun, bar(kPpRawVFull + s));
+        }
+    };
+    int32_t next_id = -1;
+    if (wid == 13) {
+        for (int j = 0; j < kPpRawStages && j < nblocks; ++j) {
+            const int32_t id = page_id(j);
+            copy_k(j, id);
+            copy_v(j, id);
+        }
+        next_id = page_id(kPpRawStages);
+    }
 
     // ---- Q rows of this CTA: one warp per row.  TQ4: rotated, scaled, split into value (staging) and
     //      residual (swizzled A tile); 8-bit: the fp16 row as it is ------------------------------------
     const uint32_t q_stage = k_t;     // 128 rows x 512 B over the tile stages
-    for (int row = wid; row < kPpCtaRows; row += kPpWarps) {
+    auto load_row = [&](int row, float (&v)[8]) {
         const int trow = row0 + row;
         const int q_off = tok0 + trow / p.gqa;
         const int q_head = kv_head * p.gqa + trow % p.gqa;
-        const bool ok = trow < rows_used &&
+        const bool ok = row < kPpCtaRows && trow < rows_used &&
                         (p.batch.valid_token_mask == nullptr || p.batch.valid_token_mask[g.q_start + q_off] != 0);
-        float tv[8];
-        const size_t q_base = ((size_t)(g.q_start + q_off) * p.num_q_heads + q_head) * kHeadDim;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) tv[j] = ok ? load_act(p.q_in, q_base + lane + 32 * j, p.io_bf16) : 0.0f;
+        for (int i = 0; i < 8; ++i) v[i] = 0.0f;
+        if (ok) load8(p.q_in, ((size_t)(g.q_start + q_off) * p.num_q_heads + q_head) * kHeadDim, lane, p.io_bf16, v);
+    };
+    float ahead[8];
+    load_row(wid, ahead);
+    for (int row = wid; row < kPpCtaRows; row += kPpWarps) {
+        float v[8];      // columns [8 lane, + 8)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = ahead[i];
+        load_row(row + kPpWarps, ahead);
         if (ROT) {
+            sign8(v, lane);
+            butterfly8<5>(v, lane);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) tv[j] = apply_sign(tv[j], lane + 32 * j);
-            wht256_lanes(tv, lane);
+            for (int i = 0; i < 8; ++i) v[i] *= p.q_scale * 0.0625f;
         }
+        uint32_t hi[4], lo[4];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int c = lane + 32 * j;
-            const float f = ROT ? tv[j] * p.q_scale : tv[j];
-            const __half h = __float2half_rn(f);
-            // staging row = 512 B; its 16-byte chunks are XOR-swizzled by the row (the reads below are thread-per-row)
-            sts16(q_stage + (uint32_t)row * 512u + (uint32_t)((((c >> 3) ^ (row & 31)) << 4) + ((c & 7) << 1)),
-                  (uint32_t)__half_as_ushort(h));
-            if (ROT) {
-                const uint32_t addr = qlo_t + (uint32_t)(c >> 6) * (kPpCtaRows * 128u) + (uint32_t)row * 128u +
-                                      (uint32_t)(((((c & 63) >> 3) ^ (row & 7)) << 4) + ((c & 7) << 1));
-                sts16(addr, (uint32_t)__half_as_ushort(__float2half_rn(f - __half2float(h))));
-            }
+        for (int i = 0; i < 4; ++i) {
+            const __half2 h = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+            const float2 hf = __half22float2(h);
+            hi[i] = *reinterpret_cast<const uint32_t*>(&h);
+            lo[i] = pack_half2(v[2 * i] - hf.x, v[2 * i + 1] - hf.y);
+        }
+        // staging row = 512 B; its 16-byte chunks are XOR-swizzled by the row (the reads below are thread-per-row)
+        sts128(q_stage + (uint32_t)row * 512u + (uint32_t)((lane ^ (row & 31)) << 4), hi[0], hi[1], hi[2], hi[3]);
+        if (ROT) {
+            sts128(qlo_t + (uint32_t)(lane >> 3) * (kPpCtaRows * 128u) + (uint32_t)row * 128u + (uint32_t)(((lane & 7) ^ (row & 7)) << 4),
+                   lo[0], lo[1], lo[2], lo[3]);
         }
     }
     if (ROT) fence_proxy_async();     // the residual tile is read by the tensor core
     tc_fence_before();
-    cluster_sync_all();               // barriers of both CTAs exist, TMEM of both is allocated, staging is written
+    __syncthreads();                  // staging is written
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     if (wid < 4) {
@@ -314,11 +424,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
         tc_wait_st();
     }
     tc_fence_before();
-    cluster_sync_all();               // Q' of both CTAs is in place, the staging area becomes the tile stages
+    cluster_sync_all();               // both CTAs: barriers, TMEM and Q' are in place, the staging area becomes the tile stages
     tc_fence_after();
 
-    const int32_t* blocks = p.batch.block_tables + (size_t)req * p.batch.max_blocks_per_req;
-    float l_run = 0.0f;
+    float l_run = 0.0f, m_ref = -1e30f;     // consumers: of this thread's row
 
     if (wid == 12) {
         // ======================= MMA issue: lane 0 of CTA 0 feeds both tensor cores ====================
@@ -371,9 +480,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
 #pragma unroll
                         for (int ks = 0; ks < 2; ++ks) {
                             const uint64_t b = b0 + (uint64_t)((2048 / 16) * ks);
-                            const uint32_t a = a0 + 8u * (uint32_t)(2 * h + ks);
+                            const uint32_t a = a0 + 32u * (uint32_t)h + 8u * (uint32_t)ks;
                             tc2_mma_f16_ts(tmem + kPpColO, a, b, kIdescPv, (i > 0 || h > 0 || ks > 0) ? 1u : 0u);
-                            tc2_mma_f16_ts(tmem + kPpColO, a + 32u, b, kIdescPv, 1u);
+                            tc2_mma_f16_ts(tmem + kPpColO, a + 16u, b, kIdescPv, 1u);
                             tc2_mma_f16_ts(tmem + kPpColO, a, b + kPpPart / 16, kIdescPv, 1u);
                         }
                         tc2_commit_both(bar(kPpEmptyV + (int)vst));
@@ -390,37 +499,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
         if (!wait_all(bar(kPpDrain), 0u)) *abort_flag = 1u;
     } else if (wid == 13) {
         // ======================= copy issue: raw (page, head) runs of a block ===========================
-        const uint8_t* k_head_base = (const uint8_t*)(uintptr_t)p.layout.k_base + (size_t)kv_head * p.layout.k_head_stride_bytes;
-        const uint8_t* v_head_base = (const uint8_t*)(uintptr_t)p.layout.v_base + (size_t)kv_head * p.layout.v_head_stride_bytes;
-        auto page_id = [&](int j) -> int32_t {      // lane pp < 4: page pp of block j, -1 outside the visible range
-            const int pg = 4 * (kb_lo + j) + (lane & 3);
-            return (j < nblocks && pg >= pg_lo && pg <= pg_hi) ? block_table_page(blocks, pg, p.batch.max_blocks_per_req, ROT ? kInPrefillExact : kInKv8) : -1;
-        };
-        int32_t id = page_id(0);
-        int issued = 0;
+        int issued = 2 * min(nblocks, kPpRawStages);
 #pragma unroll 1
-        for (int j = 0; j < nblocks; ++j) {
+        for (int j = kPpRawStages; j < nblocks; ++j) {
             if (aborted_any()) break;
             const int s = j % kPpRawStages;
-            const int32_t next_id = page_id(j + 1);
-            const uint32_t mask = __ballot_sync(0xffffffffu, id >= 0) & 15u;
-            const uint32_t kmask = (mask >> (2 * rank)) & 3u;
-            if (j >= kPpRawStages && !wait_all(bar(kPpRawKFree + s), (uint32_t)((j / kPpRawStages - 1) & 1))) { *abort_flag = 1u; break; }
-            const uint32_t rk = raw + (uint32_t)s * S::kRaw, rv = rk + S::kRawK;
-            if (lane == 0) mbar_expect_tx(bar(kPpRawKFull + s), (uint32_t)__popc(kmask) * S::kRun);
-            __syncwarp();
-            if (lane < 4 && (lane >> 1) == (int)rank && id >= 0) {
-                bulk_g2s(rk + (uint32_t)(lane & 1) * S::kRun, k_head_base + (size_t)id * p.layout.k_page_stride_bytes, S::kRun, bar(kPpRawKFull + s));
-            }
+            const int32_t id = next_id;
+            next_id = page_id(j + 1);
+            if (!wait_all(bar(kPpRawKFree + s), (uint32_t)((j / kPpRawStages - 1) & 1))) { *abort_flag = 1u; break; }
+            copy_k(j, id);
             issued = 2 * j + 1;
-            if (j >= kPpRawStages && !wait_all(bar(kPpRawVFree + s), (uint32_t)((j / kPpRawStages - 1) & 1))) { *abort_flag = 1u; break; }
-            if (lane == 0) mbar_expect_tx(bar(kPpRawVFull + s), (uint32_t)__popc(mask) * S::kRun);
-            __syncwarp();
-            if (lane < 4 && id >= 0) {
-                bulk_g2s(rv + (uint32_t)lane * S::kRun, v_head_base + (size_t)id * p.layout.v_page_stride_bytes, S::kRun, bar(kPpRawVFull + s));
-            }
+            if (!wait_all(bar(kPpRawVFree + s), (uint32_t)((j / kPpRawStages - 1) & 1))) { *abort_flag = 1u; break; }
+            copy_v(j, id);
             issued = 2 * j + 2;
-            id = next_id;
         }
         // copies in flight must land before the CTA leaves
         const int kn = (issued + 1) / 2, vn = issued / 2;
@@ -544,7 +635,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
         const uint32_t lane_base = (uint32_t)(32 * wid) << 16;
         const uint32_t t_o = tmem + lane_base + kPpColO, t_s = tmem + lane_base + kPpColS;
         const uint32_t leader_pready = map_to_rank(bar(kPpPReady), 0u);
-        float m_ref = -1e30f;
 #pragma unroll 1
         for (int j = 0; j < nblocks; ++j) {
             if (aborted_any()) break;
@@ -553,30 +643,33 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
             // PV(j - 2) precedes QK(j) in the pipe; waiting for every phase of kPpPv keeps its parity unambiguous
             if (j >= 2 && !wait_all(bar(kPpPv), (uint32_t)(j & 1))) { *abort_flag = 1u; break; }
             const uint32_t t_sj = t_s + 64u * (uint32_t)(j & 1);
-            float sv[64];
-            {
-                uint32_t r0[32], r1[32];
-                tc_ld32(r0, t_sj);
-                tc_ld32(r1, t_sj + 32u);
+            const int kbase = (kb_lo + j) << 6;
+            const bool all_seen = kbase >= rmin && kbase + 63 <= rmax;
+            // Scores of keys [32 c, + 32) of the block, scaled and masked.
+            auto scores = [&](int c, float (&sv)[32]) {
+                uint32_t r[32];
+                tc_ld32(r, t_sj + 32u * (uint32_t)c);
                 tc_wait_ld();
 #pragma unroll
-                for (int i = 0; i < 32; ++i) { sv[i] = __uint_as_float(r0[i]); sv[32 + i] = __uint_as_float(r1[i]); }
-            }
-            if (!ROT) {
+                for (int i = 0; i < 32; ++i) sv[i] = ROT ? __uint_as_float(r[i]) : __uint_as_float(r[i]) * p.q_scale;
+                if (!all_seen) {
 #pragma unroll
-                for (int i = 0; i < 64; ++i) sv[i] *= p.q_scale;
-            }
-            const int kbase = (kb_lo + j) << 6;
-            if (!(kbase >= rmin && kbase + 63 <= rmax)) {
-#pragma unroll
-                for (int i = 0; i < 64; ++i) {
-                    const int pos = kbase + i;
-                    if (!(pos >= rmin && pos <= rmax)) sv[i] = -1e30f;
+                    for (int i = 0; i < 32; ++i) {
+                        const int pos = kbase + 32 * c + i;
+                        if (!(pos >= rmin && pos <= rmax)) sv[i] = -1e30f;
+                    }
                 }
-            }
-            float mx4[4] = {sv[0], sv[1], sv[2], sv[3]};     // four independent chains
+            };
+            // TQ4 reads them twice (maximum, then weights): holding all 64 spills there (92 bytes a thread, five ragged
+            // prompts 270 us instead of 245), while the 8-bit builds have room and the second read costs them 10 %.
+            float sv[2][32];
+            float mx4[4] = {-1e30f, -1e30f, -1e30f, -1e30f};     // four independent chains
 #pragma unroll
-            for (int i = 4; i < 64; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], sv[i]);
+            for (int c = 0; c < 2; ++c) {
+                scores(c, sv[ROT ? 0 : c]);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], sv[ROT ? 0 : c][i]);
+            }
             const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
             // the reference maximum moves only when the true maximum ran ahead by more than the threshold
             const bool need = mx > m_ref + kPpRescaleThreshold;
@@ -604,18 +697,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
                 uint32_t hi[16], lo[16];
+                if (ROT) scores(c, sv[0]);
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
                     // masked scores are -1e30: ex2 gives exactly 0 against any finite reference
-                    const float pa = ex2(sv[32 * c + 2 * i] - m_use), pb = ex2(sv[32 * c + 2 * i + 1] - m_use);
+                    const float pa = ex2(sv[ROT ? 0 : c][2 * i] - m_use), pb = ex2(sv[ROT ? 0 : c][2 * i + 1] - m_use);
                     ls4[i & 3] += pa + pb;
                     const __half2 h = __floats2half2_rn(pa, pb);
                     const float2 hf = __half22float2(h);
                     hi[i] = *reinterpret_cast<const uint32_t*>(&h);
                     lo[i] = pack_half2(pa - hf.x, pb - hf.y);
                 }
-                tc_st16(t_sj + 16u * c, hi);
-                tc_st16(t_sj + 32u + 16u * c, lo);
+                // P takes the place of the scores it came from: value in columns 32 c .. + 15, residual in the next 16
+                tc_st16(t_sj + 32u * c, hi);
+                tc_st16(t_sj + 32u * c + 16u, lo);
             }
             tc_wait_st();
             l_run = l_run * alpha + ((ls4[0] + ls4[1]) + (ls4[2] + ls4[3]));
@@ -636,18 +731,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
     __syncthreads();
     const bool aborted = *abort_flag != 0u;
     float* stage = reinterpret_cast<float*>(gen);
-    if (wid < 4 && nblocks > 0 && !aborted) {
-        const uint32_t t_o = tmem + ((uint32_t)(32 * wid) << 16) + kPpColO;
-        const float inv = (l_run > 0.0f) ? (1.0f / (ROT ? l_run * kPpLutScale : l_run)) : 0.0f;
+    if (wid < 4 && !aborted) {
+        float* mine = stage + tid * kPpOutStride;
+        if (nblocks > 0) {
+            const uint32_t t_o = tmem + ((uint32_t)(32 * wid) << 16) + kPpColO;
 #pragma unroll 1
-        for (int c = 0; c < 8; ++c) {
-            uint32_t o[32];
-            tc_ld32(o, t_o + 32u * c);
-            tc_wait_ld();
+            for (int c = 0; c < 8; ++c) {
+                uint32_t o[32];
+                tc_ld32(o, t_o + 32u * c);
+                tc_wait_ld();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) stage[tid * kPpOutStride + 32 * c + i] = __uint_as_float(o[i]) * inv;
+                for (int i = 0; i < 8; ++i) {
+                    *reinterpret_cast<uint4*>(mine + 32 * c + 4 * i) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+                }
+            }
         }
-        stage[tid * kPpOutStride + 256] = l_run;
+        mine[256] = l_run;
+        mine[257] = m_ref;
     }
     tc_fence_before();
     __syncthreads();
@@ -658,19 +758,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
             const int q_off = tok0 + trow / p.gqa;
             const int q_head = kv_head * p.gqa + trow % p.gqa;
             if (p.batch.valid_token_mask != nullptr && p.batch.valid_token_mask[g.q_start + q_off] == 0) continue;
-            float tv[8];
-            const bool has = nblocks > 0 && stage[row * kPpOutStride + 256] > 0.0f;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) tv[j] = has ? stage[row * kPpOutStride + lane + 32 * j] : 0.0f;
-            const size_t out_base = ((size_t)(g.q_start + q_off) * p.num_q_heads + q_head) * kHeadDim;
-            if (ROT) {
-                wht256_lanes(tv, lane);
-                store_output_row(p.attn_out, out_base, tv, lane, p.io_bf16, p.og);
-            } else {
-                apply_output_gate(tv, p.og, out_base, lane, p.io_bf16);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) store_act(p.attn_out, out_base + lane + 32 * j, tv[j], p.io_bf16);
+            const float* src = stage + row * kPpOutStride;
+            const float l = src[256];
+            float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            if (l > 0.0f) {
+                const float4 a = *reinterpret_cast<const float4*>(src + 8 * lane), b = *reinterpret_cast<const float4*>(src + 8 * lane + 4);
+                v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
             }
+            const size_t out_row = (size_t)(g.q_start + q_off) * p.num_q_heads + q_head;
+            if (p.splits > 1) {
+                const size_t part_row = (size_t)blockIdx.z * p.batch.total_tokens * p.num_q_heads + out_row;
+                float4* dst = reinterpret_cast<float4*>(p.parts + part_row * kHeadDim + 8 * lane);
+                dst[0] = make_float4(v[0], v[1], v[2], v[3]);
+                dst[1] = make_float4(v[4], v[5], v[6], v[7]);
+                if (lane == 0) p.parts_ml[part_row] = make_float2(src[257], l);
+                continue;
+            }
+            prefill_finish_row<ROT>(p, v, l, out_row * kHeadDim, lane);
         }
     } else if (tid == 0 && p.status != nullptr) {
         atomicOr(p.status, 1);
@@ -686,10 +790,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
 }  // namespace w34
 
 namespace w34 {
-// The pair kernel for one layer's chunk: no workspace beyond the status word.
+// The pair kernel for one layer's chunk.  Workspace: a status word, and room for the parts when it splits.
 template <int FMT>
 static int launch_prefill_pair(const warp34_exec* ex, const warp34_kv_layer_layout* layout, const warp34_attention_batch* batch,
-                               const void* q_in, void* attn_out, int num_q_heads, int io_bf16, int32_t* status, const OutputGate& og) {
+                               const void* q_in, void* attn_out, int num_q_heads, int io_bf16, const OutputGate& og, int sm_count) {
+    int32_t* status = nullptr;      // the first word of the workspace, when there is one
+    if (ex->scratch_ptr != 0 && (ex->scratch_ptr & 3u) == 0 && ex->scratch_size >= sizeof(PlanHeader)) {
+        status = reinterpret_cast<int32_t*>((uintptr_t)ex->scratch_ptr);   // PlanHeader::status
+    }
     if (layout->local_kv_heads > 65535) return (int)cudaErrorInvalidValue;
     PrefillPairParams pp;
     pp.layout = *layout;
@@ -706,8 +814,40 @@ static int launch_prefill_pair(const warp34_exec* ex, const warp34_kv_layer_layo
     pp.og = og;
     const long long tiles = (long long)batch->total_tokens / pp.tok_per_tile + batch->num_reqs;
     if (tiles > 0x3fffffffll) return (int)cudaErrorInvalidValue;
-    const dim3 grid(2u * (unsigned)tiles, (unsigned)layout->local_kv_heads);
-    attention_prefill_pair_kernel<FMT><<<grid, kPpThreads, PpSmem<FMT>::kBytes, (cudaStream_t)ex->stream>>>(pp);
-    return (int)cudaGetLastError();
+    // Key ranges per tile, by an estimate in units of one 64-key block (about 1.8 us).  A CTA pair costs its blocks and about 7
+    // more for its start, query and output; pairs run in waves of sm_count / 2; a split adds a merge launch (3) and its rows,
+    // written and read (1e-4 each).  Measured on chunks of 16 to 2048 tokens after 0 to 30 000: within 10 % of the best split.
+    // A split needs workspace for its rows.
+    const long long rows = (long long)batch->total_tokens * num_q_heads;
+    const long long blocks = batch->max_seq_len > 0 ? (batch->max_seq_len + kPpKeys - 1) / kPpKeys : 0;
+    const long long by_longest = (long long)batch->num_reqs * ((batch->max_q_len + pp.tok_per_tile - 1) / pp.tok_per_tile);
+    const long long pairs = (by_longest > 0 && by_longest < tiles ? by_longest : tiles) * layout->local_kv_heads, at_once = sm_count / 2 > 0 ? sm_count / 2 : 1;
+    pp.splits = 1;
+    pp.parts = nullptr;
+    pp.parts_ml = nullptr;
+    if (ex->scratch_ptr != 0 && (ex->scratch_ptr & 15u) == 0 && ex->scratch_size > 256 && rows > 0) {
+        long long fit = (long long)((ex->scratch_size - 256) / ((size_t)rows * (kHeadDim + 2) * sizeof(float)));
+        if (fit > kPpMaxSplits) fit = kPpMaxSplits;
+        const float mean = (float)blocks - 0.5f * (float)batch->max_q_len / kPpKeys;      // a causal chunk's tiles differ
+        float best = 0.0f;
+        for (int n = 1; n <= fit && n <= blocks; ++n) {
+            const float waves = (float)((pairs * n + at_once - 1) / at_once);
+            float cost = waves * (mean / (float)n + 7.0f);
+            if (cost < (float)blocks / (float)n + 7.0f) cost = (float)blocks / (float)n + 7.0f;
+            if (n > 1) cost += 3.0f + 1e-4f * (float)n * (float)rows;
+            if (n == 1 || cost < best) { best = cost; pp.splits = n; }
+        }
+        if (pp.splits > 1) {
+            pp.parts = reinterpret_cast<float*>((uintptr_t)ex->scratch_ptr + 256);
+            pp.parts_ml = reinterpret_cast<float2*>(pp.parts + (size_t)pp.splits * rows * kHeadDim);
+        }
+    }
+    cudaStream_t st = (cudaStream_t)ex->stream;
+    const dim3 grid(2u * (unsigned)tiles, (unsigned)layout->local_kv_heads, (unsigned)pp.splits);
+    int rc = launch_behind(attention_prefill_pair_kernel<FMT>, grid, kPpThreads, PpSmem<FMT>::kBytes, st, pp);
+    if (rc == 0 && pp.splits > 1) {
+        rc = launch_behind(prefill_merge_kernel<PpFormat<FMT>::kRotated>, dim3((unsigned)((rows + 3) / 4)), 128, 0, st, pp);
+    }
+    return rc;
 }
 }  // namespace w34

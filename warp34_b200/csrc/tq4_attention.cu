@@ -372,6 +372,23 @@ __device__ __forceinline__ void sign8(float (&v)[8], int lane) {
     for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(__float_as_uint(v[i]) ^ ((bits >> i) << 31));
 }
 
+// The epilogue of apply_output_gate() on a row held that way.
+__device__ __forceinline__ void apply_output_gate8(float (&v)[8], const OutputGate& og, size_t row_base, int lane, int io_bf16) {
+    if (og.mode == 0) return;
+    if (og.gate != nullptr) {
+        float g[8];
+        load8(og.gate, row_base, lane, io_bf16, g);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = ((og.mode & 4) ? v[i] : round_act(v[i], io_bf16)) * sigmoid_gate(g[i]);
+    }
+    if ((og.mode & 3) != 2) return;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = round_act(v[i], io_bf16);
+    butterfly8<3>(v, lane);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] *= 0.125f;
+}
+
 // ---------------------------------------------------------------------------------------
 // Scalar dequant-then-attend: one block of four warps per (token, q head), fp32, any strides.
 // ---------------------------------------------------------------------------------------
@@ -597,9 +614,9 @@ __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepco
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
 
 template <class Params>
-static int launch_behind(void (*kernel)(const Params), unsigned grid, unsigned threads, size_t smem, cudaStream_t st, const Params& p) {
+static int launch_behind(void (*kernel)(const Params), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, const Params& p) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -2438,13 +2455,6 @@ static bool takes_kv8_chunk_path(uint64_t flags, const warp34_kv_layer_layout* l
     return gqa <= kPpCtaRows && (long long)b->max_q_len * gqa > 24;
 }
 
-// The chunk kernels report through the first word of the workspace, when there is one.
-static int chunk_status_word(const warp34_exec* ex, int32_t** status) {
-    if (ex->scratch_ptr == 0 || (ex->scratch_ptr & 3u) != 0 || ex->scratch_size < sizeof(PlanHeader)) return 0;
-    *status = reinterpret_cast<int32_t*>((uintptr_t)ex->scratch_ptr);   // PlanHeader::status
-    return (int)cudaMemsetAsync(*status, 0, sizeof(int32_t), (cudaStream_t)ex->stream);
-}
-
 // Shared body of the attention entry points.  triple_out != nullptr: stop after the split-KV
 // merge and write per-row (acc, m, l) instead of attn_out (streaming path only).
 // force: -1 = dispatch by batch geometry and flags; otherwise the kernel family the reference's
@@ -2467,13 +2477,11 @@ static int launch_attention(const warp34_exec* ex, const warp34_kv_layer_layout*
         if (triple_out != nullptr) return (int)cudaErrorNotSupported;
         if (force <= 0 && takes_kv8_chunk_path(ex->flags, layout, batch, num_q_heads)) {
             int rc = 0;
-            if (device_info(&rc) == nullptr) return rc;
-            int32_t* status = nullptr;
-            rc = chunk_status_word(ex, &status);
-            if (rc != 0) return rc;
+            const DeviceInfo* dev = device_info(&rc);
+            if (dev == nullptr) return rc;
             return layout->k_format == WARP34_KV_FORMAT_FP8_E4M3
-                       ? launch_prefill_pair<WARP34_KV_FORMAT_FP8_E4M3>(ex, layout, batch, q_in, attn_out, num_q_heads, io_bf16, status, og)
-                       : launch_prefill_pair<WARP34_KV_FORMAT_Q8_0>(ex, layout, batch, q_in, attn_out, num_q_heads, io_bf16, status, og);
+                       ? launch_prefill_pair<WARP34_KV_FORMAT_FP8_E4M3>(ex, layout, batch, q_in, attn_out, num_q_heads, io_bf16, og, dev->sm_count)
+                       : launch_prefill_pair<WARP34_KV_FORMAT_Q8_0>(ex, layout, batch, q_in, attn_out, num_q_heads, io_bf16, og, dev->sm_count);
         }
         const int rc8 = launch_kv8_attention(ex, layout, batch, q_in, attn_out, num_q_heads, io_bf16,
                                              (ex->flags & WARP34_B200_EXEC_FLAG_PRECISE_ATTENTION) == 0 && force <= 0);
@@ -2495,14 +2503,17 @@ static int launch_attention(const warp34_exec* ex, const warp34_kv_layer_layout*
     const bool chunk_geometry_ok = stream_layout_ok(layout) && batch->max_blocks_per_req > 0 && gqa <= kPpCtaRows;
     if (force >= 1 && (!chunk_geometry_ok || triple_out != nullptr)) return (int)cudaErrorNotSupported;
     if (force >= 1 || (force < 0 && triple_out == nullptr && takes_prefill_path(ex->flags, layout, batch, gqa))) {
-        int32_t* status = nullptr;
-        rc = chunk_status_word(ex, &status);
-        if (rc != 0) return rc;
         const bool tc = force == 2 || (force < 0 && (ex->flags & (WARP34_B200_EXEC_FLAG_FAST_ATTENTION |
                                                                   WARP34_B200_EXEC_FLAG_TCGEN05_VERIFY)) != 0);
         if (tc) {
             if (layout->local_kv_heads > 65535) return (int)cudaErrorInvalidValue;
             if ((size_t)dev->smem_optin < kTcSmemBytes) return (int)cudaErrorNotSupported;
+            int32_t* status = nullptr;
+            if (ex->scratch_ptr != 0 && (ex->scratch_ptr & 3u) == 0 && ex->scratch_size >= sizeof(PlanHeader)) {
+                status = reinterpret_cast<int32_t*>((uintptr_t)ex->scratch_ptr);   // PlanHeader::status
+                rc = (int)cudaMemsetAsync(status, 0, sizeof(int32_t), (cudaStream_t)ex->stream);
+                if (rc != 0) return rc;
+            }
             PrefillTcParams tp;
             tp.layout = *layout;
             tp.batch = *batch;
@@ -2521,7 +2532,7 @@ static int launch_attention(const warp34_exec* ex, const warp34_kv_layer_layout*
             tq4_attention_prefill_tc_kernel<<<grid, kTcThreads, kTcSmemBytes, (cudaStream_t)ex->stream>>>(tp);
             return (int)cudaGetLastError();
         }
-        return launch_prefill_pair<WARP34_KV_FORMAT_TQ4>(ex, layout, batch, q_in, attn_out, num_q_heads, io_bf16, status, og);
+        return launch_prefill_pair<WARP34_KV_FORMAT_TQ4>(ex, layout, batch, q_in, attn_out, num_q_heads, io_bf16, og, dev->sm_count);
     }
 
     // Streaming path: canonical layout, scratch that holds the plan plus at least one partial
