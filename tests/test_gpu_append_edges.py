@@ -1,0 +1,51 @@
+"""TQ4 append at the edges of its layout (rows off 16-byte boundaries, rows whose destination is 2-byte aligned, one to nine
+heads, fewer rows than a warp takes, NaN, infinity, zeros, values at the fp16 limits) against the CPU oracle: the same codes,
+scales within the oracle's one unit in the last place."""
+import numpy as np
+import pytest
+
+from util import host_layout, tq4_rows_equal_up_to_scale_ulp
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("hkv,n,shift", [(1, 1, 0), (1, 3, 2), (3, 5, 8), (4, 33, 1), (9, 7, 4)])
+def test_rows_of_any_alignment_and_value(native_libs, hkv, n, shift):
+    import oracle
+    from warp34_b200 import kv, synth
+    wl = synth.PagedWorkload([0], [n], hkv, seed=3, fill=0x3C)
+    b = wl.step()
+    k, v = synth.make_kv(n, hkv, 4)
+    k[0, :7] = torch.tensor([65504.0, -65504.0, 6e-8, -0.0, 0.0, 1.0, -1.0], dtype=torch.float16)
+    v[n - 1] = 0
+    stride = hkv * 256 + 16
+    kd = torch.zeros(n, stride, dtype=torch.float16, device="cuda")
+    vd = torch.zeros(n, stride, dtype=torch.float16, device="cuda")
+    kd[:, shift:shift + hkv * 256], vd[:, shift:shift + hkv * 256] = k.cuda(), v.cuda()
+    kv.kv_cache_write(kv.Executor(1 << 16), wl.layer, b, kd[:, shift:], vd[:, shift:])
+    torch.cuda.synchronize()
+    hk, hv = np.full(wl.layer.k.numel(), 0x3C, np.uint8), np.full(wl.layer.v.numel(), 0x3C, np.uint8)
+    oracle.kv_cache_write(host_layout(wl.layer.layout, hk, hv), b.host_desc(), k.numpy().view(np.uint16), v.numpy().view(np.uint16),
+                          hkv * 256, hkv * 256, nthreads=2)
+    for got, want in ((wl.layer.k, hk), (wl.layer.v, hv)):
+        codes, scales, ulp = tq4_rows_equal_up_to_scale_ulp(got.cpu().numpy(), want)
+        assert codes == 0 and ulp <= 1, (codes, scales, ulp)
+
+
+def test_two_byte_aligned_destinations_and_non_finite_rows(native_libs):
+    """The 16-bit store path writes what the 32-bit one does; a row with NaN or infinity leaves its neighbours alone."""
+    from warp34_b200 import kv, synth
+    n, hkv = 20, 2
+    k, v = synth.make_kv(n, hkv, 9, device="cuda")
+    k[3, 5], v[7, 300] = float("nan"), float("inf")
+    pools = []
+    for off in (0, 2):
+        wl = synth.PagedWorkload([0], [n], hkv, seed=3, fill=0x3C)
+        base = torch.full((wl.layer.k.numel() + 16,), 0x3C, dtype=torch.uint8, device="cuda")
+        wl.layer.layout.k_base = base.data_ptr() + off
+        kv.kv_cache_write(kv.Executor(1 << 16), wl.layer, wl.step(), k, v)
+        torch.cuda.synchronize()
+        pools.append((base[off:off + wl.layer.k.numel()].cpu(), wl.layer.v.cpu()))
+    assert torch.equal(pools[0][0], pools[1][0]) and torch.equal(pools[0][1], pools[1][1])
+    assert (pools[0][0] != 0x3C).any()

@@ -130,6 +130,8 @@ __device__ __forceinline__ void kv8_encode_row_by_element(const __half* src_row,
 // strides), so the kernel holds the 128-bit path alone.
 template <bool ALIGNED>
 __global__ void __launch_bounds__(128) kv8_append_kernel(const AppendParams p) {
+    grid_dependency_wait();
+    grid_launch_dependents();
     const int lane = threadIdx.x & 31;
     const int heads = p.layout.local_kv_heads;
     const long long th_ll = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);

@@ -605,29 +605,6 @@ __host__ __device__ inline size_t qfrag_item_bytes() { return (size_t)kQFragWord
 __device__ void qprep_block(const StreamParams& p, int idx);
 constexpr int kPlanThreads = 32 * kRowsPerGroup;  // the query-fragment blocks use one warp per query row
 
-// ---- dependent launches ---------------------------------------------------------------------------
-// The kernels of one attention call are launched behind each other with programmatic stream serialization: a kernel may
-// begin while the last blocks of the one before it finish, which hides the launch latency (about 2 us each on a stream).
-// Every kernel therefore waits for its predecessor's end before it touches global memory, and lets its successor start
-// being scheduled once its own blocks run.
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
-
-template <class Params>
-static int launch_behind(void (*kernel)(const Params), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, const Params& p) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return (int)cudaLaunchKernelEx(&cfg, kernel, p);
-}
-
 // Block 0 plans the split.  Blocks 1.. (one-warp items only) each rotate and scale the query rows
 // of one (request, kv head, row group) and store them as the B fragments of S^T = K Q'^T, so that
 // the stream kernel's warps (several per item, and again for every further item a warp reaches)

@@ -95,6 +95,29 @@ __device__ __forceinline__ int last_not_above(const int32_t* __restrict__ prefix
     return (int)__reduce_add_sync(0xffffffffu, (unsigned)count);
 }
 
+// ---- dependent launches ---------------------------------------------------------------------------
+// The kernels of one attention call are launched behind each other with programmatic stream serialization: a kernel may
+// begin while the last blocks of the one before it finish, which hides the launch latency (about 2 us each on a stream).
+// Every kernel therefore waits for its predecessor's end before it touches global memory, and lets its successor start
+// being scheduled once its own blocks run.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
+
+template <class Params>
+static int launch_behind(void (*kernel)(const Params), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, const Params& p) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return (int)cudaLaunchKernelEx(&cfg, kernel, p);
+}
+
 // ---- bounds-checked build (-DW34_BOUNDS) ----------------------------------------------------------
 // Every index into a block table, every page id read from one and every write slot is range-checked
 // before an address is formed from it.  The first violation is recorded in a device word (what, the
