@@ -1846,7 +1846,7 @@ constexpr int kRowTripleFloats = kHeadDim + 2;
 // hundreds of partials per row and only a few rows, for which MW = 32.
 template <bool PARTIAL_OUT, int MW>
 __global__ void __launch_bounds__(MW * 32) tq4_attention_merge_kernel(const StreamParams p) {
-    __shared__ float s_acc[MW][kHeadDim];
+    __shared__ __align__(16) float s_acc[MW][kHeadDim];
     __shared__ float s_m[MW], s_l[MW];
     grid_dependency_wait();
     grid_launch_dependents();
@@ -1864,12 +1864,12 @@ __global__ void __launch_bounds__(MW * 32) tq4_attention_merge_kernel(const Stre
         if (PARTIAL_OUT && wid == 0) {
             float* dst = p.triple_out + ((size_t)tok * p.num_q_heads + q_head) * (kHeadDim + 2);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) dst[lane + 32 * j] = 0.0f;
+            for (int j = 0; j < 8; ++j) dst[8 * lane + j] = 0.0f;
             if (lane == 0) { dst[kHeadDim] = -1e30f; dst[kHeadDim + 1] = 0.0f; }
         }
         if (!PARTIAL_OUT && wid == 0 && p.sel_phys != nullptr) {   // query-sparse: masked rows are zeros
-#pragma unroll
-            for (int j = 0; j < 8; ++j) store_act(p.attn_out, ((size_t)tok * p.num_q_heads + q_head) * kHeadDim + lane + 32 * j, 0.0f, p.io_bf16);
+            const float zero[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            store8(p.attn_out, ((size_t)tok * p.num_q_heads + q_head) * kHeadDim, lane, p.io_bf16, zero);
         }
     };
     if (p.batch.valid_token_mask != nullptr && p.batch.valid_token_mask[tok] == 0) { skip_row(); return; }
@@ -1898,7 +1898,7 @@ __global__ void __launch_bounds__(MW * 32) tq4_attention_merge_kernel(const Stre
     const int npages = npages_a[r];
     const int per = hdr->units_per_warp;
 
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};      // columns [8 lane, + 8)
     float l_tot = 0.0f;
     float m_tot = -1e30f;
     if (npages > 0 && per > 0) {
@@ -1935,28 +1935,29 @@ __global__ void __launch_bounds__(MW * 32) tq4_attention_merge_kernel(const Stre
             l_tot += lw;
             uint32_t full = __ballot_sync(0xffffffffu, w_s > 0.0f);
             while (full != 0u) {
-                float wgt[4], v[4][8];
+                float wgt[4];
+                float4 va[4], vb[4];
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     const int src = full != 0u ? __ffs((int)full) - 1 : 0;
                     wgt[k] = full != 0u ? __shfl_sync(0xffffffffu, w_s, src) : 0.0f;
                     const int slot = __shfl_sync(0xffffffffu, mine, src);
-                    const float* pa = base + (size_t)slot * part_floats + row8 * kHeadDim;
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) v[k][j] = full != 0u ? pa[lane + 32 * j] : 0.0f;
+                    const float4* pa = reinterpret_cast<const float4*>(base + (size_t)slot * part_floats + row8 * kHeadDim + 8 * lane);
+                    va[k] = full != 0u ? pa[0] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    vb[k] = full != 0u ? pa[1] : make_float4(0.f, 0.f, 0.f, 0.f);
                     full &= full - 1u;
                 }
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) acc[j] += v[k][j] * wgt[k];
+                    acc[0] += va[k].x * wgt[k]; acc[1] += va[k].y * wgt[k]; acc[2] += va[k].z * wgt[k]; acc[3] += va[k].w * wgt[k];
+                    acc[4] += vb[k].x * wgt[k]; acc[5] += vb[k].y * wgt[k]; acc[6] += vb[k].z * wgt[k]; acc[7] += vb[k].w * wgt[k];
                 }
             }
         }
     }
     // combine the warps
-#pragma unroll
-    for (int j = 0; j < 8; ++j) s_acc[wid][lane + 32 * j] = acc[j];
+    *reinterpret_cast<float4*>(&s_acc[wid][8 * lane]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    *reinterpret_cast<float4*>(&s_acc[wid][8 * lane + 4]) = make_float4(acc[4], acc[5], acc[6], acc[7]);
     if (lane == 0) { s_m[wid] = m_tot; s_l[wid] = l_tot; }
     __syncthreads();
     if (wid != 0) return;
@@ -1970,31 +1971,27 @@ __global__ void __launch_bounds__(MW * 32) tq4_attention_merge_kernel(const Stre
     for (int w = 0; w < MW; ++w) {
         const float wgt = (s_l[w] > 0.0f) ? ex2(s_m[w] - m_tot) : 0.0f;
         l_tot += s_l[w] * wgt;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[j] += s_acc[w][lane + 32 * j] * wgt;
+        const float4 a = *reinterpret_cast<const float4*>(&s_acc[w][8 * lane]), b = *reinterpret_cast<const float4*>(&s_acc[w][8 * lane + 4]);
+        acc[0] += a.x * wgt; acc[1] += a.y * wgt; acc[2] += a.z * wgt; acc[3] += a.w * wgt;
+        acc[4] += b.x * wgt; acc[5] += b.y * wgt; acc[6] += b.z * wgt; acc[7] += b.w * wgt;
     }
     if (PARTIAL_OUT) {
         float* dst = p.triple_out + ((size_t)tok * p.num_q_heads + q_head) * kRowTripleFloats;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) dst[lane + 32 * j] = acc[j];
+        for (int j = 0; j < 8; ++j) dst[8 * lane + j] = acc[j];
         if (lane == 0) { dst[kHeadDim] = m_tot; dst[kHeadDim + 1] = l_tot; }
         return;
     }
     const size_t out_base = ((size_t)tok * p.num_q_heads + q_head) * kHeadDim;
-    if (p.natural) {
-        const float inv = (l_tot > 0.0f) ? (1.0f / l_tot) : 0.0f;
+    const float inv = (l_tot > 0.0f) ? (1.0f / (p.natural ? l_tot : l_tot * (kLutScale * 16.0f))) : 0.0f;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[j] *= inv;
-        apply_output_gate(acc, p.og, out_base, lane, p.io_bf16);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) store_act(p.attn_out, out_base + lane + 32 * j, acc[j], p.io_bf16);
-        return;
+    for (int j = 0; j < 8; ++j) acc[j] *= inv;
+    if (!p.natural) {
+        butterfly8<5>(acc, lane);
+        sign8(acc, lane);
     }
-    const float inv_l = (l_tot > 0.0f) ? (1.0f / (l_tot * kLutScale)) : 0.0f;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] *= inv_l;
-    wht256_lanes(acc, lane);
-    store_output_row(p.attn_out, out_base, acc, lane, p.io_bf16, p.og);
+    apply_output_gate8(acc, p.og, out_base, lane, p.io_bf16);
+    store8(p.attn_out, out_base, lane, p.io_bf16, acc);
 }
 
 // Cross-shard merge: parts is [num_parts][rows][258]; one warp per row.

@@ -486,11 +486,13 @@ class StepIo:
     changed since the last upload (graph_io.rs:109-195): a decode step adds a page to one sequence
     in sixteen."""
 
-    def __init__(self, max_reqs, max_tokens, max_blocks_per_req, device="cuda"):
+    def __init__(self, max_reqs, max_tokens, max_blocks_per_req, device="cuda", front_words=0):
         self.max_reqs, self.max_tokens, self.max_blocks = max_reqs, max_tokens, max_blocks_per_req
+        # front_words: 32-bit words in front of the metadata that the caller fills itself (a multiple of 4)
+        self.front_words = front_words
         # arena order: query_start_loc | context_lens_before | seq_lens_after | write_slot_mapping | block_tables
         sizes = [max_reqs + 1, max_reqs, max_reqs, max_tokens, max_reqs * max_blocks_per_req]
-        offs = np.concatenate([[0], np.cumsum([(s + 3) // 4 * 4 for s in sizes])])
+        offs = front_words + np.concatenate([[0], np.cumsum([(s + 3) // 4 * 4 for s in sizes])])
         self._offs, self._sizes = offs, sizes
         total = int(offs[-1])
         self.host = torch.zeros(total, dtype=torch.int32).pin_memory() if device != "cpu" else torch.zeros(total, dtype=torch.int32)
@@ -516,7 +518,7 @@ class StepIo:
         self.desc.block_tables = base + 4 * int(offs[4])
         self.desc.max_blocks_per_req = max_blocks_per_req
         self._arena_ptrs = (self._ptr(0), self._ptr(1), self._ptr(2), self._ptr(4), self._ptr(3))
-        self.nbytes = total * 4          # a full upload
+        self.nbytes = (total - front_words) * 4          # a full upload of the metadata
         self.last_upload_bytes = 0
 
     def _ptr(self, i):
@@ -549,8 +551,8 @@ class StepIo:
         return rc
 
     def upload(self, full=False, tables_only=False):
-        """One copy of the arena up to the last block-table entry that changed since the previous
-        upload (the length and slot arrays sit in front of the tables); returns the bytes copied.
+        """One copy of the arena (with what the caller put in front of it) up to the last block-table entry that
+        changed since the previous upload (the length and slot arrays sit in front of the tables); returns the bytes copied.
         tables_only: the copy starts at the block tables (the caller uploads the front part itself,
         e.g. from a captured graph) and is skipped when no entry changed."""
         bt0, bt1 = int(self._offs[4]), int(self._offs[5])
@@ -578,7 +580,7 @@ class StepIo:
 
     @property
     def head_words(self):
-        """Words in front of the block tables: lengths and slots."""
+        """Words in front of the block tables: the caller's, lengths and slots."""
         return int(self._offs[4])
 
 
@@ -591,21 +593,26 @@ class DecodeStep:
     """The call a user of this path makes once per model step and layer: new K/V rows and Q in
     HOST memory in, attention output in HOST memory out (append then attend, forward.rs:1141-1188)."""
 
+    SMALL_PAYLOAD = 16 << 10
+
     def __init__(self, layer, seqs, num_q_heads, max_q_len=1, scratch_bytes=64 << 20, device="cuda", extra_blocks=0):
         self.layer, self.seqs, self.hq = layer, seqs, num_q_heads
         hkv = layer.layout.local_kv_heads
         n_tok = len(seqs) * max_q_len
         max_blocks = max(s.num_pages for s in seqs) + extra_blocks   # room for sequences that grow
-        self.io = StepIo(len(seqs), n_tok, max_blocks, device=device)
+        # K, V and Q of the step sit in front of its metadata, in the pinned arena and in the device's: one copy takes both.
+        shapes = ((n_tok, hkv * 256), (n_tok, hkv * 256), (n_tok, num_q_heads, 256))
+        ends = np.cumsum([int(np.prod(s)) // 2 for s in shapes])        # in 32-bit words; rows are 512 bytes
+        self.payload_words = int(ends[-1])
+        self.io = StepIo(len(seqs), n_tok, max_blocks, device=device, front_words=self.payload_words)
         self.ex = Executor(scratch_bytes, device=device)
-        pin = lambda *shape: torch.zeros(*shape, dtype=torch.float16).pin_memory()  # noqa: E731
-        self.k_host, self.v_host = pin(n_tok, hkv * 256), pin(n_tok, hkv * 256)
-        self.q_host, self.out_host = pin(n_tok, num_q_heads, 256), pin(n_tok, num_q_heads, 256)
-        self.k_dev = torch.zeros_like(self.k_host, device=device)
-        self.v_dev = torch.zeros_like(self.v_host, device=device)
-        self.q_dev = torch.zeros_like(self.q_host, device=device)
+        views = lambda arena: [arena[e - int(np.prod(s)) // 2:e].view(torch.float16).view(*s)  # noqa: E731
+                               for s, e in zip(shapes, ends)]
+        self.k_host, self.v_host, self.q_host = views(self.io.host)
+        self.k_dev, self.v_dev, self.q_dev = views(self.io.dev)
+        self.out_host = torch.zeros(*shapes[2], dtype=torch.float16).pin_memory()
         self.out_dev = torch.zeros_like(self.out_host, device=device)
-        self.payload_bytes = 2 * self.k_host.numel() * 2 + self.q_host.numel() * 2
+        self.payload_bytes = self.payload_words * 4
         self.h2d_bytes = self.io.nbytes + self.payload_bytes      # upper bound: a full metadata upload
         self.h2d_bytes_total = 0                                  # bytes actually copied by run() so far
         self._graphs = {}
@@ -613,34 +620,38 @@ class DecodeStep:
         self._fence = None      # recorded after a step's last use of the pinned buffers when sync=False
 
     def _capture(self, lib):
-        """Two CUDA graphs for the whole step (the reference replays its decode steps the same way,
-        crates/warp34-host/src/model/graphs.rs:199-259): the first uploads K, V and Q from pinned
-        memory and is launched before the host packs the step's metadata, so that the copies run
-        while the CPU works; the second uploads lengths and slots, appends, attends and downloads
-        the output.  Block tables are in neither: their changed part is copied between the two."""
+        """CUDA graphs for the whole step (the reference replays its decode steps the same way,
+        crates/warp34-host/src/model/graphs.rs:199-259): upload K, V, Q, lengths and slots, append, attend with the
+        output written to pinned memory.  Block tables are not in them: their changed part is copied in front.  K, V and Q get a graph of their own,
+        launched before the host packs the step's metadata so that the copy runs while the CPU works; up to SMALL_PAYLOAD
+        bytes are copied faster than a second graph is launched, and go with the metadata (one sequence 51 us a step instead
+        of 53; two sequences already 73 instead of 65)."""
+        split = 0 if self.payload_bytes <= self.SMALL_PAYLOAD else self.payload_words
         head = self.io.head_words
         b = _DescOnly(self.io.desc)
 
         def payload():
-            self.k_dev.copy_(self.k_host, non_blocking=True)
-            self.v_dev.copy_(self.v_host, non_blocking=True)
-            self.q_dev.copy_(self.q_host, non_blocking=True)
+            self.io.dev[:split].copy_(self.io.host[:split], non_blocking=True)
 
         def body():
             self.ex.set_stream()
-            self.io.dev[:head].copy_(self.io.host[:head], non_blocking=True)
+            self.io.dev[split:head].copy_(self.io.host[split:head], non_blocking=True)
             kv_cache_write(self.ex, self.layer, b, self.k_dev, self.v_dev, lib=lib)
-            paged_attention(self.ex, self.layer, b, self.q_dev, self.out_dev, self.hq, lib=lib)
-            self.out_host.copy_(self.out_dev, non_blocking=True)
+            # the output goes straight to the pinned buffer: a row is one 512-byte write across the bus, and no copy follows
+            paged_attention(self.ex, self.layer, b, self.q_dev, self.out_host, self.hq, lib=lib)
 
         side = torch.cuda.Stream()
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):
-            payload()
+            if split:
+                payload()
             body()                      # warm-up outside the capture (one-time attribute calls)
         torch.cuda.current_stream().wait_stream(side)
         graphs = []
         for fn in (payload, body):
+            if fn is payload and not split:
+                graphs.append(None)
+                continue
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g):
                 fn()
@@ -662,24 +673,22 @@ class DecodeStep:
             key = (id(lib), len(self.seqs), int(sum(q_lens)), int(max(q_lens)), float(sm_scale),
                    int(mask_mode), int(sliding_window), int(self.ex.ex.flags))
             g = self._graphs.get(key)
-            if g is not None:
+            if g is not None and g[0] is not None:
                 g[0].replay()           # K, V, Q on their way while the metadata is packed
             self.io.pack(self.seqs, q_lens, sm_scale, mask_mode, sliding_window)
             if g is None:
                 self.io.upload(full=True)
                 g = self._graphs[key] = self._capture(lib)
-                g[0].replay()
-            self.meta_bytes_last = self.io.upload(tables_only=True) + 4 * self.io.head_words
+                if g[0] is not None:
+                    g[0].replay()
+            self.meta_bytes_last = self.io.upload(tables_only=True) + 4 * self.io.head_words - self.payload_bytes
             self.h2d_bytes_total += self.meta_bytes_last + self.payload_bytes
             g[1].replay()
             self._finish(sync)
             return self.out_host
         self.io.pack(self.seqs, q_lens, sm_scale, mask_mode, sliding_window)
-        self.meta_bytes_last = self.io.upload()
+        self.meta_bytes_last = self.io.upload() - self.payload_bytes      # K, V and Q with it
         self.h2d_bytes_total += self.meta_bytes_last + self.payload_bytes
-        self.k_dev.copy_(self.k_host, non_blocking=True)
-        self.v_dev.copy_(self.v_host, non_blocking=True)
-        self.q_dev.copy_(self.q_host, non_blocking=True)
         self.ex.set_stream()
         b = _DescOnly(self.io.desc)
         kv_cache_write(self.ex, self.layer, b, self.k_dev, self.v_dev, lib=lib)
