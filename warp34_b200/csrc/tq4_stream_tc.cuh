@@ -1,0 +1,222 @@
+// Decode and verify attention over TQ4 pages on the 5th-generation tensor cores, with value + residual operands.  Included by
+// tq4_attention.cu (shares the plan, the table, the PTX wrappers and the merge with the other streaming kernels).
+//
+// One CTA per SM is one worker: it takes an equal contiguous share of the step's (request, kv head, group of R query rows,
+// page) units and walks it in blocks of 128 keys.  The cached keys are the M dimension of both products, so that every code
+// is dequantised once for up to 24 query rows, and straight into tensor memory, where it is the MMAs' A operand:
+//   S^T[128 keys x 2R]      per 128-half = Khi [Q'hi | Q'lo]^T + Klo [Q'hi | Q'lo]^T        lane = key
+//   O^T[128 channels x 2R]  per 128-half += Vhi^T [(P d_v)hi | (P d_v)lo]^T                  lane = channel
+// (on blocks with a large weight also the V centroids' residual).  Scales stay outside the operands: a thread holds a key's
+// scores of both halves and applies its K scales there, and P is multiplied by the V scale of its key and half.
+//
+//   warps 0-3   softmax: thread = key.  P goes to shared memory as the B operand; the running maximum is a reference that
+//               moves only when it is exceeded by 2^3, so a block usually needs no reduction over its keys
+//   warps 4-7   K: thread = key, 32 channels at a time into a ring of four TMEM granules
+//   warps 8-15  V: thread = fragment position (16x256b stores put channel pairs of four keys in place), half x quadrant
+//   warp 16 copies raw pages, warp 17 issues the score products, warp 18 the output products
+// Work is split by role because query fragments, table look-ups and accumulators in one warp need 255 registers, which left two
+// warps per scheduler and every pipe below half (see tq4_stream_exact.cuh, still used for steps of few pages).
+#pragma once
+
+namespace w34 {
+
+constexpr int kXtKeys = 128, kXtPages = kXtKeys / kPageTokens;
+constexpr int kXtWarps = 20, kXtThreads = kXtWarps * 32;      // the last warp only fills the fourth quadrant
+constexpr uint32_t kXtRun = (uint32_t)kXtPages * kTq4PageHeadBytes;       // 16896: K or V of a block
+constexpr uint32_t kXtColK = 0, kXtColV = 128, kXtColS = 256, kXtColO = 384;
+constexpr int kXtKRing = 4;                                   // granules of 32 channels: 16 columns of values, 16 of residuals
+constexpr float kXtLag = 3.0f;                                // log2 units the reference maximum may lag; P is carried times 2^-3
+
+__host__ __device__ constexpr int xt_stages(int rows) { return rows <= 8 ? 3 : 2; }
+__host__ __device__ constexpr uint32_t xt_query_bytes(int rows) { return 2u * (uint32_t)rows * 512u; }
+
+struct XtShared {
+    float2 k_scale[2][kXtKeys], v_scale[2][kXtKeys];
+    float m_ref[24], alpha[24], mass[24];
+    float red[4][24];
+    int row_min[24], row_max[24];
+    __align__(16) int peak[2][4];
+    uint32_t tmem;
+    uint32_t aborted;
+    uint64_t bars[48];
+};
+enum { kXtRawKFull = 0, kXtRawKFree = 4, kXtRawVFull = 8, kXtRawVFree = 12, kXtKFull = 16, kXtKEmpty = 20, kXtVFull = 24, kXtVEmpty = 26,
+       kXtQFull = 28, kXtQFree = 30, kXtSReady = 32, kXtSFree, kXtPReady, kXtPvDone, kXtKScale, kXtVScale = kXtKScale + 2,
+       kXtDrain = kXtVScale + 2, kXtBarCount };
+static_assert(kXtBarCount <= 48, "barrier slots");
+
+__device__ __forceinline__ void tc_ld8(uint32_t (&r)[8], uint32_t taddr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tc_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+// 16 lanes x 256 bits, four times: registers 4 i + {0, 1} go to lane t / 4, columns 8 i + 2 (t % 4) + {0, 1}; 4 i + {2, 3} eight
+// lanes further (t: thread of the warp).
+__device__ __forceinline__ void tc_st_16x256b_x4(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+                 :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+// Barrier of the four softmax warps.
+__device__ __forceinline__ void xt_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ bool xt_any(bool x) {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(r) : "r"((uint32_t)x) : "memory");
+    return r != 0;
+}
+
+// Query rows of item idx = (request * kv heads + kv head) * q_groups_max + group as the B operand: 2R rows (R values, then R
+// residuals) of 256 rotated columns, four blocks of 64 columns, 16-byte chunks swizzled by the row.  Eight warps.
+__device__ void xt_prepare_query(const StreamParams& p, int idx) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, R = p.rows_per_group;
+    const int hkv = p.layout.local_kv_heads;
+    const int group = idx % p.q_groups_max, kv_head = (idx / p.q_groups_max) % hkv, r = idx / (p.q_groups_max * hkv);
+    if (r >= p.batch.num_reqs) return;
+    const ReqGeom g = load_req(p.batch, r);
+    const int rows_in_req = g.q_len * p.gqa;
+    if (!g.valid || group * R >= rows_in_req) return;
+    uint8_t* dst = reinterpret_cast<uint8_t*>(p.qfrag) + (size_t)idx * xt_query_bytes(R);
+    for (int i = wid; i < R; i += kRowsPerGroup) {
+        const int row = group * R + i;
+        const int q_off = row / p.gqa, q_head = kv_head * p.gqa + (row - q_off * p.gqa);
+        float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (row < rows_in_req && (p.batch.valid_token_mask == nullptr || p.batch.valid_token_mask[g.q_start + q_off] != 0)) {
+            load8(p.q_in, ((size_t)(g.q_start + q_off) * p.num_q_heads + q_head) * kHeadDim, lane, p.io_bf16, v);
+            sign8(v, lane);
+            butterfly8<5>(v, lane);
+        }
+        uint32_t hi[4], lo[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float a = v[2 * k] * (p.q_scale * 0.0625f), b = v[2 * k + 1] * (p.q_scale * 0.0625f);
+            const __half2 h = __floats2half2_rn(a, b);
+            const float2 hf = __half22float2(h);
+            hi[k] = *reinterpret_cast<const uint32_t*>(&h);
+            lo[k] = pack_half2(a - hf.x, b - hf.y);
+        }
+        // (i and i + R share their low three bits: R is a multiple of 8)
+        uint4* out = reinterpret_cast<uint4*>(dst + (size_t)(lane >> 3) * (2 * R * 128) + (size_t)i * 128 + (((lane & 7) ^ (i & 7)) << 4));
+        out[0] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        out[R * 8] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    }
+}
+
+// A worker's position in the step's unit list; every role warp advances its own.
+struct XtWalk {
+    int u, u_end, r;
+};
+struct XtSegment {
+    int r, kv_head, group, pg0, pages, slot;
+};
+__device__ __forceinline__ bool xt_next(const StreamParams& p, XtWalk& w, XtSegment& s) {
+    if (w.u >= w.u_end) return false;
+    const int R = p.batch.num_reqs;
+    const int32_t* unit_prefix = plan_array(p.scratch, 0, R);
+    while (unit_prefix[w.r + 1] <= w.u) ++w.r;  // skips requests without units
+    const int npages = plan_array(p.scratch, 3, R)[w.r], ngroups = plan_array(p.scratch, 4, R)[w.r];
+    const int in_req = w.u - unit_prefix[w.r];
+    const int item = in_req / npages, page = in_req - item * npages;
+    s.r = w.r;
+    s.kv_head = item / ngroups;
+    s.group = item - s.kv_head * ngroups;
+    s.pg0 = plan_array(p.scratch, 2, R)[w.r] + page;
+    s.pages = min(w.u_end - w.u, npages - page);
+    s.slot = (int)blockIdx.x + plan_array(p.scratch, 1, R)[w.r] + item;
+    w.u += s.pages;
+    return true;
+}
+
+template <int R>
+__global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(const StreamParams p) {
+    constexpr int N = 2 * R, STAGES = xt_stages(R);
+    constexpr uint32_t kQueryBytes = xt_query_bytes(R), kPBytes = (uint32_t)N * 256u;      // P of one half: [2 x 64 keys][N][128 B]
+    extern __shared__ __align__(1024) uint8_t smem[];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const uint32_t win_lo = smem_u32(smem);
+    const uint32_t lut_addr = (win_lo + 0xffffu) & ~0xffffu;
+    PlanHeader* hdr = reinterpret_cast<PlanHeader*>(p.scratch);
+    SmemCarver carve(win_lo, lut_addr, win_lo + p.smem_bytes);
+    const uint32_t q_t[2] = {carve.take(kQueryBytes, 1024), carve.take(kQueryBytes, 1024)};
+    const uint32_t p_t = carve.take(2u * kPBytes, 1024);
+    uint32_t raw[2 * STAGES];
+#pragma unroll
+    for (int i = 0; i < 2 * STAGES; ++i) raw[i] = carve.take(kXtRun, 128);
+    const uint32_t sh_addr = carve.take((uint32_t)sizeof(XtShared), 16);
+    if (!carve.ok) {
+        grid_dependency_wait();
+        if (tid == 0) atomicOr(&hdr->status, 2);  // shared-memory window cannot hold the layout
+        return;
+    }
+    XtShared& sh = *reinterpret_cast<XtShared*>(smem + (sh_addr - win_lo));
+    auto raw_k = [&](int s) { return s == 0 ? raw[0] : (STAGES == 2 || s == 1) ? raw[1] : raw[STAGES - 1]; };
+    auto raw_v = [&](int s) { return s == 0 ? raw[STAGES] : (STAGES == 2 || s == 1) ? raw[STAGES + 1] : raw[2 * STAGES - 1]; };
+    const uint32_t bars = smem_u32(sh.bars);
+    auto bar = [&](int which) { return bars + 8u * (uint32_t)which; };
+    volatile uint32_t* aborted = &sh.aborted;
+    // Waits are bounded and warp-uniform; one that gives up ends every loop.
+    auto wait_all = [&](uint32_t b, uint32_t parity) {
+        const bool ok = mbar_wait(b, parity) && *aborted == 0u;
+        if (__all_sync(0xffffffffu, ok)) return true;
+        *aborted = 1u;
+        return false;
+    };
+
+    for (int i = tid; i < 256 * 32; i += kXtThreads) {      // table as in the exact streaming kernel, residuals unscaled
+        const int byte = i >> 5, ln = i & 31;
+        const float c0 = kLutScale * tq4_centroid(byte & 15), c1 = kLutScale * tq4_centroid(byte >> 4);
+        const uint32_t hi = pack_half2(c0, c1);
+        const float2 hf = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+        sts32(lut_addr + (uint32_t)(byte * 256 + ln * 4), (ln & 1) ? pack_half2(c0 - hf.x, c1 - hf.y) : hi);
+        sts32(lut_addr + (uint32_t)(byte * 256 + 128 + ln * 4), hi);
+    }
+    if (tid == 0) {
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(bar(kXtRawKFull + s), 1u);
+            mbar_init(bar(kXtRawKFree + s), 4u);
+            mbar_init(bar(kXtRawVFull + s), 1u);
+            mbar_init(bar(kXtRawVFree + s), 8u);
+        }
+        for (int s = 0; s < kXtKRing; ++s) { mbar_init(bar(kXtKFull + s), 4u); mbar_init(bar(kXtKEmpty + s), 1u); }
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(bar(kXtVFull + s), 8u);
+            mbar_init(bar(kXtVEmpty + s), 1u);
+            mbar_init(bar(kXtQFull + s), 1u);
+            mbar_init(bar(kXtQFree + s), 1u);
+            mbar_init(bar(kXtKScale + s), 4u);
+            mbar_init(bar(kXtVScale + s), 8u);
+        }
+        mbar_init(bar(kXtSReady), 1u);
+        mbar_init(bar(kXtSFree), 4u);
+        mbar_init(bar(kXtPReady), 4u);
+        mbar_init(bar(kXtPvDone), 1u);
+        mbar_init(bar(kXtDrain), 2u);
+        sh.aborted = 0u;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    grid_dependency_wait();      // nothing above touches global memory
+    grid_launch_dependents();
+
+    const int per = hdr->units_per_warp, total_units = hdr->total_units;
+    XtWalk walk;
+    {
+        const long long u0 = (long long)blockIdx.x * per;
+        walk.u = (int)min(u0, (long long)total_units);
+        walk.u_end = min(walk.u + per, total_units);
+    }
+    if (walk.u >= walk.u_end) return;      // block-uniform
+    walk.r = last_not_above(plan_array(p.scratch, 0, p.batch.num_reqs), p.batch.num_reqs, walk.u);
+    __syncwarp();
+    if (wid == 0) {
+        tc_alloc(smem_u32(&sh.tmem), 512);
+        tc_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&sh.tmem);
+    const uint32_t quad = (uint32_t)(wid & 3) << 21;      // this warp's 32 TMEM lanes
+    XtSegment sg;
+    uint32_t c = 0;                                       // blocks so far
