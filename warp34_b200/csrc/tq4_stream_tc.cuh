@@ -220,3 +220,255 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
     const uint32_t quad = (uint32_t)(wid & 3) << 21;      // this warp's 32 TMEM lanes
     XtSegment sg;
     uint32_t c = 0;                                       // blocks so far
+
+    if (wid == 16) {
+        // ======================= raw pages and query rows ==========================================
+        uint32_t seg = 0, k_issued = 0, v_issued = 0;
+        bool ok = true;
+        while (ok && xt_next(p, walk, sg)) {
+            const int32_t* blocks = p.batch.block_tables + (size_t)sg.r * p.batch.max_blocks_per_req;
+            const uint8_t* kb = (const uint8_t*)(uintptr_t)p.layout.k_base + (size_t)sg.kv_head * p.layout.k_head_stride_bytes;
+            const uint8_t* vb = (const uint8_t*)(uintptr_t)p.layout.v_base + (size_t)sg.kv_head * p.layout.v_head_stride_bytes;
+            auto page_id = [&](int b) -> int32_t {
+                const int pg = kXtPages * b + lane;
+                return (lane < kXtPages && pg < sg.pages) ? block_table_page(blocks, sg.pg0 + pg, p.batch.max_blocks_per_req, kInStream) : -1;
+            };
+            int32_t id = page_id(0);
+            ok = wait_all(bar(kXtQFree + (int)(seg & 1)), ((seg >> 1) & 1) ^ 1u);
+            if (!ok) break;
+            if (lane == 0) {
+                const size_t idx = (size_t)(sg.r * p.layout.local_kv_heads + sg.kv_head) * p.q_groups_max + sg.group;
+                mbar_expect_tx(bar(kXtQFull + (int)(seg & 1)), kQueryBytes);
+                bulk_g2s((seg & 1) ? q_t[1] : q_t[0], reinterpret_cast<const uint8_t*>(p.qfrag) + idx * kQueryBytes, kQueryBytes,
+                         bar(kXtQFull + (int)(seg & 1)));
+            }
+            __syncwarp();
+            ++seg;
+            for (int b = 0; kXtPages * b < sg.pages; ++b, ++c) {
+                const int s = (int)(c % STAGES);
+                const uint32_t lap = (c / STAGES) & 1u, bytes = (uint32_t)min(kXtPages, sg.pages - kXtPages * b) * kTq4PageHeadBytes;
+                const int32_t next = page_id(b + 1);
+                if (!(ok = wait_all(bar(kXtRawKFree + s), lap ^ 1u))) break;
+                if (lane == 0) mbar_expect_tx(bar(kXtRawKFull + s), bytes);
+                __syncwarp();
+                if (id >= 0) {
+                    bulk_g2s(raw_k(s) + (uint32_t)lane * kTq4PageHeadBytes, kb + (size_t)id * p.layout.k_page_stride_bytes, kTq4PageHeadBytes,
+                             bar(kXtRawKFull + s));
+                }
+                k_issued = c + 1;
+                if (!(ok = wait_all(bar(kXtRawVFree + s), lap ^ 1u))) break;
+                if (lane == 0) mbar_expect_tx(bar(kXtRawVFull + s), bytes);
+                __syncwarp();
+                if (id >= 0) {
+                    bulk_g2s(raw_v(s) + (uint32_t)lane * kTq4PageHeadBytes, vb + (size_t)id * p.layout.v_page_stride_bytes, kTq4PageHeadBytes,
+                             bar(kXtRawVFull + s));
+                }
+                v_issued = c + 1;
+                id = next;
+            }
+        }
+        // copies in flight must land before the CTA leaves
+        for (uint32_t j = k_issued > STAGES ? k_issued - STAGES : 0; j < k_issued; ++j) (void)mbar_wait(bar(kXtRawKFull + (int)(j % STAGES)), (j / STAGES) & 1u);
+        for (uint32_t j = v_issued > STAGES ? v_issued - STAGES : 0; j < v_issued; ++j) (void)mbar_wait(bar(kXtRawVFull + (int)(j % STAGES)), (j / STAGES) & 1u);
+        for (uint32_t j = seg > 2 ? seg - 2 : 0; j < seg; ++j) (void)mbar_wait(bar(kXtQFull + (int)(j & 1)), (j >> 1) & 1u);
+        __syncwarp();
+    } else if (wid == 17) {
+        // ======================= score products: one thread =======================================
+        if (elect_one()) {
+            constexpr uint32_t kIdesc = tc_idesc(kXtKeys, N, 0);
+            const uint64_t desc_q[2] = {tc_smem_desc(q_t[0], 16u, 1024u), tc_smem_desc(q_t[1], 16u, 1024u)};
+            uint32_t seg = 0;
+            bool ok = true;
+            while (ok && xt_next(p, walk, sg)) {
+                ok = mbar_wait(bar(kXtQFull + (int)(seg & 1)), (seg >> 1) & 1u);
+                const uint64_t dq = (seg & 1) ? desc_q[1] : desc_q[0];
+                for (int b = 0; ok && kXtPages * b < sg.pages; ++b, ++c) {
+                    ok = mbar_wait(bar(kXtSFree), (c & 1u) ^ 1u);      // the scores of the block before are in registers
+#pragma unroll 1
+                    for (int gr = 0; gr < 8 && ok; ++gr) {
+                        const uint32_t slot = (uint32_t)gr & (kXtKRing - 1), lap = 2u * c + ((uint32_t)gr >> 2);
+                        ok = mbar_wait(bar(kXtKFull + (int)slot), lap & 1u) && *aborted == 0u;
+                        if (!ok) break;
+                        tc_fence_after();
+                        const uint32_t d = tmem + kXtColS + (uint32_t)(gr >> 2) * (uint32_t)N, a = tmem + kXtColK + 32u * slot;
+#pragma unroll
+                        for (int ks = 0; ks < 2; ++ks) {
+                            // channels 32 gr + 16 ks: block of 64 gr >> 1, 32 bytes per k-step
+                            const uint64_t bq = dq + (uint64_t)((gr >> 1) * (N * 128 / 16) + 2 * (2 * (gr & 1) + ks));
+                            tc_mma_f16_ts(d, a + 8u * (uint32_t)ks, bq, kIdesc, ((gr & 3) || ks) ? 1u : 0u);
+                            tc_mma_f16_ts(d, a + 16u + 8u * (uint32_t)ks, bq, kIdesc, 1u);
+                        }
+                        tc_commit(bar(kXtKEmpty + (int)slot));
+                    }
+                    if (ok) tc_commit(bar(kXtSReady));
+                }
+                if (ok) tc_commit(bar(kXtQFree + (int)(seg & 1)));
+                ++seg;
+            }
+            if (!ok) *aborted = 1u;
+            tc_commit(bar(kXtDrain));      // nothing may be in flight when the CTA leaves
+        }
+        __syncwarp();
+        (void)mbar_wait(bar(kXtDrain), 0u);
+        __syncwarp();
+    } else if (wid == 18) {
+        // ======================= output products: one thread =======================================
+        if (elect_one()) {
+            constexpr uint32_t kIdesc = tc_idesc(128, N, 0);
+            const uint64_t desc_p = tc_smem_desc(p_t, 16u, 1024u);
+            uint32_t laps = 0;      // fills of each V granule so far
+            bool ok = true;
+            while (ok && xt_next(p, walk, sg)) {
+                for (int b = 0; ok && kXtPages * b < sg.pages; ++b, ++c) {
+                    ok = mbar_wait(bar(kXtPReady), c & 1u) && *aborted == 0u;
+                    if (!ok) break;
+                    volatile int* pk = sh.peak[c & 1];
+                    const int passes = (pk[0] | pk[1] | pk[2] | pk[3]) != 0 ? 2 : 1;
+                    for (int pass = 0; pass < passes && ok; ++pass, ++laps) {
+#pragma unroll 1
+                        for (int kk = 0; kk < 2 && ok; ++kk) {
+                            ok = mbar_wait(bar(kXtVFull + kk), laps & 1u) && *aborted == 0u;
+                            if (!ok) break;
+                            tc_fence_after();
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+#pragma unroll
+                                for (int ks = 0; ks < 4; ++ks) {
+                                    const uint64_t bp = desc_p + (uint64_t)(h * (int)(kPBytes / 16) + kk * (N * 128 / 16) + 2 * ks);
+                                    tc_mma_f16_ts(tmem + kXtColO + (uint32_t)(h * N),
+                                                  tmem + kXtColV + 64u * (uint32_t)h + 32u * (uint32_t)kk + 8u * (uint32_t)ks,
+                                                  bp, kIdesc, (b | pass | kk | ks) ? 1u : 0u);
+                                }
+                            }
+                            tc_commit(bar(kXtVEmpty + kk));
+                        }
+                    }
+                    if (ok) tc_commit(bar(kXtPvDone));
+                }
+            }
+            if (!ok) *aborted = 1u;
+            tc_commit(bar(kXtDrain));
+        }
+        __syncwarp();
+        (void)mbar_wait(bar(kXtDrain), 0u);
+        __syncwarp();
+    } else if (wid >= 8 && wid < 16) {
+        // ======================= V: 32 channels of a half, fragments of four keys a thread ===============
+        const int gid = lane >> 2, tig = lane & 3, half = (wid - 8) >> 2;
+        const int vw = 4 * (wid & 3) + (gid >> 1);                           // this thread's code word of the half
+        const uint32_t word_off = 4u * ((half ? 17u : 0u) + (uint32_t)vw);
+        const bool splice = half == 0 && vw == 0;                            // virtual word 0: (W0 >> 16) | (W16 << 16)
+        const uint32_t lut_v = lut_addr + 128u + 4u * (uint32_t)lane, lut_r = lut_addr + 8u * (uint32_t)(lane & 15);
+        // byte 2 (gid & 1) + T of the paired codes belongs to tile T
+        const uint32_t sel[2] = {0x7604u + ((uint32_t)(2 * (gid & 1)) << 4), 0x7604u + ((uint32_t)(2 * (gid & 1) + 1) << 4)};
+        uint32_t laps = 0;
+        bool ok = true;
+        while (ok && xt_next(p, walk, sg)) {
+            for (int b = 0; ok && kXtPages * b < sg.pages; ++b, ++c) {
+                const int s = (int)(c % STAGES);
+                if (!(ok = wait_all(bar(kXtRawVFull + s), (c / STAGES) & 1u))) break;
+                const uint32_t run = raw_v(s);
+                if (lane < 16) {      // the scales of 16 keys
+                    const int key = 16 * (wid - 8) + lane;
+                    const uint32_t rowp = run + (uint32_t)key * kTq4RowBytes;
+                    sh.v_scale[c & 1][key] = make_float2(__half2float(__ushort_as_half((unsigned short)(lds32(rowp) & 0xffffu))),
+                                                         __half2float(__ushort_as_half((unsigned short)(lds32(rowp + 64) >> 16))));
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar(kXtVScale + (int)(c & 1)));
+                const uint32_t rows = run + (uint32_t)(4 * tig) * kTq4RowBytes;
+                int passes = 1;
+#pragma unroll 1
+                for (int pass = 0; pass < passes && ok; ++pass, ++laps) {
+#pragma unroll 1
+                    for (int kk = 0; kk < 2; ++kk) {
+                        uint32_t a[2][16];
+                        if (!(ok = wait_all(bar(kXtVEmpty + kk), (laps & 1u) ^ 1u))) break;
+#pragma unroll
+                        for (int pg = 0; pg < 4; ++pg) {
+                            const uint32_t at = rows + (uint32_t)(4 * kk + pg) * kTq4PageHeadBytes;
+                            uint32_t w[4];
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) {
+                                w[k] = lds32(at + (uint32_t)k * kTq4RowBytes + word_off);
+                                if (splice) w[k] = (w[k] >> 16) | (lds32(at + (uint32_t)k * kTq4RowBytes + 64) << 16);
+                            }
+                            // byte t of ab -> (key 0, key 1) of channel 2 t (first) and 2 t + 1 (second); cd: keys 2 and 3
+                            const uint32_t ab[2] = {(w[0] & 0x0f0f0f0fu) | ((w[1] << 4) & 0xf0f0f0f0u), ((w[0] >> 4) & 0x0f0f0f0fu) | (w[1] & 0xf0f0f0f0u)};
+                            const uint32_t cd[2] = {(w[2] & 0x0f0f0f0fu) | ((w[3] << 4) & 0xf0f0f0f0u), ((w[2] >> 4) & 0x0f0f0f0fu) | (w[3] & 0xf0f0f0f0u)};
+#pragma unroll
+                            for (int T = 0; T < 2; ++T) {
+#pragma unroll
+                                for (int o = 0; o < 2; ++o) {
+                                    if (pass == 0) {
+                                        a[T][4 * pg + 2 * o] = lds32_lut(__byte_perm(ab[o], lut_v, sel[T]));
+                                        a[T][4 * pg + 2 * o + 1] = lds32_lut(__byte_perm(cd[o], lut_v, sel[T]));
+                                    } else {
+                                        a[T][4 * pg + 2 * o] = lds32_lut_residual(__byte_perm(ab[o], lut_r, sel[T]));
+                                        a[T][4 * pg + 2 * o + 1] = lds32_lut_residual(__byte_perm(cd[o], lut_r, sel[T]));
+                                    }
+                                }
+                            }
+                        }
+                        const uint32_t dst = tmem + quad + kXtColV + 64u * (uint32_t)half + 32u * (uint32_t)kk;
+                        tc_st_16x256b_x4(dst, a[0]);
+                        tc_st_16x256b_x4(dst + (16u << 16), a[1]);
+                        tc_wait_st();
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar(kXtVFull + kk));
+                    }
+                    if (ok && pass == 0) {      // does the block need its centroids' residuals?
+                        ok = wait_all(bar(kXtPReady), c & 1u);
+                        volatile int* pk = sh.peak[c & 1];
+                        if (ok && (pk[0] | pk[1] | pk[2] | pk[3]) != 0) passes = 2;
+                    }
+                }
+                __syncwarp();
+                if (ok && lane == 0) mbar_arrive(bar(kXtRawVFree + s));
+            }
+        }
+    } else if (wid >= 4 && wid < 8) {
+        // ======================= K: thread = key ===================================================
+        const int key = tid - 128;
+        const uint32_t lutk_lane = lut_addr + 8u * (uint32_t)(lane & 15);
+        bool ok = true;
+        while (ok && xt_next(p, walk, sg)) {
+            for (int b = 0; ok && kXtPages * b < sg.pages; ++b, ++c) {
+                const int s = (int)(c % STAGES);
+                if (!(ok = wait_all(bar(kXtRawKFull + s), (c / STAGES) & 1u))) break;
+                const uint32_t rowp = raw_k(s) + (uint32_t)key * kTq4RowBytes;
+                sh.k_scale[c & 1][key] = make_float2(__half2float(__ushort_as_half((unsigned short)(lds32(rowp) & 0xffffu))),
+                                                     __half2float(__ushort_as_half((unsigned short)(lds32(rowp + 64) >> 16))));
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar(kXtKScale + (int)(c & 1)));
+#pragma unroll 1
+                for (int gr = 0; gr < 8; ++gr) {
+                    const uint32_t slot = (uint32_t)gr & (kXtKRing - 1), lap = 2u * c + ((uint32_t)gr >> 2);
+                    uint32_t x[5], w[4];
+                    const uint32_t at = rowp + 16u * (uint32_t)(gr & 3) + (gr >= 4 ? 68u : 0u);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) x[i] = lds32(at + 4u * i);
+                    x[4] = gr < 4 ? lds32(at + 16u) : 0u;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) w[i] = gr < 4 ? __funnelshift_r(x[i], x[i + 1], 16) : x[i];   // half 0 starts at byte 2
+                    uint32_t hi[16], lo[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        const uint2 e = lds64_lut(__byte_perm(w[i >> 2], lutk_lane, 0x7604 + ((i & 3) << 4)));
+                        hi[i] = e.x;
+                        lo[i] = e.y;
+                    }
+                    if (!(ok = wait_all(bar(kXtKEmpty + (int)slot), (lap & 1u) ^ 1u))) break;
+                    tc_st16(tmem + quad + kXtColK + 32u * slot, hi);
+                    tc_st16(tmem + quad + kXtColK + 32u * slot + 16u, lo);
+                    tc_wait_st();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar(kXtKFull + (int)slot));
+                }
+                __syncwarp();
+                if (ok && lane == 0) mbar_arrive(bar(kXtRawKFree + s));
+            }
+        }
+    } else if (wid < 4) {
