@@ -472,3 +472,198 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
             }
         }
     } else if (wid < 4) {
+        // ======================= softmax: thread = key =============================================
+        const uint32_t t_s = tmem + quad + kXtColS, t_o = tmem + quad + kXtColO;
+        float* partials = reinterpret_cast<float*>(p.scratch + plan_bytes(p.batch.num_reqs));
+        bool ok = true;
+        while (ok && xt_next(p, walk, sg)) {
+            const ReqGeom g = load_req(p.batch, sg.r);
+            if (tid < R) {
+                const int row = sg.group * R + tid, q_off = row / p.gqa;
+                const bool valid = row < g.q_len * p.gqa && (p.batch.valid_token_mask == nullptr || p.batch.valid_token_mask[g.q_start + q_off] != 0);
+                sh.row_max[tid] = valid ? row_max_kv(p.batch, g, q_off) : -1;
+                sh.row_min[tid] = valid ? row_min_kv(p.batch, g, q_off) : 0x7fffffff;
+                sh.m_ref[tid] = -1e30f;
+                sh.mass[tid] = 0.0f;
+            }
+            xt_sync();
+            int safe_lo = 0, safe_hi = 0x7fffffff;      // keys every valid row can see
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                if (sh.row_max[i] >= 0) {
+                    safe_lo = max(safe_lo, sh.row_min[i]);
+                    safe_hi = min(safe_hi, sh.row_max[i]);
+                }
+            }
+            float l[R];
+#pragma unroll
+            for (int i = 0; i < R; ++i) l[i] = 0.0f;
+            // mass of every row over all keys so far, into sh.mass (a lower bound from then on)
+            auto reduce_mass = [&]() {
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    float t = l[i];
+#pragma unroll
+                    for (int d = 16; d > 0; d >>= 1) t += __shfl_xor_sync(0xffffffffu, t, d);
+                    if (lane == 0) sh.red[wid][i] = t;
+                }
+                xt_sync();
+                if (tid < R) sh.mass[tid] = (sh.red[0][tid] + sh.red[1][tid]) + (sh.red[2][tid] + sh.red[3][tid]);
+                xt_sync();
+            };
+            const int nblocks = (sg.pages + kXtPages - 1) / kXtPages;
+#pragma unroll 1
+            for (int b = 0; b < nblocks; ++b, ++c) {
+                if (!(ok = wait_all(bar(kXtKScale + (int)(c & 1)), (c >> 1) & 1u))) break;
+                const float2 dk = sh.k_scale[c & 1][tid];
+                if (!(ok = wait_all(bar(kXtSReady), c & 1u))) break;
+                tc_fence_after();
+                float sc[R];
+#pragma unroll
+                for (int i0 = 0; i0 < R; i0 += 8) {
+                    uint32_t h0[8], l0[8], h1[8], l1[8];
+                    tc_ld8(h0, t_s + (uint32_t)i0);
+                    tc_ld8(l0, t_s + (uint32_t)(R + i0));
+                    tc_ld8(h1, t_s + (uint32_t)(N + i0));
+                    tc_ld8(l1, t_s + (uint32_t)(N + R + i0));
+                    tc_wait_ld();
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        sc[i0 + i] = dk.x * (__uint_as_float(h0[i]) + __uint_as_float(l0[i])) + dk.y * (__uint_as_float(h1[i]) + __uint_as_float(l1[i]));
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar(kXtSFree));
+                const int kv_base = (sg.pg0 + kXtPages * b) << 4;
+                const int last = (min(kXtPages, sg.pages - kXtPages * b) << 4) - 1;       // keys past it are not in the block
+                const bool full = kv_base >= safe_lo && kv_base + kXtKeys - 1 <= safe_hi && last == kXtKeys - 1;
+                const int pos = kv_base + tid;
+                if (!full) {
+#pragma unroll
+                    for (int i = 0; i < R; ++i) {
+                        if (tid > last || pos < sh.row_min[i] || pos > sh.row_max[i]) sc[i] = -1e30f;
+                    }
+                }
+                bool ahead = false;
+#pragma unroll
+                for (int i = 0; i < R; ++i) ahead = ahead || sc[i] > sh.m_ref[i] + kXtLag;
+                const bool moved = xt_any(ahead);
+                if (moved) {      // the reference maximum of some row moves: take the block's maxima
+#pragma unroll
+                    for (int i = 0; i < R; ++i) {
+                        float t = sc[i];
+#pragma unroll
+                        for (int d = 16; d > 0; d >>= 1) t = fmaxf(t, __shfl_xor_sync(0xffffffffu, t, d));
+                        if (lane == 0) sh.red[wid][i] = t;
+                    }
+                    xt_sync();
+                    if (tid < R) {
+                        const float old = sh.m_ref[tid];
+                        const float now = fmaxf(fmaxf(fmaxf(sh.red[0][tid], sh.red[1][tid]), fmaxf(sh.red[2][tid], sh.red[3][tid])), old);
+                        const float a = ex2(old - now);      // 0 when nothing was visible before
+                        sh.m_ref[tid] = now;
+                        sh.alpha[tid] = a;
+                        sh.mass[tid] *= a;
+                    }
+                    xt_sync();
+#pragma unroll
+                    for (int i = 0; i < R; ++i) l[i] *= sh.alpha[i];
+                }
+                if (!(ok = wait_all(bar(kXtVScale + (int)(c & 1)), (c >> 1) & 1u))) break;
+                float2 dv = sh.v_scale[c & 1][tid];
+                // P and O are in use until the output product of the block before has completed
+                if (c > 0 && !(ok = wait_all(bar(kXtPvDone), (c - 1) & 1u))) break;
+                if (moved && b > 0) {
+                    tc_fence_after();
+#pragma unroll 1
+                    for (int h = 0; h < 2; ++h) {
+#pragma unroll
+                        for (int i0 = 0; i0 < N; i0 += 8) {
+                            uint32_t o[8];
+                            tc_ld8(o, t_o + (uint32_t)(h * N + i0));
+                            tc_wait_ld();
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * sh.alpha[(i0 + i) % R]);
+                            tc_st8(t_o + (uint32_t)(h * N + i0), o);
+                        }
+                    }
+                    tc_wait_st();
+                    tc_fence_before();
+                }
+                // weights; a key no row can see may hold never-written bytes, its scale must not meet a zero weight
+                bool peaked = false, seen = false;
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    float w = ex2(sc[i] - (sh.m_ref[i] + kXtLag));
+                    if (!full && sc[i] <= -1e30f) w = 0.0f;      // (a row that has seen nothing yet: masked scores equal its maximum)
+                    l[i] += w;
+                    // a key with more than kPeakedWeight of a row's mass so far (of what is known of it)
+                    peaked = peaked || w > kPeakedWeight * sh.mass[i];
+                    seen = seen || w != 0.0f;
+                    sc[i] = w;
+                }
+                if (!seen) dv = make_float2(0.0f, 0.0f);
+                const uint32_t at = p_t + (uint32_t)(tid >> 6) * (uint32_t)(N * 128) + 2u * (uint32_t)(tid & 7);
+                const uint32_t chunk = (uint32_t)(tid & 63) >> 3;
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    const uint32_t a = at + (uint32_t)i * 128u + ((chunk ^ (uint32_t)(i & 7)) << 4);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const float x = sc[i] * (h ? dv.y : dv.x);
+                        const __half xh = __float2half_rn(x);
+                        const __half xl = __float2half_rn(x - __half2float(xh));
+                        sts16(a + (uint32_t)h * kPBytes, (uint32_t)__half_as_ushort(xh));
+                        sts16(a + (uint32_t)h * kPBytes + (uint32_t)R * 128u, (uint32_t)__half_as_ushort(xl));
+                    }
+                }
+                const bool any_peak = __any_sync(0xffffffffu, peaked);
+                if (lane == 0) sh.peak[c & 1][wid] = any_peak ? 1 : 0;
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar(kXtPReady));
+                if (b < 2 || (b & 3) == 3) reduce_mass();
+            }
+            if (!ok) break;
+            // ---- the item's share is done: write the partial (lane = channel) ----------------------
+            reduce_mass();
+            if (!(ok = wait_all(bar(kXtPvDone), (c - 1) & 1u))) break;
+            tc_fence_after();
+            if (sg.slot < p.max_slots) {
+                float* dst = partials + (size_t)sg.slot * (R * kHeadDim + 2 * R);
+                // TMEM lane 32 q + 16 T + gid (+ 8): code word 4 q + gid / 2, channels 2 (2 (gid & 1) + T) (+ 1) of it
+                const int T = lane >> 4, gid = lane & 7, odd = (lane >> 3) & 1;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int ch = vword_col(h, 4 * (wid & 3) + (gid >> 1), 2 * (2 * (gid & 1) + T) + odd);
+#pragma unroll
+                    for (int i0 = 0; i0 < R; i0 += 8) {
+                        uint32_t a[8], b8[8];
+                        tc_ld8(a, t_o + (uint32_t)(h * N + i0));
+                        tc_ld8(b8, t_o + (uint32_t)(h * N + R + i0));
+                        tc_wait_ld();
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) dst[(i0 + i) * kHeadDim + ch] = __uint_as_float(a[i]) + __uint_as_float(b8[i]);
+                    }
+                }
+                if (tid < R) {
+                    dst[R * kHeadDim + tid] = sh.m_ref[tid] + kXtLag;
+                    dst[R * kHeadDim + R + tid] = sh.mass[tid];
+                }
+            }
+            tc_fence_before();
+            xt_sync();
+        }
+        if (!ok) *aborted = 1u;
+    }
+
+    __syncthreads();
+    if (wid == 0) {
+        tc_fence_after();
+        tc_dealloc(tmem, 512);
+    }
+    if (*aborted != 0u && tid == 0) atomicOr(&hdr->status, 1);
+}
+
+}  // namespace w34
