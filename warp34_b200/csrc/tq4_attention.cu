@@ -571,6 +571,8 @@ struct StreamParams {
     int q_floor = 0;       // query fragments for the exact build: hi rounded down, residual bytes 0..255
     int rows_from_first_token = 0;   // merge: block x is row x of the batch (0) or row x counted from the batch's first token (1)
     int keep_status = 0;             // plan: OR into the status word instead of clearing it (second and later passes)
+    int query_tiles = 0;             // qfrag holds tcgen05 operand tiles of rows_per_group rows instead of fragments
+    int min_units = kMinUnitsPerWarp;    // smallest share of a worker
     const int32_t* sel_phys = nullptr;
     const int32_t* sel_logical = nullptr;
     const int32_t* num_selected = nullptr;
@@ -603,6 +605,7 @@ __device__ __forceinline__ int32_t* plan_array(uint8_t* scratch, int which, int 
 constexpr int kQFragWords = 49;
 __host__ __device__ inline size_t qfrag_item_bytes() { return (size_t)kQFragWords * 32 * sizeof(uint32_t); }
 __device__ void qprep_block(const StreamParams& p, int idx);
+__device__ void xt_prepare_query(const StreamParams& p, int idx);
 constexpr int kPlanThreads = 32 * kRowsPerGroup;  // the query-fragment blocks use one warp per query row
 
 // Block 0 plans the split.  Blocks 1.. (one-warp items only) each rotate and scale the query rows
@@ -613,7 +616,8 @@ __global__ void __launch_bounds__(kPlanThreads) tq4_attention_plan_kernel(const 
     grid_dependency_wait();
     grid_launch_dependents();
     if (blockIdx.x > 0) {
-        qprep_block(p, (int)blockIdx.x - 1);
+        if (p.query_tiles) xt_prepare_query(p, (int)blockIdx.x - 1);
+        else qprep_block(p, (int)blockIdx.x - 1);
         return;
     }
     if (threadIdx.x >= 32) return;
@@ -681,7 +685,7 @@ __global__ void __launch_bounds__(kPlanThreads) tq4_attention_plan_kernel(const 
         h->total_items = item_carry;
         h->total_units = unit_carry;
         int per = (unit_carry + p.num_warps - 1) / (p.num_warps > 0 ? p.num_warps : 1);
-        if (unit_carry > 0 && per < kMinUnitsPerWarp) per = kMinUnitsPerWarp;
+        if (unit_carry > 0 && per < p.min_units) per = p.min_units;
         h->units_per_warp = per;
     }
 }
@@ -1832,6 +1836,7 @@ W34_BOUNDS_HOST_HOOKS(attention)
 #include "tq4_stream_exact.cuh"
 #include "tq4_prefill_tc.cuh"
 #include "prefill_pair.cuh"
+#include "tq4_stream_tc.cuh"
 namespace w34 {
 
 // Row triple written when the caller merges across page shards itself: 256 un-normalised
@@ -2201,6 +2206,12 @@ static DeviceInfo* device_info(int* rc) {
         *rc = (int)cudaFuncSetAttribute(tq4_attention_prefill_tc_kernel,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmemBytes);
         if (*rc != 0) return nullptr;
+        *rc = (int)cudaFuncSetAttribute(tq4_attention_stream_tc_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+        if (*rc != 0) return nullptr;
+        *rc = (int)cudaFuncSetAttribute(tq4_attention_stream_tc_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+        if (*rc != 0) return nullptr;
+        *rc = (int)cudaFuncSetAttribute(tq4_attention_stream_tc_kernel<24>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+        if (*rc != 0) return nullptr;
         d->smem_optin = optin;
         d->sm_count = sms;
         d->configured = true;
@@ -2258,6 +2269,25 @@ static size_t stream_scratch_bytes(const warp34_kv_layer_layout* l, const warp34
     const long long slots = workers + items_bound(l, b, hq, rpg);
     const size_t qfrag = (nt == 1) ? (size_t)qfrag_items(l, b, gqa) * qfrag_item_bytes() : 0;
     return plan_bytes(b->num_reqs) + (size_t)slots * (size_t)(rpg * kHeadDim + 2 * rpg) * sizeof(float) + qfrag;
+}
+
+// The tcgen05 stream kernel: rows per item (8, 16 or 24: all of a request's rows per kv head, 0: too many) and its workspace.
+static int xt_rows(const warp34_attention_batch* b, int gqa) {
+    const long long rows = (long long)(b->max_q_len > 0 ? b->max_q_len : 1) * gqa;
+    return rows <= 8 ? 8 : rows <= 16 ? 16 : rows <= 24 ? 24 : 0;
+}
+static size_t xt_scratch_bytes(const warp34_kv_layer_layout* l, const warp34_attention_batch* b, int hq, int rows, int grid) {
+    return plan_bytes(b->num_reqs) + ((size_t)grid + (size_t)items_bound(l, b, hq, rows)) * (size_t)(rows * kHeadDim + 2 * rows) * sizeof(float) +
+           (size_t)b->num_reqs * l->local_kv_heads * xt_query_bytes(rows);
+}
+// It is taken where the CTAs' shares are long enough: a CTA needs a few blocks of 128 keys to fill its roles, and a share below
+// that leaves the small-step kernel's 8 workers per SM ahead.  max_seq_len is a hint (0: unknown).
+static bool takes_tiles(const warp34_exec* ex, const warp34_kv_layer_layout* l, const warp34_attention_batch* b, int hq, int rows, int sms) {
+    if (rows == 0 || b->max_seq_len <= 0) return false;
+    const long long pages = ((long long)b->max_seq_len + kPageTokens - 1) / kPageTokens;
+    const long long items = (long long)b->num_reqs * l->local_kv_heads;
+    if (items * pages < (long long)kXtMinPages * sms || items * b->max_blocks_per_req >= 0x7fffffffll) return false;
+    return ex->scratch_size >= xt_scratch_bytes(l, b, hq, rows, sms);
 }
 
 // ---- a batch in several passes ------------------------------------------------------------------
@@ -2405,7 +2435,10 @@ extern "C" size_t warp34_paged_attention_scratch_bytes(const warp34_kv_layer_lay
     const size_t fast = w34::stream_scratch_bytes(layout, batch, num_q_heads, true,
                                                   (long long)sms * (nt_fast == 1 ? w34::kFastWarps : w34::kTeams));
     const size_t exact = w34::stream_scratch_bytes(layout, batch, num_q_heads, false, (long long)sms * w34::kExactWarps);
-    return fast > exact ? fast : exact;
+    const int rows = w34::xt_rows(batch, gqa);
+    const size_t tiles = rows != 0 ? w34::xt_scratch_bytes(layout, batch, num_q_heads, rows, sms) : 0;
+    const size_t most = fast > exact ? fast : exact;
+    return most > tiles ? most : tiles;
 }
 
 namespace w34 {
@@ -2522,6 +2555,41 @@ static int launch_attention(const warp34_exec* ex, const warp34_kv_layer_layout*
                            stream_layout_ok(layout) && ex->scratch_ptr != 0 && (ex->scratch_ptr & 15u) == 0u &&
                            batch->max_blocks_per_req > 0;
     if (nt == 1 && qfrag_items(layout, batch, gqa) > 0x3fffffffll) return (int)cudaErrorInvalidValue;
+
+    const int tile_rows = xt_rows(batch, gqa);
+    if (stream_ok && !fast && force < 0 && takes_tiles(ex, layout, batch, num_q_heads, tile_rows, dev->sm_count)) {
+        cudaStream_t st = (cudaStream_t)ex->stream;
+        const long long items = items_bound(layout, batch, num_q_heads, tile_rows);
+        const long long q_items = (long long)batch->num_reqs * layout->local_kv_heads;
+        StreamParams p;
+        p.layout = *layout;
+        p.batch = *batch;
+        p.q_in = q_in;
+        p.attn_out = attn_out;
+        p.io_bf16 = io_bf16;
+        p.triple_out = triple_out;
+        p.scratch = reinterpret_cast<uint8_t*>((uintptr_t)ex->scratch_ptr);
+        p.num_q_heads = num_q_heads;
+        p.gqa = gqa;
+        p.num_warps = dev->sm_count;
+        p.max_slots = (int)(dev->sm_count + items);
+        p.rows_per_group = tile_rows;
+        p.q_scale = batch->sm_scale * 1.4426950408889634f / kLutScale;
+        p.natural = 0;
+        p.og = og;
+        p.qfrag = reinterpret_cast<uint32_t*>(p.scratch + plan_bytes(batch->num_reqs) + (size_t)p.max_slots * (size_t)(tile_rows * kHeadDim + 2 * tile_rows) * sizeof(float));
+        p.smem_bytes = (uint32_t)dev->smem_optin;
+        p.q_groups_max = 1;
+        p.query_tiles = 1;
+        p.min_units = kXtPages;
+        rc = launch_behind(tq4_attention_plan_kernel, 1 + (unsigned)q_items, kPlanThreads, 0, st, p);
+        if (rc != 0) return rc;
+        auto* kernel = tile_rows == 8 ? tq4_attention_stream_tc_kernel<8> : tile_rows == 16 ? tq4_attention_stream_tc_kernel<16> : tq4_attention_stream_tc_kernel<24>;
+        rc = launch_behind(kernel, (unsigned)dev->sm_count, kXtThreads, (size_t)dev->smem_optin, st, p);
+        if (rc != 0) return rc;
+        const long long rows = (long long)batch->total_tokens * num_q_heads;
+        return triple_out != nullptr ? launch_merge<true>(p, rows, st) : launch_merge<false>(p, rows, st);
+    }
 
     // Worker slots the workspace leaves for a batch of `reqs` requests with at most `tokens` query tokens
     // (-1: its unit count does not fit 32 bits).  Each of its items needs a slot and, one-warp items, a set

@@ -24,6 +24,7 @@ constexpr int kXtKeys = 128, kXtPages = kXtKeys / kPageTokens;
 constexpr int kXtWarps = 20, kXtThreads = kXtWarps * 32;      // the last warp only fills the fourth quadrant
 constexpr uint32_t kXtRun = (uint32_t)kXtPages * kTq4PageHeadBytes;       // 16896: K or V of a block
 constexpr uint32_t kXtColK = 0, kXtColV = 128, kXtColS = 256, kXtColO = 384;
+constexpr int kXtMinPages = 24;                               // per SM, see takes_tiles
 constexpr int kXtKRing = 4;                                   // granules of 32 channels: 16 columns of values, 16 of residuals
 constexpr float kXtLag = 3.0f;                                // log2 units the reference maximum may lag; P is carried times 2^-3
 
@@ -383,7 +384,6 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
 #pragma unroll 1
                     for (int kk = 0; kk < 2; ++kk) {
                         uint32_t a[2][16];
-                        if (!(ok = wait_all(bar(kXtVEmpty + kk), (laps & 1u) ^ 1u))) break;
 #pragma unroll
                         for (int pg = 0; pg < 4; ++pg) {
                             const uint32_t at = rows + (uint32_t)(4 * kk + pg) * kTq4PageHeadBytes;
@@ -410,6 +410,7 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                                 }
                             }
                         }
+                        if (!(ok = wait_all(bar(kXtVEmpty + kk), (laps & 1u) ^ 1u))) break;
                         const uint32_t dst = tmem + quad + kXtColV + 64u * (uint32_t)half + 32u * (uint32_t)kk;
                         tc_st_16x256b_x4(dst, a[0]);
                         tc_st_16x256b_x4(dst + (16u << 16), a[1]);
@@ -475,8 +476,10 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
         // ======================= softmax: thread = key =============================================
         const uint32_t t_s = tmem + quad + kXtColS, t_o = tmem + quad + kXtColO;
         float* partials = reinterpret_cast<float*>(p.scratch + plan_bytes(p.batch.num_reqs));
-        bool ok = true;
-        while (ok && xt_next(p, walk, sg)) {
+        // The four warps share barriers, so that one whose wait gave up carries on (nothing it reads can be out of bounds) and
+        // all leave together behind a vote at the end of a segment; no wait after the first that gave up takes any time.
+        bool failed = false;
+        while (xt_next(p, walk, sg)) {
             const ReqGeom g = load_req(p.batch, sg.r);
             if (tid < R) {
                 const int row = sg.group * R + tid, q_off = row / p.gqa;
@@ -514,9 +517,9 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
             const int nblocks = (sg.pages + kXtPages - 1) / kXtPages;
 #pragma unroll 1
             for (int b = 0; b < nblocks; ++b, ++c) {
-                if (!(ok = wait_all(bar(kXtKScale + (int)(c & 1)), (c >> 1) & 1u))) break;
+                bool bad = *aborted != 0u || !wait_all(bar(kXtKScale + (int)(c & 1)), (c >> 1) & 1u);
                 const float2 dk = sh.k_scale[c & 1][tid];
-                if (!(ok = wait_all(bar(kXtSReady), c & 1u))) break;
+                bad = bad || !wait_all(bar(kXtSReady), c & 1u);
                 tc_fence_after();
                 float sc[R];
 #pragma unroll
@@ -570,10 +573,10 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
 #pragma unroll
                     for (int i = 0; i < R; ++i) l[i] *= sh.alpha[i];
                 }
-                if (!(ok = wait_all(bar(kXtVScale + (int)(c & 1)), (c >> 1) & 1u))) break;
+                bad = bad || !wait_all(bar(kXtVScale + (int)(c & 1)), (c >> 1) & 1u);
                 float2 dv = sh.v_scale[c & 1][tid];
                 // P and O are in use until the output product of the block before has completed
-                if (c > 0 && !(ok = wait_all(bar(kXtPvDone), (c - 1) & 1u))) break;
+                bad = bad || (c > 0 && !wait_all(bar(kXtPvDone), (c - 1) & 1u));
                 if (moved && b > 0) {
                     tc_fence_after();
 #pragma unroll 1
@@ -618,6 +621,7 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                         sts16(a + (uint32_t)h * kPBytes + (uint32_t)R * 128u, (uint32_t)__half_as_ushort(xl));
                     }
                 }
+                if (bad) failed = true;
                 const bool any_peak = __any_sync(0xffffffffu, peaked);
                 if (lane == 0) sh.peak[c & 1][wid] = any_peak ? 1 : 0;
                 fence_proxy_async();
@@ -625,10 +629,9 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                 if (lane == 0) mbar_arrive(bar(kXtPReady));
                 if (b < 2 || (b & 3) == 3) reduce_mass();
             }
-            if (!ok) break;
             // ---- the item's share is done: write the partial (lane = channel) ----------------------
             reduce_mass();
-            if (!(ok = wait_all(bar(kXtPvDone), (c - 1) & 1u))) break;
+            if (failed || !wait_all(bar(kXtPvDone), (c - 1) & 1u)) failed = true;
             tc_fence_after();
             if (sg.slot < p.max_slots) {
                 float* dst = partials + (size_t)sg.slot * (R * kHeadDim + 2 * R);
@@ -653,9 +656,8 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                 }
             }
             tc_fence_before();
-            xt_sync();
+            if (xt_any(failed)) break;
         }
-        if (!ok) *aborted = 1u;
     }
 
     __syncthreads();
