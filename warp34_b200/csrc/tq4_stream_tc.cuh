@@ -21,7 +21,7 @@
 namespace w34 {
 
 constexpr int kXtKeys = 128, kXtPages = kXtKeys / kPageTokens;
-constexpr int kXtWarps = 20, kXtThreads = kXtWarps * 32;      // the last warp only fills the fourth quadrant
+constexpr int kXtWarps = 28, kXtThreads = kXtWarps * 32;      // the last warp is idle
 constexpr uint32_t kXtRun = (uint32_t)kXtPages * kTq4PageHeadBytes;       // 16896: K or V of a block
 constexpr uint32_t kXtColK = 0, kXtColV = 128, kXtColS = 256, kXtColO = 384;
 constexpr int kXtMinPages = 24;                               // per SM, see takes_tiles
@@ -34,9 +34,9 @@ __host__ __device__ constexpr uint32_t xt_query_bytes(int rows) { return 2u * (u
 struct XtShared {
     float2 k_scale[2][kXtKeys], v_scale[2][kXtKeys];
     float m_ref[24], alpha[24], mass[24];
-    float red[4][24];
+    float red[4][24];                // [warp of the part][row]
     int row_min[24], row_max[24];
-    __align__(16) int peak[2][4];
+    int peak[2];               // of the block's parity: some key has a large weight
     uint32_t tmem;
     uint32_t aborted;
     uint64_t bars[48];
@@ -46,13 +46,13 @@ enum { kXtRawKFull = 0, kXtRawKFree = 4, kXtRawVFull = 8, kXtRawVFree = 12, kXtK
        kXtDrain = kXtVScale + 2, kXtBarCount };
 static_assert(kXtBarCount <= 48, "barrier slots");
 
-__device__ __forceinline__ void tc_ld8(uint32_t (&r)[8], uint32_t taddr) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+__device__ __forceinline__ void tc_ld4(uint32_t (&r)[4], uint32_t taddr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
 }
-__device__ __forceinline__ void tc_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                 :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+__device__ __forceinline__ void tc_st4(uint32_t taddr, const uint32_t (&r)[4]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};"
+                 :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
 }
 // 16 lanes x 256 bits, four times: registers 4 i + {0, 1} go to lane t / 4, columns 8 i + 2 (t % 4) + {0, 1}; 4 i + {2, 3} eight
 // lanes further (t: thread of the warp).
@@ -60,12 +60,12 @@ __device__ __forceinline__ void tc_st_16x256b_x4(uint32_t taddr, const uint32_t 
     asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
                  :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
-// Barrier of the four softmax warps.
-__device__ __forceinline__ void xt_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
-__device__ __forceinline__ bool xt_any(bool x) {
+// Barrier of the four warps of a softmax part.
+__device__ __forceinline__ void xt_sync(int part) { asm volatile("bar.sync %0, 128;" :: "r"(1 + part) : "memory"); }
+__device__ __forceinline__ bool xt_any(bool x, int part) {
     uint32_t r;
-    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
-                 : "=r"(r) : "r"((uint32_t)x) : "memory");
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, %2, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(r) : "r"((uint32_t)x), "r"(1 + part) : "memory");
     return r != 0;
 }
 
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(bar(kXtRawKFull + s), 1u);
-            mbar_init(bar(kXtRawKFree + s), 4u);
+            mbar_init(bar(kXtRawKFree + s), 8u);
             mbar_init(bar(kXtRawVFull + s), 1u);
             mbar_init(bar(kXtRawVFree + s), 8u);
         }
@@ -190,10 +190,11 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
             mbar_init(bar(kXtVScale + s), 8u);
         }
         mbar_init(bar(kXtSReady), 1u);
-        mbar_init(bar(kXtSFree), 4u);
-        mbar_init(bar(kXtPReady), 4u);
+        mbar_init(bar(kXtSFree), 8u);
+        mbar_init(bar(kXtPReady), 8u);
         mbar_init(bar(kXtPvDone), 1u);
         mbar_init(bar(kXtDrain), 2u);
+        sh.peak[0] = sh.peak[1] = 0;
         sh.aborted = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -222,7 +223,7 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
     XtSegment sg;
     uint32_t c = 0;                                       // blocks so far
 
-    if (wid == 16) {
+    if (wid == 24) {
         // ======================= raw pages and query rows ==========================================
         uint32_t seg = 0, k_issued = 0, v_issued = 0;
         bool ok = true;
@@ -273,7 +274,7 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
         for (uint32_t j = v_issued > STAGES ? v_issued - STAGES : 0; j < v_issued; ++j) (void)mbar_wait(bar(kXtRawVFull + (int)(j % STAGES)), (j / STAGES) & 1u);
         for (uint32_t j = seg > 2 ? seg - 2 : 0; j < seg; ++j) (void)mbar_wait(bar(kXtQFull + (int)(j & 1)), (j >> 1) & 1u);
         __syncwarp();
-    } else if (wid == 17) {
+    } else if (wid == 25) {
         // ======================= score products: one thread =======================================
         if (elect_one()) {
             constexpr uint32_t kIdesc = tc_idesc(kXtKeys, N, 0);
@@ -312,7 +313,7 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
         __syncwarp();
         (void)mbar_wait(bar(kXtDrain), 0u);
         __syncwarp();
-    } else if (wid == 18) {
+    } else if (wid == 26) {
         // ======================= output products: one thread =======================================
         if (elect_one()) {
             constexpr uint32_t kIdesc = tc_idesc(128, N, 0);
@@ -323,8 +324,7 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                 for (int b = 0; ok && kXtPages * b < sg.pages; ++b, ++c) {
                     ok = mbar_wait(bar(kXtPReady), c & 1u) && *aborted == 0u;
                     if (!ok) break;
-                    volatile int* pk = sh.peak[c & 1];
-                    const int passes = (pk[0] | pk[1] | pk[2] | pk[3]) != 0 ? 2 : 1;
+                    const int passes = *reinterpret_cast<volatile int*>(&sh.peak[c & 1]) == (int)c + 1 ? 2 : 1;
                     for (int pass = 0; pass < passes && ok; ++pass, ++laps) {
 #pragma unroll 1
                         for (int kk = 0; kk < 2 && ok; ++kk) {
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
         const int gid = lane >> 2, tig = lane & 3, half = (wid - 8) >> 2;
         const int vw = 4 * (wid & 3) + (gid >> 1);                           // this thread's code word of the half
         const uint32_t word_off = 4u * ((half ? 17u : 0u) + (uint32_t)vw);
-        const bool splice = half == 0 && vw == 0;                            // virtual word 0: (W0 >> 16) | (W16 << 16)
+        const bool splice_warp = half == 0 && (wid & 3) == 0;                // virtual word 0: (W0 >> 16) | (W16 << 16)
         const uint32_t lut_v = lut_addr + 128u + 4u * (uint32_t)lane, lut_r = lut_addr + 8u * (uint32_t)(lane & 15);
         // byte 2 (gid & 1) + T of the paired codes belongs to tile T
         const uint32_t sel[2] = {0x7604u + ((uint32_t)(2 * (gid & 1)) << 4), 0x7604u + ((uint32_t)(2 * (gid & 1) + 1) << 4)};
@@ -384,15 +384,25 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
 #pragma unroll 1
                     for (int kk = 0; kk < 2; ++kk) {
                         uint32_t a[2][16];
+                        uint32_t x[4][4];
 #pragma unroll
                         for (int pg = 0; pg < 4; ++pg) {
-                            const uint32_t at = rows + (uint32_t)(4 * kk + pg) * kTq4PageHeadBytes;
-                            uint32_t w[4];
 #pragma unroll
-                            for (int k = 0; k < 4; ++k) {
-                                w[k] = lds32(at + (uint32_t)k * kTq4RowBytes + word_off);
-                                if (splice) w[k] = (w[k] >> 16) | (lds32(at + (uint32_t)k * kTq4RowBytes + 64) << 16);
+                            for (int k = 0; k < 4; ++k) x[pg][k] = lds32(rows + (uint32_t)(4 * kk + pg) * kTq4PageHeadBytes + (uint32_t)k * kTq4RowBytes + word_off);
+                        }
+                        if (splice_warp) {
+#pragma unroll
+                            for (int pg = 0; pg < 4; ++pg) {
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) {
+                                    const uint32_t y = lds32(rows + (uint32_t)(4 * kk + pg) * kTq4PageHeadBytes + (uint32_t)k * kTq4RowBytes + 64u);
+                                    if (vw == 0) x[pg][k] = (x[pg][k] >> 16) | (y << 16);
+                                }
                             }
+                        }
+#pragma unroll
+                        for (int pg = 0; pg < 4; ++pg) {
+                            const uint32_t (&w)[4] = x[pg];
                             // byte t of ab -> (key 0, key 1) of channel 2 t (first) and 2 t + 1 (second); cd: keys 2 and 3
                             const uint32_t ab[2] = {(w[0] & 0x0f0f0f0fu) | ((w[1] << 4) & 0xf0f0f0f0u), ((w[0] >> 4) & 0x0f0f0f0fu) | (w[1] & 0xf0f0f0f0u)};
                             const uint32_t cd[2] = {(w[2] & 0x0f0f0f0fu) | ((w[3] << 4) & 0xf0f0f0f0u), ((w[2] >> 4) & 0x0f0f0f0fu) | (w[3] & 0xf0f0f0f0u)};
@@ -421,17 +431,16 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                     }
                     if (ok && pass == 0) {      // does the block need its centroids' residuals?
                         ok = wait_all(bar(kXtPReady), c & 1u);
-                        volatile int* pk = sh.peak[c & 1];
-                        if (ok && (pk[0] | pk[1] | pk[2] | pk[3]) != 0) passes = 2;
+                        if (ok && *reinterpret_cast<volatile int*>(&sh.peak[c & 1]) == (int)c + 1) passes = 2;
                     }
                 }
                 __syncwarp();
                 if (ok && lane == 0) mbar_arrive(bar(kXtRawVFree + s));
             }
         }
-    } else if (wid >= 4 && wid < 8) {
+    } else if (wid >= 16 && wid < 24) {
         // ======================= K: thread = key ===================================================
-        const int key = tid - 128;
+        const int part = (wid - 16) >> 2, key = tid & 127;          // part 0 takes the even granules, part 1 the odd ones
         const uint32_t lutk_lane = lut_addr + 8u * (uint32_t)(lane & 15);
         bool ok = true;
         while (ok && xt_next(p, walk, sg)) {
@@ -439,12 +448,14 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                 const int s = (int)(c % STAGES);
                 if (!(ok = wait_all(bar(kXtRawKFull + s), (c / STAGES) & 1u))) break;
                 const uint32_t rowp = raw_k(s) + (uint32_t)key * kTq4RowBytes;
-                sh.k_scale[c & 1][key] = make_float2(__half2float(__ushort_as_half((unsigned short)(lds32(rowp) & 0xffffu))),
-                                                     __half2float(__ushort_as_half((unsigned short)(lds32(rowp + 64) >> 16))));
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar(kXtKScale + (int)(c & 1)));
+                if (part == 0) {
+                    sh.k_scale[c & 1][key] = make_float2(__half2float(__ushort_as_half((unsigned short)(lds32(rowp) & 0xffffu))),
+                                                         __half2float(__ushort_as_half((unsigned short)(lds32(rowp + 64) >> 16))));
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar(kXtKScale + (int)(c & 1)));
+                }
 #pragma unroll 1
-                for (int gr = 0; gr < 8; ++gr) {
+                for (int gr = part; gr < 8; gr += 2) {
                     const uint32_t slot = (uint32_t)gr & (kXtKRing - 1), lap = 2u * c + ((uint32_t)gr >> 2);
                     uint32_t x[5], w[4];
                     const uint32_t at = rowp + 16u * (uint32_t)(gr & 3) + (gr >= 4 ? 68u : 0u);
@@ -472,66 +483,73 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                 if (ok && lane == 0) mbar_arrive(bar(kXtRawKFree + s));
             }
         }
-    } else if (wid < 4) {
-        // ======================= softmax: thread = key =============================================
-        const uint32_t t_s = tmem + quad + kXtColS, t_o = tmem + quad + kXtColO;
+    } else if (wid < 8) {
+        // ======================= softmax: thread = key, a part = half of the rows =============================================
+        constexpr int P = R / 2;
+        const int part = wid >> 2, row0 = part * P, key = tid & 127;
+        const uint32_t t_s = tmem + quad + kXtColS + (uint32_t)row0, t_o = tmem + quad + kXtColO + (uint32_t)row0;
+        float* m_ref = sh.m_ref + row0;      // this part's rows
+        float* alpha = sh.alpha + row0;
+        float* mass = sh.mass + row0;
+        int *row_min = sh.row_min + row0, *row_max = sh.row_max + row0;
+        float* red = &sh.red[0][row0];
         float* partials = reinterpret_cast<float*>(p.scratch + plan_bytes(p.batch.num_reqs));
         // The four warps share barriers, so that one whose wait gave up carries on (nothing it reads can be out of bounds) and
         // all leave together behind a vote at the end of a segment; no wait after the first that gave up takes any time.
         bool failed = false;
         while (xt_next(p, walk, sg)) {
             const ReqGeom g = load_req(p.batch, sg.r);
-            if (tid < R) {
-                const int row = sg.group * R + tid, q_off = row / p.gqa;
+            if (key < P) {
+                const int row = sg.group * R + row0 + key, q_off = row / p.gqa;
                 const bool valid = row < g.q_len * p.gqa && (p.batch.valid_token_mask == nullptr || p.batch.valid_token_mask[g.q_start + q_off] != 0);
-                sh.row_max[tid] = valid ? row_max_kv(p.batch, g, q_off) : -1;
-                sh.row_min[tid] = valid ? row_min_kv(p.batch, g, q_off) : 0x7fffffff;
-                sh.m_ref[tid] = -1e30f;
-                sh.mass[tid] = 0.0f;
+                row_max[key] = valid ? row_max_kv(p.batch, g, q_off) : -1;
+                row_min[key] = valid ? row_min_kv(p.batch, g, q_off) : 0x7fffffff;
+                m_ref[key] = -1e30f;
+                mass[key] = 0.0f;
             }
-            xt_sync();
+            xt_sync(part);
             int safe_lo = 0, safe_hi = 0x7fffffff;      // keys every valid row can see
 #pragma unroll
-            for (int i = 0; i < R; ++i) {
-                if (sh.row_max[i] >= 0) {
-                    safe_lo = max(safe_lo, sh.row_min[i]);
-                    safe_hi = min(safe_hi, sh.row_max[i]);
+            for (int i = 0; i < P; ++i) {
+                if (row_max[i] >= 0) {
+                    safe_lo = max(safe_lo, row_min[i]);
+                    safe_hi = min(safe_hi, row_max[i]);
                 }
             }
-            float l[R];
+            float l[P];
 #pragma unroll
-            for (int i = 0; i < R; ++i) l[i] = 0.0f;
+            for (int i = 0; i < P; ++i) l[i] = 0.0f;
             // mass of every row over all keys so far, into sh.mass (a lower bound from then on)
             auto reduce_mass = [&]() {
 #pragma unroll
-                for (int i = 0; i < R; ++i) {
+                for (int i = 0; i < P; ++i) {
                     float t = l[i];
 #pragma unroll
                     for (int d = 16; d > 0; d >>= 1) t += __shfl_xor_sync(0xffffffffu, t, d);
-                    if (lane == 0) sh.red[wid][i] = t;
+                    if (lane == 0) red[(wid & 3) * 24 + i] = t;
                 }
-                xt_sync();
-                if (tid < R) sh.mass[tid] = (sh.red[0][tid] + sh.red[1][tid]) + (sh.red[2][tid] + sh.red[3][tid]);
-                xt_sync();
+                xt_sync(part);
+                if (key < P) mass[key] = (red[0 + key] + red[24 + key]) + (red[48 + key] + red[72 + key]);
+                xt_sync(part);
             };
             const int nblocks = (sg.pages + kXtPages - 1) / kXtPages;
 #pragma unroll 1
             for (int b = 0; b < nblocks; ++b, ++c) {
                 bool bad = *aborted != 0u || !wait_all(bar(kXtKScale + (int)(c & 1)), (c >> 1) & 1u);
-                const float2 dk = sh.k_scale[c & 1][tid];
+                const float2 dk = sh.k_scale[c & 1][key];
                 bad = bad || !wait_all(bar(kXtSReady), c & 1u);
                 tc_fence_after();
-                float sc[R];
+                float sc[P];
 #pragma unroll
-                for (int i0 = 0; i0 < R; i0 += 8) {
-                    uint32_t h0[8], l0[8], h1[8], l1[8];
-                    tc_ld8(h0, t_s + (uint32_t)i0);
-                    tc_ld8(l0, t_s + (uint32_t)(R + i0));
-                    tc_ld8(h1, t_s + (uint32_t)(N + i0));
-                    tc_ld8(l1, t_s + (uint32_t)(N + R + i0));
+                for (int i0 = 0; i0 < P; i0 += 4) {
+                    uint32_t h0[4], l0[4], h1[4], l1[4];
+                    tc_ld4(h0, t_s + (uint32_t)i0);
+                    tc_ld4(l0, t_s + (uint32_t)(R + i0));
+                    tc_ld4(h1, t_s + (uint32_t)(N + i0));
+                    tc_ld4(l1, t_s + (uint32_t)(N + R + i0));
                     tc_wait_ld();
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
+                    for (int i = 0; i < 4; ++i) {
                         sc[i0 + i] = dk.x * (__uint_as_float(h0[i]) + __uint_as_float(l0[i])) + dk.y * (__uint_as_float(h1[i]) + __uint_as_float(l1[i]));
                     }
                 }
@@ -541,54 +559,54 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                 const int kv_base = (sg.pg0 + kXtPages * b) << 4;
                 const int last = (min(kXtPages, sg.pages - kXtPages * b) << 4) - 1;       // keys past it are not in the block
                 const bool full = kv_base >= safe_lo && kv_base + kXtKeys - 1 <= safe_hi && last == kXtKeys - 1;
-                const int pos = kv_base + tid;
+                const int pos = kv_base + key;
                 if (!full) {
 #pragma unroll
-                    for (int i = 0; i < R; ++i) {
-                        if (tid > last || pos < sh.row_min[i] || pos > sh.row_max[i]) sc[i] = -1e30f;
+                    for (int i = 0; i < P; ++i) {
+                        if (key > last || pos < row_min[i] || pos > row_max[i]) sc[i] = -1e30f;
                     }
                 }
                 bool ahead = false;
 #pragma unroll
-                for (int i = 0; i < R; ++i) ahead = ahead || sc[i] > sh.m_ref[i] + kXtLag;
-                const bool moved = xt_any(ahead);
+                for (int i = 0; i < P; ++i) ahead = ahead || sc[i] > m_ref[i] + kXtLag;
+                const bool moved = xt_any(ahead, part);
                 if (moved) {      // the reference maximum of some row moves: take the block's maxima
 #pragma unroll
-                    for (int i = 0; i < R; ++i) {
+                    for (int i = 0; i < P; ++i) {
                         float t = sc[i];
 #pragma unroll
                         for (int d = 16; d > 0; d >>= 1) t = fmaxf(t, __shfl_xor_sync(0xffffffffu, t, d));
-                        if (lane == 0) sh.red[wid][i] = t;
+                        if (lane == 0) red[(wid & 3) * 24 + i] = t;
                     }
-                    xt_sync();
-                    if (tid < R) {
-                        const float old = sh.m_ref[tid];
-                        const float now = fmaxf(fmaxf(fmaxf(sh.red[0][tid], sh.red[1][tid]), fmaxf(sh.red[2][tid], sh.red[3][tid])), old);
+                    xt_sync(part);
+                    if (key < P) {
+                        const float old = m_ref[key];
+                        const float now = fmaxf(fmaxf(fmaxf(red[0 + key], red[24 + key]), fmaxf(red[48 + key], red[72 + key])), old);
                         const float a = ex2(old - now);      // 0 when nothing was visible before
-                        sh.m_ref[tid] = now;
-                        sh.alpha[tid] = a;
-                        sh.mass[tid] *= a;
+                        m_ref[key] = now;
+                        alpha[key] = a;
+                        mass[key] *= a;
                     }
-                    xt_sync();
+                    xt_sync(part);
 #pragma unroll
-                    for (int i = 0; i < R; ++i) l[i] *= sh.alpha[i];
+                    for (int i = 0; i < P; ++i) l[i] *= alpha[i];
                 }
                 bad = bad || !wait_all(bar(kXtVScale + (int)(c & 1)), (c >> 1) & 1u);
-                float2 dv = sh.v_scale[c & 1][tid];
+                float2 dv = sh.v_scale[c & 1][key];
                 // P and O are in use until the output product of the block before has completed
                 bad = bad || (c > 0 && !wait_all(bar(kXtPvDone), (c - 1) & 1u));
                 if (moved && b > 0) {
                     tc_fence_after();
 #pragma unroll 1
-                    for (int h = 0; h < 2; ++h) {
+                    for (int q = 0; q < 4; ++q) {      // value and residual columns of both halves
 #pragma unroll
-                        for (int i0 = 0; i0 < N; i0 += 8) {
-                            uint32_t o[8];
-                            tc_ld8(o, t_o + (uint32_t)(h * N + i0));
+                        for (int i0 = 0; i0 < P; i0 += 4) {
+                            uint32_t o[4];
+                            tc_ld4(o, t_o + (uint32_t)(q * R + i0));
                             tc_wait_ld();
 #pragma unroll
-                            for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * sh.alpha[(i0 + i) % R]);
-                            tc_st8(t_o + (uint32_t)(h * N + i0), o);
+                            for (int i = 0; i < 4; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha[i0 + i]);
+                            tc_st4(t_o + (uint32_t)(q * R + i0), o);
                         }
                     }
                     tc_wait_st();
@@ -597,20 +615,20 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                 // weights; a key no row can see may hold never-written bytes, its scale must not meet a zero weight
                 bool peaked = false, seen = false;
 #pragma unroll
-                for (int i = 0; i < R; ++i) {
-                    float w = ex2(sc[i] - (sh.m_ref[i] + kXtLag));
+                for (int i = 0; i < P; ++i) {
+                    float w = ex2(sc[i] - (m_ref[i] + kXtLag));
                     if (!full && sc[i] <= -1e30f) w = 0.0f;      // (a row that has seen nothing yet: masked scores equal its maximum)
                     l[i] += w;
                     // a key with more than kPeakedWeight of a row's mass so far (of what is known of it)
-                    peaked = peaked || w > kPeakedWeight * sh.mass[i];
+                    peaked = peaked || w > kPeakedWeight * mass[i];
                     seen = seen || w != 0.0f;
                     sc[i] = w;
                 }
                 if (!seen) dv = make_float2(0.0f, 0.0f);
-                const uint32_t at = p_t + (uint32_t)(tid >> 6) * (uint32_t)(N * 128) + 2u * (uint32_t)(tid & 7);
-                const uint32_t chunk = (uint32_t)(tid & 63) >> 3;
+                const uint32_t at = p_t + (uint32_t)(key >> 6) * (uint32_t)(N * 128) + (uint32_t)row0 * 128u + 2u * (uint32_t)(key & 7);
+                const uint32_t chunk = ((uint32_t)(key & 63) >> 3) ^ (uint32_t)(row0 & 4);      // (row0 is a multiple of 4: row & 7 = (row0 & 4) ^ (i & 7))
 #pragma unroll
-                for (int i = 0; i < R; ++i) {
+                for (int i = 0; i < P; ++i) {
                     const uint32_t a = at + (uint32_t)i * 128u + ((chunk ^ (uint32_t)(i & 7)) << 4);
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
@@ -623,7 +641,7 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                 }
                 if (bad) failed = true;
                 const bool any_peak = __any_sync(0xffffffffu, peaked);
-                if (lane == 0) sh.peak[c & 1][wid] = any_peak ? 1 : 0;
+                if (any_peak && lane == 0) sh.peak[c & 1] = (int)c + 1;
                 fence_proxy_async();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar(kXtPReady));
@@ -641,22 +659,22 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                 for (int h = 0; h < 2; ++h) {
                     const int ch = vword_col(h, 4 * (wid & 3) + (gid >> 1), 2 * (2 * (gid & 1) + T) + odd);
 #pragma unroll
-                    for (int i0 = 0; i0 < R; i0 += 8) {
-                        uint32_t a[8], b8[8];
-                        tc_ld8(a, t_o + (uint32_t)(h * N + i0));
-                        tc_ld8(b8, t_o + (uint32_t)(h * N + R + i0));
+                    for (int i0 = 0; i0 < P; i0 += 4) {
+                        uint32_t a[4], b4[4];
+                        tc_ld4(a, t_o + (uint32_t)(h * N + i0));
+                        tc_ld4(b4, t_o + (uint32_t)(h * N + R + i0));
                         tc_wait_ld();
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) dst[(i0 + i) * kHeadDim + ch] = __uint_as_float(a[i]) + __uint_as_float(b8[i]);
+                        for (int i = 0; i < 4; ++i) dst[(row0 + i0 + i) * kHeadDim + ch] = __uint_as_float(a[i]) + __uint_as_float(b4[i]);
                     }
                 }
-                if (tid < R) {
-                    dst[R * kHeadDim + tid] = sh.m_ref[tid] + kXtLag;
-                    dst[R * kHeadDim + R + tid] = sh.mass[tid];
+                if (key < P) {
+                    dst[R * kHeadDim + row0 + key] = m_ref[key] + kXtLag;
+                    dst[R * kHeadDim + R + row0 + key] = mass[key];
                 }
             }
             tc_fence_before();
-            if (xt_any(failed)) break;
+            if (xt_any(failed, part)) break;
         }
     }
 
