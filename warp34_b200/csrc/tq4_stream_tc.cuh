@@ -33,7 +33,7 @@ __host__ __device__ constexpr uint32_t xt_query_bytes(int rows) { return 2u * (u
 
 struct XtShared {
     float2 k_scale[2][kXtKeys], v_scale[2][kXtKeys];
-    float m_ref[24], alpha[24], mass[24];
+    __align__(16) float m_ref[24], alpha[24], mass[24];
     float red[4][24];                // [warp of the part][row]
     int row_min[24], row_max[24];
     int peak[2];               // of the block's parity: some key has a large weight
@@ -60,6 +60,14 @@ __device__ __forceinline__ void tc_st_16x256b_x4(uint32_t taddr, const uint32_t 
     asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
                  :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
+// D (+)= A B with A in tensor memory, all output lanes.
+template <bool ACC>
+__device__ __forceinline__ void xt_mma(uint32_t d, uint32_t a, uint64_t b_desc, uint32_t idesc) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                 :: "r"(d), "r"(a), "l"(b_desc), "r"(idesc), "n"(ACC ? 1 : 0) : "memory");
+}
+// A descriptor like `like` with another start address (low word).
+__device__ __forceinline__ uint64_t xt_desc(uint32_t low, uint64_t like) { return (like & 0xffffffff00000000ull) | low; }
 // Barrier of the four warps of a softmax part.
 __device__ __forceinline__ void xt_sync(int part) { asm volatile("bar.sync %0, 128;" :: "r"(1 + part) : "memory"); }
 __device__ __forceinline__ bool xt_any(bool x, int part) {
@@ -159,7 +167,8 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
     volatile uint32_t* aborted = &sh.aborted;
     // Waits are bounded and warp-uniform; one that gives up ends every loop.
     auto wait_all = [&](uint32_t b, uint32_t parity) {
-        const bool ok = mbar_wait(b, parity) && *aborted == 0u;
+        if (__all_sync(0xffffffffu, mbar_try_wait(b, parity))) return true;
+        const bool ok = *aborted == 0u && mbar_wait(b, parity) && *aborted == 0u;
         if (__all_sync(0xffffffffu, ok)) return true;
         *aborted = 1u;
         return false;
@@ -275,81 +284,87 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
         for (uint32_t j = seg > 2 ? seg - 2 : 0; j < seg; ++j) (void)mbar_wait(bar(kXtQFull + (int)(j & 1)), (j >> 1) & 1u);
         __syncwarp();
     } else if (wid == 25) {
-        // ======================= score products: one thread =======================================
-        if (elect_one()) {
-            constexpr uint32_t kIdesc = tc_idesc(kXtKeys, N, 0);
-            const uint64_t desc_q[2] = {tc_smem_desc(q_t[0], 16u, 1024u), tc_smem_desc(q_t[1], 16u, 1024u)};
-            uint32_t seg = 0;
-            bool ok = true;
-            while (ok && xt_next(p, walk, sg)) {
-                ok = mbar_wait(bar(kXtQFull + (int)(seg & 1)), (seg >> 1) & 1u);
-                const uint64_t dq = (seg & 1) ? desc_q[1] : desc_q[0];
-                for (int b = 0; ok && kXtPages * b < sg.pages; ++b, ++c) {
-                    ok = mbar_wait(bar(kXtSFree), (c & 1u) ^ 1u);      // the scores of the block before are in registers
-#pragma unroll 1
-                    for (int gr = 0; gr < 8 && ok; ++gr) {
-                        const uint32_t slot = (uint32_t)gr & (kXtKRing - 1), lap = 2u * c + ((uint32_t)gr >> 2);
-                        ok = mbar_wait(bar(kXtKFull + (int)slot), lap & 1u) && *aborted == 0u;
-                        if (!ok) break;
+        // ======================= score products =====================================================
+        // An MMA of this size takes the tensor cores some 40 cycles, so that operands are kept where an issue needs no more than a
+        // few instructions: warp-uniform bases, everything else constant.
+        constexpr uint32_t kIdesc = tc_idesc(kXtKeys, N, 0);
+        const uint64_t desc_q0 = tc_smem_desc(q_t[0], 16u, 1024u), desc_q1 = tc_smem_desc(q_t[1], 16u, 1024u);
+        const uint32_t base = __shfl_sync(0xffffffffu, tmem, 0);
+        uint32_t seg = 0;
+        bool ok = true;
+        while (ok && xt_next(p, walk, sg)) {
+            ok = wait_all(bar(kXtQFull + (int)(seg & 1)), (seg >> 1) & 1u);
+            const uint64_t dq = xt_desc(__shfl_sync(0xffffffffu, (uint32_t)((seg & 1) ? desc_q1 : desc_q0), 0), desc_q0);
+            for (int b = 0; ok && kXtPages * b < sg.pages; ++b, ++c) {
+                ok = wait_all(bar(kXtSFree), (c & 1u) ^ 1u);      // the scores of the block before are in registers
+#pragma unroll
+                for (int gr = 0; gr < 8; ++gr) {
+                    ok = ok && wait_all(bar(kXtKFull + (gr & 3)), (uint32_t)(gr >> 2));      // fills 2 c + (gr >> 2)
+                    if (ok && elect_one()) {
                         tc_fence_after();
-                        const uint32_t d = tmem + kXtColS + (uint32_t)(gr >> 2) * (uint32_t)N, a = tmem + kXtColK + 32u * slot;
 #pragma unroll
                         for (int ks = 0; ks < 2; ++ks) {
                             // channels 32 gr + 16 ks: block of 64 gr >> 1, 32 bytes per k-step
                             const uint64_t bq = dq + (uint64_t)((gr >> 1) * (N * 128 / 16) + 2 * (2 * (gr & 1) + ks));
-                            tc_mma_f16_ts(d, a + 8u * (uint32_t)ks, bq, kIdesc, ((gr & 3) || ks) ? 1u : 0u);
-                            tc_mma_f16_ts(d, a + 16u + 8u * (uint32_t)ks, bq, kIdesc, 1u);
+                            const uint32_t d = base + kXtColS + (uint32_t)((gr >> 2) * N), a = base + kXtColK + (uint32_t)(32 * (gr & 3) + 8 * ks);
+                            if ((gr & 3) || ks) xt_mma<true>(d, a, bq, kIdesc);
+                            else xt_mma<false>(d, a, bq, kIdesc);
+                            xt_mma<true>(d, a + 16u, bq, kIdesc);
                         }
-                        tc_commit(bar(kXtKEmpty + (int)slot));
+                        tc_commit(bar(kXtKEmpty + (gr & 3)));
+                        if (gr == 7) tc_commit(bar(kXtSReady));
                     }
-                    if (ok) tc_commit(bar(kXtSReady));
+                    __syncwarp();
                 }
-                if (ok) tc_commit(bar(kXtQFree + (int)(seg & 1)));
-                ++seg;
             }
-            if (!ok) *aborted = 1u;
-            tc_commit(bar(kXtDrain));      // nothing may be in flight when the CTA leaves
+            if (ok && elect_one()) tc_commit(bar(kXtQFree + (int)(seg & 1)));
+            __syncwarp();
+            ++seg;
         }
+        if (!ok) *aborted = 1u;
+        if (elect_one()) tc_commit(bar(kXtDrain));      // nothing may be in flight when the CTA leaves
         __syncwarp();
         (void)mbar_wait(bar(kXtDrain), 0u);
         __syncwarp();
     } else if (wid == 26) {
-        // ======================= output products: one thread =======================================
-        if (elect_one()) {
-            constexpr uint32_t kIdesc = tc_idesc(128, N, 0);
-            const uint64_t desc_p = tc_smem_desc(p_t, 16u, 1024u);
-            uint32_t laps = 0;      // fills of each V granule so far
-            bool ok = true;
-            while (ok && xt_next(p, walk, sg)) {
-                for (int b = 0; ok && kXtPages * b < sg.pages; ++b, ++c) {
-                    ok = mbar_wait(bar(kXtPReady), c & 1u) && *aborted == 0u;
-                    if (!ok) break;
-                    const int passes = *reinterpret_cast<volatile int*>(&sh.peak[c & 1]) == (int)c + 1 ? 2 : 1;
-                    for (int pass = 0; pass < passes && ok; ++pass, ++laps) {
-#pragma unroll 1
-                        for (int kk = 0; kk < 2 && ok; ++kk) {
-                            ok = mbar_wait(bar(kXtVFull + kk), laps & 1u) && *aborted == 0u;
-                            if (!ok) break;
+        // ======================= output products ====================================================
+        constexpr uint32_t kIdesc = tc_idesc(128, N, 0);
+        const uint64_t desc_p = tc_smem_desc(p_t, 16u, 1024u);
+        const uint32_t base = __shfl_sync(0xffffffffu, tmem, 0);
+        uint32_t laps = 0;      // fills of each V granule so far
+        bool ok = true;
+        while (ok && xt_next(p, walk, sg)) {
+            for (int b = 0; ok && kXtPages * b < sg.pages; ++b, ++c) {
+                ok = wait_all(bar(kXtPReady), c & 1u);
+                const int passes = *reinterpret_cast<volatile int*>(&sh.peak[c & 1]) == (int)c + 1 ? 2 : 1;
+                for (int pass = 0; pass < passes && ok; ++pass, ++laps) {
+#pragma unroll
+                    for (int kk = 0; kk < 2; ++kk) {
+                        ok = ok && wait_all(bar(kXtVFull + kk), laps & 1u);
+                        const bool more = (b | pass) != 0;
+                        if (ok && elect_one()) {
                             tc_fence_after();
 #pragma unroll
                             for (int h = 0; h < 2; ++h) {
 #pragma unroll
                                 for (int ks = 0; ks < 4; ++ks) {
                                     const uint64_t bp = desc_p + (uint64_t)(h * (int)(kPBytes / 16) + kk * (N * 128 / 16) + 2 * ks);
-                                    tc_mma_f16_ts(tmem + kXtColO + (uint32_t)(h * N),
-                                                  tmem + kXtColV + 64u * (uint32_t)h + 32u * (uint32_t)kk + 8u * (uint32_t)ks,
-                                                  bp, kIdesc, (b | pass | kk | ks) ? 1u : 0u);
+                                    const uint32_t d = base + kXtColO + (uint32_t)(h * N), a = base + kXtColV + (uint32_t)(64 * h + 32 * kk + 8 * ks);
+                                    if ((kk | ks) || more) xt_mma<true>(d, a, bp, kIdesc);
+                                    else xt_mma<false>(d, a, bp, kIdesc);
                                 }
                             }
                             tc_commit(bar(kXtVEmpty + kk));
                         }
+                        __syncwarp();
                     }
-                    if (ok) tc_commit(bar(kXtPvDone));
                 }
+                if (ok && elect_one()) tc_commit(bar(kXtPvDone));
+                __syncwarp();
             }
-            if (!ok) *aborted = 1u;
-            tc_commit(bar(kXtDrain));
         }
+        if (!ok) *aborted = 1u;
+        if (elect_one()) tc_commit(bar(kXtDrain));
         __syncwarp();
         (void)mbar_wait(bar(kXtDrain), 0u);
         __syncwarp();
@@ -359,7 +374,7 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
         const int vw = 4 * (wid & 3) + (gid >> 1);                           // this thread's code word of the half
         const uint32_t word_off = 4u * ((half ? 17u : 0u) + (uint32_t)vw);
         const bool splice_warp = half == 0 && (wid & 3) == 0;                // virtual word 0: (W0 >> 16) | (W16 << 16)
-        const uint32_t lut_v = lut_addr + 128u + 4u * (uint32_t)lane, lut_r = lut_addr + 8u * (uint32_t)(lane & 15);
+        const uint32_t lut_v = lut_addr + 128u + 4u * (uint32_t)lane, lut_r = lut_addr + 8u * (uint32_t)(lane & 15) + 4u;
         // byte 2 (gid & 1) + T of the paired codes belongs to tile T
         const uint32_t sel[2] = {0x7604u + ((uint32_t)(2 * (gid & 1)) << 4), 0x7604u + ((uint32_t)(2 * (gid & 1) + 1) << 4)};
         uint32_t laps = 0;
@@ -381,6 +396,7 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                 int passes = 1;
 #pragma unroll 1
                 for (int pass = 0; pass < passes && ok; ++pass, ++laps) {
+                    const uint32_t lut = pass == 0 ? lut_v : lut_r;
 #pragma unroll 1
                     for (int kk = 0; kk < 2; ++kk) {
                         uint32_t a[2][16];
@@ -410,13 +426,8 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                             for (int T = 0; T < 2; ++T) {
 #pragma unroll
                                 for (int o = 0; o < 2; ++o) {
-                                    if (pass == 0) {
-                                        a[T][4 * pg + 2 * o] = lds32_lut(__byte_perm(ab[o], lut_v, sel[T]));
-                                        a[T][4 * pg + 2 * o + 1] = lds32_lut(__byte_perm(cd[o], lut_v, sel[T]));
-                                    } else {
-                                        a[T][4 * pg + 2 * o] = lds32_lut_residual(__byte_perm(ab[o], lut_r, sel[T]));
-                                        a[T][4 * pg + 2 * o + 1] = lds32_lut_residual(__byte_perm(cd[o], lut_r, sel[T]));
-                                    }
+                                    a[T][4 * pg + 2 * o] = lds32_lut(__byte_perm(ab[o], lut, sel[T]));
+                                    a[T][4 * pg + 2 * o + 1] = lds32_lut(__byte_perm(cd[o], lut, sel[T]));
                                 }
                             }
                         }
@@ -461,9 +472,10 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                     const uint32_t at = rowp + 16u * (uint32_t)(gr & 3) + (gr >= 4 ? 68u : 0u);
 #pragma unroll
                     for (int i = 0; i < 4; ++i) x[i] = lds32(at + 4u * i);
-                    x[4] = gr < 4 ? lds32(at + 16u) : 0u;
+                    x[4] = lds32(at + (gr < 4 ? 16u : 12u));
+                    const uint32_t shift = gr < 4 ? 16u : 0u;            // half 0 starts at byte 2
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) w[i] = gr < 4 ? __funnelshift_r(x[i], x[i + 1], 16) : x[i];   // half 0 starts at byte 2
+                    for (int i = 0; i < 4; ++i) w[i] = __funnelshift_r(x[i], x[i + 1], shift);
                     uint32_t hi[16], lo[16];
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
@@ -516,9 +528,12 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                     safe_hi = min(safe_hi, row_max[i]);
                 }
             }
-            float l[P];
+            float l[P], m_lag[P];      // this key's mass of every row; the reference maxima plus the lag
 #pragma unroll
-            for (int i = 0; i < P; ++i) l[i] = 0.0f;
+            for (int i = 0; i < P; ++i) {
+                l[i] = 0.0f;
+                m_lag[i] = -1e30f;
+            }
             // mass of every row over all keys so far, into sh.mass (a lower bound from then on)
             auto reduce_mass = [&]() {
 #pragma unroll
@@ -535,7 +550,7 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
             const int nblocks = (sg.pages + kXtPages - 1) / kXtPages;
 #pragma unroll 1
             for (int b = 0; b < nblocks; ++b, ++c) {
-                bool bad = *aborted != 0u || !wait_all(bar(kXtKScale + (int)(c & 1)), (c >> 1) & 1u);
+                bool bad = !wait_all(bar(kXtKScale + (int)(c & 1)), (c >> 1) & 1u);
                 const float2 dk = sh.k_scale[c & 1][key];
                 bad = bad || !wait_all(bar(kXtSReady), c & 1u);
                 tc_fence_after();
@@ -563,12 +578,12 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                 if (!full) {
 #pragma unroll
                     for (int i = 0; i < P; ++i) {
-                        if (key > last || pos < row_min[i] || pos > row_max[i]) sc[i] = -1e30f;
+                        if (key > last || pos < row_min[i] || pos > row_max[i]) sc[i] = -INFINITY;
                     }
                 }
                 bool ahead = false;
 #pragma unroll
-                for (int i = 0; i < P; ++i) ahead = ahead || sc[i] > m_ref[i] + kXtLag;
+                for (int i = 0; i < P; ++i) ahead = ahead || sc[i] > m_lag[i];
                 const bool moved = xt_any(ahead, part);
                 if (moved) {      // the reference maximum of some row moves: take the block's maxima
 #pragma unroll
@@ -589,7 +604,10 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                     }
                     xt_sync(part);
 #pragma unroll
-                    for (int i = 0; i < P; ++i) l[i] *= alpha[i];
+                    for (int i = 0; i < P; ++i) {
+                        l[i] *= alpha[i];
+                        m_lag[i] = m_ref[i] + kXtLag;
+                    }
                 }
                 bad = bad || !wait_all(bar(kXtVScale + (int)(c & 1)), (c >> 1) & 1u);
                 float2 dv = sh.v_scale[c & 1][key];
@@ -612,32 +630,36 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                     tc_wait_st();
                     tc_fence_before();
                 }
-                // weights; a key no row can see may hold never-written bytes, its scale must not meet a zero weight
-                bool peaked = false, seen = false;
+                if (!full) {      // a key no row can see may hold never-written bytes: its scale must not meet a zero weight
+                    bool seen = false;
 #pragma unroll
-                for (int i = 0; i < P; ++i) {
-                    float w = ex2(sc[i] - (m_ref[i] + kXtLag));
-                    if (!full && sc[i] <= -1e30f) w = 0.0f;      // (a row that has seen nothing yet: masked scores equal its maximum)
-                    l[i] += w;
-                    // a key with more than kPeakedWeight of a row's mass so far (of what is known of it)
-                    peaked = peaked || w > kPeakedWeight * mass[i];
-                    seen = seen || w != 0.0f;
-                    sc[i] = w;
+                    for (int i = 0; i < P; ++i) seen = seen || sc[i] > -INFINITY;
+                    if (!seen) dv = make_float2(0.0f, 0.0f);
                 }
-                if (!seen) dv = make_float2(0.0f, 0.0f);
-                const uint32_t at = p_t + (uint32_t)(key >> 6) * (uint32_t)(N * 128) + (uint32_t)row0 * 128u + 2u * (uint32_t)(key & 7);
-                const uint32_t chunk = ((uint32_t)(key & 63) >> 3) ^ (uint32_t)(row0 & 4);      // (row0 is a multiple of 4: row & 7 = (row0 & 4) ^ (i & 7))
+                float known[P];
+#pragma unroll
+                for (int i = 0; i < P; i += 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(&mass[i]);
+                    known[i] = v.x; known[i + 1] = v.y; known[i + 2] = v.z; known[i + 3] = v.w;
+                }
+                bool peaked = false;      // a key with more than kPeakedWeight of a row's mass so far (of what is known of it)
+                // 16-byte chunk of the key's column, swizzled by the row (row0 is a multiple of 4: row & 7 = (row0 & 4) ^ (i & 7))
+                const uint32_t at = p_t + (uint32_t)(key >> 6) * (uint32_t)(N * 128) + (uint32_t)row0 * 128u + 2u * (uint32_t)(key & 7) +
+                                    ((((uint32_t)(key & 63) >> 3) ^ (uint32_t)(row0 & 4)) << 4);
 #pragma unroll
                 for (int i = 0; i < P; ++i) {
-                    const uint32_t a = at + (uint32_t)i * 128u + ((chunk ^ (uint32_t)(i & 7)) << 4);
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const float x = sc[i] * (h ? dv.y : dv.x);
-                        const __half xh = __float2half_rn(x);
-                        const __half xl = __float2half_rn(x - __half2float(xh));
-                        sts16(a + (uint32_t)h * kPBytes, (uint32_t)__half_as_ushort(xh));
-                        sts16(a + (uint32_t)h * kPBytes + (uint32_t)R * 128u, (uint32_t)__half_as_ushort(xl));
-                    }
+                    const float w = ex2(sc[i] - m_lag[i]);
+                    l[i] += w;
+                    peaked = peaked || w > kPeakedWeight * known[i];
+                    const float x0 = w * dv.x, x1 = w * dv.y;
+                    const __half2 h = __floats2half2_rn(x0, x1);
+                    const float2 hf = __half22float2(h);
+                    const uint32_t hi = *reinterpret_cast<const uint32_t*>(&h), lo = pack_half2(x0 - hf.x, x1 - hf.y);
+                    const uint32_t a = (at ^ (uint32_t)((i & 7) << 4)) + (uint32_t)i * 128u;
+                    sts16(a, hi);
+                    sts16(a + (uint32_t)R * 128u, lo);
+                    sts16(a + kPBytes, hi >> 16);
+                    sts16(a + kPBytes + (uint32_t)R * 128u, lo >> 16);
                 }
                 if (bad) failed = true;
                 const bool any_peak = __any_sync(0xffffffffu, peaked);
