@@ -2206,8 +2206,6 @@ static DeviceInfo* device_info(int* rc) {
         *rc = (int)cudaFuncSetAttribute(tq4_attention_prefill_tc_kernel,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmemBytes);
         if (*rc != 0) return nullptr;
-        *rc = (int)cudaFuncSetAttribute(tq4_attention_stream_tc_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-        if (*rc != 0) return nullptr;
         *rc = (int)cudaFuncSetAttribute(tq4_attention_stream_tc_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
         if (*rc != 0) return nullptr;
         *rc = (int)cudaFuncSetAttribute(tq4_attention_stream_tc_kernel<24>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
@@ -2271,10 +2269,10 @@ static size_t stream_scratch_bytes(const warp34_kv_layer_layout* l, const warp34
     return plan_bytes(b->num_reqs) + (size_t)slots * (size_t)(rpg * kHeadDim + 2 * rpg) * sizeof(float) + qfrag;
 }
 
-// The tcgen05 stream kernel: rows per item (8, 16 or 24: all of a request's rows per kv head, 0: too many) and its workspace.
+// The tcgen05 stream kernel: rows per item (16 or 24: all of a request's rows per kv head, 0: too few or too many) and its workspace.
 static int xt_rows(const warp34_attention_batch* b, int gqa) {
     const long long rows = (long long)(b->max_q_len > 0 ? b->max_q_len : 1) * gqa;
-    return rows <= 8 ? 8 : rows <= 16 ? 16 : rows <= 24 ? 24 : 0;
+    return rows <= 8 ? 0 : rows <= 16 ? 16 : rows <= 24 ? 24 : 0;
 }
 static size_t xt_scratch_bytes(const warp34_kv_layer_layout* l, const warp34_attention_batch* b, int hq, int rows, int grid) {
     return plan_bytes(b->num_reqs) + ((size_t)grid + (size_t)items_bound(l, b, hq, rows)) * (size_t)(rows * kHeadDim + 2 * rows) * sizeof(float) +
@@ -2584,8 +2582,8 @@ static int launch_attention(const warp34_exec* ex, const warp34_kv_layer_layout*
         p.min_units = kXtPages;
         rc = launch_behind(tq4_attention_plan_kernel, 1 + (unsigned)q_items, kPlanThreads, 0, st, p);
         if (rc != 0) return rc;
-        auto* kernel = tile_rows == 8 ? tq4_attention_stream_tc_kernel<8> : tile_rows == 16 ? tq4_attention_stream_tc_kernel<16> : tq4_attention_stream_tc_kernel<24>;
-        rc = launch_behind(kernel, (unsigned)dev->sm_count, kXtThreads, (size_t)dev->smem_optin, st, p);
+        auto* kernel = tile_rows == 16 ? tq4_attention_stream_tc_kernel<16> : tq4_attention_stream_tc_kernel<24>;
+        rc = launch_behind(kernel, (unsigned)dev->sm_count, (unsigned)xt_threads(tile_rows), (size_t)dev->smem_optin, st, p);
         if (rc != 0) return rc;
         const long long rows = (long long)batch->total_tokens * num_q_heads;
         return triple_out != nullptr ? launch_merge<true>(p, rows, st) : launch_merge<false>(p, rows, st);

@@ -21,18 +21,19 @@
 namespace w34 {
 
 constexpr int kXtKeys = 128, kXtPages = kXtKeys / kPageTokens;
-constexpr int kXtWarps = 28, kXtThreads = kXtWarps * 32;      // the last warp is idle
+// four softmax warps per eight rows, 8 V warps, 8 K warps, copies, two MMA warps, one idle
+__host__ __device__ constexpr int xt_threads(int rows) { return (rows / 2 + 20) * 32; }
+constexpr int kXtStages = 2;                                  // blocks of raw K and V in shared memory
 constexpr uint32_t kXtRun = (uint32_t)kXtPages * kTq4PageHeadBytes;       // 16896: K or V of a block
 constexpr uint32_t kXtColK = 0, kXtColV = 128, kXtColS = 256, kXtColO = 384;
 constexpr int kXtMinPages = 24;                               // per SM, see takes_tiles
 constexpr int kXtKRing = 4;                                   // granules of 32 channels: 16 columns of values, 16 of residuals
 constexpr float kXtLag = 3.0f;                                // log2 units the reference maximum may lag; P is carried times 2^-3
 
-__host__ __device__ constexpr int xt_stages(int rows) { return rows <= 8 ? 3 : 2; }
 __host__ __device__ constexpr uint32_t xt_query_bytes(int rows) { return 2u * (uint32_t)rows * 512u; }
 
 struct XtShared {
-    float2 k_scale[2][kXtKeys], v_scale[2][kXtKeys];
+    float2 k_scale[2][kXtKeys];
     __align__(16) float m_ref[24], alpha[24], mass[24];
     float red[4][24];                // [warp of the part][row]
     int row_min[24], row_max[24];
@@ -42,8 +43,8 @@ struct XtShared {
     uint64_t bars[48];
 };
 enum { kXtRawKFull = 0, kXtRawKFree = 4, kXtRawVFull = 8, kXtRawVFree = 12, kXtKFull = 16, kXtKEmpty = 20, kXtVFull = 24, kXtVEmpty = 26,
-       kXtQFull = 28, kXtQFree = 30, kXtSReady = 32, kXtSFree, kXtPReady, kXtPvDone, kXtKScale, kXtVScale = kXtKScale + 2,
-       kXtDrain = kXtVScale + 2, kXtBarCount };
+       kXtQFull = 28, kXtQFree = 30, kXtSReady = 32, kXtSFree, kXtPReady, kXtPvDone, kXtKScale,
+       kXtDrain = kXtKScale + 2, kXtBarCount };
 static_assert(kXtBarCount <= 48, "barrier slots");
 
 __device__ __forceinline__ void tc_ld4(uint32_t (&r)[4], uint32_t taddr) {
@@ -139,8 +140,8 @@ __device__ __forceinline__ bool xt_next(const StreamParams& p, XtWalk& w, XtSegm
 }
 
 template <int R>
-__global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(const StreamParams p) {
-    constexpr int N = 2 * R, STAGES = xt_stages(R);
+__global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kernel(const StreamParams p) {
+    constexpr int N = 2 * R, STAGES = kXtStages, PARTS = R / 8, W0 = 4 * PARTS;      // W0: first V warp
     constexpr uint32_t kQueryBytes = xt_query_bytes(R), kPBytes = (uint32_t)N * 256u;      // P of one half: [2 x 64 keys][N][128 B]
     extern __shared__ __align__(1024) uint8_t smem[];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -160,8 +161,8 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
         return;
     }
     XtShared& sh = *reinterpret_cast<XtShared*>(smem + (sh_addr - win_lo));
-    auto raw_k = [&](int s) { return s == 0 ? raw[0] : (STAGES == 2 || s == 1) ? raw[1] : raw[STAGES - 1]; };
-    auto raw_v = [&](int s) { return s == 0 ? raw[STAGES] : (STAGES == 2 || s == 1) ? raw[STAGES + 1] : raw[2 * STAGES - 1]; };
+    auto raw_k = [&](int s) { return s == 0 ? raw[0] : raw[1]; };
+    auto raw_v = [&](int s) { return s == 0 ? raw[2] : raw[3]; };
     const uint32_t bars = smem_u32(sh.bars);
     auto bar = [&](int which) { return bars + 8u * (uint32_t)which; };
     volatile uint32_t* aborted = &sh.aborted;
@@ -174,7 +175,7 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
         return false;
     };
 
-    for (int i = tid; i < 256 * 32; i += kXtThreads) {      // table as in the exact streaming kernel, residuals unscaled
+    for (int i = tid; i < 256 * 32; i += xt_threads(R)) {      // table as in the exact streaming kernel, residuals unscaled
         const int byte = i >> 5, ln = i & 31;
         const float c0 = kLutScale * tq4_centroid(byte & 15), c1 = kLutScale * tq4_centroid(byte >> 4);
         const uint32_t hi = pack_half2(c0, c1);
@@ -187,7 +188,7 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
             mbar_init(bar(kXtRawKFull + s), 1u);
             mbar_init(bar(kXtRawKFree + s), 8u);
             mbar_init(bar(kXtRawVFull + s), 1u);
-            mbar_init(bar(kXtRawVFree + s), 8u);
+            mbar_init(bar(kXtRawVFree + s), 8u + W0);
         }
         for (int s = 0; s < kXtKRing; ++s) { mbar_init(bar(kXtKFull + s), 4u); mbar_init(bar(kXtKEmpty + s), 1u); }
         for (int s = 0; s < 2; ++s) {
@@ -196,11 +197,10 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
             mbar_init(bar(kXtQFull + s), 1u);
             mbar_init(bar(kXtQFree + s), 1u);
             mbar_init(bar(kXtKScale + s), 4u);
-            mbar_init(bar(kXtVScale + s), 8u);
         }
         mbar_init(bar(kXtSReady), 1u);
-        mbar_init(bar(kXtSFree), 8u);
-        mbar_init(bar(kXtPReady), 8u);
+        mbar_init(bar(kXtSFree), W0);
+        mbar_init(bar(kXtPReady), W0);
         mbar_init(bar(kXtPvDone), 1u);
         mbar_init(bar(kXtDrain), 2u);
         sh.peak[0] = sh.peak[1] = 0;
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
     XtSegment sg;
     uint32_t c = 0;                                       // blocks so far
 
-    if (wid == 24) {
+    if (wid == W0 + 16) {
         // ======================= raw pages and query rows ==========================================
         uint32_t seg = 0, k_issued = 0, v_issued = 0;
         bool ok = true;
@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
         for (uint32_t j = v_issued > STAGES ? v_issued - STAGES : 0; j < v_issued; ++j) (void)mbar_wait(bar(kXtRawVFull + (int)(j % STAGES)), (j / STAGES) & 1u);
         for (uint32_t j = seg > 2 ? seg - 2 : 0; j < seg; ++j) (void)mbar_wait(bar(kXtQFull + (int)(j & 1)), (j >> 1) & 1u);
         __syncwarp();
-    } else if (wid == 25) {
+    } else if (wid == W0 + 17) {
         // ======================= score products =====================================================
         // An MMA of this size takes the tensor cores some 40 cycles, so that operands are kept where an issue needs no more than a
         // few instructions: warp-uniform bases, everything else constant.
@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
         __syncwarp();
         (void)mbar_wait(bar(kXtDrain), 0u);
         __syncwarp();
-    } else if (wid == 26) {
+    } else if (wid == W0 + 18) {
         // ======================= output products ====================================================
         constexpr uint32_t kIdesc = tc_idesc(128, N, 0);
         const uint64_t desc_p = tc_smem_desc(p_t, 16u, 1024u);
@@ -368,9 +368,9 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
         __syncwarp();
         (void)mbar_wait(bar(kXtDrain), 0u);
         __syncwarp();
-    } else if (wid >= 8 && wid < 16) {
+    } else if (wid >= W0 && wid < W0 + 8) {
         // ======================= V: 32 channels of a half, fragments of four keys a thread ===============
-        const int gid = lane >> 2, tig = lane & 3, half = (wid - 8) >> 2;
+        const int gid = lane >> 2, tig = lane & 3, half = (wid - W0) >> 2;
         const int vw = 4 * (wid & 3) + (gid >> 1);                           // this thread's code word of the half
         const uint32_t word_off = 4u * ((half ? 17u : 0u) + (uint32_t)vw);
         const bool splice_warp = half == 0 && (wid & 3) == 0;                // virtual word 0: (W0 >> 16) | (W16 << 16)
@@ -384,14 +384,6 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                 const int s = (int)(c % STAGES);
                 if (!(ok = wait_all(bar(kXtRawVFull + s), (c / STAGES) & 1u))) break;
                 const uint32_t run = raw_v(s);
-                if (lane < 16) {      // the scales of 16 keys
-                    const int key = 16 * (wid - 8) + lane;
-                    const uint32_t rowp = run + (uint32_t)key * kTq4RowBytes;
-                    sh.v_scale[c & 1][key] = make_float2(__half2float(__ushort_as_half((unsigned short)(lds32(rowp) & 0xffffu))),
-                                                         __half2float(__ushort_as_half((unsigned short)(lds32(rowp + 64) >> 16))));
-                }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar(kXtVScale + (int)(c & 1)));
                 const uint32_t rows = run + (uint32_t)(4 * tig) * kTq4RowBytes;
                 int passes = 1;
 #pragma unroll 1
@@ -449,9 +441,9 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                 if (ok && lane == 0) mbar_arrive(bar(kXtRawVFree + s));
             }
         }
-    } else if (wid >= 16 && wid < 24) {
+    } else if (wid >= W0 + 8 && wid < W0 + 16) {
         // ======================= K: thread = key ===================================================
-        const int part = (wid - 16) >> 2, key = tid & 127;          // part 0 takes the even granules, part 1 the odd ones
+        const int part = (wid - W0 - 8) >> 2, key = tid & 127;          // part 0 takes the even granules, part 1 the odd ones
         const uint32_t lutk_lane = lut_addr + 8u * (uint32_t)(lane & 15);
         bool ok = true;
         while (ok && xt_next(p, walk, sg)) {
@@ -495,9 +487,9 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                 if (ok && lane == 0) mbar_arrive(bar(kXtRawKFree + s));
             }
         }
-    } else if (wid < 8) {
-        // ======================= softmax: thread = key, a part = half of the rows =============================================
-        constexpr int P = R / 2;
+    } else if (wid < W0) {
+        // ======================= softmax: thread = key, a part = eight rows =============================================
+        constexpr int P = 8;
         const int part = wid >> 2, row0 = part * P, key = tid & 127;
         const uint32_t t_s = tmem + quad + kXtColS + (uint32_t)row0, t_o = tmem + quad + kXtColO + (uint32_t)row0;
         float* m_ref = sh.m_ref + row0;      // this part's rows
@@ -609,8 +601,10 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                         m_lag[i] = m_ref[i] + kXtLag;
                     }
                 }
-                bad = bad || !wait_all(bar(kXtVScale + (int)(c & 1)), (c >> 1) & 1u);
-                float2 dv = sh.v_scale[c & 1][key];
+                bad = bad || !wait_all(bar(kXtRawVFull + (int)(c % STAGES)), (c / STAGES) & 1u);
+                const uint32_t v_row = raw_v((int)(c % STAGES)) + (uint32_t)key * kTq4RowBytes;
+                float2 dv = make_float2(__half2float(__ushort_as_half((unsigned short)(lds32(v_row) & 0xffffu))),
+                                        __half2float(__ushort_as_half((unsigned short)(lds32(v_row + 64) >> 16))));
                 // P and O are in use until the output product of the block before has completed
                 bad = bad || (c > 0 && !wait_all(bar(kXtPvDone), (c - 1) & 1u));
                 if (moved && b > 0) {
@@ -643,9 +637,9 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                     known[i] = v.x; known[i + 1] = v.y; known[i + 2] = v.z; known[i + 3] = v.w;
                 }
                 bool peaked = false;      // a key with more than kPeakedWeight of a row's mass so far (of what is known of it)
-                // 16-byte chunk of the key's column, swizzled by the row (row0 is a multiple of 4: row & 7 = (row0 & 4) ^ (i & 7))
+                // 16-byte chunk of the key's column, swizzled by the row
                 const uint32_t at = p_t + (uint32_t)(key >> 6) * (uint32_t)(N * 128) + (uint32_t)row0 * 128u + 2u * (uint32_t)(key & 7) +
-                                    ((((uint32_t)(key & 63) >> 3) ^ (uint32_t)(row0 & 4)) << 4);
+                                    (((uint32_t)(key & 63) >> 3) << 4);
 #pragma unroll
                 for (int i = 0; i < P; ++i) {
                     const float w = ex2(sc[i] - m_lag[i]);
@@ -655,7 +649,7 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                     const __half2 h = __floats2half2_rn(x0, x1);
                     const float2 hf = __half22float2(h);
                     const uint32_t hi = *reinterpret_cast<const uint32_t*>(&h), lo = pack_half2(x0 - hf.x, x1 - hf.y);
-                    const uint32_t a = (at ^ (uint32_t)((i & 7) << 4)) + (uint32_t)i * 128u;
+                    const uint32_t a = (at ^ (uint32_t)(i << 4)) + (uint32_t)i * 128u;
                     sts16(a, hi);
                     sts16(a + (uint32_t)R * 128u, lo);
                     sts16(a + kPBytes, hi >> 16);
@@ -666,8 +660,11 @@ __global__ void __launch_bounds__(kXtThreads, 1) tq4_attention_stream_tc_kernel(
                 if (any_peak && lane == 0) sh.peak[c & 1] = (int)c + 1;
                 fence_proxy_async();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(bar(kXtPReady));
-                if (b < 2 || (b & 3) == 3) reduce_mass();
+                if (lane == 0) {
+                    mbar_arrive(bar(kXtPReady));
+                    mbar_arrive(bar(kXtRawVFree + (int)(c % STAGES)));
+                }
+                if ((b & (b + 1)) == 0) reduce_mass();      // after 1, 2, 4, 8 ... blocks
             }
             // ---- the item's share is done: write the partial (lane = channel) ----------------------
             reduce_mass();
