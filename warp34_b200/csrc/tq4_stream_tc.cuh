@@ -34,7 +34,7 @@ __host__ __device__ constexpr uint32_t xt_query_bytes(int rows) { return 2u * (u
 
 struct XtShared {
     float2 k_scale[2][kXtKeys];
-    __align__(16) float m_ref[24], alpha[24], mass[24];
+    __align__(16) float m_ref[24], alpha[24], mass[24], cut[24];      // cut: kPeakedWeight of the mass known so far
     float red[4][24];                // [warp of the part][row]
     int row_min[24], row_max[24];
     int peak[2];               // of the block's parity: some key has a large weight
@@ -169,8 +169,10 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
     // Waits are bounded and warp-uniform; one that gives up ends every loop.
     auto wait_all = [&](uint32_t b, uint32_t parity) {
         if (__all_sync(0xffffffffu, mbar_try_wait(b, parity))) return true;
-        const bool ok = *aborted == 0u && mbar_wait(b, parity) && *aborted == 0u;
-        if (__all_sync(0xffffffffu, ok)) return true;
+        const long long t0 = clock64();
+        do {
+            if (__all_sync(0xffffffffu, mbar_try_wait(b, parity))) return true;
+        } while (*aborted == 0u && clock64() - t0 < kWaitCycleLimit);
         *aborted = 1u;
         return false;
     };
@@ -495,6 +497,7 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
         float* m_ref = sh.m_ref + row0;      // this part's rows
         float* alpha = sh.alpha + row0;
         float* mass = sh.mass + row0;
+        float* cut = sh.cut + row0;
         int *row_min = sh.row_min + row0, *row_max = sh.row_max + row0;
         float* red = &sh.red[0][row0];
         float* partials = reinterpret_cast<float*>(p.scratch + plan_bytes(p.batch.num_reqs));
@@ -510,6 +513,7 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                 row_min[key] = valid ? row_min_kv(p.batch, g, q_off) : 0x7fffffff;
                 m_ref[key] = -1e30f;
                 mass[key] = 0.0f;
+                cut[key] = 0.0f;
             }
             xt_sync(part);
             int safe_lo = 0, safe_hi = 0x7fffffff;      // keys every valid row can see
@@ -536,7 +540,11 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                     if (lane == 0) red[(wid & 3) * 24 + i] = t;
                 }
                 xt_sync(part);
-                if (key < P) mass[key] = (red[0 + key] + red[24 + key]) + (red[48 + key] + red[72 + key]);
+                if (key < P) {
+                    const float t = (red[0 + key] + red[24 + key]) + (red[48 + key] + red[72 + key]);
+                    mass[key] = t;
+                    cut[key] = kPeakedWeight * t;
+                }
                 xt_sync(part);
             };
             const int nblocks = (sg.pages + kXtPages - 1) / kXtPages;
@@ -592,7 +600,7 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                         const float a = ex2(old - now);      // 0 when nothing was visible before
                         m_ref[key] = now;
                         alpha[key] = a;
-                        mass[key] *= a;
+                        cut[key] *= a;
                     }
                     xt_sync(part);
 #pragma unroll
@@ -630,13 +638,13 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                     for (int i = 0; i < P; ++i) seen = seen || sc[i] > -INFINITY;
                     if (!seen) dv = make_float2(0.0f, 0.0f);
                 }
+                bool peaked = false;      // a key with more than kPeakedWeight of a row's mass so far (of what is known of it)
                 float known[P];
 #pragma unroll
                 for (int i = 0; i < P; i += 4) {
-                    const float4 v = *reinterpret_cast<const float4*>(&mass[i]);
+                    const float4 v = *reinterpret_cast<const float4*>(&cut[i]);
                     known[i] = v.x; known[i + 1] = v.y; known[i + 2] = v.z; known[i + 3] = v.w;
                 }
-                bool peaked = false;      // a key with more than kPeakedWeight of a row's mass so far (of what is known of it)
                 // 16-byte chunk of the key's column, swizzled by the row
                 const uint32_t at = p_t + (uint32_t)(key >> 6) * (uint32_t)(N * 128) + (uint32_t)row0 * 128u + 2u * (uint32_t)(key & 7) +
                                     (((uint32_t)(key & 63) >> 3) << 4);
@@ -644,7 +652,8 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                 for (int i = 0; i < P; ++i) {
                     const float w = ex2(sc[i] - m_lag[i]);
                     l[i] += w;
-                    peaked = peaked || w > kPeakedWeight * known[i];
+                    sc[i] = w;
+                    peaked = peaked || w > known[i];
                     const float x0 = w * dv.x, x1 = w * dv.y;
                     const __half2 h = __floats2half2_rn(x0, x1);
                     const float2 hf = __half22float2(h);
@@ -656,15 +665,20 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                     sts16(a + kPBytes + (uint32_t)R * 128u, lo >> 16);
                 }
                 if (bad) failed = true;
-                const bool any_peak = __any_sync(0xffffffffu, peaked);
-                if (any_peak && lane == 0) sh.peak[c & 1] = (int)c + 1;
+                if (xt_any(peaked, part)) {      // bring the known mass up to date and look again
+                    reduce_mass();
+                    peaked = false;
+#pragma unroll
+                    for (int i = 0; i < P; ++i) peaked = peaked || sc[i] > cut[i];
+                    const bool any_peak = __any_sync(0xffffffffu, peaked);
+                    if (any_peak && lane == 0) sh.peak[c & 1] = (int)c + 1;
+                }
                 fence_proxy_async();
                 __syncwarp();
                 if (lane == 0) {
                     mbar_arrive(bar(kXtPReady));
                     mbar_arrive(bar(kXtRawVFree + (int)(c % STAGES)));
                 }
-                if ((b & (b + 1)) == 0) reduce_mass();      // after 1, 2, 4, 8 ... blocks
             }
             // ---- the item's share is done: write the partial (lane = channel) ----------------------
             reduce_mass();
