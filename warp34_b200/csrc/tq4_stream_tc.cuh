@@ -27,10 +27,10 @@ constexpr int kXtStages = 2;                                  // blocks of raw K
 constexpr uint32_t kXtRun = (uint32_t)kXtPages * kTq4PageHeadBytes;       // 16896: K or V of a block
 constexpr uint32_t kXtColK = 0, kXtColV = 128, kXtColS = 256, kXtColO = 384;
 constexpr int kXtMinPages = 24;                               // per SM, see takes_tiles
-constexpr int kXtKRing = 4;                                   // granules of 32 channels: 16 columns of values, 16 of residuals
+constexpr int kXtKRing = 4;                                   // granules of 32 channels: a column of values, one of residuals in turn
 constexpr float kXtLag = 3.0f;                                // log2 units the reference maximum may lag; P is carried times 2^-3
 
-__host__ __device__ constexpr uint32_t xt_query_bytes(int rows) { return 2u * (uint32_t)rows * 512u; }
+__host__ __device__ constexpr uint32_t xt_query_bytes(int rows) { return 2u * (uint32_t)rows * 1024u; }
 
 struct XtShared {
     float2 k_scale[2][kXtKeys];
@@ -43,7 +43,7 @@ struct XtShared {
     uint64_t bars[48];
 };
 enum { kXtRawKFull = 0, kXtRawKFree = 4, kXtRawVFull = 8, kXtRawVFree = 12, kXtKFull = 16, kXtKEmpty = 20, kXtVFull = 24, kXtVEmpty = 26,
-       kXtQFull = 28, kXtQFree = 30, kXtSReady = 32, kXtSFree, kXtPReady, kXtPvDone, kXtKScale,
+       kXtQFull = 28, kXtQFree, kXtSReady, kXtSFree, kXtPReady, kXtPvDone, kXtKScale,
        kXtDrain = kXtKScale + 2, kXtBarCount };
 static_assert(kXtBarCount <= 48, "barrier slots");
 
@@ -67,8 +67,6 @@ __device__ __forceinline__ void xt_mma(uint32_t d, uint32_t a, uint64_t b_desc, 
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
                  :: "r"(d), "r"(a), "l"(b_desc), "r"(idesc), "n"(ACC ? 1 : 0) : "memory");
 }
-// A descriptor like `like` with another start address (low word).
-__device__ __forceinline__ uint64_t xt_desc(uint32_t low, uint64_t like) { return (like & 0xffffffff00000000ull) | low; }
 // Barrier of the four warps of a softmax part.
 __device__ __forceinline__ void xt_sync(int part) { asm volatile("bar.sync %0, 128;" :: "r"(1 + part) : "memory"); }
 __device__ __forceinline__ bool xt_any(bool x, int part) {
@@ -79,7 +77,9 @@ __device__ __forceinline__ bool xt_any(bool x, int part) {
 }
 
 // Query rows of item idx = (request * kv heads + kv head) * q_groups_max + group as the B operand: 2R rows (R values, then R
-// residuals) of 256 rotated columns, four blocks of 64 columns, 16-byte chunks swizzled by the row.  Eight warps.
+// residuals) of the 256 rotated columns, every pair of columns twice in a row (K's table entries hold a pair's values and, next to
+// them, its residuals, and go to tensor memory as they are): eight blocks of 32 columns, 16-byte chunks swizzled by the row.
+// Eight warps.
 __device__ void xt_prepare_query(const StreamParams& p, int idx) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, R = p.rows_per_group;
     const int hkv = p.layout.local_kv_heads;
@@ -108,9 +108,13 @@ __device__ void xt_prepare_query(const StreamParams& p, int idx) {
             lo[k] = pack_half2(a - hf.x, b - hf.y);
         }
         // (i and i + R share their low three bits: R is a multiple of 8)
-        uint4* out = reinterpret_cast<uint4*>(dst + (size_t)(lane >> 3) * (2 * R * 128) + (size_t)i * 128 + (((lane & 7) ^ (i & 7)) << 4));
-        out[0] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-        out[R * 8] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        uint8_t* out = dst + (size_t)(lane >> 2) * (2 * R * 128) + (size_t)i * 128;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            uint4* at = reinterpret_cast<uint4*>(out + (((2 * (lane & 3) + k) ^ (i & 7)) << 4));
+            at[0] = make_uint4(hi[2 * k], hi[2 * k], hi[2 * k + 1], hi[2 * k + 1]);
+            at[R * 8] = make_uint4(lo[2 * k], lo[2 * k], lo[2 * k + 1], lo[2 * k + 1]);
+        }
     }
 }
 
@@ -149,7 +153,7 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
     const uint32_t lut_addr = (win_lo + 0xffffu) & ~0xffffu;
     PlanHeader* hdr = reinterpret_cast<PlanHeader*>(p.scratch);
     SmemCarver carve(win_lo, lut_addr, win_lo + p.smem_bytes);
-    const uint32_t q_t[2] = {carve.take(kQueryBytes, 1024), carve.take(kQueryBytes, 1024)};
+    const uint32_t q_t = carve.take(kQueryBytes, 1024);
     const uint32_t p_t = carve.take(2u * kPBytes, 1024);
     uint32_t raw[2 * STAGES];
 #pragma unroll
@@ -196,10 +200,10 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
         for (int s = 0; s < 2; ++s) {
             mbar_init(bar(kXtVFull + s), 8u);
             mbar_init(bar(kXtVEmpty + s), 1u);
-            mbar_init(bar(kXtQFull + s), 1u);
-            mbar_init(bar(kXtQFree + s), 1u);
             mbar_init(bar(kXtKScale + s), 4u);
         }
+        mbar_init(bar(kXtQFull), 1u);
+        mbar_init(bar(kXtQFree), 1u);
         mbar_init(bar(kXtSReady), 1u);
         mbar_init(bar(kXtSFree), W0);
         mbar_init(bar(kXtPReady), W0);
@@ -247,13 +251,12 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                 return (lane < kXtPages && pg < sg.pages) ? block_table_page(blocks, sg.pg0 + pg, p.batch.max_blocks_per_req, kInStream) : -1;
             };
             int32_t id = page_id(0);
-            ok = wait_all(bar(kXtQFree + (int)(seg & 1)), ((seg >> 1) & 1) ^ 1u);
+            ok = wait_all(bar(kXtQFree), (seg & 1u) ^ 1u);
             if (!ok) break;
             if (lane == 0) {
                 const size_t idx = (size_t)(sg.r * p.layout.local_kv_heads + sg.kv_head) * p.q_groups_max + sg.group;
-                mbar_expect_tx(bar(kXtQFull + (int)(seg & 1)), kQueryBytes);
-                bulk_g2s((seg & 1) ? q_t[1] : q_t[0], reinterpret_cast<const uint8_t*>(p.qfrag) + idx * kQueryBytes, kQueryBytes,
-                         bar(kXtQFull + (int)(seg & 1)));
+                mbar_expect_tx(bar(kXtQFull), kQueryBytes);
+                bulk_g2s(q_t, reinterpret_cast<const uint8_t*>(p.qfrag) + idx * kQueryBytes, kQueryBytes, bar(kXtQFull));
             }
             __syncwarp();
             ++seg;
@@ -283,20 +286,19 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
         // copies in flight must land before the CTA leaves
         for (uint32_t j = k_issued > STAGES ? k_issued - STAGES : 0; j < k_issued; ++j) (void)mbar_wait(bar(kXtRawKFull + (int)(j % STAGES)), (j / STAGES) & 1u);
         for (uint32_t j = v_issued > STAGES ? v_issued - STAGES : 0; j < v_issued; ++j) (void)mbar_wait(bar(kXtRawVFull + (int)(j % STAGES)), (j / STAGES) & 1u);
-        for (uint32_t j = seg > 2 ? seg - 2 : 0; j < seg; ++j) (void)mbar_wait(bar(kXtQFull + (int)(j & 1)), (j >> 1) & 1u);
+        if (seg > 0) (void)mbar_wait(bar(kXtQFull), (seg - 1) & 1u);
         __syncwarp();
     } else if (wid == W0 + 17) {
         // ======================= score products =====================================================
         // An MMA of this size takes the tensor cores some 40 cycles, so that operands are kept where an issue needs no more than a
         // few instructions: warp-uniform bases, everything else constant.
         constexpr uint32_t kIdesc = tc_idesc(kXtKeys, N, 0);
-        const uint64_t desc_q0 = tc_smem_desc(q_t[0], 16u, 1024u), desc_q1 = tc_smem_desc(q_t[1], 16u, 1024u);
+        const uint64_t desc_q = tc_smem_desc(q_t, 16u, 1024u);
         const uint32_t base = __shfl_sync(0xffffffffu, tmem, 0);
         uint32_t seg = 0;
         bool ok = true;
         while (ok && xt_next(p, walk, sg)) {
-            ok = wait_all(bar(kXtQFull + (int)(seg & 1)), (seg >> 1) & 1u);
-            const uint64_t dq = xt_desc(__shfl_sync(0xffffffffu, (uint32_t)((seg & 1) ? desc_q1 : desc_q0), 0), desc_q0);
+            ok = wait_all(bar(kXtQFull), seg & 1u);
             for (int b = 0; ok && kXtPages * b < sg.pages; ++b, ++c) {
                 ok = wait_all(bar(kXtSFree), (c & 1u) ^ 1u);      // the scores of the block before are in registers
 #pragma unroll
@@ -305,13 +307,11 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                     if (ok && elect_one()) {
                         tc_fence_after();
 #pragma unroll
-                        for (int ks = 0; ks < 2; ++ks) {
-                            // channels 32 gr + 16 ks: block of 64 gr >> 1, 32 bytes per k-step
-                            const uint64_t bq = dq + (uint64_t)((gr >> 1) * (N * 128 / 16) + 2 * (2 * (gr & 1) + ks));
+                        for (int ks = 0; ks < 4; ++ks) {      // eight channels each
+                            const uint64_t bq = desc_q + (uint64_t)(gr * (N * 128 / 16) + 2 * ks);
                             const uint32_t d = base + kXtColS + (uint32_t)((gr >> 2) * N), a = base + kXtColK + (uint32_t)(32 * (gr & 3) + 8 * ks);
                             if ((gr & 3) || ks) xt_mma<true>(d, a, bq, kIdesc);
                             else xt_mma<false>(d, a, bq, kIdesc);
-                            xt_mma<true>(d, a + 16u, bq, kIdesc);
                         }
                         tc_commit(bar(kXtKEmpty + (gr & 3)));
                         if (gr == 7) tc_commit(bar(kXtSReady));
@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                     __syncwarp();
                 }
             }
-            if (ok && elect_one()) tc_commit(bar(kXtQFree + (int)(seg & 1)));
+            if (ok && elect_one()) tc_commit(bar(kXtQFree));
             __syncwarp();
             ++seg;
         }
@@ -470,16 +470,15 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                     const uint32_t shift = gr < 4 ? 16u : 0u;            // half 0 starts at byte 2
 #pragma unroll
                     for (int i = 0; i < 4; ++i) w[i] = __funnelshift_r(x[i], x[i + 1], shift);
-                    uint32_t hi[16], lo[16];
+                    uint32_t e[32];      // values and residuals of 16 pairs of channels
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
-                        const uint2 e = lds64_lut(__byte_perm(w[i >> 2], lutk_lane, 0x7604 + ((i & 3) << 4)));
-                        hi[i] = e.x;
-                        lo[i] = e.y;
+                        const uint2 v = lds64_lut(__byte_perm(w[i >> 2], lutk_lane, 0x7604 + ((i & 3) << 4)));
+                        e[2 * i] = v.x;
+                        e[2 * i + 1] = v.y;
                     }
                     if (!(ok = wait_all(bar(kXtKEmpty + (int)slot), (lap & 1u) ^ 1u))) break;
-                    tc_st16(tmem + quad + kXtColK + 32u * slot, hi);
-                    tc_st16(tmem + quad + kXtColK + 32u * slot + 16u, lo);
+                    tc_st32(tmem + quad + kXtColK + 32u * slot, e);
                     tc_wait_st();
                     tc_fence_before();
                     __syncwarp();
