@@ -26,7 +26,6 @@ __host__ __device__ constexpr int xt_threads(int rows) { return (rows / 2 + 20) 
 constexpr int kXtStages = 2;                                  // blocks of raw K and V in shared memory
 constexpr uint32_t kXtRun = (uint32_t)kXtPages * kTq4PageHeadBytes;       // 16896: K or V of a block
 constexpr uint32_t kXtColK = 0, kXtColV = 128, kXtColS = 256, kXtColO = 384;
-constexpr int kXtMinPages = 24;                               // per SM, see takes_tiles
 constexpr int kXtKRing = 4;                                   // granules of 32 channels: a column of values, one of residuals in turn
 constexpr float kXtLag = 3.0f;                                // log2 units the reference maximum may lag; P is carried times 2^-3
 
