@@ -54,7 +54,7 @@ enum {
 #define WARP34_EXEC_FLAG_ALLOW_W4A8_PREFILL (1ull << 0)
 #define WARP34_B200_EXEC_FLAG_PRECISE_ATTENTION (1ull << 40)
 /* Additive: multi-token verify batches (more than 8 query rows per request and KV head) take the
- * tcgen05 kernel, one 128-row CTA per request and KV head, instead of the split-KV team kernel. */
+ * tcgen05 kernel, one 128-row CTA per request and KV head, instead of the split-KV kernel. */
 #define WARP34_B200_EXEC_FLAG_TCGEN05_VERIFY (1ull << 42)
 /* Additive: the tensor-core kernels feed every operand as one fp16 value, as the reference's own
  * tensor-core kernel does (op_paged_attn.cu:357, :47-50, :470).  Faster; a softmax weight is then
@@ -492,7 +492,7 @@ int warp34_qsa_sparse_paged_attn_hadamard_f16(const warp34_exec* ex, const void*
  * (0 = unknown: only block-table indices are checked).  A violating access goes to entry 0 / page 0
  * (reads) or is skipped (writes); nothing traps.  warp34_bounds_report() fills
  *   out4[0] = what | where << 8   what: 1 block-table index, 2 page id, 3 write slot; 0 = no violation
- *                                 where: 1 append, 2 fp32 attention, 3 decode stream, 4 verify team,
+ *                                 where: 1 append, 2 fp32 attention, 3 decode stream, 4 unused,
  *                                        5 / 6 prefill kernels, 7 bf16 KV, 8 8-bit KV
  *   out4[1] = the offending value, out4[2] = its limit     (of the first violation seen)
  *   out4[3] = number of violations since the last reset

@@ -559,7 +559,7 @@ struct StreamParams {
     int num_warps;         // worker warps over the whole grid
     int max_slots;
     uint32_t smem_bytes;   // dynamic shared memory given to the stream kernel
-    int rows_per_group;    // query rows per work item: 8 (one warp per item) or 8 * NT (teams)
+    int rows_per_group;    // query rows per work item: 8 (one warp per item), 16 or 24 (tcgen05 stream kernel)
     float q_scale;         // sm_scale * log2(e) / kLutScale, folded into Q'
     int natural;           // partials are in natural (unrotated, unscaled) coordinates: uncompressed KV
     uint32_t* qfrag;       // rotated queries as MMA fragments, written by the plan launch (or null)
@@ -1325,41 +1325,6 @@ __global__ void __launch_bounds__(WARPS * 32, 1) tq4_attention_stream_kernel(con
     }
 }
 
-// ---------------------------------------------------------------------------------------
-// Team kernel: 8 * NT query rows (GQA heads x draft tokens of a verify step) share ONE pass
-// over the KV pages.  A team is four warps; warp t owns a quarter of the 256 channels (half
-// t >> 1 of the row, every other pair of 8-channel words), for the score product and for the
-// output alike, so every code is looked up once per page however many query rows read it and
-// each looked-up fragment feeds NT MMAs.  The team meets once per page, after the partial
-// scores: they are summed through shared memory by the warp that owns an 8-row tile, which
-// runs its online softmax and publishes P fragments and rescale factors (double-buffered);
-// the output product of a page runs after the next meeting, so one page's softmax overlaps the
-// next page's score product.  Three teams per CTA, one CTA per SM, each team with its own ring.
-// ---------------------------------------------------------------------------------------
-constexpr int kTeams = 3;
-constexpr int kTeamWarps = 4;
-constexpr int kTeamStages = 8;
-
-__device__ __forceinline__ void team_barrier(int team) {
-    asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "r"(kTeamWarps * 32) : "memory");
-}
-__device__ __forceinline__ float4 lds128f(uint32_t addr) {
-    float4 v;
-    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
-    return v;
-}
-__device__ __forceinline__ void sts128f(uint32_t addr, float4 v) {
-    asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
-}
-__device__ __forceinline__ float2 lds64f(uint32_t addr) {
-    float2 v;
-    asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
-    return v;
-}
-__device__ __forceinline__ void sts64f(uint32_t addr, float2 v) {
-    asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(addr), "f"(v.x), "f"(v.y) : "memory");
-}
-
 // Carves [lo, hi) minus the 64 KB table at `lut` into chunks: first fit below the table, then above.
 struct SmemCarver {
     uint32_t a_cur, a_end, b_cur, b_end;
@@ -1375,445 +1340,6 @@ struct SmemCarver {
         return b_end >= bytes ? b_end - bytes : 0;
     }
 };
-
-template <int NT>
-__global__ void __launch_bounds__(kTeams * kTeamWarps * 32, 1) tq4_attention_team_kernel(const StreamParams p) {
-    extern __shared__ __align__(1024) uint8_t smem[];
-    constexpr int RG = 8 * NT;
-    constexpr int PARTIAL = RG * kHeadDim + 2 * RG;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int team = wid >> 2, t = wid & 3;     // warp t of its team
-    const int half = t >> 1, cset = t & 1;      // 128-half and word set owned by this warp
-    const uint32_t win_lo = smem_u32(smem);
-    const uint32_t win_hi = win_lo + p.smem_bytes;
-    const uint32_t lut_addr = (win_lo + 0xffffu) & ~0xffffu;
-    PlanHeader* hdr = reinterpret_cast<PlanHeader*>(p.scratch);
-
-    SmemCarver carve(win_lo, lut_addr, win_hi);
-    uint32_t ring = 0, sx = 0, px = 0, ax = 0, bars = 0;
-    for (int tm = 0; tm < kTeams; ++tm) {
-        const uint32_t r_ = carve.take(kTeamStages * kStageStride, 128);
-        if (tm == team) ring = r_;
-    }
-    for (int tm = 0; tm < kTeams; ++tm) {
-        // all three are double-buffered by page parity
-        const uint32_t s_ = carve.take(2 * kTeamWarps * NT * 512, 16);   // partial scores [buf][warp][tile][lane] float4
-        const uint32_t p_ = carve.take(2 * NT * 2 * 2 * 128, 16);         // P fragments [buf][tile][half][reg][lane]
-        const uint32_t a_ = carve.take(2 * NT * 4 * 8, 8);                // rescale factors [buf][tile][tig] float2
-        const uint32_t b_ = carve.take(kTeamStages * 8, 8);
-        if (tm == team) { sx = s_; px = p_; ax = a_; bars = b_; }
-    }
-    if (!carve.ok) {
-        if (threadIdx.x == 0) atomicOr(&hdr->status, 2);
-        return;
-    }
-    uint8_t* ring_gen = smem + (ring - win_lo);
-
-    for (int i = threadIdx.x; i < 256 * 32; i += blockDim.x) {
-        const int byte = i >> 5, ln = i & 31;
-        sts32(lut_addr + (uint32_t)(byte * 256 + ln * 4),
-              pack_half2(kLutScale * tq4_centroid(byte & 15), kLutScale * tq4_centroid(byte >> 4)));
-    }
-    if (t == 0 && lane == 0) {
-        for (int s = 0; s < kTeamStages; ++s) mbar_init(bars + 8u * s, 1u);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-
-    const int R = p.batch.num_reqs;
-    const int32_t* unit_prefix = plan_array(p.scratch, 0, R);
-    const int32_t* item_prefix = plan_array(p.scratch, 1, R);
-    const int32_t* page_lo_a = plan_array(p.scratch, 2, R);
-    const int32_t* npages_a = plan_array(p.scratch, 3, R);
-    const int32_t* ngroups_a = plan_array(p.scratch, 4, R);
-    float* partials = reinterpret_cast<float*>(p.scratch + plan_bytes(R));
-
-    const int worker = blockIdx.x * kTeams + team;
-    const int per = hdr->units_per_warp;
-    const int total_units = hdr->total_units;
-    const long long u_ll = (long long)worker * per;
-    if (per <= 0 || u_ll >= total_units) return;   // whole team leaves together
-    int u = (int)u_ll;
-    const int u_end = min(u + per, total_units);
-
-    const int gid = lane >> 2, tig = lane & 3;
-    const int key_a = (gid & 3) + 8 * (gid >> 2);
-    const int kv0 = 2 * (tig & 1) + 8 * (tig >> 1);
-    const uint32_t lut_lane = lut_addr + 4u * lane;
-    // Softmax owners are rotated from team to team so that the schedulers, which each host one
-    // warp of every team, share the softmax work evenly.
-    const int tile = (t + 4 - (team & 3)) & 3;   // query tile this warp owns, if < NT
-    const bool owner = tile < NT;
-    uint32_t phase_bits = 0, pending = 0;
-    bool failed = false;
-
-    int r;
-    {
-        int lo = 0, hi = R;
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (unit_prefix[mid] <= u) lo = mid; else hi = mid;
-        }
-        r = lo;
-    }
-
-    while (u < u_end) {
-        while (unit_prefix[r + 1] <= u) ++r;
-        const int npages = npages_a[r];
-        const int ngroups = ngroups_a[r];
-        const int in_req = u - unit_prefix[r];
-        const int item = in_req / npages;
-        const int page_in_item = in_req - item * npages;
-        const int n_here = min(u_end - u, npages - page_in_item);
-        const int kv_head = item / ngroups;
-        const int group = item - kv_head * ngroups;
-        const int pg0 = page_lo_a[r] + page_in_item;
-        const int slot = worker + item_prefix[r] + item;
-        const ReqGeom g = load_req(p.batch, r);
-        const int rows_in_req = g.q_len * p.gqa;
-
-        // ---- limits: this lane's two rows of the tile it owns, and the group-wide safe range ----
-        int rmax[2] = {-1, -1}, rmin[2] = {0x7fffffff, 0x7fffffff};
-        int safe_hi = 0x7fffffff, safe_lo = 0;
-        for (int row = group * RG + lane; row < group * RG + RG; row += 32) {   // RG <= 32: one pass
-            const int q_off = row / p.gqa;
-            const bool ok = row < rows_in_req &&
-                            (p.batch.valid_token_mask == nullptr || p.batch.valid_token_mask[g.q_start + q_off] != 0);
-            if (ok) {
-                safe_hi = row_max_kv(p.batch, g, q_off);
-                safe_lo = row_min_kv(p.batch, g, q_off);
-            }
-        }
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-            safe_hi = min(safe_hi, __shfl_xor_sync(0xffffffffu, safe_hi, d));
-            safe_lo = max(safe_lo, __shfl_xor_sync(0xffffffffu, safe_lo, d));
-        }
-        if (owner) {
-#pragma unroll
-            for (int x = 0; x < 2; ++x) {
-                const int row = group * RG + 8 * tile + 2 * tig + x;
-                const int q_off = row / p.gqa;
-                const bool ok = row < rows_in_req &&
-                                (p.batch.valid_token_mask == nullptr || p.batch.valid_token_mask[g.q_start + q_off] != 0);
-                if (ok) { rmax[x] = row_max_kv(p.batch, g, q_off); rmin[x] = row_min_kv(p.batch, g, q_off); }
-            }
-        }
-
-        // ---- stage Q' (fp16 [RG][256], pre-scaled) in the idle ring; warp t rotates rows t, t+4, ...
-        __half* q_stage = reinterpret_cast<__half*>(ring_gen);
-        for (int row8 = t; row8 < RG; row8 += kTeamWarps) {
-            const int row = group * RG + row8;
-            const int q_off = row / p.gqa;
-            const int q_head = kv_head * p.gqa + (row - q_off * p.gqa);
-            const bool ok = row < rows_in_req &&
-                            (p.batch.valid_token_mask == nullptr || p.batch.valid_token_mask[g.q_start + q_off] != 0);
-            float tv[8];
-            if (ok) {
-                const size_t q_base = ((size_t)(g.q_start + q_off) * p.num_q_heads + q_head) * kHeadDim;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) tv[j] = apply_sign(load_act(p.q_in, q_base + lane + 32 * j, p.io_bf16), lane + 32 * j);
-                wht256_lanes(tv, lane);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) tv[j] = 0.0f;
-            }
-#pragma unroll
-            for (int j = 0; j < 8; ++j) q_stage[row8 * kHeadDim + lane + 32 * j] = __float2half_rn(tv[j] * p.q_scale);
-        }
-        team_barrier(team);
-        // B fragments: k-step ks = 2 j + hk covers elements 4 hk .. 4 hk + 3 of virtual word
-        // vw_j = 2 cset + j + 4 tig of this warp's half.
-        uint32_t qb[4][NT][2];
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int vw = 2 * cset + j + 4 * tig;
-#pragma unroll
-            for (int hk = 0; hk < 2; ++hk) {
-#pragma unroll
-                for (int nt = 0; nt < NT; ++nt) {
-#pragma unroll
-                    for (int x = 0; x < 2; ++x) {
-                        const int e = 4 * hk + 2 * x;
-                        const __half lo = q_stage[(8 * nt + gid) * kHeadDim + vword_col(half, vw, e)];
-                        const __half hi = q_stage[(8 * nt + gid) * kHeadDim + vword_col(half, vw, e + 1)];
-                        qb[2 * j + hk][nt][x] = (uint32_t)__half_as_ushort(lo) | ((uint32_t)__half_as_ushort(hi) << 16);
-                    }
-                }
-            }
-        }
-        team_barrier(team);   // everyone has its fragments before copies overwrite the staging area
-
-        float o[4][NT][4];
-#pragma unroll
-        for (int mt = 0; mt < 4; ++mt) {
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt) { o[mt][nt][0] = o[mt][nt][1] = o[mt][nt][2] = o[mt][nt][3] = 0.0f; }
-        }
-        float m_run[2] = {-1e30f, -1e30f};
-        float l_run[2] = {0.0f, 0.0f};
-
-        const int32_t* blocks = p.batch.block_tables + (size_t)r * p.batch.max_blocks_per_req;
-        const uint8_t* k_head_base = (const uint8_t*)(uintptr_t)p.layout.k_base + (size_t)kv_head * p.layout.k_head_stride_bytes;
-        const uint8_t* v_head_base = (const uint8_t*)(uintptr_t)p.layout.v_base + (size_t)kv_head * p.layout.v_head_stride_bytes;
-        // page ids are only needed by the issuing warp (t == 0)
-        int32_t my_page = (t == 0 && lane < n_here) ? block_table_page(blocks, pg0 + lane, p.batch.max_blocks_per_req, kInTeam) : 0;
-        int32_t next_page = (t == 0 && 32 + lane < n_here) ? block_table_page(blocks, pg0 + 32 + lane, p.batch.max_blocks_per_req, kInTeam) : 0;
-
-        fence_proxy_async();
-        auto issue = [&](int idx) {
-            pending |= 1u << (idx % kTeamStages);
-            if (t == 0) {
-                const int32_t page = __shfl_sync(0xffffffffu, (idx & 32) ? next_page : my_page, idx & 31);
-                if (lane == 0) {
-                    const int s = idx % kTeamStages;
-                    const uint32_t bar = bars + 8u * s;
-                    const uint32_t dst = ring + (uint32_t)s * kStageStride;
-                    const uint8_t* ksrc = k_head_base + (size_t)page * p.layout.k_page_stride_bytes;
-                    const uint8_t* vsrc = v_head_base + (size_t)page * p.layout.v_page_stride_bytes;
-                    mbar_expect_tx(bar, 4 * kHalfBytes);
-                    bulk_g2s(dst, ksrc, kHalfBytes, bar);
-                    bulk_g2s(dst + kHalfStride, ksrc + kHalfBytes, kHalfBytes, bar);
-                    bulk_g2s(dst + kRunStride, vsrc, kHalfBytes, bar);
-                    bulk_g2s(dst + kRunStride + kHalfStride, vsrc + kHalfBytes, kHalfBytes, bar);
-                }
-            }
-        };
-        // The page ids of units [32 c, 32 c + 32) alternate between my_page (c even) and next_page
-        // (c odd); a window is replaced once every unit in it has been issued.
-#pragma unroll 1
-        for (int i = 0; i < kTeamStages && i < n_here; ++i) issue(i);
-
-        // One meeting per page.  Iteration i: partial scores of page i -> meet -> (output product
-        // of page i - 1, whose P fragments the owners published before arriving) -> owners'
-        // softmax of page i -> V look-ups of page i.  The softmax of one page thus overlaps the
-        // score product of the next in the other warps.
-        uint32_t av[4][4];
-        auto pv_product = [&](int buf) {
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt) {
-                const float2 al = lds64f(ax + (uint32_t)(buf * (NT * 32) + (nt * 4 + tig) * 8));
-                const uint32_t pb0 = lds32(px + (uint32_t)(buf * (NT * 512) + nt * 512 + half * 256 + lane * 4));
-                const uint32_t pb1 = lds32(px + (uint32_t)(buf * (NT * 512) + nt * 512 + half * 256 + 128 + lane * 4));
-                if (__any_sync(0xffffffffu, al.x != 1.0f || al.y != 1.0f)) {
-#pragma unroll
-                    for (int mt = 0; mt < 4; ++mt) {
-                        o[mt][nt][0] *= al.x; o[mt][nt][1] *= al.y; o[mt][nt][2] *= al.x; o[mt][nt][3] *= al.y;
-                    }
-                }
-#pragma unroll
-                for (int mt = 0; mt < 4; ++mt) mma16816(o[mt][nt], av[mt][0], av[mt][1], av[mt][2], av[mt][3], pb0, pb1);
-            }
-        };
-
-#pragma unroll 1
-        for (int i = 0; i < n_here; ++i) {
-            const int s = i % kTeamStages;
-            const int buf = i & 1;
-            if (!failed && !mbar_wait(bars + 8u * s, (phase_bits >> s) & 1u)) {
-                failed = true;                      // results are void; keep meeting the team's barriers
-                if (lane == 0) atomicOr(&hdr->status, 1);
-            }
-            phase_bits ^= 1u << s;
-            pending &= ~(1u << s);
-
-            const uint32_t kst = ring + (uint32_t)s * kStageStride;
-            const uint32_t vst = kst + kRunStride;
-            const int kv_base = (pg0 + i) << 4;
-            const bool full = (kv_base >= safe_lo) && (kv_base + 15 <= safe_hi);
-#define W34_LUT(word, k) lds32(__byte_perm((word), lut_lane, 0x7604 + ((k) << 4)))
-
-            // ---- partial scores over this warp's 64 channels -------------------------------
-            {
-                float sa[NT][4];
-#pragma unroll
-                for (int nt = 0; nt < NT; ++nt) { sa[nt][0] = sa[nt][1] = sa[nt][2] = sa[nt][3] = 0.0f; }
-                const uint32_t krow_a = kst + token_offset(key_a);
-                const uint32_t krow_b = krow_a + 4u * kTq4RowBytes;
-                const uint32_t sw_a = lds32(krow_a + (half ? 64u : 0u));   // word holding this half's scale
-                const uint32_t sw_b = lds32(krow_b + (half ? 64u : 0u));
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    const uint32_t off = 4u * ((half ? 17u : 0u) + 2u * cset + j + 4u * tig);
-                    uint32_t wa = lds32(krow_a + off);
-                    uint32_t wb = lds32(krow_b + off);
-                    if (j == 0 && t == 0 && tig == 0) {   // virtual word 0 of half 0: splice
-                        wa = (wa >> 16) | (lds32(krow_a + 64) << 16);
-                        wb = (wb >> 16) | (lds32(krow_b + 64) << 16);
-                    }
-#pragma unroll
-                    for (int hk = 0; hk < 2; ++hk) {
-                        const uint32_t a0 = W34_LUT(wa, 2 * hk);
-                        const uint32_t a1 = W34_LUT(wb, 2 * hk);
-                        const uint32_t a2 = W34_LUT(wa, 2 * hk + 1);
-                        const uint32_t a3 = W34_LUT(wb, 2 * hk + 1);
-#pragma unroll
-                        for (int nt = 0; nt < NT; ++nt) {
-                            mma16816(sa[nt], a0, a1, a2, a3, qb[2 * j + hk][nt][0], qb[2 * j + hk][nt][1]);
-                        }
-                    }
-                }
-                const float dka = __half2float(__ushort_as_half((unsigned short)(half ? (sw_a >> 16) : (sw_a & 0xffffu))));
-                const float dkb = __half2float(__ushort_as_half((unsigned short)(half ? (sw_b >> 16) : (sw_b & 0xffffu))));
-#pragma unroll
-                for (int nt = 0; nt < NT; ++nt) {
-                    sts128f(sx + (uint32_t)(buf * (kTeamWarps * NT * 512) + (t * NT + nt) * 512 + lane * 16),
-                            make_float4(dka * sa[nt][0], dka * sa[nt][1], dkb * sa[nt][2], dkb * sa[nt][3]));
-                }
-            }
-            team_barrier(team);   // scores of page i are in shared memory; so is everything of page i - 1
-
-            // page i - 1 is finished by every warp once it has passed this point's output product,
-            // which the NEXT meeting certifies: refill the stage of page i - 1 now that all warps
-            // have passed the meeting of page i (they read stage i - 1 before arriving).
-            if (i >= 1 && i - 1 + kTeamStages < n_here) {
-                if (t == 0 && ((i - 1 + kTeamStages) & 31) == 0) {
-                    // entering a new id window: the window being replaced was fully issued long ago
-                    const int base = i - 1 + kTeamStages + 32;
-                    const int32_t fresh = (base + lane < n_here) ? block_table_page(blocks, pg0 + base + lane, p.batch.max_blocks_per_req, kInTeam) : 0;
-                    if ((i - 1 + kTeamStages) & 32) my_page = fresh; else next_page = fresh;
-                }
-                issue(i - 1 + kTeamStages);
-            }
-            if (i >= 1) pv_product(buf ^ 1);
-
-            // ---- the owner of query tile t sums the partials and runs the online softmax -------
-            if (owner) {
-                float sc[4];
-                {
-                    const uint32_t sb = sx + (uint32_t)(buf * (kTeamWarps * NT * 512) + tile * 512 + lane * 16);
-                    const float4 p0 = lds128f(sb + 0 * NT * 512);
-                    const float4 p1 = lds128f(sb + 1 * NT * 512);
-                    const float4 p2 = lds128f(sb + 2 * NT * 512);
-                    const float4 p3 = lds128f(sb + 3 * NT * 512);
-                    sc[0] = ((p0.x + p1.x) + p2.x) + p3.x;
-                    sc[1] = ((p0.y + p1.y) + p2.y) + p3.y;
-                    sc[2] = ((p0.z + p1.z) + p2.z) + p3.z;
-                    sc[3] = ((p0.w + p1.w) + p2.w) + p3.w;
-                }
-                const uint32_t vrow_a = vst + token_offset(key_a);
-                const uint32_t va0 = lds32(vrow_a), va16 = lds32(vrow_a + 64);
-                const uint32_t vb0 = lds32(vrow_a + 4u * kTq4RowBytes), vb16 = lds32(vrow_a + 4u * kTq4RowBytes + 64);
-                float dva0 = __half2float(__ushort_as_half((unsigned short)(va0 & 0xffffu)));
-                float dva1 = __half2float(__ushort_as_half((unsigned short)(va16 >> 16)));
-                float dvb0 = __half2float(__ushort_as_half((unsigned short)(vb0 & 0xffffu)));
-                float dvb1 = __half2float(__ushort_as_half((unsigned short)(vb16 >> 16)));
-                bool msk[4] = {false, false, false, false};
-                if (!full) {
-                    const int pos_a = kv_base + key_a, pos_b = pos_a + 4;
-                    msk[0] = !(pos_a >= rmin[0] && pos_a <= rmax[0]);
-                    msk[1] = !(pos_a >= rmin[1] && pos_a <= rmax[1]);
-                    msk[2] = !(pos_b >= rmin[0] && pos_b <= rmax[0]);
-                    msk[3] = !(pos_b >= rmin[1] && pos_b <= rmax[1]);
-#pragma unroll
-                    for (int x = 0; x < 4; ++x) if (msk[x]) sc[x] = -1e30f;
-                }
-                float mx0 = fmaxf(sc[0], sc[2]), mx1 = fmaxf(sc[1], sc[3]);
-#pragma unroll
-                for (int d = 4; d < 32; d <<= 1) {
-                    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, d));
-                    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, d));
-                }
-                const float mn0 = fmaxf(m_run[0], mx0), mn1 = fmaxf(m_run[1], mx1);
-                const float al0 = ex2(m_run[0] - mn0), al1 = ex2(m_run[1] - mn1);  // 1 when the max did not grow
-                l_run[0] *= al0;
-                l_run[1] *= al1;
-                m_run[0] = mn0;
-                m_run[1] = mn1;
-                float pr[4];
-                pr[0] = ex2(sc[0] - mn0);
-                pr[1] = ex2(sc[1] - mn1);
-                pr[2] = ex2(sc[2] - mn0);
-                pr[3] = ex2(sc[3] - mn1);
-                if (!full) {
-#pragma unroll
-                    for (int x = 0; x < 4; ++x) if (msk[x]) pr[x] = 0.0f;
-                    if (msk[0] && msk[1]) { dva0 = 0.0f; dva1 = 0.0f; }
-                    if (msk[2] && msk[3]) { dvb0 = 0.0f; dvb1 = 0.0f; }
-                }
-                l_run[0] += pr[0] + pr[2];
-                l_run[1] += pr[1] + pr[3];
-                const uint32_t pbase = px + (uint32_t)(buf * (NT * 512) + tile * 512 + lane * 4);
-                sts32(pbase + 0, movmatrix_trans(pack_half2(pr[0] * dva0, pr[1] * dva0)));
-                sts32(pbase + 128, movmatrix_trans(pack_half2(pr[2] * dvb0, pr[3] * dvb0)));
-                sts32(pbase + 256, movmatrix_trans(pack_half2(pr[0] * dva1, pr[1] * dva1)));
-                sts32(pbase + 384, movmatrix_trans(pack_half2(pr[2] * dvb1, pr[3] * dvb1)));
-                if (gid == 0) sts64f(ax + (uint32_t)(buf * (NT * 32) + (tile * 4 + tig) * 8), make_float2(al0, al1));
-            }
-
-            // ---- V look-ups of page i (its product runs after the next meeting) ----------------
-            {
-                const uint32_t vr = vst + token_offset(kv0);
-                const uint32_t vw = 4u * (uint32_t)(gid >> 1) + (uint32_t)(gid & 1) + 2u * cset;
-                const uint32_t off = 4u * ((half ? 17u : 0u) + vw);
-                uint32_t w[4];
-                w[0] = lds32(vr + off);
-                w[1] = lds32(vr + kTq4RowBytes + off);
-                w[2] = lds32(vr + 4u * kTq4RowBytes + off);
-                w[3] = lds32(vr + 5u * kTq4RowBytes + off);
-                if (t == 0 && gid == 0) {
-                    w[0] = (w[0] >> 16) | (lds32(vr + 64) << 16);
-                    w[1] = (w[1] >> 16) | (lds32(vr + kTq4RowBytes + 64) << 16);
-                    w[2] = (w[2] >> 16) | (lds32(vr + 4u * kTq4RowBytes + 64) << 16);
-                    w[3] = (w[3] >> 16) | (lds32(vr + 5u * kTq4RowBytes + 64) << 16);
-                }
-                const uint32_t lo_ab = (w[0] & 0x0f0f0f0fu) | ((w[1] << 4) & 0xf0f0f0f0u);
-                const uint32_t hi_ab = ((w[0] >> 4) & 0x0f0f0f0fu) | (w[1] & 0xf0f0f0f0u);
-                const uint32_t lo_cd = (w[2] & 0x0f0f0f0fu) | ((w[3] << 4) & 0xf0f0f0f0u);
-                const uint32_t hi_cd = ((w[2] >> 4) & 0x0f0f0f0fu) | (w[3] & 0xf0f0f0f0u);
-#pragma unroll
-                for (int mt = 0; mt < 4; ++mt) {
-                    av[mt][0] = W34_LUT(lo_ab, mt);
-                    av[mt][1] = W34_LUT(hi_ab, mt);
-                    av[mt][2] = W34_LUT(lo_cd, mt);
-                    av[mt][3] = W34_LUT(hi_cd, mt);
-                }
-            }
-#undef W34_LUT
-        }
-        team_barrier(team);   // the owners' last softmax is published
-        if (n_here > 0) pv_product((n_here - 1) & 1);
-
-        // ---- write the partial of this segment ------------------------------------------------
-        if (slot < p.max_slots) {
-            float* dst = partials + (size_t)slot * PARTIAL;
-            const int vw = 4 * (gid >> 1) + (gid & 1) + 2 * cset;
-#pragma unroll
-            for (int mt = 0; mt < 4; ++mt) {
-                const int ca = vword_col(half, vw, 2 * mt), cb = vword_col(half, vw, 2 * mt + 1);
-#pragma unroll
-                for (int nt = 0; nt < NT; ++nt) {
-                    const int r0 = 8 * nt + 2 * tig;
-                    dst[r0 * kHeadDim + ca] = o[mt][nt][0];
-                    dst[(r0 + 1) * kHeadDim + ca] = o[mt][nt][1];
-                    dst[r0 * kHeadDim + cb] = o[mt][nt][2];
-                    dst[(r0 + 1) * kHeadDim + cb] = o[mt][nt][3];
-                }
-            }
-            if (owner) {
-#pragma unroll
-                for (int d = 4; d < 32; d <<= 1) {
-                    l_run[0] += __shfl_xor_sync(0xffffffffu, l_run[0], d);
-                    l_run[1] += __shfl_xor_sync(0xffffffffu, l_run[1], d);
-                }
-                if (gid == 0) {
-                    const int r0 = 8 * tile + 2 * tig;
-                    dst[RG * kHeadDim + r0] = m_run[0];
-                    dst[RG * kHeadDim + r0 + 1] = m_run[1];
-                    dst[RG * kHeadDim + RG + r0] = l_run[0];
-                    dst[RG * kHeadDim + RG + r0 + 1] = l_run[1];
-                }
-            }
-        }
-        team_barrier(team);   // the staging area is rewritten by the next segment
-        u += n_here;
-    }
-    if (failed) {
-        for (int s = 0; s < kTeamStages; ++s) {
-            if (pending & (1u << s)) (void)mbar_wait(bars + 8u * s, (phase_bits >> s) & 1u);
-        }
-    }
-}
 
 // ---------------------------------------------------------------------------------------
 // Helpers shared by the tile-based kernels (tcgen05 prefill, uncompressed bf16 KV).
@@ -2188,12 +1714,6 @@ static DeviceInfo* device_info(int* rc) {
         *rc = (int)cudaFuncSetAttribute(tq4_attention_stream_exact_kernel<true>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
         if (*rc != 0) return nullptr;
-        *rc = (int)cudaFuncSetAttribute(tq4_attention_team_kernel<2>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-        if (*rc != 0) return nullptr;
-        *rc = (int)cudaFuncSetAttribute(tq4_attention_team_kernel<3>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-        if (*rc != 0) return nullptr;
         *rc = (int)cudaFuncSetAttribute(attention_prefill_pair_kernel<WARP34_KV_FORMAT_TQ4>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PpSmem<WARP34_KV_FORMAT_TQ4>::kBytes);
         if (*rc != 0) return nullptr;
@@ -2247,26 +1767,13 @@ static long long qfrag_items(const warp34_kv_layer_layout* l, const warp34_atten
     return (long long)b->num_reqs * l->local_kv_heads * groups;
 }
 
-// Query rows that share one KV pass.  Exact build: 8, one warp per work item; a request with more
-// rows per kv head (several draft tokens) becomes several items that read the same pages, close
-// enough in time for the second and third read to come from L2.  Fast build: 8 with one warp per
-// item, 16 or 24 with four-warp teams.
-static int pick_row_tiles(const warp34_attention_batch* b, int gqa, bool fast) {
-    const long long rows = (long long)(b->max_q_len > 0 ? b->max_q_len : 1) * gqa;
-    if (!fast || rows <= 8) return 1;
-    return rows <= 16 ? 2 : 3;
-}
-
-// Workspace of the streaming path with `workers` worker warps (or teams): plan, one partial slot
-// per worker and per work item, and the query fragments of one-warp items.
-static size_t stream_scratch_bytes(const warp34_kv_layer_layout* l, const warp34_attention_batch* b, int hq,
-                                   bool fast, long long workers) {
-    const int gqa = hq / l->local_kv_heads;
-    const int nt = pick_row_tiles(b, gqa, fast);
-    const int rpg = 8 * nt;
-    const long long slots = workers + items_bound(l, b, hq, rpg);
-    const size_t qfrag = (nt == 1) ? (size_t)qfrag_items(l, b, gqa) * qfrag_item_bytes() : 0;
-    return plan_bytes(b->num_reqs) + (size_t)slots * (size_t)(rpg * kHeadDim + 2 * rpg) * sizeof(float) + qfrag;
+// Workspace of the one-warp streaming path with `workers` worker warps: plan, one partial slot per worker and per work item (8
+// query rows; a request with more becomes several items that read the same pages, close enough in time for the second and third
+// read to come from L2), and the query fragments.
+static size_t stream_scratch_bytes(const warp34_kv_layer_layout* l, const warp34_attention_batch* b, int hq, long long workers) {
+    const long long slots = workers + items_bound(l, b, hq, kRowsPerGroup);
+    return plan_bytes(b->num_reqs) + (size_t)slots * kPartialFloats * sizeof(float) +
+           (size_t)qfrag_items(l, b, hq / l->local_kv_heads) * qfrag_item_bytes();
 }
 
 // The tcgen05 stream kernel: rows per item (16 or 24: all of a request's rows per kv head, 0: too few or too many) and its workspace.
@@ -2278,9 +1785,10 @@ static size_t xt_scratch_bytes(const warp34_kv_layer_layout* l, const warp34_att
     return plan_bytes(b->num_reqs) + ((size_t)grid + (size_t)items_bound(l, b, hq, rows)) * (size_t)(rows * kHeadDim + 2 * rows) * sizeof(float) +
            (size_t)b->num_reqs * l->local_kv_heads * xt_query_bytes(rows);
 }
-// It is taken from one block of 128 keys up.  Measured against the one-warp kernel over 9 to 24 rows, 1 to 128 requests of 128 to
-// 65536 keys: never behind by more than 4 %, 1.1 to 1.5 times as fast from 512 keys; at 64 keys, where a block is mostly padding,
-// 0.85 to 1.04.  (At 8 rows and below half of its score columns would be empty: 700 against 520 us on 64 sequences of 4096 to 16384.)
+// It is taken from one block of 128 keys up, with the fast flag too.  Measured against the one-warp kernel over 9 to 24 rows, 1 to
+// 128 requests of 128 to 65536 keys: never behind by more than 4 %, 1.1 to 1.5 times as fast from 512 keys; at 64 keys, where a block
+// is mostly padding, 0.85 to 1.04.  (At 8 rows and below half of its score columns would be empty: 577 against 520 us on 64
+// sequences of 4096 to 16384.)
 static bool takes_tiles(const warp34_exec* ex, const warp34_kv_layer_layout* l, const warp34_attention_batch* b, int hq, int rows, int sms) {
     if (rows == 0) return false;
     const long long keys = b->max_seq_len > 0 ? b->max_seq_len : (long long)b->max_blocks_per_req * kPageTokens;   // max_seq_len is optional
@@ -2430,13 +1938,10 @@ extern "C" size_t warp34_paged_attention_scratch_bytes(const warp34_kv_layer_lay
     const int sms = d ? d->sm_count : 148;
     // enough for a full grid in either build
     const int gqa = num_q_heads / layout->local_kv_heads;
-    const int nt_fast = w34::pick_row_tiles(batch, gqa, true);
-    const size_t fast = w34::stream_scratch_bytes(layout, batch, num_q_heads, true,
-                                                  (long long)sms * (nt_fast == 1 ? w34::kFastWarps : w34::kTeams));
-    const size_t exact = w34::stream_scratch_bytes(layout, batch, num_q_heads, false, (long long)sms * w34::kExactWarps);
+    const size_t most = w34::stream_scratch_bytes(layout, batch, num_q_heads,
+                                                  (long long)sms * (w34::kFastWarps > w34::kExactWarps ? w34::kFastWarps : w34::kExactWarps));
     const int rows = w34::xt_rows(batch, gqa);
     const size_t tiles = rows != 0 ? w34::xt_scratch_bytes(layout, batch, num_q_heads, rows, sms) : 0;
-    const size_t most = fast > exact ? fast : exact;
     return most > tiles ? most : tiles;
 }
 
@@ -2542,21 +2047,18 @@ static int launch_attention(const warp34_exec* ex, const warp34_kv_layer_layout*
     }
 
     // Streaming path: canonical layout, scratch that holds the plan plus at least one partial
-    // per item and per worker, unit count within int32.  Workers are warps (8 query rows per
-    // item) or four-warp teams (16 / 24 rows per item).
+    // per item and per worker, unit count within int32.
     const bool fast = (ex->flags & WARP34_B200_EXEC_FLAG_FAST_ATTENTION) != 0;
-    const int nt = pick_row_tiles(batch, gqa, fast);
-    const int rpg = 8 * nt;
-    const int workers_per_cta = (nt == 1) ? (fast ? kFastWarps : kExactWarps) : kTeams;
-    const size_t slot_bytes = (size_t)(rpg * kHeadDim + 2 * rpg) * sizeof(float);
+    const int workers_per_cta = fast ? kFastWarps : kExactWarps;
+    const size_t slot_bytes = (size_t)kPartialFloats * sizeof(float);
     const long long full_workers = (long long)dev->sm_count * workers_per_cta;
     const bool stream_ok = (ex->flags & WARP34_B200_EXEC_FLAG_PRECISE_ATTENTION) == 0 &&
                            stream_layout_ok(layout) && ex->scratch_ptr != 0 && (ex->scratch_ptr & 15u) == 0u &&
                            batch->max_blocks_per_req > 0;
-    if (nt == 1 && qfrag_items(layout, batch, gqa) > 0x3fffffffll) return (int)cudaErrorInvalidValue;
+    if (qfrag_items(layout, batch, gqa) > 0x3fffffffll) return (int)cudaErrorInvalidValue;
 
     const int tile_rows = xt_rows(batch, gqa);
-    if (stream_ok && !fast && force < 0 && takes_tiles(ex, layout, batch, num_q_heads, tile_rows, dev->sm_count)) {
+    if (stream_ok && force < 0 && takes_tiles(ex, layout, batch, num_q_heads, tile_rows, dev->sm_count)) {
         cudaStream_t st = (cudaStream_t)ex->stream;
         const long long items = items_bound(layout, batch, num_q_heads, tile_rows);
         const long long q_items = (long long)batch->num_reqs * layout->local_kv_heads;
@@ -2597,9 +2099,9 @@ static int launch_attention(const warp34_exec* ex, const warp34_kv_layer_layout*
         warp34_attention_batch b = *batch;
         b.num_reqs = reqs;
         b.total_tokens = (int)tokens;
-        const long long items = items_bound(layout, &b, num_q_heads, rpg);
+        const long long items = items_bound(layout, &b, num_q_heads, kRowsPerGroup);
         if (items * (long long)batch->max_blocks_per_req >= 0x7fffffffll) return -1;
-        const size_t fixed = plan_bytes(reqs) + ((nt == 1) ? (size_t)qfrag_items(layout, &b, gqa) * qfrag_item_bytes() : 0);
+        const size_t fixed = plan_bytes(reqs) + (size_t)qfrag_items(layout, &b, gqa) * qfrag_item_bytes();
         const size_t avail = ex->scratch_size > fixed ? ex->scratch_size - fixed : 0;
         const long long w = (long long)(avail / slot_bytes) - items;
         return w < 0 ? 0 : w;
@@ -2625,8 +2127,8 @@ static int launch_attention(const warp34_exec* ex, const warp34_kv_layer_layout*
         p.layout = *layout;
         p.batch = *batch;
         if (in_parts) p.batch = batch_part(batch, r0, reqs);
-        const long long items = items_bound(layout, &p.batch, num_q_heads, rpg);
-        const long long q_items = (nt == 1) ? qfrag_items(layout, &p.batch, gqa) : 0;
+        const long long items = items_bound(layout, &p.batch, num_q_heads, kRowsPerGroup);
+        const long long q_items = qfrag_items(layout, &p.batch, gqa);
         long long part_workers = in_parts ? workers_for(reqs, p.batch.total_tokens) : workers;   // the last part is smaller
         if (part_workers > full_workers) part_workers = full_workers;
         const int grid = (int)(part_workers / workers_per_cta);
@@ -2641,26 +2143,20 @@ static int launch_attention(const warp34_exec* ex, const warp34_kv_layer_layout*
         p.gqa = gqa;
         p.num_warps = grid * workers_per_cta;
         p.max_slots = (int)(p.num_warps + items);
-        p.rows_per_group = rpg;
+        p.rows_per_group = kRowsPerGroup;
         p.q_scale = batch->sm_scale * 1.4426950408889634f / kLutScale;
         p.natural = 0;
         p.q_floor = fast ? 0 : 1;
         p.og = og;
         p.rows_from_first_token = in_parts ? 1 : 0;
         p.keep_status = r0 > 0 ? 1 : 0;
-        p.qfrag = (nt == 1) ? reinterpret_cast<uint32_t*>(p.scratch + plan + (size_t)p.max_slots * slot_bytes) : nullptr;
+        p.qfrag = reinterpret_cast<uint32_t*>(p.scratch + plan + (size_t)p.max_slots * slot_bytes);
         p.smem_bytes = (uint32_t)smem;
-        p.q_groups_max = (nt == 1) ? (int)(q_items / ((long long)reqs * layout->local_kv_heads)) : 0;
+        p.q_groups_max = (int)(q_items / ((long long)reqs * layout->local_kv_heads));
         rc = launch_behind(tq4_attention_plan_kernel, 1 + (unsigned)q_items, q_items > 0 ? kPlanThreads : 32, 0, st, p);
         if (rc != 0) return rc;
-        if (nt == 1) {
-            if (fast) tq4_attention_stream_kernel<kFastStages, kFastWarps><<<grid, kFastWarps * 32, smem, st>>>(p);
-            else rc = launch_behind(tq4_attention_stream_exact_kernel<false>, (unsigned)grid, kXThreads, smem, st, p);
-        } else if (nt == 2) {
-            tq4_attention_team_kernel<2><<<grid, kTeams * kTeamWarps * 32, smem, st>>>(p);
-        } else {
-            tq4_attention_team_kernel<3><<<grid, kTeams * kTeamWarps * 32, smem, st>>>(p);
-        }
+        if (fast) tq4_attention_stream_kernel<kFastStages, kFastWarps><<<grid, kFastWarps * 32, smem, st>>>(p);
+        else rc = launch_behind(tq4_attention_stream_exact_kernel<false>, (unsigned)grid, kXThreads, smem, st, p);
         // rows of the merge: every token of the batch, or (a part) as many as the part can hold, counted
         // from its first token
         const long long rows = (long long)p.batch.total_tokens * num_q_heads;
@@ -2918,7 +2414,7 @@ extern "C" int warp34_paged_attention_f16_static_scratch(uintptr_t stream, const
     const int gqa = num_q_heads / layout->local_kv_heads;
     const size_t needed = w34::takes_prefill_path(0, layout, batch, gqa)
                               ? sizeof(w34::PlanHeader)
-                              : w34::stream_scratch_bytes(layout, batch, num_q_heads, false, w34::kExactWarps);
+                              : w34::stream_scratch_bytes(layout, batch, num_q_heads, w34::kExactWarps);
     if (scratch_needed != nullptr) *scratch_needed = needed;
     if (needed > kStaticScratchBytes) return (int)cudaErrorInvalidValue;  // batch too large for the built-in workspace
     warp34_exec ex;

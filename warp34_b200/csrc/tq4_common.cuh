@@ -126,7 +126,7 @@ static int launch_behind(void (*kernel)(const Params), dim3 grid, unsigned threa
 // layer descriptor does not carry the pool's page count, so the host states it once with
 // warp34_bounds_set_pool_pages().  Without the define these helpers cost nothing.
 enum { kBoundsBlockIndex = 1, kBoundsPageId = 2, kBoundsWriteSlot = 3 };
-enum { kInAppend = 1, kInScalar = 2, kInStream = 3, kInTeam = 4, kInPrefillExact = 5, kInPrefillTc = 6,
+enum { kInAppend = 1, kInScalar = 2, kInStream = 3, kInPrefillExact = 5, kInPrefillTc = 6,
        kInBf16 = 7, kInKv8 = 8, kInSparse = 9 };
 #ifdef W34_BOUNDS
 struct BoundsWord { int what, value, limit, count; };
