@@ -5,22 +5,23 @@
 // page) units and walks it in blocks of 128 keys.  The cached keys are the M dimension of both products, so that every code
 // is dequantised once for up to 24 query rows, and straight into tensor memory, where it is the MMAs' A operand:
 //   S^T[128 keys x 2R]      per 128-half = Khi [Q'hi | Q'lo]^T + Klo [Q'hi | Q'lo]^T        lane = key
-//   O^T[128 channels x 2R]  per 128-half += Vhi^T [(P d_v)hi | (P d_v)lo]^T                  lane = channel
-// (on blocks with a large weight also the V centroids' residual).  Scales stay outside the operands: a thread holds a key's
+//   O^T[128 channels x 2R]  per 128-half += (Vhi + Vlo)^T [(P d_v)hi | (P d_v)lo]^T          lane = channel
+// (the centroids' residuals on every block: leaving them out where no key has a large weight takes one more vote of the softmax
+// warps a block, 920 us against 914, and an error three times as large).  Scales stay outside the operands: a thread holds a key's
 // scores of both halves and applies its K scales there, and P is multiplied by the V scale of its key and half.
 //
 //   softmax: four warps per eight rows, thread = key.  P goes to shared memory as the B operand; the running maximum is a
-//            reference that moves only when it is exceeded by 2^3, so a block usually needs no reduction over its keys, and
-//            the mass known of a row is brought up to date only when a weight looks large against it
-//   V:       eight warps, thread = fragment position (16x256b stores put channel pairs of four keys in place), half x quadrant
+//            reference that moves only when it is exceeded by 2^3, so a block usually needs no reduction over its keys
+//   V:       eight warps, thread = fragment position (16x256b stores put channel pairs of four keys in place), half x quadrant;
+//            64 keys at a time, values into one granule, residuals into the next
 //   K:       eight warps, thread = key, 32 channels at a time into a ring of four TMEM granules; values and residuals lie next
 //            to each other as the table returns them, and the query operand repeats each pair of columns to match
 //   one warp copies raw pages and query rows, one issues the score products, one the output products
 //
-// Measured on 128 requests of 2048 to 16384 keys, four query tokens, 24 / 4 heads (1.26 GB of pages): 920 us against 1458 with
+// Measured on 128 requests of 2048 to 16384 keys, four query tokens, 24 / 4 heads (1.26 GB of pages): 914 us against 1454 with
 // three 8-row items of the one-warp kernel (tq4_stream_exact.cuh), which looks every code up three times.  Bound by the softmax
-// warps' serial chain from scores to P: a block of 128 keys takes about 6700 cycles at 13800 instructions (2.5 per cycle and SM;
-// the shared-memory pipe is 56 % busy, the tensor pipe 22 %).  Taking the weights before the vote on the reference (one barrier
+// warps' serial chain from scores to P: a block of 128 keys takes about 6700 cycles at some 14000 instructions (2.5 per cycle
+// and SM; with the residuals on a fifth of the blocks only, the shared-memory pipe was 56 % and the tensor pipe 22 % busy).  Taking the weights before the vote on the reference (one barrier
 // a block fewer) put them behind the wait for the previous output product: 1008 us.
 #pragma once
 
@@ -39,10 +40,9 @@ __host__ __device__ constexpr uint32_t xt_query_bytes(int rows) { return 2u * (u
 
 struct XtShared {
     float2 k_scale[2][kXtKeys];
-    __align__(16) float m_ref[24], alpha[24], mass[24], cut[24];      // cut: kPeakedWeight of the mass known so far
+    __align__(16) float m_ref[24], alpha[24], mass[24];
     float red[4][24];                // [warp of the part][row]
     int row_min[24], row_max[24];
-    int peak[2];               // of the block's parity: some key has a large weight
     uint32_t tmem;
     uint32_t aborted;
     uint64_t bars[48];
@@ -214,7 +214,6 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
         mbar_init(bar(kXtPReady), W0);
         mbar_init(bar(kXtPvDone), 1u);
         mbar_init(bar(kXtDrain), 2u);
-        sh.peak[0] = sh.peak[1] = 0;
         sh.aborted = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -338,17 +337,15 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
         constexpr uint32_t kIdesc = tc_idesc(128, N, 0);
         const uint64_t desc_p = tc_smem_desc(p_t, 16u, 1024u);
         const uint32_t base = __shfl_sync(0xffffffffu, tmem, 0);
-        uint32_t laps = 0;      // fills of each V granule so far
         bool ok = true;
         while (ok && xt_next(p, walk, sg)) {
             for (int b = 0; ok && kXtPages * b < sg.pages; ++b, ++c) {
                 ok = wait_all(bar(kXtPReady), c & 1u);
-                const int passes = *reinterpret_cast<volatile int*>(&sh.peak[c & 1]) == (int)c + 1 ? 2 : 1;
-                for (int pass = 0; pass < passes && ok; ++pass, ++laps) {
 #pragma unroll
-                    for (int kk = 0; kk < 2; ++kk) {
-                        ok = ok && wait_all(bar(kXtVFull + kk), laps & 1u);
-                        const bool more = (b | pass) != 0;
+                for (int kk = 0; kk < 2; ++kk) {
+#pragma unroll
+                    for (int res = 0; res < 2; ++res) {      // the centroids' values, then their residuals
+                        ok = ok && wait_all(bar(kXtVFull + res), (uint32_t)kk);      // fills 2 c + kk
                         if (ok && elect_one()) {
                             tc_fence_after();
 #pragma unroll
@@ -356,12 +353,12 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
 #pragma unroll
                                 for (int ks = 0; ks < 4; ++ks) {
                                     const uint64_t bp = desc_p + (uint64_t)(h * (int)(kPBytes / 16) + kk * (N * 128 / 16) + 2 * ks);
-                                    const uint32_t d = base + kXtColO + (uint32_t)(h * N), a = base + kXtColV + (uint32_t)(64 * h + 32 * kk + 8 * ks);
-                                    if ((kk | ks) || more) xt_mma<true>(d, a, bp, kIdesc);
+                                    const uint32_t d = base + kXtColO + (uint32_t)(h * N), a = base + kXtColV + (uint32_t)(64 * h + 32 * res + 8 * ks);
+                                    if ((kk | res | ks) || b != 0) xt_mma<true>(d, a, bp, kIdesc);
                                     else xt_mma<false>(d, a, bp, kIdesc);
                                 }
                             }
-                            tc_commit(bar(kXtVEmpty + kk));
+                            tc_commit(bar(kXtVEmpty + res));
                         }
                         __syncwarp();
                     }
@@ -384,7 +381,6 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
         const uint32_t lut_v = lut_addr + 128u + 4u * (uint32_t)lane, lut_r = lut_addr + 8u * (uint32_t)(lane & 15) + 4u;
         // byte 2 (gid & 1) + T of the paired codes belongs to tile T
         const uint32_t sel[2] = {0x7604u + ((uint32_t)(2 * (gid & 1)) << 4), 0x7604u + ((uint32_t)(2 * (gid & 1) + 1) << 4)};
-        uint32_t laps = 0;
         bool ok = true;
         while (ok && xt_next(p, walk, sg)) {
             for (int b = 0; ok && kXtPages * b < sg.pages; ++b, ++c) {
@@ -392,57 +388,58 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                 if (!(ok = wait_all(bar(kXtRawVFull + s), (c / STAGES) & 1u))) break;
                 const uint32_t run = raw_v(s);
                 const uint32_t rows = run + (uint32_t)(4 * tig) * kTq4RowBytes;
-                int passes = 1;
 #pragma unroll 1
-                for (int pass = 0; pass < passes && ok; ++pass, ++laps) {
-                    const uint32_t lut = pass == 0 ? lut_v : lut_r;
-#pragma unroll 1
-                    for (int kk = 0; kk < 2; ++kk) {
-                        uint32_t a[2][16];
-                        uint32_t x[4][4];
+                for (int kk = 0; kk < 2; ++kk) {
+                    uint32_t x[4][4];
+#pragma unroll
+                    for (int pg = 0; pg < 4; ++pg) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) x[pg][k] = lds32(rows + (uint32_t)(4 * kk + pg) * kTq4PageHeadBytes + (uint32_t)k * kTq4RowBytes + word_off);
+                    }
+                    if (splice_warp) {
 #pragma unroll
                         for (int pg = 0; pg < 4; ++pg) {
 #pragma unroll
-                            for (int k = 0; k < 4; ++k) x[pg][k] = lds32(rows + (uint32_t)(4 * kk + pg) * kTq4PageHeadBytes + (uint32_t)k * kTq4RowBytes + word_off);
-                        }
-                        if (splice_warp) {
-#pragma unroll
-                            for (int pg = 0; pg < 4; ++pg) {
-#pragma unroll
-                                for (int k = 0; k < 4; ++k) {
-                                    const uint32_t y = lds32(rows + (uint32_t)(4 * kk + pg) * kTq4PageHeadBytes + (uint32_t)k * kTq4RowBytes + 64u);
-                                    if (vw == 0) x[pg][k] = (x[pg][k] >> 16) | (y << 16);
-                                }
+                            for (int k = 0; k < 4; ++k) {
+                                const uint32_t y = lds32(rows + (uint32_t)(4 * kk + pg) * kTq4PageHeadBytes + (uint32_t)k * kTq4RowBytes + 64u);
+                                if (vw == 0) x[pg][k] = (x[pg][k] >> 16) | (y << 16);
                             }
                         }
+                    }
+#pragma unroll
+                    for (int pg = 0; pg < 4; ++pg) {
+                        // byte t of x[0] -> keys 0 and 1 of channel 2 t, x[1]: of channel 2 t + 1; x[2], x[3]: keys 2 and 3
+                        const uint32_t w0 = x[pg][0], w1 = x[pg][1], w2 = x[pg][2], w3 = x[pg][3];
+                        x[pg][0] = (w0 & 0x0f0f0f0fu) | ((w1 << 4) & 0xf0f0f0f0u);
+                        x[pg][1] = ((w0 >> 4) & 0x0f0f0f0fu) | (w1 & 0xf0f0f0f0u);
+                        x[pg][2] = (w2 & 0x0f0f0f0fu) | ((w3 << 4) & 0xf0f0f0f0u);
+                        x[pg][3] = ((w2 >> 4) & 0x0f0f0f0fu) | (w3 & 0xf0f0f0f0u);
+                    }
+#pragma unroll 1
+                    for (int res = 0; res < 2; ++res) {
+                        const uint32_t lut = res == 0 ? lut_v : lut_r;
+                        uint32_t a[2][16];
 #pragma unroll
                         for (int pg = 0; pg < 4; ++pg) {
-                            const uint32_t (&w)[4] = x[pg];
-                            // byte t of ab -> (key 0, key 1) of channel 2 t (first) and 2 t + 1 (second); cd: keys 2 and 3
-                            const uint32_t ab[2] = {(w[0] & 0x0f0f0f0fu) | ((w[1] << 4) & 0xf0f0f0f0u), ((w[0] >> 4) & 0x0f0f0f0fu) | (w[1] & 0xf0f0f0f0u)};
-                            const uint32_t cd[2] = {(w[2] & 0x0f0f0f0fu) | ((w[3] << 4) & 0xf0f0f0f0u), ((w[2] >> 4) & 0x0f0f0f0fu) | (w[3] & 0xf0f0f0f0u)};
 #pragma unroll
                             for (int T = 0; T < 2; ++T) {
 #pragma unroll
                                 for (int o = 0; o < 2; ++o) {
-                                    a[T][4 * pg + 2 * o] = lds32_lut(__byte_perm(ab[o], lut, sel[T]));
-                                    a[T][4 * pg + 2 * o + 1] = lds32_lut(__byte_perm(cd[o], lut, sel[T]));
+                                    a[T][4 * pg + 2 * o] = lds32_lut(__byte_perm(x[pg][o], lut, sel[T]));
+                                    a[T][4 * pg + 2 * o + 1] = lds32_lut(__byte_perm(x[pg][2 + o], lut, sel[T]));
                                 }
                             }
                         }
-                        if (!(ok = wait_all(bar(kXtVEmpty + kk), (laps & 1u) ^ 1u))) break;
-                        const uint32_t dst = tmem + quad + kXtColV + 64u * (uint32_t)half + 32u * (uint32_t)kk;
+                        if (!(ok = wait_all(bar(kXtVEmpty + res), (uint32_t)(kk ^ 1)))) break;
+                        const uint32_t dst = tmem + quad + kXtColV + 64u * (uint32_t)half + 32u * (uint32_t)res;
                         tc_st_16x256b_x4(dst, a[0]);
                         tc_st_16x256b_x4(dst + (16u << 16), a[1]);
                         tc_wait_st();
                         tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(bar(kXtVFull + kk));
+                        if (lane == 0) mbar_arrive(bar(kXtVFull + res));
                     }
-                    if (ok && pass == 0) {      // does the block need its centroids' residuals?
-                        ok = wait_all(bar(kXtPReady), c & 1u);
-                        if (ok && *reinterpret_cast<volatile int*>(&sh.peak[c & 1]) == (int)c + 1) passes = 2;
-                    }
+                    if (!ok) break;
                 }
                 __syncwarp();
                 if (ok && lane == 0) mbar_arrive(bar(kXtRawVFree + s));
@@ -501,7 +498,6 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
         float* m_ref = sh.m_ref + row0;      // this part's rows
         float* alpha = sh.alpha + row0;
         float* mass = sh.mass + row0;
-        float* cut = sh.cut + row0;
         int *row_min = sh.row_min + row0, *row_max = sh.row_max + row0;
         float* red = &sh.red[0][row0];
         float* partials = reinterpret_cast<float*>(p.scratch + plan_bytes(p.batch.num_reqs));
@@ -517,7 +513,6 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                 row_min[key] = valid ? row_min_kv(p.batch, g, q_off) : 0x7fffffff;
                 m_ref[key] = -1e30f;
                 mass[key] = 0.0f;
-                cut[key] = 0.0f;
             }
             xt_sync(part);
             int safe_lo = 0, safe_hi = 0x7fffffff;      // keys every valid row can see
@@ -534,7 +529,7 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                 l[i] = 0.0f;
                 m_lag[i] = -1e30f;
             }
-            // mass of every row over all keys so far, into sh.mass (a lower bound from then on)
+            // mass of every row over all keys, into sh.mass
             auto reduce_mass = [&]() {
 #pragma unroll
                 for (int i = 0; i < P; ++i) {
@@ -544,11 +539,7 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                     if (lane == 0) red[(wid & 3) * 24 + i] = t;
                 }
                 xt_sync(part);
-                if (key < P) {
-                    const float t = (red[0 + key] + red[24 + key]) + (red[48 + key] + red[72 + key]);
-                    mass[key] = t;
-                    cut[key] = kPeakedWeight * t;
-                }
+                if (key < P) mass[key] = (red[0 + key] + red[24 + key]) + (red[48 + key] + red[72 + key]);
                 xt_sync(part);
             };
             const int nblocks = (sg.pages + kXtPages - 1) / kXtPages;
@@ -604,7 +595,6 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                         const float a = ex2(old - now);      // 0 when nothing was visible before
                         m_ref[key] = now;
                         alpha[key] = a;
-                        cut[key] *= a;
                     }
                     xt_sync(part);
 #pragma unroll
@@ -642,13 +632,6 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                     for (int i = 0; i < P; ++i) seen = seen || sc[i] > -INFINITY;
                     if (!seen) dv = make_float2(0.0f, 0.0f);
                 }
-                bool peaked = false;      // a key with more than kPeakedWeight of a row's mass so far (of what is known of it)
-                float known[P];
-#pragma unroll
-                for (int i = 0; i < P; i += 4) {
-                    const float4 v = *reinterpret_cast<const float4*>(&cut[i]);
-                    known[i] = v.x; known[i + 1] = v.y; known[i + 2] = v.z; known[i + 3] = v.w;
-                }
                 // 16-byte chunk of the key's column, swizzled by the row
                 const uint32_t at = p_t + (uint32_t)(key >> 6) * (uint32_t)(N * 128) + (uint32_t)row0 * 128u + 2u * (uint32_t)(key & 7) +
                                     (((uint32_t)(key & 63) >> 3) << 4);
@@ -656,8 +639,6 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                 for (int i = 0; i < P; ++i) {
                     const float w = ex2(sc[i] - m_lag[i]);
                     l[i] += w;
-                    sc[i] = w;
-                    peaked = peaked || w > known[i];
                     const float x0 = w * dv.x, x1 = w * dv.y;
                     const __half2 h = __floats2half2_rn(x0, x1);
                     const float2 hf = __half22float2(h);
@@ -669,14 +650,6 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                     sts16(a + kPBytes + (uint32_t)R * 128u, lo >> 16);
                 }
                 if (bad) failed = true;
-                if (xt_any(peaked, part)) {      // bring the known mass up to date and look again
-                    reduce_mass();
-                    peaked = false;
-#pragma unroll
-                    for (int i = 0; i < P; ++i) peaked = peaked || sc[i] > cut[i];
-                    const bool any_peak = __any_sync(0xffffffffu, peaked);
-                    if (any_peak && lane == 0) sh.peak[c & 1] = (int)c + 1;
-                }
                 fence_proxy_async();
                 __syncwarp();
                 if (lane == 0) {
