@@ -1090,7 +1090,8 @@ def main():
     peaks, peak_kind = measured_peaks()
     peak = float(peaks.get("hbm_gbs", FALLBACK_HBM_GBS))
     achieved = kv_bytes / (attn_ms * 1e-3) / 1e9
-    traffic_ratio, traffic_rec = (None, None) if reference else measured_traffic_ratio("tq4_attention_stream_exact_kernel")
+    attn_kernel = "tq4_attention_stream_exact_kernel" if q_len * hq // hkv <= 8 else "tq4_attention_stream_tc_kernel"
+    traffic_ratio, traffic_rec = (None, None) if reference else measured_traffic_ratio(attn_kernel)
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_per_step, "higher_is_better": True,
@@ -1106,7 +1107,7 @@ def main():
                                    if sharded else f"batch-sharded x{world}, no collective")},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_kind": f"of {peak_kind}", "frac_of_nominal_8TBs": achieved / NOMINAL_HBM_GBS,
-                     "kernel": "tq4_attention_stream_exact_kernel (+ plan and merge launches, timed together)",
+                     "kernel": f"{attn_kernel} (+ plan and merge launches, timed together)",
                      "launch_ms": attn_ms,
                      # DRAM bytes of one stream-kernel launch: the ratio measured by ncu on a smaller case of
                      # the same kernel (recorded with its date and workload) times this run's bytes

@@ -20,8 +20,9 @@
 //
 // Measured on 128 requests of 2048 to 16384 keys, four query tokens, 24 / 4 heads (1.26 GB of pages): 914 us against 1454 with
 // three 8-row items of the one-warp kernel (tq4_stream_exact.cuh), which looks every code up three times.  Bound by the softmax
-// warps' serial chain from scores to P: a block of 128 keys takes about 6700 cycles at some 14000 instructions (2.5 per cycle
-// and SM; with the residuals on a fifth of the blocks only, the shared-memory pipe was 56 % and the tensor pipe 22 % busy).  Taking the weights before the vote on the reference (one barrier
+// warps' serial chain from scores to P: and by the shared-memory data pipe that the look-ups share with them: a block of 128
+// keys takes about 6700 cycles at 14100 instructions; the pipe is 72 % busy, the issue slots 60 %, the tensor pipe 26 %.
+// Taking the weights before the vote on the reference (one barrier
 // a block fewer) put them behind the wait for the previous output product: 1008 us.
 #pragma once
 
