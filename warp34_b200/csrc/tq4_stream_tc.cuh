@@ -20,10 +20,10 @@
 //
 // Measured on 128 requests of 2048 to 16384 keys, four query tokens, 24 / 4 heads (1.26 GB of pages): 914 us against 1454 with
 // three 8-row items of the one-warp kernel (tq4_stream_exact.cuh), which looks every code up three times.  Bound by the softmax
-// warps' serial chain from scores to P: and by the shared-memory data pipe that the look-ups share with them: a block of 128
-// keys takes about 6700 cycles at 14100 instructions; the pipe is 72 % busy, the issue slots 60 %, the tensor pipe 26 %.
-// Taking the weights before the vote on the reference (one barrier
-// a block fewer) put them behind the wait for the previous output product: 1008 us.
+// warps' serial chain from scores to P and by the shared-memory data pipe that the look-ups share with them: a block of 128 keys
+// takes about 6700 cycles at 14100 instructions; the pipe is 72 % busy, the issue slots 60 %, the tensor pipe 26 %.  Taking the
+// weights before the vote on the reference (one barrier a block fewer) put them behind the wait for the previous output
+// product: 1008 us.
 #pragma once
 
 namespace w34 {
@@ -187,13 +187,14 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
         return false;
     };
 
-    for (int i = tid; i < 256 * 32; i += xt_threads(R)) {      // table as in the exact streaming kernel, residuals unscaled
+    for (int i = tid; i < 256 * 32; i += xt_threads(R)) {      // per byte: {values, residuals} x 16, {residuals, values} x 16
         const int byte = i >> 5, ln = i & 31;
         const float c0 = kLutScale * tq4_centroid(byte & 15), c1 = kLutScale * tq4_centroid(byte >> 4);
         const uint32_t hi = pack_half2(c0, c1);
         const float2 hf = __half22float2(*reinterpret_cast<const __half2*>(&hi));
-        sts32(lut_addr + (uint32_t)(byte * 256 + ln * 4), (ln & 1) ? pack_half2(c0 - hf.x, c1 - hf.y) : hi);
-        sts32(lut_addr + (uint32_t)(byte * 256 + 128 + ln * 4), hi);
+        const uint32_t lo = pack_half2(c0 - hf.x, c1 - hf.y);
+        sts32(lut_addr + (uint32_t)(byte * 256 + ln * 4), (ln & 1) ? lo : hi);
+        sts32(lut_addr + (uint32_t)(byte * 256 + 128 + ln * 4), (ln & 1) ? hi : lo);
     }
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -379,7 +380,8 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
         const int vw = 4 * (wid & 3) + (gid >> 1);                           // this thread's code word of the half
         const uint32_t word_off = 4u * ((half ? 17u : 0u) + (uint32_t)vw);
         const bool splice_warp = half == 0 && (wid & 3) == 0;                // virtual word 0: (W0 >> 16) | (W16 << 16)
-        const uint32_t lut_v = lut_addr + 128u + 4u * (uint32_t)lane, lut_r = lut_addr + 8u * (uint32_t)(lane & 15) + 4u;
+        // lanes 0-15 read the first half of a table entry, lanes 16-31 the second: 32 banks for the values and for the residuals
+        const uint32_t lut_v = lut_addr + (uint32_t)(lane >> 4) * 132u + 8u * (uint32_t)(lane & 15), lut_r = lut_v ^ 4u;
         // byte 2 (gid & 1) + T of the paired codes belongs to tile T
         const uint32_t sel[2] = {0x7604u + ((uint32_t)(2 * (gid & 1)) << 4), 0x7604u + ((uint32_t)(2 * (gid & 1) + 1) << 4)};
         bool ok = true;
