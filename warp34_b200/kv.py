@@ -642,20 +642,25 @@ class DecodeStep:
 
         side = torch.cuda.Stream()
         side.wait_stream(torch.cuda.current_stream())
+        graphs = []
         with torch.cuda.stream(side):
             if split:
                 payload()
             body()                      # warm-up outside the capture (one-time attribute calls)
+            for fn in (payload, body):
+                if fn is payload and not split:
+                    graphs.append(None)
+                    continue
+                # captured directly: torch.cuda.graph() would also collect garbage and return every cached block to the
+                # driver, milliseconds of a new step's first run, for a capture that allocates nothing
+                g = torch.cuda.CUDAGraph()
+                g.capture_begin()
+                try:
+                    fn()
+                finally:
+                    g.capture_end()
+                graphs.append(g)
         torch.cuda.current_stream().wait_stream(side)
-        graphs = []
-        for fn in (payload, body):
-            if fn is payload and not split:
-                graphs.append(None)
-                continue
-            g = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(g):
-                fn()
-            graphs.append(g)
         self.ex.set_stream()
         return tuple(graphs)
 
