@@ -84,7 +84,7 @@ template <int FMT> struct PpSmem {
 // barrier slots (8 bytes each).  Full / PReady: waited for by the MMA warp of CTA 0, arrivals from both CTAs.
 // Empty, S, Pv: one arrival per CTA from the MMA warp's commits.  Raw*: within a CTA.
 enum { kPpFullK = 0, kPpFullV = kPpFullK + kPpStages, kPpEmptyK = kPpFullV + kPpStages, kPpEmptyV = kPpEmptyK + kPpStages,
-       kPpS = kPpEmptyV + kPpStages, kPpPReady = kPpS + 2, kPpPv = kPpPReady + 2, kPpDrain, kPpRawKFull,
+       kPpS = kPpEmptyV + kPpStages, kPpPReady = kPpS + 2, kPpPv = kPpPReady + 2, kPpDrain = kPpPv + 2, kPpRawKFull,
        kPpRawKFree = kPpRawKFull + kPpRawStages, kPpRawVFull = kPpRawKFree + kPpRawStages,
        kPpRawVFree = kPpRawVFull + kPpRawStages, kPpBarCount = kPpRawVFree + kPpRawStages };
 static_assert(kPpBarCount * 8 <= 240, "barrier slots end before the TMEM address and abort words");
@@ -270,6 +270,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
         mbar_init(bar(kPpS), 1u);
         mbar_init(bar(kPpS + 1), 1u);
         mbar_init(bar(kPpPv), 1u);
+        mbar_init(bar(kPpPv + 1), 1u);
         mbar_init(bar(kPpPReady), 8u);             // four consumer warps of each CTA
         mbar_init(bar(kPpPReady + 1), 8u);
         mbar_init(bar(kPpDrain), 1u);
@@ -486,7 +487,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
                             tc2_mma_f16_ts(tmem + kPpColO, a, b + kPpPart / 16, kIdescPv, 1u);
                         }
                         tc2_commit_both(bar(kPpEmptyV + (int)vst));
-                        if (h == 1) tc2_commit_both(bar(kPpPv));
+                        if (h == 1) tc2_commit_both(bar(kPpPv + (i & 1)));
                         if (++vst == kPpStages) { vst = 0; vph ^= 1u; }
                     }
                 }
@@ -640,8 +641,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
             if (aborted_any()) break;
             if (!wait_all(bar(kPpS + (j & 1)), (uint32_t)((j >> 1) & 1))) { *abort_flag = 1u; break; }
             tc_fence_after();
-            // PV(j - 2) precedes QK(j) in the pipe; waiting for every phase of kPpPv keeps its parity unambiguous
-            if (j >= 2 && !wait_all(bar(kPpPv), (uint32_t)(j & 1))) { *abort_flag = 1u; break; }
+            // PV(j - 2) precedes QK(j) in the pipe.  Every phase is waited for: the next one of the same barrier, PV(j), needs this
+            // block's weights, so that no delay of this warp lets two go by.  (One barrier for all blocks would have: PV(j - 1) needs
+            // nothing more from here, and once it had completed the parity meant PV(j).)
+            if (j >= 2 && !wait_all(bar(kPpPv + (j & 1)), (uint32_t)(((j - 2) >> 1) & 1))) { *abort_flag = 1u; break; }
             const uint32_t t_sj = t_s + 64u * (uint32_t)(j & 1);
             const int kbase = (kb_lo + j) << 6;
             const bool all_seen = kbase >= rmin && kbase + 63 <= rmax;
@@ -680,7 +683,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
             }
             if (j > 0 && __any_sync(0xffffffffu, need)) {
                 // O is at rest once the previous output product has completed (the next one waits for this block's P)
-                if (!wait_all(bar(kPpPv), (uint32_t)((j - 1) & 1))) { *abort_flag = 1u; break; }
+                if (!wait_all(bar(kPpPv + ((j - 1) & 1)), (uint32_t)(((j - 1) >> 1) & 1))) { *abort_flag = 1u; break; }
                 tc_fence_after();
 #pragma unroll 1
                 for (int c = 0; c < 16; ++c) {
@@ -720,8 +723,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
         }
         // the last output product
         if (nblocks > 0 && !aborted_any()) {
-            if (nblocks > 1 && !wait_all(bar(kPpPv), (uint32_t)(nblocks & 1))) *abort_flag = 1u;
-            if (!wait_all(bar(kPpPv), (uint32_t)((nblocks - 1) & 1))) *abort_flag = 1u;
+            if (nblocks > 1 && !wait_all(bar(kPpPv + (nblocks & 1)), (uint32_t)(((nblocks - 2) >> 1) & 1))) *abort_flag = 1u;
+            if (!wait_all(bar(kPpPv + ((nblocks - 1) & 1)), (uint32_t)(((nblocks - 1) >> 1) & 1))) *abort_flag = 1u;
         }
         tc_fence_after();
     }
