@@ -100,3 +100,54 @@ def test_split_chunks_equal_the_unsplit_ones(env, fmt, hq, hkv, ctx, new, gate):
         torch.cuda.synchronize()
         ok, msg = plain_parity(outs[0], want.float().cpu().numpy())
         assert ok, msg
+
+
+@pytest.mark.parametrize("fmt", ["TQ4", "FP8_E4M3", "Q8_0"])
+@pytest.mark.parametrize("k_exp,v_exp,where", [(-10, 0, "all"), (0, -9, "all"), (-13, 0, "all"), (6, 6, "all"), (-10, -9, "pages"),
+                                               (-13, 0, "ends"), (0, -13, "ends"), (-13, -13, "ends")])
+def test_accuracy_does_not_depend_on_the_magnitude_of_k_and_v(env, fmt, k_exp, v_exp, where):
+    """K times 2^a under Q times 2^-a, or V times 2^b: the stored codes are the same and every scale is the same but for a power
+    of two, so the outputs are those of magnitude 1 (times 2^b).  At magnitude 1 about 3 % of the outputs are not the float64
+    result's nearest fp16 value (1 % for 8-bit rows), so at most twice that many may differ here (measured: 2.6 and 0.5 %).
+    `pages`: only the tokens of every other page are scaled; `ends`: only the first and the last 64 tokens, all others are times 4 (the exponents that
+    a tile takes from its ends do not fit the rows between): the comparison is then with the fp32 kernel."""
+    ffi, kv, synth = env["ffi"], env["kv"], env["synth"]
+    f = getattr(ffi, "KV_FORMAT_" + fmt)
+    tr = ffi.KV_TRANSFORM_RADEMACHER_WHT256 if fmt == "TQ4" else ffi.KV_TRANSFORM_IDENTITY
+    hq, hkv, ctx, new = 12, 2, [400, 77], [70, 130]
+    total, n = sum(ctx) + sum(new), sum(new)
+    tok = torch.cat([torch.arange(c + m) for c, m in zip(ctx, new)]).cuda()
+    left = torch.cat([torch.arange(c + m).flip(0) for c, m in zip(ctx, new)]).cuda()
+    scaled = {"all": tok >= 0, "pages": tok // 16 % 2 == 0, "ends": (tok < 64) | (left < 64 + 15)}[where]
+    outs = {}
+    for a, b in ((0, 0), (k_exp, v_exp)):
+        wl = synth.PagedWorkload([0, 0], [c + m for c, m in zip(ctx, new)], hkv, seed=7, fill=0x7F, formats=(f, f, tr, tr))
+        k, v = synth.make_kv(total, hkv, 9, device="cuda")
+        q = synth.make_q(n, hq, 9, device="cuda").float()
+        k, v = (k.float() * 16).round() / 16, (v.float() * 16).round() / 16      # eleven bits or fewer, so exact at every scale
+        other = 4.0 if where == "ends" else 1.0
+        k, v = (k * torch.where(scaled, 2.0 ** x, other if x else 1.0)[:, None] for k, x in ((k, a), (v, b)))
+        q = (q * 2.0 ** -a if where == "all" else q).half()
+        kv.kv_cache_write(env["ex"], wl.layer, wl.step(), k.half(), v.half())
+        for s, c in zip(wl.seqs, ctx):
+            s.commit(c)
+        step = wl.step(q_lens=new)
+        out = torch.zeros(n, hq, 256, dtype=torch.float16, device="cuda")
+        kv.paged_attention(env["ex"], wl.layer, step, q, out, hq)
+        torch.cuda.synchronize()
+        assert int(env["ex"].scratch[:4].view(torch.int32).item()) == 0
+        outs[(a, b)] = out.float()
+        if where != "all":
+            want = torch.zeros_like(out)
+            kv.paged_attention(env["ex"], wl.layer, step, q, want, hq, scalar=True)
+            torch.cuda.synchronize()
+            ok, msg = plain_parity(out.float().cpu().numpy(), want.float().cpu().numpy())
+            assert ok, msg
+    if where != "all":
+        return
+    base, got = outs[(0, 0)], outs[(k_exp, v_exp)] * 2.0 ** -v_exp
+    ok, msg = plain_parity(got.cpu().numpy(), base.cpu().numpy())
+    assert ok, msg
+    normal = base.abs() >= 2.0 ** (-13 - min(v_exp, 0))     # fp16 has all its bits on both sides
+    differ = float((got != base)[normal].float().mean())
+    assert differ <= (0.06 if fmt == "TQ4" else 0.025), differ

@@ -19,7 +19,12 @@
 //   S[256 x 64]   = Q'hi Khi^T + Q'lo Khi^T + Q'hi Klo^T      A in TMEM (Q'hi) or shared memory (Q'lo)
 //   O[256 x 256] += Phi Vhi + Plo Vhi + Phi Vlo               A in TMEM
 //
-// K and V elements are row scale x centroid (or code): hi = fp16(d c), lo = fp16(d c - hi), about 22 bits together.
+// K and V elements are row scale x centroid (or code): hi = fp16(d c), lo = fp16(d c - hi), about 22 bits together as long as
+// lo is not far below fp16's normal range.  Where a sample of a tile's rows is small (PpScales: below about 2^-3), K or V
+// is therefore held divided by a power of two for the whole tile, which the consumers take out again in fp32 at no cost: a factor
+// of the scores for K, of the normalised output for V.  (Without it 21 % of the outputs of a TQ4 chunk over K of magnitude 2^-10
+// under Q of magnitude 2^10 were not the nearest fp16 value, against 3 % at magnitude 1, and one missed 2e-3 + 1e-2 |b| by 16 %.
+// A power of two for every key or every 32 keys took 10 to 35 % more time on long contexts: each block then waits for its scales.)
 // What bounds it: the tensor pipe under the power cap.  Six (TQ4) or five (8-bit) products per visible pair instead of
 // two; 8 x 2048 tokens after 8192 (16 / 4 heads) take 5.6 ms = 440 TFLOP/s of attention = 1320 TFLOP/s issued, against
 // 21.6 ms for register MMAs (mma.sync) over the same operands.  A pair rather than one CTA because dequantising once per
@@ -65,6 +70,30 @@ template <> struct PpFormat<WARP34_KV_FORMAT_Q8_0> {
     static constexpr bool kRotated = false;
 };
 
+// A row's scales, as bits: non-negative floats order like them.
+template <int FMT> struct PpScales {
+    static constexpr uint32_t kFirst = FMT == WARP34_KV_FORMAT_FP8_E4M3 ? (uint32_t)kHeadDim : 0u;
+    // How large a row is, from its scale: about its root mean square (TQ4: the centroids' is 1/16), or its largest element.
+    static __device__ __forceinline__ float magnitude(uint32_t bits) {
+        if (FMT == WARP34_KV_FORMAT_TQ4) return __half2float(__ushort_as_half((unsigned short)bits)) * 0.0625f;
+        return __uint_as_float(bits) * (FMT == WARP34_KV_FORMAT_FP8_E4M3 ? 448.0f : 127.0f);
+    }
+    // The first scale of a row in global memory, without its sign.
+    static __device__ __forceinline__ uint32_t first(const uint8_t* row) {
+        return FMT == WARP34_KV_FORMAT_TQ4 ? *reinterpret_cast<const uint16_t*>(row + kFirst) & 0x7fffu : *reinterpret_cast<const uint32_t*>(row + kFirst) & 0x7fffffffu;
+    }
+    // The exponent of the power of two by which rows of this magnitude are divided: 0 from 2^-3 on (the tile of a TQ4 row holds a
+    // quarter of it, and the residual's step of 2^-24 is then 2^-19 of a typical element; of an 8-bit row's largest element it is 2^-21),
+    // so that ordinary activations pass as they are, and for zeros, NaN and infinities; smaller rows are brought to [1, 2).
+    static __device__ __forceinline__ int exponent(uint32_t bits) {
+        const float m = magnitude(bits);
+        return m > 0.0f && m < 0.125f ? max((int)(__float_as_uint(m) >> 23) - 127, -60) : 0;
+    }
+    // Rows divided by 2^e are finite, scale and elements, up to here.
+    static __device__ __forceinline__ bool fits(uint32_t bits, int e) { return e == 0 || !(magnitude(bits) >= 2048.0f * __uint_as_float((uint32_t)(127 + e) << 23)); }
+};
+__device__ __forceinline__ float power_of_two(int e) { return __uint_as_float((uint32_t)(127 + e) << 23); }
+
 template <int FMT> struct PpSmem {
     static constexpr uint32_t kRun = kPageTokens * PpFormat<FMT>::kRow;      // one (page, head) run
     static constexpr uint32_t kRawK = 2u * kRun, kRawV = 4u * kRun;
@@ -87,7 +116,7 @@ enum { kPpFullK = 0, kPpFullV = kPpFullK + kPpStages, kPpEmptyK = kPpFullV + kPp
        kPpS = kPpEmptyV + kPpStages, kPpPReady = kPpS + 2, kPpPv = kPpPReady + 2, kPpDrain = kPpPv + 2, kPpRawKFull,
        kPpRawKFree = kPpRawKFull + kPpRawStages, kPpRawVFull = kPpRawKFree + kPpRawStages,
        kPpRawVFree = kPpRawVFull + kPpRawStages, kPpBarCount = kPpRawVFree + kPpRawStages };
-static_assert(kPpBarCount * 8 <= 240, "barrier slots end before the TMEM address and abort words");
+static_assert(kPpBarCount * 8 <= 224, "barrier slots end before the words behind them");
 
 // ---- CTA-pair wrappers ------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -161,7 +190,9 @@ struct PrefillPairParams {
     int num_q_heads;
     int gqa;
     int tok_per_tile;      // 256 / gqa
-    float q_scale;         // TQ4: sm_scale * log2(e) / kPpLutScale, folded into Q'; 8-bit: sm_scale * log2(e), applied to the scores
+    // The scores are multiplied by score_scale, which is positive.  TQ4: 1, and sm_scale * log2(e) / kPpLutScale is folded into Q' as
+    // q_scale.  8-bit: |sm_scale| * log2(e), and q_scale is its sign; 1 and 0 where sm_scale is 0.
+    float q_scale, score_scale;
     int32_t* status;       // may be null; bit 0: a wait gave up, bit 1: shared-memory window misaligned
     OutputGate og;
     // A chunk of few tiles after a long context: blockIdx.z takes one of `splits` equal ranges of a tile's key blocks and
@@ -183,6 +214,71 @@ __device__ __forceinline__ void prefill_finish_row(const PrefillPairParams& p, f
     }
     apply_output_gate8(v, p.og, row_base, lane, p.io_bf16);
     store8(p.attn_out, row_base, lane, p.io_bf16, v);
+}
+
+// One query row over its keys in [lo, hi] in fp32 by one warp, as the attention kernel leaves it (columns [8 lane, + 8) of the accumulator,
+// mass, maximum): for tiles whose rows differ so much in magnitude that those the exponents were chosen by are not the others' kind.
+template <int FMT>
+__device__ __forceinline__ void prefill_row_fp32(const PrefillPairParams& p, int req, int q_off, int q_head, int lo, int hi, float (&acc)[8], float& l,
+                                                 float& m) {
+    constexpr bool ROT = PpFormat<FMT>::kRotated;
+    const int lane = threadIdx.x & 31, kv_head = q_head / p.gqa;
+    const ReqGeom g = load_req(p.batch, req);
+    const int32_t* blocks = p.batch.block_tables + (size_t)req * p.batch.max_blocks_per_req;
+    const uint8_t* k_head_base = (const uint8_t*)(uintptr_t)p.layout.k_base + (size_t)kv_head * p.layout.k_head_stride_bytes;
+    const uint8_t* v_head_base = (const uint8_t*)(uintptr_t)p.layout.v_base + (size_t)kv_head * p.layout.v_head_stride_bytes;
+    lo = max(lo, row_min_kv(p.batch, g, q_off));
+    hi = min(hi, row_max_kv(p.batch, g, q_off));
+    float q[8];
+    load8(p.q_in, ((size_t)(g.q_start + q_off) * p.num_q_heads + q_head) * kHeadDim, lane, p.io_bf16, q);
+    if (ROT) {
+        sign8(q, lane);
+        butterfly8<5>(q, lane);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        q[i] *= ROT ? p.q_scale * (0.0625f * kPpLutScale) : p.q_scale;
+        acc[i] = 0.0f;
+    }
+    auto elements = [&](const uint8_t* row, float (&x)[8]) {
+        if (FMT == WARP34_KV_FORMAT_TQ4) {
+            const uint8_t* half = row + kTq4BlockBytes * (lane >> 4);
+            const uint16_t* codes = reinterpret_cast<const uint16_t*>(half + 2 + 4 * (lane & 15));
+            const float d = __half2float(*reinterpret_cast<const __half*>(half));
+            const uint32_t w = (uint32_t)codes[0] | ((uint32_t)codes[1] << 16);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) x[i] = d * tq4_centroid((int)((w >> (4 * i)) & 15u));
+        } else {
+            constexpr bool FP8 = FMT == WARP34_KV_FORMAT_FP8_E4M3;
+            const uint32_t* codes = reinterpret_cast<const uint32_t*>(row + (FP8 ? 8 * lane : 68 * (lane >> 3) + 4 + 8 * (lane & 7)));
+            const float d = *reinterpret_cast<const float*>(row + (FP8 ? kHeadDim + 4 * (lane >> 4) : 68 * (lane >> 3)));
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                uint32_t a, b;
+                kv8x4_to_f16x4<FMT>(codes[i], a, b);
+                const float2 fa = __half22float2(*reinterpret_cast<const __half2*>(&a)), fb = __half22float2(*reinterpret_cast<const __half2*>(&b));
+                x[4 * i] = d * fa.x; x[4 * i + 1] = d * fa.y; x[4 * i + 2] = d * fb.x; x[4 * i + 3] = d * fb.y;
+            }
+        }
+    };
+    l = 0.0f;
+    m = -1e30f;
+#pragma unroll 1
+    for (int pos = lo; pos <= hi; ++pos) {
+        const int32_t page = block_table_page(blocks, pos >> 4, p.batch.max_blocks_per_req, ROT ? kInPrefillExact : kInKv8);
+        const size_t row = (size_t)(pos & 15) * PpFormat<FMT>::kRow;
+        float x[8], s = 0.0f;
+        elements(k_head_base + (size_t)page * p.layout.k_page_stride_bytes + row, x);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s += q[i] * x[i];
+        s = warp_sum(s) * p.score_scale;
+        const float m_new = fmaxf(m, s), alpha = ex2(m - m_new), w = ex2(s - m_new);
+        l = l * alpha + w;
+        m = m_new;
+        elements(v_head_base + (size_t)page * p.layout.v_page_stride_bytes + row, x);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i] = acc[i] * alpha + w * (ROT ? x[i] * kPpLutScale : x[i]);
+    }
 }
 
 // Combines the splits of every row that takes part: one warp per (token, q head).
@@ -236,6 +332,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
     const uint32_t raw = base + S::kOffRaw, lut = base + S::kOffLut, bars = base + S::kOffBars;
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + S::kOffBars + 240);
     volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(gen + S::kOffBars + 244);
+    uint32_t* row_max = reinterpret_cast<uint32_t*>(gen + S::kOffBars + 224);                      // largest scale of the tile's K, V rows
+    volatile int* exponents = reinterpret_cast<volatile int*>(gen + S::kOffBars + 232);            // of K, of V
+    volatile int* place = reinterpret_cast<volatile int*>(gen + S::kOffBars + 248);                // request, first block (for prefill_row_fp32)
     auto bar = [&](int which) { return bars + 8u * (uint32_t)which; };
     // Waits and abort checks are warp-uniform: no lane leaves a loop alone.
     auto wait_all = [&](uint32_t b, uint32_t parity) {
@@ -281,6 +380,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
             mbar_init(bar(kPpRawVFree + s), 4u);
         }
         *abort_flag = 0u;
+        row_max[0] = row_max[1] = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     grid_dependency_wait();          // nothing above touches global memory
@@ -311,10 +411,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
     const int kv_lo = row_min_kv(p.batch, g, tok0);
     const int kv_hi = row_max_kv(p.batch, g, tok0 + ntok - 1);
     const bool any_keys = kv_hi >= kv_lo;
+    const int pg_lo = any_keys ? (kv_lo >> 4) : 0, pg_hi = any_keys ? (kv_hi >> 4) : -1;
     const int all_lo = any_keys ? (kv_lo >> 6) : 0, all = any_keys ? ((kv_hi >> 6) - all_lo + 1) : 0;
     const int kb_lo = all_lo + (int)((long long)all * blockIdx.z / p.splits);     // this split's key blocks
     const int nblocks = all_lo + (int)((long long)all * (blockIdx.z + 1) / p.splits) - kb_lo;
-    const int pg_lo = any_keys ? (kv_lo >> 4) : 0, pg_hi = any_keys ? (kv_hi >> 4) : -1;
 
     __syncwarp();
     if (wid == 0) {
@@ -361,6 +461,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
         }
         next_id = page_id(kPpRawStages);
     }
+    // The sample that exponents are chosen by: the first scales of the first block's rows, the same in both CTAs.  Requested here,
+    // looked at behind the query's rows.
+    uint32_t sample_k[2] = {0u, 0u}, sample_v[2] = {0u, 0u};
+    if (wid == 12) {
+        const int32_t id = page_id(0);
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            const int pos = (kb_lo << 6) + lane + 32 * x;
+            const int32_t page = __shfl_sync(0xffffffffu, id, 2 * x + (lane >> 4));
+            if (page >= 0 && pos >= kv_lo && pos <= kv_hi) {
+                const size_t row = (size_t)(lane & 15) * ROW;
+                sample_k[x] = PpScales<FMT>::first(k_head_base + (size_t)page * p.layout.k_page_stride_bytes + row);
+                sample_v[x] = PpScales<FMT>::first(v_head_base + (size_t)page * p.layout.v_page_stride_bytes + row);
+            }
+        }
+    }
 
     // ---- Q rows of this CTA: one warp per row.  TQ4: rotated, scaled, split into value (staging) and
     //      residual (swizzled A tile); 8-bit: the fp16 row as it is ------------------------------------
@@ -387,6 +503,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
             butterfly8<5>(v, lane);
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] *= p.q_scale * 0.0625f;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] *= p.q_scale;
         }
         uint32_t hi[4], lo[4];
 #pragma unroll
@@ -402,6 +521,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
             sts128(qlo_t + (uint32_t)(lane >> 3) * (kPpCtaRows * 128u) + (uint32_t)row * 128u + (uint32_t)(((lane & 7) ^ (row & 7)) << 4),
                    lo[0], lo[1], lo[2], lo[3]);
         }
+    }
+    if (wid == 12) {
+        const int ek = PpScales<FMT>::exponent(__reduce_max_sync(0xffffffffu, max(sample_k[0], sample_k[1])));
+        const int ev = PpScales<FMT>::exponent(__reduce_max_sync(0xffffffffu, max(sample_v[0], sample_v[1])));
+        if (lane == 0) { exponents[0] = ek; exponents[1] = ev; place[0] = req; place[1] = kb_lo; }
     }
     if (ROT) fence_proxy_async();     // the residual tile is read by the tensor core
     tc_fence_before();
@@ -429,6 +553,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
     tc_fence_after();
 
     float l_run = 0.0f, m_ref = -1e30f;     // consumers: of this thread's row
+    const int ek = exponents[0], ev = exponents[1];
 
     if (wid == 12) {
         // ======================= MMA issue: lane 0 of CTA 0 feeds both tensor cores ====================
@@ -529,6 +654,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
         const uint32_t dst0 = (uint32_t)(quarter >> 1) * 4096u + (uint32_t)lane * 128u;
         const uint32_t lut_lane = lut + 8u * (uint32_t)(lane & 15);
         const uint32_t leader_full = map_to_rank(bar(full), 0u);
+        const int exponent = is_v ? ev : ek;
+        const float down = power_of_two(-exponent);
+        uint32_t most = 0u;           // largest scale seen, where that matters
         uint32_t st = 0, ph = 1;      // parity 1: the first pass over the ring does not wait
 #pragma unroll 1
         for (int j = 0; j < nblocks; ++j) {
@@ -562,6 +690,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
                         for (int i = 0; i < 4; ++i) w[i] = lds32(rowp + 68u + 16u * quarter + 4u * i);
                     }
                     if (!key_ok) dbits = 0u;
+                    if (exponent != 0) {
+                        most = max(most, dbits & 0x7fffu);
+                        dbits = __half_as_ushort(__float2half_rn(__half2float(__ushort_as_half((unsigned short)dbits)) * down));
+                    }
                 } else if (FMT == WARP34_KV_FORMAT_FP8_E4M3) {
 #pragma unroll
                     for (int i = 0; i < 8; ++i) w[i] = lds32(rowp + 128u * half + 32u * quarter + 4u * i);
@@ -576,6 +708,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
                     d = 0.0f;
 #pragma unroll
                     for (int i = 0; i < 8; ++i) w[i] = 0u;      // e4m3 codes of unwritten rows can be NaN patterns
+                }
+                if (FMT != WARP34_KV_FORMAT_TQ4 && exponent != 0) {
+                    most = max(most, __float_as_uint(d) & 0x7fffffffu);
+                    d *= down;
                 }
                 __syncwarp();
                 if (h == 1 && lane == 0) mbar_arrive(bar(raw_free + rs));     // the runs are in registers
@@ -625,6 +761,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
             }
             if (!ok) { *abort_flag = 1u; break; }
         }
+        if (exponent != 0) {
+            most = __reduce_max_sync(0xffffffffu, most);
+            if (lane == 0) {
+#pragma unroll
+                for (uint32_t r = 0; r < 2; ++r) {
+                    asm volatile("red.relaxed.cluster.shared::cluster.max.u32 [%0], %1;" ::"r"(map_to_rank(smem_u32(row_max + (is_v ? 1 : 0)), r)), "r"(most) : "memory");
+                }
+            }
+        }
     } else {
         // ======================= consumers: softmax, P, rescale =========================================
         const int trow = row0 + tid;
@@ -636,6 +781,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
         const uint32_t lane_base = (uint32_t)(32 * wid) << 16;
         const uint32_t t_o = tmem + lane_base + kPpColO, t_s = tmem + lane_base + kPpColS;
         const uint32_t leader_pready = map_to_rank(bar(kPpPReady), 0u);
+        const float factor = fmaxf(power_of_two(ek) * p.score_scale, 1.2e-38f);      // never 0: masked scores are -infinity
 #pragma unroll 1
         for (int j = 0; j < nblocks; ++j) {
             if (aborted_any()) break;
@@ -648,32 +794,32 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
             const uint32_t t_sj = t_s + 64u * (uint32_t)(j & 1);
             const int kbase = (kb_lo + j) << 6;
             const bool all_seen = kbase >= rmin && kbase + 63 <= rmax;
-            // Scores of keys [32 c, + 32) of the block, scaled and masked.
+            // Scores of keys [32 c, + 32) of the block, masked; `factor` is still to be applied.
             auto scores = [&](int c, float (&sv)[32]) {
                 uint32_t r[32];
                 tc_ld32(r, t_sj + 32u * (uint32_t)c);
                 tc_wait_ld();
 #pragma unroll
-                for (int i = 0; i < 32; ++i) sv[i] = ROT ? __uint_as_float(r[i]) : __uint_as_float(r[i]) * p.q_scale;
+                for (int i = 0; i < 32; ++i) sv[i] = __uint_as_float(r[i]);
                 if (!all_seen) {
 #pragma unroll
                     for (int i = 0; i < 32; ++i) {
                         const int pos = kbase + 32 * c + i;
-                        if (!(pos >= rmin && pos <= rmax)) sv[i] = -1e30f;
+                        if (!(pos >= rmin && pos <= rmax)) sv[i] = -INFINITY;
                     }
                 }
             };
             // TQ4 reads them twice (maximum, then weights): holding all 64 spills there (92 bytes a thread, five ragged
             // prompts 270 us instead of 245), while the 8-bit builds have room and the second read costs them 10 %.
             float sv[2][32];
-            float mx4[4] = {-1e30f, -1e30f, -1e30f, -1e30f};     // four independent chains
+            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};     // four independent chains
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
                 scores(c, sv[ROT ? 0 : c]);
 #pragma unroll
                 for (int i = 0; i < 32; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], sv[ROT ? 0 : c][i]);
             }
-            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * factor;
             // the reference maximum moves only when the true maximum ran ahead by more than the threshold
             const bool need = mx > m_ref + kPpRescaleThreshold;
             float alpha = 1.0f;
@@ -703,8 +849,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
                 if (ROT) scores(c, sv[0]);
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                    // masked scores are -1e30: ex2 gives exactly 0 against any finite reference
-                    const float pa = ex2(sv[ROT ? 0 : c][2 * i] - m_use), pb = ex2(sv[ROT ? 0 : c][2 * i + 1] - m_use);
+                    // masked scores are -infinity: ex2 gives exactly 0 against any finite reference
+                    const float pa = ex2(__fmaf_rn(sv[ROT ? 0 : c][2 * i], factor, -m_use)), pb = ex2(__fmaf_rn(sv[ROT ? 0 : c][2 * i + 1], factor, -m_use));
                     ls4[i & 3] += pa + pb;
                     const __half2 h = __floats2half2_rn(pa, pb);
                     const float2 hf = __half22float2(h);
@@ -732,6 +878,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
     // ---- epilogue: O / l -> staging -> inverse rotation -> global ---------------------------------
     // (staging aliases the tiles: every MMA of the pair that read them has completed, see kPpDrain)
     __syncthreads();
+    const int k_exp = exponents[0], v_exp = exponents[1];      // (read again: in registers throughout, they would make the kernel spill)
+    bool fits = true;
+    if ((k_exp | v_exp) != 0) {      // does every row of the tile fit the sample's exponents?  (K rows are spread over both CTAs.)
+        cluster_sync_all();
+        fits = PpScales<FMT>::fits(row_max[0], k_exp) && PpScales<FMT>::fits(row_max[1], v_exp);
+    }
     const bool aborted = *abort_flag != 0u;
     float* stage = reinterpret_cast<float*>(gen);
     if (wid < 4 && !aborted) {
@@ -762,11 +914,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
             const int q_head = kv_head * p.gqa + trow % p.gqa;
             if (p.batch.valid_token_mask != nullptr && p.batch.valid_token_mask[g.q_start + q_off] == 0) continue;
             const float* src = stage + row * kPpOutStride;
-            const float l = src[256];
+            float l = src[256], m = src[257];
             float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            if (l > 0.0f) {
+            if (!fits) {
+                prefill_row_fp32<FMT>(p, place[0], q_off, q_head, place[1] << 6, ((place[1] + nblocks) << 6) - 1, v, l, m);
+            } else if (l > 0.0f) {
                 const float4 a = *reinterpret_cast<const float4*>(src + 8 * lane), b = *reinterpret_cast<const float4*>(src + 8 * lane + 4);
                 v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+                if (v_exp != 0) {
+                    const float up = power_of_two(v_exp);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) v[i] *= up;
+                }
             }
             const size_t out_row = (size_t)(g.q_start + q_off) * p.num_q_heads + q_head;
             if (p.splits > 1) {
@@ -774,7 +933,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
                 float4* dst = reinterpret_cast<float4*>(p.parts + part_row * kHeadDim + 8 * lane);
                 dst[0] = make_float4(v[0], v[1], v[2], v[3]);
                 dst[1] = make_float4(v[4], v[5], v[6], v[7]);
-                if (lane == 0) p.parts_ml[part_row] = make_float2(src[257], l);
+                if (lane == 0) p.parts_ml[part_row] = make_float2(m, l);
                 continue;
             }
             prefill_finish_row<ROT>(p, v, l, out_row * kHeadDim, lane);
@@ -812,7 +971,13 @@ static int launch_prefill_pair(const warp34_exec* ex, const warp34_kv_layer_layo
     pp.gqa = num_q_heads / layout->local_kv_heads;
     pp.tok_per_tile = kPpRows / pp.gqa;
     pp.q_scale = batch->sm_scale * 1.4426950408889634f;
-    if (PpFormat<FMT>::kRotated) pp.q_scale /= kPpLutScale;
+    pp.score_scale = 1.0f;
+    if (PpFormat<FMT>::kRotated) {
+        pp.q_scale /= kPpLutScale;
+    } else if (pp.q_scale != 0.0f) {
+        pp.score_scale = fabsf(pp.q_scale);
+        pp.q_scale = pp.q_scale < 0.0f ? -1.0f : 1.0f;
+    }
     pp.status = status;
     pp.og = og;
     const long long tiles = (long long)batch->total_tokens / pp.tok_per_tile + batch->num_reqs;
