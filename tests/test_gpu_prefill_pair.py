@@ -151,3 +151,25 @@ def test_accuracy_does_not_depend_on_the_magnitude_of_k_and_v(env, fmt, k_exp, v
     normal = base.abs() >= 2.0 ** (-13 - min(v_exp, 0))     # fp16 has all its bits on both sides
     differ = float((got != base)[normal].float().mean())
     assert differ <= (0.06 if fmt == "TQ4" else 0.025), differ
+
+
+@pytest.mark.parametrize("ctx,new", [([300, 20], [70, 50]), ([3000], [20])])      # one range of keys; several, merged
+def test_nan_rows_of_a_tq4_chunk_come_out_as_nan(env, ctx, new):
+    """A query row with a NaN, and only that row, gives NaN, as the fp32 kernel's does; it is not passed off as zeros."""
+    kv, synth = env["kv"], env["synth"]
+    hq, hkv, n = 12, 2, sum(new)
+    wl = synth.PagedWorkload(ctx, new, hkv, seed=7, fill=0x7F)
+    wl.fill_context(env["ex"], 7)
+    k, v = synth.make_kv(n, hkv, 9, device="cuda")
+    q = synth.make_q(n, hq, 9, device="cuda")
+    b = wl.step()
+    kv.kv_cache_write(env["ex"], wl.layer, b, k, v)
+    clean = torch.zeros_like(q)
+    kv.paged_attention(env["ex"], wl.layer, b, q, clean, hq)
+    q[5, 3, 100] = float("nan")
+    out = torch.zeros_like(q)
+    kv.paged_attention(env["ex"], wl.layer, b, q, out, hq)
+    torch.cuda.synchronize()
+    assert torch.isnan(out[5, 3]).all()
+    out[5, 3] = clean[5, 3]
+    assert torch.equal(out, clean)

@@ -57,17 +57,22 @@ constexpr int kPpOutStride = 260;                    // floats per row of the ep
 constexpr int kPpMaxSplits = 24;                     // at most 32: a lane per split in the merge
 
 template <int FMT> struct PpFormat;
+// has_keys: whether a row of mass l has a result.  A row whose query or keys hold a NaN has a NaN mass: it comes out as NaN on TQ4
+// layers and as zeros on 8-bit ones, as it does from the kernels that serve smaller batches of them.
 template <> struct PpFormat<WARP34_KV_FORMAT_TQ4> {
     static constexpr uint32_t kRow = kTq4RowBytes;
     static constexpr bool kRotated = true;
+    static __device__ __forceinline__ bool has_keys(float l) { return !(l <= 0.0f); }
 };
 template <> struct PpFormat<WARP34_KV_FORMAT_FP8_E4M3> {
     static constexpr uint32_t kRow = kHeadDim + 8;
     static constexpr bool kRotated = false;
+    static __device__ __forceinline__ bool has_keys(float l) { return l > 0.0f; }
 };
 template <> struct PpFormat<WARP34_KV_FORMAT_Q8_0> {
     static constexpr uint32_t kRow = 4 * 68;
     static constexpr bool kRotated = false;
+    static __device__ __forceinline__ bool has_keys(float l) { return l > 0.0f; }
 };
 
 // A row's scales, as bits: non-negative floats order like them.
@@ -298,11 +303,12 @@ __global__ void __launch_bounds__(128) prefill_merge_kernel(const PrefillPairPar
     if (p.batch.valid_req_mask != nullptr && p.batch.valid_req_mask[r] == 0) return;
     float2 ml = make_float2(-1e30f, 0.0f);
     if (lane < p.splits) ml = p.parts_ml[(size_t)lane * rows + row];
-    float m_tot = ml.y > 0.0f ? ml.x : -1e30f;
+    const bool part = ROT ? !(ml.y <= 0.0f) : ml.y > 0.0f;      // PpFormat::has_keys
+    float m_tot = part ? ml.x : -1e30f;
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) m_tot = fmaxf(m_tot, __shfl_xor_sync(0xffffffffu, m_tot, d));
-    const float w = ml.y > 0.0f ? ex2(ml.x - m_tot) : 0.0f;
-    float l_tot = ml.y * w;
+    const float w = part ? ex2(ml.x - m_tot) : 0.0f;
+    float l_tot = part ? ml.y * w : 0.0f;
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) l_tot += __shfl_xor_sync(0xffffffffu, l_tot, d);
     float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -918,7 +924,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
             float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             if (!fits) {
                 prefill_row_fp32<FMT>(p, place[0], q_off, q_head, place[1] << 6, ((place[1] + nblocks) << 6) - 1, v, l, m);
-            } else if (l > 0.0f) {
+            } else if (PpFormat<FMT>::has_keys(l)) {
                 const float4 a = *reinterpret_cast<const float4*>(src + 8 * lane), b = *reinterpret_cast<const float4*>(src + 8 * lane + 4);
                 v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
                 if (v_exp != 0) {
