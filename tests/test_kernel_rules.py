@@ -1,0 +1,30 @@
+"""Rules of the kernels' source whose breach no run is sure to show: orderings between pipeline stages that hold by timing until
+they do not.  Read from the text, on the CPU."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "warp34_b200", "csrc")
+
+
+def _code(name):
+    with open(os.path.join(CSRC, name)) as f:
+        return [x.split("//")[0] for x in f]
+
+
+@pytest.mark.parametrize("name", ["tq4_stream_tc.cuh", "prefill_pair.cuh", "tq4_prefill_tc.cuh"])
+def test_tensor_memory_accesses_are_fenced_from_the_wait_before_them(name):
+    """An access to tensor memory behind a wait on an mbarrier needs tcgen05.fence::after_thread_sync in between: the wait alone does
+    not order the access behind the MMAs whose completion it saw.  (Waits on other barriers in between are no matter; the
+    rescaling and epilogue accesses that follow a fenced one without a new wait are covered by it.)"""
+    waited = None
+    for i, line in enumerate(_code(name), 1):
+        if re.match(r"__device__|template|static", line):
+            waited = None
+        if re.search(r"\b(wait_all|mbar_wait)\(bar\(", line) and not re.search(r"Raw|KScale|QFull|QFree|KXtQ|Drain|RawFull|RawFree", line):
+            waited = i
+        if "tc_fence_after()" in line:
+            waited = None
+        if re.search(r"\btc_(ld|st)\w*\(", line) and "tc_wait" not in line and waited is not None:
+            raise AssertionError(f"{name}:{i}: access to tensor memory, unfenced since the wait in line {waited}")

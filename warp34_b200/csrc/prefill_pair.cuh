@@ -792,11 +792,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
         for (int j = 0; j < nblocks; ++j) {
             if (aborted_any()) break;
             if (!wait_all(bar(kPpS + (j & 1)), (uint32_t)((j >> 1) & 1))) { *abort_flag = 1u; break; }
-            tc_fence_after();
             // PV(j - 2) precedes QK(j) in the pipe.  Every phase is waited for: the next one of the same barrier, PV(j), needs this
             // block's weights, so that no delay of this warp lets two go by.  (One barrier for all blocks would have: PV(j - 1) needs
             // nothing more from here, and once it had completed the parity meant PV(j).)
             if (j >= 2 && !wait_all(bar(kPpPv + (j & 1)), (uint32_t)(((j - 2) >> 1) & 1))) { *abort_flag = 1u; break; }
+            tc_fence_after();
             const uint32_t t_sj = t_s + 64u * (uint32_t)(j & 1);
             const int kbase = (kb_lo + j) << 6;
             const bool all_seen = kbase >= rmin && kbase + 63 <= rmax;

@@ -434,6 +434,7 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                             }
                         }
                         if (!(ok = wait_all(bar(kXtVEmpty + res), (uint32_t)(kk ^ 1)))) break;
+                        tc_fence_after();      // the MMAs that read the granule come before the stores over it
                         const uint32_t dst = tmem + quad + kXtColV + 64u * (uint32_t)half + 32u * (uint32_t)res;
                         tc_st_16x256b_x4(dst, a[0]);
                         tc_st_16x256b_x4(dst + (16u << 16), a[1]);
@@ -483,6 +484,7 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                         e[2 * i + 1] = v.y;
                     }
                     if (!(ok = wait_all(bar(kXtKEmpty + (int)slot), (lap & 1u) ^ 1u))) break;
+                    tc_fence_after();
                     tc_st32(tmem + quad + kXtColK + 32u * slot, e);
                     tc_wait_st();
                     tc_fence_before();
