@@ -28,3 +28,14 @@ def test_tensor_memory_accesses_are_fenced_from_the_wait_before_them(name):
             waited = None
         if re.search(r"\btc_(ld|st)\w*\(", line) and "tc_wait" not in line and waited is not None:
             raise AssertionError(f"{name}:{i}: access to tensor memory, unfenced since the wait in line {waited}")
+
+
+def test_what_the_kernel_in_front_writes_is_not_read_through_the_non_coherent_path():
+    """Kernels launched behind each other overlap (tq4_common.cuh), so the plan's output (query fragments, prefix arrays) and the
+    partials change during the lifetime of the kernel that reads them: no __ldg and no const __restrict__ on them."""
+    for name in ("tq4_stream_exact.cuh", "tq4_stream_tc.cuh", "prefill_pair.cuh"):
+        for i, line in enumerate(_code(name), 1):
+            assert "__ldg(" not in line and ".nc." not in line, f"{name}:{i}: {line.strip()}"
+    for line in _code("tq4_common.cuh"):
+        if "last_not_above(" in line and "__device__" in line:
+            assert "__restrict__" not in line, line.strip()

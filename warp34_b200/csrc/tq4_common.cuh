@@ -81,7 +81,7 @@ __device__ __forceinline__ int find_request(const int32_t* __restrict__ qsl, int
 
 // The largest r in [0, n) with prefix[r] <= v, for prefix[0] <= v, by one warp: every lane counts its share of the entries
 // (one round trip to memory; a binary search makes log2(n)).  Long arrays are searched.
-__device__ __forceinline__ int last_not_above(const int32_t* __restrict__ prefix, int n, int v) {
+__device__ __forceinline__ int last_not_above(const int32_t* prefix, int n, int v) {
     if (n > 1024) {
         int lo = 0, hi = n;
         while (hi - lo > 1) {
@@ -99,7 +99,9 @@ __device__ __forceinline__ int last_not_above(const int32_t* __restrict__ prefix
 // The kernels of one attention call are launched behind each other with programmatic stream serialization: a kernel may
 // begin while the last blocks of the one before it finish, which hides the launch latency (about 2 us each on a stream).
 // Every kernel therefore waits for its predecessor's end before it touches global memory, and lets its successor start
-// being scheduled once its own blocks run.
+// being scheduled once its own blocks run.  What the predecessor writes is not read-only for such a kernel's lifetime: it is read
+// with plain loads, never through the non-coherent path (__ldg, const __restrict__).  Memory that kernels before that one wrote
+// is: a kernel lets its successor start only behind its own wait.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
 

@@ -532,7 +532,8 @@ __global__ void __launch_bounds__(kXThreads, 1) tq4_attention_stream_exact_kerne
         float o[16][4], m_run[2], l_row[2];
         const uint32_t* qf = p.qfrag + ((size_t)(r * p.layout.local_kv_heads + kv_head) * p.q_groups_max + group) * (kQFragWords * 32) + lane;
         x_stream<SPARSE>(p, x, r, g, kv_head, group, pg0, n_here,
-                         [&](uint32_t (&qb)[16][2], uint32_t (&ql)[16][2]) { x_load_query([&](int i) { return __ldg(qf + i * 32); }, qb, ql); },
+                         // (not __ldg: the plan kernel was still writing these words when this one started)
+                         [&](uint32_t (&qb)[16][2], uint32_t (&ql)[16][2]) { x_load_query([&](int i) { return qf[i * 32]; }, qb, ql); },
                          o, m_run, l_row);
         if (x.failed) {
             x_drain(x);
