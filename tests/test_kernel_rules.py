@@ -39,3 +39,21 @@ def test_what_the_kernel_in_front_writes_is_not_read_through_the_non_coherent_pa
     for line in _code("tq4_common.cuh"):
         if "last_not_above(" in line and "__device__" in line:
             assert "__restrict__" not in line, line.strip()
+
+
+@pytest.mark.parametrize("name", ["tq4_stream_tc.cuh", "prefill_pair.cuh", "tq4_prefill_tc.cuh"])
+def test_a_loop_that_votes_is_left_by_a_vote(name):
+    """Every lane takes part in each __all_sync of a polling loop, so the clock and the abort flag, which lanes read at different
+    times, may end the loop through a vote only."""
+    code = "".join(_code(name))
+    for m in re.finditer(r"\b(do|for \(;;\))\s*\{", code):
+        depth, end = 1, m.end()
+        while depth:
+            depth += {"{": 1, "}": -1}.get(code[end], 0)
+            end += 1
+        body = code[m.end():end - 1] + code[end:code.index(";", end) + 1] if m.group(1) == "do" else code[m.end():end - 1]
+        if "__all_sync" not in body:
+            continue
+        for line in body.splitlines() if "\n" in body else [body]:
+            if "clock64()" in line and "t0 =" not in line:
+                assert re.search(r"__any_sync|__all_sync", line), f"{name}: {line.strip()}"

@@ -176,13 +176,15 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
     const uint32_t bars = smem_u32(sh.bars);
     auto bar = [&](int which) { return bars + 8u * (uint32_t)which; };
     volatile uint32_t* aborted = &sh.aborted;
-    // Waits are bounded and warp-uniform; one that gives up ends every loop.
+    // Waits are bounded and warp-uniform, the decision to give up included: a lane that left alone would leave the others in a vote
+    // that never completes.  One that gives up ends every loop.
     auto wait_all = [&](uint32_t b, uint32_t parity) {
         if (__all_sync(0xffffffffu, mbar_try_wait(b, parity))) return true;
         const long long t0 = clock64();
-        do {
+        for (;;) {
             if (__all_sync(0xffffffffu, mbar_try_wait(b, parity))) return true;
-        } while (*aborted == 0u && clock64() - t0 < kWaitCycleLimit);
+            if (__any_sync(0xffffffffu, *aborted != 0u || clock64() - t0 >= kWaitCycleLimit)) break;
+        }
         *aborted = 1u;
         return false;
     };
