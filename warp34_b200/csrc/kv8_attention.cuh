@@ -820,26 +820,31 @@ static bool kv8_stream_ok(const warp34_exec* ex, const warp34_kv_layer_layout* l
     return ex->scratch_ptr != 0 && (ex->scratch_ptr & 15u) == 0;
 }
 
+// Worker slots the workspace leaves for `reqs` requests with at most `tokens` query tokens (-1: too many units).
+static long long kv8_stream_workers(const warp34_exec* ex, const warp34_kv_layer_layout* layout, const warp34_attention_batch* batch, int num_q_heads,
+                                    int reqs, long long tokens) {
+    warp34_attention_batch b = *batch;
+    b.num_reqs = reqs;
+    b.total_tokens = (int)tokens;
+    const long long items = items_bound(layout, &b, num_q_heads, kRowsPerGroup);
+    if (items * (long long)batch->max_blocks_per_req >= 0x7fffffffll) return -1;
+    const size_t plan = plan_bytes(reqs);
+    const size_t avail = ex->scratch_size > plan ? ex->scratch_size - plan : 0;
+    const long long w = (long long)(avail / ((size_t)kPartialFloats * sizeof(float))) - items;
+    return w < 0 ? 0 : w;
+}
+
+// short_og: the requests of at most batch->max_q_len tokens only, behind the pair kernel that has served the others; the merge applies
+// this epilogue.
 static int launch_kv8_stream(const warp34_exec* ex, const warp34_kv_layer_layout* layout,
                              const warp34_attention_batch* batch, const void* q_in, void* attn_out,
-                             int num_q_heads, int io_bf16, bool* taken) {
+                             int num_q_heads, int io_bf16, bool* taken, const OutputGate* short_og = nullptr) {
     *taken = false;
     int rc = 0;
     DeviceInfo* dev = device_info(&rc);
     if (dev == nullptr) return rc;
-    const size_t slot_bytes = (size_t)kPartialFloats * sizeof(float);
     const long long full_workers = (long long)dev->sm_count * kKv8StreamWarps;
-    auto workers_for = [&](int reqs, long long tokens) -> long long {
-        warp34_attention_batch b = *batch;
-        b.num_reqs = reqs;
-        b.total_tokens = (int)tokens;
-        const long long items = items_bound(layout, &b, num_q_heads, kRowsPerGroup);
-        if (items * (long long)batch->max_blocks_per_req >= 0x7fffffffll) return -1;
-        const size_t plan = plan_bytes(reqs);
-        const size_t avail = ex->scratch_size > plan ? ex->scratch_size - plan : 0;
-        const long long w = (long long)(avail / slot_bytes) - items;
-        return w < 0 ? 0 : w;
-    };
+    auto workers_for = [&](int reqs, long long tokens) { return kv8_stream_workers(ex, layout, batch, num_q_heads, reqs, tokens); };
     long long workers = 0;
     const int reqs_per_pass = pick_reqs_per_pass(batch, full_workers, kKv8StreamWarps, true, workers_for, &workers);
     if (workers < kKv8StreamWarps) return 0;      // the caller falls back to the fp32 kernel
@@ -899,7 +904,12 @@ static int launch_kv8_stream(const warp34_exec* ex, const warp34_kv_layer_layout
         p.qfrag = nullptr;
         p.q_groups_max = 0;
         p.rows_from_first_token = in_parts ? 1 : 0;
-        p.keep_status = r0 > 0 ? 1 : 0;
+        p.keep_status = r0 > 0 || short_og != nullptr ? 1 : 0;
+        if (short_og != nullptr) {
+            p.og = *short_og;
+            p.tokens_per_req = batch->max_q_len;
+            p.max_rows = batch->max_q_len * p.gqa;
+        }
         rc = launch_behind(tq4_attention_plan_kernel, 1u, 32, 0, st, p);
         if (rc != 0) return rc;
         if (fp8) {
@@ -907,7 +917,7 @@ static int launch_kv8_stream(const warp34_exec* ex, const warp34_kv_layer_layout
         } else {
             rc = launch_behind(kv8_attention_stream_kernel<WARP34_KV_FORMAT_Q8_0, kKv8StreamStages>, (unsigned)grid, kKv8StreamWarps * 32, smem, st, p);
         }
-        const long long rows = (long long)p.batch.total_tokens * num_q_heads;
+        const long long rows = (short_og != nullptr ? (long long)reqs * batch->max_q_len : (long long)p.batch.total_tokens) * num_q_heads;
         if (rc == 0) rc = launch_merge<false>(p, rows, st);
         if (rc != 0) return rc;
         rc = (int)cudaGetLastError();

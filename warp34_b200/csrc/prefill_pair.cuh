@@ -195,6 +195,7 @@ struct PrefillPairParams {
     int num_q_heads;
     int gqa;
     int tok_per_tile;      // 256 / gqa
+    int skip_rows;         // requests of at most this many query rows per kv head are left alone
     // The scores are multiplied by score_scale, which is positive.  TQ4: 1, and sm_scale * log2(e) / kPpLutScale is folded into Q' as
     // q_scale.  8-bit: |sm_scale| * log2(e), and q_scale is its sign; 1 and 0 where sm_scale is 0.
     float q_scale, score_scale;
@@ -300,6 +301,7 @@ __global__ void __launch_bounds__(128) prefill_merge_kernel(const PrefillPairPar
     const int R = p.batch.num_reqs;
     if (tok < p.batch.query_start_loc[0] || tok >= p.batch.query_start_loc[R]) return;
     const int r = last_not_above(p.batch.query_start_loc, R, tok);
+    if (p.skip_rows != 0 && p.batch.query_start_loc[r + 1] - p.batch.query_start_loc[r] <= p.skip_rows / p.gqa) return;
     if (p.batch.valid_req_mask != nullptr && p.batch.valid_req_mask[r] == 0) return;
     float2 ml = make_float2(-1e30f, 0.0f);
     if (lane < p.splits) ml = p.parts_ml[(size_t)lane * rows + row];
@@ -401,7 +403,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
         int t = (int)(blockIdx.x >> 1);
         for (int r = 0; r < p.batch.num_reqs; ++r) {
             const int ql = p.batch.query_start_loc[r + 1] - p.batch.query_start_loc[r];
-            const int nt = (ql + tpt - 1) / tpt;
+            const int nt = ql <= p.skip_rows / p.gqa ? 0 : (ql + tpt - 1) / tpt;
             if (t < nt) { req = r; tile_in_req = nt - 1 - t; break; }    // the tiles with the most keys first
             t -= nt;
         }
@@ -958,10 +960,60 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
 }  // namespace w34
 
 namespace w34 {
+// Tiles and key ranges of a launch, and an estimate of its time in units of one 64-key block (about 1.8 us).  A CTA pair costs its
+// blocks and about 7 more for its start, query and output; pairs run in waves of sm_count / 2; a split adds a merge launch (3) and
+// its rows, written and read (1e-4 each).  Measured on chunks of 16 to 2048 tokens after 0 to 30 000: within 10 % of the best split.
+// A split needs workspace for its rows.
+struct PrefillPairPlan {
+    long long tiles;
+    int splits;
+    float cost;
+};
+// Requests of the longest one's length that leave one token for each of the others.
+static long long likely_longs(const warp34_attention_batch* batch) {
+    if (batch->max_q_len < 2) return batch->num_reqs;
+    const long long n = ((long long)batch->total_tokens - batch->num_reqs + batch->max_q_len - 2) / (batch->max_q_len - 1);
+    return n < 1 ? 1 : n > batch->num_reqs ? batch->num_reqs : n;
+}
+static PrefillPairPlan prefill_pair_plan(const warp34_exec* ex, const warp34_kv_layer_layout* layout, const warp34_attention_batch* batch, int num_q_heads,
+                                         int sm_count, int skip_rows) {
+    const int gqa = num_q_heads / layout->local_kv_heads, tok_per_tile = kPpRows / gqa;
+    long long reqs = batch->num_reqs;      // with tiles: those that are not skipped have more tokens than skip_rows / gqa
+    if (skip_rows != 0 && batch->total_tokens / (skip_rows / gqa + 1) < reqs) reqs = batch->total_tokens / (skip_rows / gqa + 1);
+    PrefillPairPlan plan;
+    plan.tiles = (long long)batch->total_tokens / tok_per_tile + reqs;
+    long long likely = plan.tiles;      // that have work
+    if (skip_rows != 0) {
+        const long long longs = likely_longs(batch);
+        if (longs < reqs) { likely -= reqs - longs; reqs = longs; }
+    }
+    plan.splits = 1;
+    plan.cost = 0.0f;
+    const long long rows = (long long)batch->total_tokens * num_q_heads;
+    const long long blocks = batch->max_seq_len > 0 ? (batch->max_seq_len + kPpKeys - 1) / kPpKeys : 0;
+    const long long by_longest = reqs * ((batch->max_q_len + tok_per_tile - 1) / tok_per_tile);
+    const long long pairs = (by_longest > 0 && by_longest < likely ? by_longest : likely) * layout->local_kv_heads, at_once = sm_count / 2 > 0 ? sm_count / 2 : 1;
+    long long fit = 1;
+    if (ex->scratch_ptr != 0 && (ex->scratch_ptr & 15u) == 0 && ex->scratch_size > 256 && rows > 0) {
+        fit = (long long)((ex->scratch_size - 256) / ((size_t)rows * (kHeadDim + 2) * sizeof(float)));
+        if (fit > kPpMaxSplits) fit = kPpMaxSplits;
+        if (fit < 1) fit = 1;
+    }
+    const float mean = (float)blocks - 0.5f * (float)batch->max_q_len / kPpKeys;      // a causal chunk's tiles differ
+    for (int n = 1; n <= fit && (n == 1 || n <= blocks); ++n) {
+        const float waves = (float)((pairs * n + at_once - 1) / at_once);
+        float cost = waves * (mean / (float)n + 7.0f);
+        if (cost < (float)blocks / (float)n + 7.0f) cost = (float)blocks / (float)n + 7.0f;
+        if (n > 1) cost += 3.0f + 1e-4f * (float)n * (float)rows;
+        if (n == 1 || cost < plan.cost) { plan.cost = cost; plan.splits = n; }
+    }
+    return plan;
+}
+
 // The pair kernel for one layer's chunk.  Workspace: a status word, and room for the parts when it splits.
 template <int FMT>
 static int launch_prefill_pair(const warp34_exec* ex, const warp34_kv_layer_layout* layout, const warp34_attention_batch* batch,
-                               const void* q_in, void* attn_out, int num_q_heads, int io_bf16, const OutputGate& og, int sm_count) {
+                               const void* q_in, void* attn_out, int num_q_heads, int io_bf16, const OutputGate& og, int sm_count, int skip_rows = 0) {
     int32_t* status = nullptr;      // the first word of the workspace, when there is one
     if (ex->scratch_ptr != 0 && (ex->scratch_ptr & 3u) == 0 && ex->scratch_size >= sizeof(PlanHeader)) {
         status = reinterpret_cast<int32_t*>((uintptr_t)ex->scratch_ptr);   // PlanHeader::status
@@ -986,35 +1038,18 @@ static int launch_prefill_pair(const warp34_exec* ex, const warp34_kv_layer_layo
     }
     pp.status = status;
     pp.og = og;
-    const long long tiles = (long long)batch->total_tokens / pp.tok_per_tile + batch->num_reqs;
+    pp.skip_rows = skip_rows;
+    const PrefillPairPlan plan = prefill_pair_plan(ex, layout, batch, num_q_heads, sm_count, skip_rows);
+    const long long tiles = plan.tiles;
     if (tiles > 0x3fffffffll) return (int)cudaErrorInvalidValue;
-    // Key ranges per tile, by an estimate in units of one 64-key block (about 1.8 us).  A CTA pair costs its blocks and about 7
-    // more for its start, query and output; pairs run in waves of sm_count / 2; a split adds a merge launch (3) and its rows,
-    // written and read (1e-4 each).  Measured on chunks of 16 to 2048 tokens after 0 to 30 000: within 10 % of the best split.
-    // A split needs workspace for its rows.
+    if (tiles == 0) return 0;
     const long long rows = (long long)batch->total_tokens * num_q_heads;
-    const long long blocks = batch->max_seq_len > 0 ? (batch->max_seq_len + kPpKeys - 1) / kPpKeys : 0;
-    const long long by_longest = (long long)batch->num_reqs * ((batch->max_q_len + pp.tok_per_tile - 1) / pp.tok_per_tile);
-    const long long pairs = (by_longest > 0 && by_longest < tiles ? by_longest : tiles) * layout->local_kv_heads, at_once = sm_count / 2 > 0 ? sm_count / 2 : 1;
-    pp.splits = 1;
+    pp.splits = plan.splits;
     pp.parts = nullptr;
     pp.parts_ml = nullptr;
-    if (ex->scratch_ptr != 0 && (ex->scratch_ptr & 15u) == 0 && ex->scratch_size > 256 && rows > 0) {
-        long long fit = (long long)((ex->scratch_size - 256) / ((size_t)rows * (kHeadDim + 2) * sizeof(float)));
-        if (fit > kPpMaxSplits) fit = kPpMaxSplits;
-        const float mean = (float)blocks - 0.5f * (float)batch->max_q_len / kPpKeys;      // a causal chunk's tiles differ
-        float best = 0.0f;
-        for (int n = 1; n <= fit && n <= blocks; ++n) {
-            const float waves = (float)((pairs * n + at_once - 1) / at_once);
-            float cost = waves * (mean / (float)n + 7.0f);
-            if (cost < (float)blocks / (float)n + 7.0f) cost = (float)blocks / (float)n + 7.0f;
-            if (n > 1) cost += 3.0f + 1e-4f * (float)n * (float)rows;
-            if (n == 1 || cost < best) { best = cost; pp.splits = n; }
-        }
-        if (pp.splits > 1) {
-            pp.parts = reinterpret_cast<float*>((uintptr_t)ex->scratch_ptr + 256);
-            pp.parts_ml = reinterpret_cast<float2*>(pp.parts + (size_t)pp.splits * rows * kHeadDim);
-        }
+    if (pp.splits > 1) {
+        pp.parts = reinterpret_cast<float*>((uintptr_t)ex->scratch_ptr + 256);
+        pp.parts_ml = reinterpret_cast<float2*>(pp.parts + (size_t)pp.splits * rows * kHeadDim);
     }
     cudaStream_t st = (cudaStream_t)ex->stream;
     const dim3 grid(2u * (unsigned)tiles, (unsigned)layout->local_kv_heads, (unsigned)pp.splits);

@@ -573,6 +573,9 @@ struct StreamParams {
     int keep_status = 0;             // plan: OR into the status word instead of clearing it (second and later passes)
     int query_tiles = 0;             // qfrag holds tcgen05 operand tiles of rows_per_group rows instead of fragments
     int min_units = kMinUnitsPerWarp;    // smallest share of a worker
+    // Requests with more query rows per kv head than max_rows take no part (0: all do), and the merge's grid is tokens_per_req x q
+    // heads for every request (0: x q heads for every token).
+    int max_rows = 0, tokens_per_req = 0;
     const int32_t* sel_phys = nullptr;
     const int32_t* sel_logical = nullptr;
     const int32_t* num_selected = nullptr;
@@ -645,7 +648,7 @@ __global__ void __launch_bounds__(kPlanThreads) tq4_attention_plan_kernel(const 
             }
         } else if (r < R) {
             const ReqGeom g = load_req(p.batch, r);
-            if (g.valid) {
+            if (g.valid && (p.max_rows == 0 || g.q_len <= p.max_rows / p.gqa)) {
                 const int lo = row_min_kv(p.batch, g, 0);
                 const int hi = row_max_kv(p.batch, g, g.q_len - 1);
                 if (hi >= lo) { plo = lo >> 4; npages = (hi >> 4) - plo + 1; }
@@ -1385,7 +1388,11 @@ __global__ void __launch_bounds__(MW * 32) tq4_attention_merge_kernel(const Stre
     const long long row_ll = blockIdx.x;
     int tok = (int)(row_ll / p.num_q_heads);
     const int q_head = (int)(row_ll % p.num_q_heads);
-    if (p.rows_from_first_token) {   // a part of a larger batch: its tokens start at query_start_loc[0]
+    if (p.tokens_per_req != 0) {
+        const int req = tok / p.tokens_per_req, off = tok - req * p.tokens_per_req, first = p.batch.query_start_loc[req];
+        tok = first + off;
+        if (tok >= p.batch.query_start_loc[req + 1]) return;   // (a request with more tokens has no items, see below)
+    } else if (p.rows_from_first_token) {   // a part of a larger batch: its tokens start at query_start_loc[0]
         tok += p.batch.query_start_loc[0];
         if (tok >= p.batch.query_start_loc[p.batch.num_reqs]) return;   // the grid is sized by max_q_len
     }
@@ -1956,6 +1963,48 @@ static bool takes_prefill_path(uint64_t flags, const warp34_kv_layer_layout* l,
            b->max_blocks_per_req > 0 && gqa <= kPpCtaRows && ((long long)b->max_q_len * gqa > 24 || want_tc);
 }
 
+// ---- 8-bit layers with more than 24 query rows in some request: stream kernel, CTA-pair kernel, or each for its requests ----------
+// The stream kernel reads a request's pages once per 8 rows, the pair kernel once per 256 but takes about as long for one row as for
+// 256.  A batch of a scheduler mixes both: decode rows beside a prompt's chunk.  The requests' own lengths are known on the device
+// only, so that the choice rests on what the host knows (requests, tokens, the longest request and context) and, where both kernels
+// run, each leaves the other's requests alone.
+enum Kv8Route { kKv8Pair, kKv8Stream, kKv8Both };
+constexpr int kKv8ShortRows = 24;
+// The batch as the stream kernel sees it where both run: only requests of at most kKv8ShortRows rows.
+static warp34_attention_batch kv8_short_part(const warp34_attention_batch* batch, int gqa) {
+    warp34_attention_batch b = *batch;
+    b.max_q_len = kKv8ShortRows / gqa;
+    b.total_tokens = (int)part_tokens(&b, b.num_reqs);
+    return b;
+}
+// Times in microseconds.  Stream: 23 + 1.2 for every thousand (page, kv head, 8 rows); pair: 2.1 a block of its own estimate.  Against
+// FP8 and Q8_0 batches of 1 to 64 requests of 5 to 24 tokens (24 and 16 heads on 4) after 128 to 16384 keys: stream kernel 382 us,
+// pair kernel 611, for 64 requests of 30 rows after 4096 keys; 720 and 641 for 60 rows; 24 and 18 for one of 30 rows after 128;
+// 46 and 57 after 16384.  The choice is the slower one by at most 12 %.  63 decode rows of 16384 keys beside a chunk of 512 tokens:
+// 1831 us with the pair kernel for all, 612 with both (two requests, 16384 keys and a chunk of 64 tokens after 100: 92 and 78).
+static Kv8Route kv8_chunk_route(const warp34_exec* ex, const warp34_kv_layer_layout* l, const warp34_attention_batch* b, const void* q_in, int hq,
+                                int io_bf16, int sms) {
+    const int gqa = hq / l->local_kv_heads, short_tokens = kKv8ShortRows / gqa;
+    if (!kv8_stream_ok(ex, l, b, q_in, io_bf16)) return kKv8Pair;
+    const float keys = (float)(b->max_seq_len > 0 ? (long long)b->max_seq_len : (long long)b->max_blocks_per_req * kPageTokens);
+    const float per_item = 1.2e-3f * (float)l->local_kv_heads * (keys / kPageTokens + 1.0f);
+    const float pair_all = 2.1f * prefill_pair_plan(ex, l, b, hq, sms, 0).cost;
+    if ((long long)b->max_q_len * gqa <= 3 * kKv8ShortRows) {
+        const float items = (float)b->total_tokens * (float)gqa / kRowsPerGroup + 0.5f * (float)b->num_reqs;
+        if (23.0f + per_item * items < pair_all && kv8_stream_workers(ex, l, b, hq, b->num_reqs, b->total_tokens) >= (long long)sms * kKv8StreamWarps / 2) return kKv8Stream;
+    }
+    if (short_tokens < 1 || b->num_reqs < 2 || (long long)b->num_reqs * b->max_q_len <= b->total_tokens) return kKv8Pair;
+    // The host cannot tell a few long requests beside decode rows from ragged prompts, for which the second set of launches would be
+    // spent in vain: the others must be short on average.
+    const long long shorts = b->num_reqs - likely_longs(b);
+    const bool lopsided = ((long long)b->total_tokens - b->max_q_len) * 4 < (long long)(b->num_reqs - 1) * b->max_q_len;
+    if (shorts < 1 || !lopsided) return kKv8Pair;
+    const warp34_attention_batch rest = kv8_short_part(b, gqa);
+    if (kv8_stream_workers(ex, l, &rest, hq, rest.num_reqs, rest.total_tokens) < (long long)sms * kKv8StreamWarps / 2) return kKv8Pair;
+    const float both = 2.1f * prefill_pair_plan(ex, l, b, hq, sms, kKv8ShortRows).cost + 18.0f + per_item * (float)shorts;
+    return both < pair_all ? kKv8Both : kKv8Pair;
+}
+
 static bool takes_kv8_chunk_path(uint64_t flags, const warp34_kv_layer_layout* l, const warp34_attention_batch* b, int num_q_heads) {
     if ((flags & WARP34_B200_EXEC_FLAG_PRECISE_ATTENTION) != 0 || !kv8_canonical(l) || l->k_base == 0 || l->v_base == 0 ||
         l->local_kv_heads <= 0 || num_q_heads % l->local_kv_heads != 0 || b->num_reqs <= 0 || b->block_tables == nullptr ||
@@ -1990,9 +2039,18 @@ static int launch_attention(const warp34_exec* ex, const warp34_kv_layer_layout*
             int rc = 0;
             const DeviceInfo* dev = device_info(&rc);
             if (dev == nullptr) return rc;
-            return layout->k_format == WARP34_KV_FORMAT_FP8_E4M3
-                       ? launch_prefill_pair<WARP34_KV_FORMAT_FP8_E4M3>(ex, layout, batch, q_in, attn_out, num_q_heads, io_bf16, og, dev->sm_count)
-                       : launch_prefill_pair<WARP34_KV_FORMAT_Q8_0>(ex, layout, batch, q_in, attn_out, num_q_heads, io_bf16, og, dev->sm_count);
+            const Kv8Route route = kv8_chunk_route(ex, layout, batch, q_in, num_q_heads, io_bf16, dev->sm_count);
+            if (route != kKv8Stream) {
+                const int skip_rows = route == kKv8Both ? kKv8ShortRows : 0;
+                rc = layout->k_format == WARP34_KV_FORMAT_FP8_E4M3
+                         ? launch_prefill_pair<WARP34_KV_FORMAT_FP8_E4M3>(ex, layout, batch, q_in, attn_out, num_q_heads, io_bf16, og, dev->sm_count, skip_rows)
+                         : launch_prefill_pair<WARP34_KV_FORMAT_Q8_0>(ex, layout, batch, q_in, attn_out, num_q_heads, io_bf16, og, dev->sm_count, skip_rows);
+                if (rc != 0 || route == kKv8Pair) return rc;
+                const warp34_attention_batch rest = kv8_short_part(batch, num_q_heads / layout->local_kv_heads);
+                bool taken = false;
+                rc = launch_kv8_stream(ex, layout, &rest, q_in, attn_out, num_q_heads, io_bf16, &taken, &og);
+                return rc != 0 || taken ? rc : (int)cudaErrorInvalidValue;      // (kv8_chunk_route has seen that it is taken)
+            }
         }
         const int rc8 = launch_kv8_attention(ex, layout, batch, q_in, attn_out, num_q_heads, io_bf16,
                                              (ex->flags & WARP34_B200_EXEC_FLAG_PRECISE_ATTENTION) == 0 && force <= 0);
