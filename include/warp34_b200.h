@@ -307,7 +307,8 @@ int warp34_paged_attention_bf16(const warp34_exec* ex, const warp34_kv_layer_lay
  * ======================================================================== */
 
 /*
- * Upper bound of the scratch the split-KV path can use for a batch geometry
+ * Upper bound of the scratch that warp34_paged_attention_f16 can use for a batch geometry: the split-KV
+ * path's, or the parts of a short prefill chunk whose keys are cut into ranges
  * (only host-known fields of `batch` are read).  The reference sizes the same
  * buffer inline (op_paged_attn.cu:1301-1338).
  */

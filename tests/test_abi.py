@@ -6,6 +6,7 @@ import ctypes as C
 import os
 import re
 
+from util import canonical_layout
 from warp34_b200 import ffi
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -104,3 +105,24 @@ def test_argument_validation_needs_no_gpu(native_libs):
     lay.k_head_stride_bytes = lay.v_head_stride_bytes = 2112
     lay.k_page_stride_bytes = lay.v_page_stride_bytes = 8448
     assert qsa(C.addressof(ex), p, None, C.addressof(lay), p, p, p, p, None, p, 0, 8, 4, 0.0625) == 0    # no tokens: no launch
+
+
+def test_scratch_bytes_covers_a_short_chunk_cut_into_key_ranges():
+    """A chunk of few tiles after a long context is cut into key ranges, each with rows of 258 floats in the workspace
+    (attention_prefill_pair_kernel): a host that sizes its workspace by the bound gets as many of them as one without a limit (13 tiles
+    of 4 kv heads on 74 pairs of SMs: four ranges; 7 tiles: five; 2 tiles: nine, which the streaming path's share covers)."""
+    lib = ffi.kernels()
+    lay = canonical_layout(4)
+    b = ffi.AttentionBatch()
+    b.num_reqs, b.max_blocks_per_req = 1, 3000
+    row = 24 * 258 * 4
+
+    def bound(tokens, keys):
+        b.total_tokens = b.max_q_len = tokens
+        b.max_seq_len = keys
+        return lib.warp34_paged_attention_scratch_bytes(C.byref(lay), C.byref(b), 24)
+
+    assert bound(512, 30512) >= 4 * 512 * row
+    assert bound(256, 30256) >= 5 * 256 * row
+    assert bound(64, 30064) >= 9 * 64 * row
+    assert bound(2048, 2048) < 3 * 2048 * row          # fills the GPU by itself

@@ -969,6 +969,10 @@ struct PrefillPairPlan {
     int splits;
     float cost;
 };
+// Workspace of a launch that cuts its keys into `splits` ranges: the status word's line, then rows and their (m, l).
+static size_t prefill_pair_parts_bytes(const warp34_attention_batch* batch, int num_q_heads, int splits) {
+    return splits > 1 ? 256 + (size_t)splits * (size_t)batch->total_tokens * (size_t)num_q_heads * (kHeadDim + 2) * sizeof(float) : 0;
+}
 // Requests of the longest one's length that leave one token for each of the others.
 static long long likely_longs(const warp34_attention_batch* batch) {
     if (batch->max_q_len < 2) return batch->num_reqs;
@@ -995,9 +999,8 @@ static PrefillPairPlan prefill_pair_plan(const warp34_exec* ex, const warp34_kv_
     const long long pairs = (by_longest > 0 && by_longest < likely ? by_longest : likely) * layout->local_kv_heads, at_once = sm_count / 2 > 0 ? sm_count / 2 : 1;
     long long fit = 1;
     if (ex->scratch_ptr != 0 && (ex->scratch_ptr & 15u) == 0 && ex->scratch_size > 256 && rows > 0) {
-        fit = (long long)((ex->scratch_size - 256) / ((size_t)rows * (kHeadDim + 2) * sizeof(float)));
-        if (fit > kPpMaxSplits) fit = kPpMaxSplits;
-        if (fit < 1) fit = 1;
+        fit = kPpMaxSplits;
+        while (fit > 1 && prefill_pair_parts_bytes(batch, num_q_heads, (int)fit) > ex->scratch_size) --fit;
     }
     const float mean = (float)blocks - 0.5f * (float)batch->max_q_len / kPpKeys;      // a causal chunk's tiles differ
     for (int n = 1; n <= fit && (n == 1 || n <= blocks); ++n) {

@@ -1949,7 +1949,16 @@ extern "C" size_t warp34_paged_attention_scratch_bytes(const warp34_kv_layer_lay
                                                   (long long)sms * (w34::kFastWarps > w34::kExactWarps ? w34::kFastWarps : w34::kExactWarps));
     const int rows = w34::xt_rows(batch, gqa);
     const size_t tiles = rows != 0 ? w34::xt_scratch_bytes(layout, batch, num_q_heads, rows, sms) : 0;
-    return most > tiles ? most : tiles;
+    // a chunk: the parts of its key ranges, as many as the pair kernel would cut without a limit
+    size_t parts = 0;
+    if (gqa >= 1 && gqa <= w34::kPpCtaRows && batch->total_tokens > 0 && (long long)batch->max_q_len * gqa > 24) {
+        warp34_exec any = {};
+        any.scratch_ptr = 16;
+        any.scratch_size = ~(size_t)0;
+        parts = w34::prefill_pair_parts_bytes(batch, num_q_heads, w34::prefill_pair_plan(&any, layout, batch, num_q_heads, sms, 0).splits);
+    }
+    const size_t stream = most > tiles ? most : tiles;
+    return stream > parts ? stream : parts;
 }
 
 namespace w34 {
