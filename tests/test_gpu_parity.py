@@ -891,3 +891,28 @@ def test_graph_replayed_steps_match_eager_steps(env):
         assert torch.equal(a, b)
     for (ak, av), (bk, bv) in zip(pools[0], pools[1]):
         assert (ak == bk).all() and (av == bv).all()
+
+
+@pytest.mark.parametrize("hq,q_len,ctx", [(24, 1, [300]),                # K, V and Q of one sequence: 16 KB, copied with the metadata
+                                          (24, 1, [300, 40]),            # and beyond, with a graph of their own
+                                          (24, 4, [100, 60])])           # 24 rows, growing past 128 keys: another kernel from there on
+def test_graph_steps_match_eager_ones_at_their_switches(env, hq, q_len, ctx):
+    kv, synth = env["kv"], env["synth"]
+    hkv, outs = 4, []
+    for use_graph in (False, True):
+        wl = synth.PagedWorkload(ctx, [q_len] * len(ctx), hkv, seed=72, slack_pages=16)
+        wl.fill_context(kv.Executor(8 << 20), 72)
+        step = kv.DecodeStep(wl.layer, wl.seqs, hq, max_q_len=q_len, scratch_bytes=32 << 20, extra_blocks=4)
+        res = []
+        for it in range(12):
+            for s in wl.seqs:
+                assert s.reserve(s.committed_len + q_len) >= 0
+            n = q_len * len(ctx)
+            k, v = synth.make_kv(n, hkv, 900 + it)
+            step.k_host.copy_(k); step.v_host.copy_(v); step.q_host.copy_(synth.make_q(n, hq, 900 + it))
+            res.append(step.run([q_len] * len(ctx), graph=use_graph).clone())
+            for s in wl.seqs:
+                s.commit(q_len)
+        outs.append(res)
+    for it, (a, b) in enumerate(zip(*outs)):
+        assert torch.equal(a, b), it

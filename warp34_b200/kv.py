@@ -616,11 +616,12 @@ class DecodeStep:
         self.h2d_bytes = self.io.nbytes + self.payload_bytes      # upper bound: a full metadata upload
         self.h2d_bytes_total = 0                                  # bytes actually copied by run() so far
         self._graphs = {}
+        self._payload_graph = None      # K, V and Q: the same for every geometry
         self.d2h_bytes = self.out_host.numel() * 2
         self._fence = None      # recorded after a step's last use of the pinned buffers when sync=False
 
     def _capture(self, lib):
-        """CUDA graphs for the whole step (the reference replays its decode steps the same way,
+        """The CUDA graph of a step of this geometry and, the first time, the one of K, V and Q.  Together the whole step (the reference replays its decode steps the same way,
         crates/warp34-host/src/model/graphs.rs:199-259): upload K, V, Q, lengths and slots, append, attend with the
         output written to pinned memory.  Block tables are not in them: their changed part is copied in front.  K, V and Q get a graph of their own,
         launched before the host packs the step's metadata so that the copy runs while the CPU works; up to SMALL_PAYLOAD
@@ -648,8 +649,7 @@ class DecodeStep:
                 payload()
             body()                      # warm-up outside the capture (one-time attribute calls)
             for fn in (payload, body):
-                if fn is payload and not split:
-                    graphs.append(None)
+                if fn is payload and (not split or self._payload_graph is not None):
                     continue
                 # captured directly: torch.cuda.graph() would also collect garbage and return every cached block to the
                 # driver, milliseconds of a new step's first run, for a capture that allocates nothing
@@ -662,7 +662,9 @@ class DecodeStep:
                 graphs.append(g)
         torch.cuda.current_stream().wait_stream(side)
         self.ex.set_stream()
-        return tuple(graphs)
+        if len(graphs) > 1:
+            self._payload_graph = graphs[0]
+        return graphs[-1]
 
     def run(self, q_lens, sm_scale=1.0 / 16.0, lib=None, sync=True, attend=None, graph=False,
             mask_mode=0, sliding_window=0):
@@ -673,22 +675,26 @@ class DecodeStep:
             self._fence.synchronize()
             self._fence = None
         if graph and attend is None:
-            # baked into the captured launches (the descriptors are passed by value): the geometry,
-            # the softmax scale, the mask mode and the window, and the executor's flags
-            key = (id(lib), len(self.seqs), int(sum(q_lens)), int(max(q_lens)), float(sm_scale),
-                   int(mask_mode), int(sliding_window), int(self.ex.ex.flags))
-            g = self._graphs.get(key)
-            if g is not None and g[0] is not None:
-                g[0].replay()           # K, V, Q on their way while the metadata is packed
+            sent = self._payload_graph is not None
+            if sent:
+                self._payload_graph.replay()            # K, V, Q on their way while the metadata is packed
             self.io.pack(self.seqs, q_lens, sm_scale, mask_mode, sliding_window)
+            # baked into the captured launches (the descriptors are passed by value): the geometry, the softmax scale, the
+            # mask mode and the window, and the executor's flags; with more than 8 query rows per kv head also what is chosen
+            # by the longest sequence (the kernel and its key ranges), to the next power of two
+            rows = self.hq // self.layer.layout.local_kv_heads * int(max(q_lens))
+            longest = int(self.io.desc.max_seq_len).bit_length() if rows > 8 else 0
+            key = (id(lib), len(self.seqs), int(sum(q_lens)), int(max(q_lens)), float(sm_scale),
+                   int(mask_mode), int(sliding_window), int(self.ex.ex.flags), longest)
+            g = self._graphs.get(key)
             if g is None:
                 self.io.upload(full=True)
                 g = self._graphs[key] = self._capture(lib)
-                if g[0] is not None:
-                    g[0].replay()
+                if self._payload_graph is not None and not sent:
+                    self._payload_graph.replay()
             self.meta_bytes_last = self.io.upload(tables_only=True) + 4 * self.io.head_words - self.payload_bytes
             self.h2d_bytes_total += self.meta_bytes_last + self.payload_bytes
-            g[1].replay()
+            g.replay()
             self._finish(sync)
             return self.out_host
         self.io.pack(self.seqs, q_lens, sm_scale, mask_mode, sliding_window)
