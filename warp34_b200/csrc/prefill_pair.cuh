@@ -21,7 +21,7 @@
 //
 // K and V elements are row scale x centroid (or code): hi = fp16(d c), lo = fp16(d c - hi), about 22 bits together as long as
 // lo is not far below fp16's normal range.  Where a sample of a tile's rows is small (PpScales: below about 2^-3), K or V
-// is therefore held divided by a power of two for the whole tile, which the consumers take out again in fp32 at no cost: a factor
+// is therefore held divided by a power of two for the whole tile, which the consumers take out again in fp32: a factor
 // of the scores for K, of the normalised output for V.  (Without it 21 % of the outputs of a TQ4 chunk over K of magnitude 2^-10
 // under Q of magnitude 2^10 were not the nearest fp16 value, against 3 % at magnitude 1, and one missed 2e-3 + 1e-2 |b| by 16 %.
 // A power of two for every key or every 32 keys took 10 to 35 % more time on long contexts: each block then waits for its scales.)
@@ -109,7 +109,7 @@ template <int FMT> struct PpSmem {
     static constexpr uint32_t kOffRaw = kOffQLo + (PpFormat<FMT>::kRotated ? kPpQLoBytes : 0u);
     static constexpr uint32_t kOffLut = (kOffRaw + kPpRawStages * kRaw + 127u) & ~127u;
     static constexpr uint32_t kOffBars = kOffLut + (PpFormat<FMT>::kRotated ? kPpLutBytes : 0u);
-    static constexpr uint32_t kBytes = kOffBars + 256u;
+    static constexpr uint32_t kBytes = kOffBars + 288u;
     static_assert(kPpCtaRows * kPpOutStride * 4 <= (int)kOffLut, "epilogue staging must end before the table");
     static_assert(kPpCtaRows * 512 <= (int)kOffQLo, "Q' staging fits the tile stages");
     static_assert(kBytes <= 227u * 1024u, "shared memory");
@@ -195,7 +195,7 @@ struct PrefillPairParams {
     int num_q_heads;
     int gqa;
     int tok_per_tile;      // 256 / gqa
-    int skip_rows;         // requests of at most this many query rows per kv head are left alone
+    int skip_tokens;       // requests of at most this many tokens are left alone
     // The scores are multiplied by score_scale, which is positive.  TQ4: 1, and sm_scale * log2(e) / kPpLutScale is folded into Q' as
     // q_scale.  8-bit: |sm_scale| * log2(e), and q_scale is its sign; 1 and 0 where sm_scale is 0.
     float q_scale, score_scale;
@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(128) prefill_merge_kernel(const PrefillPairPar
     const int R = p.batch.num_reqs;
     if (tok < p.batch.query_start_loc[0] || tok >= p.batch.query_start_loc[R]) return;
     const int r = last_not_above(p.batch.query_start_loc, R, tok);
-    if (p.skip_rows != 0 && p.batch.query_start_loc[r + 1] - p.batch.query_start_loc[r] <= p.skip_rows / p.gqa) return;
+    if (p.skip_tokens != 0 && p.batch.query_start_loc[r + 1] - p.batch.query_start_loc[r] <= p.skip_tokens) return;
     if (p.batch.valid_req_mask != nullptr && p.batch.valid_req_mask[r] == 0) return;
     float2 ml = make_float2(-1e30f, 0.0f);
     if (lane < p.splits) ml = p.parts_ml[(size_t)lane * rows + row];
@@ -342,7 +342,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
     volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(gen + S::kOffBars + 244);
     uint32_t* row_max = reinterpret_cast<uint32_t*>(gen + S::kOffBars + 224);                      // largest scale of the tile's K, V rows
     volatile int* exponents = reinterpret_cast<volatile int*>(gen + S::kOffBars + 232);            // of K, of V
-    volatile int* place = reinterpret_cast<volatile int*>(gen + S::kOffBars + 248);                // request, first block (for prefill_row_fp32)
+    // request, first block, first token, rows, first token of the request: for the epilogue, which reads them again so that they take no
+    // registers from the consumers
+    volatile int* place = reinterpret_cast<volatile int*>(gen + S::kOffBars + 256);
     auto bar = [&](int which) { return bars + 8u * (uint32_t)which; };
     // Waits and abort checks are warp-uniform: no lane leaves a loop alone.
     auto wait_all = [&](uint32_t b, uint32_t parity) {
@@ -403,7 +405,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
         int t = (int)(blockIdx.x >> 1);
         for (int r = 0; r < p.batch.num_reqs; ++r) {
             const int ql = p.batch.query_start_loc[r + 1] - p.batch.query_start_loc[r];
-            const int nt = ql <= p.skip_rows / p.gqa ? 0 : (ql + tpt - 1) / tpt;
+            const int nt = min((ql + tpt - 1) / tpt, ql > p.skip_tokens ? 0x7fffffff : 0);
             if (t < nt) { req = r; tile_in_req = nt - 1 - t; break; }    // the tiles with the most keys first
             t -= nt;
         }
@@ -533,7 +535,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
     if (wid == 12) {
         const int ek = PpScales<FMT>::exponent(__reduce_max_sync(0xffffffffu, max(sample_k[0], sample_k[1])));
         const int ev = PpScales<FMT>::exponent(__reduce_max_sync(0xffffffffu, max(sample_v[0], sample_v[1])));
-        if (lane == 0) { exponents[0] = ek; exponents[1] = ev; place[0] = req; place[1] = kb_lo; }
+        if (lane == 0) { exponents[0] = ek; exponents[1] = ev; place[0] = req; place[1] = kb_lo; place[2] = tok0; place[3] = rows_used; place[4] = g.q_start; }
     }
     if (ROT) fence_proxy_async();     // the residual tile is read by the tensor core
     tc_fence_before();
@@ -789,7 +791,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
         const uint32_t lane_base = (uint32_t)(32 * wid) << 16;
         const uint32_t t_o = tmem + lane_base + kPpColO, t_s = tmem + lane_base + kPpColS;
         const uint32_t leader_pready = map_to_rank(bar(kPpPReady), 0u);
-        const float factor = fmaxf(power_of_two(ek) * p.score_scale, 1.2e-38f);      // never 0: masked scores are -infinity
+        const float factor = ROT ? power_of_two(ek) : 1.0f;
 #pragma unroll 1
         for (int j = 0; j < nblocks; ++j) {
             if (aborted_any()) break;
@@ -802,13 +804,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
             const uint32_t t_sj = t_s + 64u * (uint32_t)(j & 1);
             const int kbase = (kb_lo + j) << 6;
             const bool all_seen = kbase >= rmin && kbase + 63 <= rmax;
-            // Scores of keys [32 c, + 32) of the block, masked; `factor` is still to be applied.
+            // Scores of keys [32 c, + 32) of the block, masked.  TQ4: `factor`, the exponent's power of two, is still to be applied.  8-bit:
+            // p.score_scale is, a constant operand (in one register with the power of two it made these builds spill, and a stack
+            // frame costs this kernel several us a launch).
             auto scores = [&](int c, float (&sv)[32]) {
                 uint32_t r[32];
                 tc_ld32(r, t_sj + 32u * (uint32_t)c);
                 tc_wait_ld();
 #pragma unroll
                 for (int i = 0; i < 32; ++i) sv[i] = __uint_as_float(r[i]);
+                if (!ROT && ek != 0) {
+                    const float up = power_of_two(exponents[0]);
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) sv[i] *= up;
+                }
                 if (!all_seen) {
 #pragma unroll
                     for (int i = 0; i < 32; ++i) {
@@ -827,7 +836,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
 #pragma unroll
                 for (int i = 0; i < 32; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], sv[ROT ? 0 : c][i]);
             }
-            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * factor;
+            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * (ROT ? factor : p.score_scale);
             // the reference maximum moves only when the true maximum ran ahead by more than the threshold
             const bool need = mx > m_ref + kPpRescaleThreshold;
             float alpha = 1.0f;
@@ -858,7 +867,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
                     // masked scores are -infinity: ex2 gives exactly 0 against any finite reference
-                    const float pa = ex2(__fmaf_rn(sv[ROT ? 0 : c][2 * i], factor, -m_use)), pb = ex2(__fmaf_rn(sv[ROT ? 0 : c][2 * i + 1], factor, -m_use));
+                    const float sa = sv[ROT ? 0 : c][2 * i], sb = sv[ROT ? 0 : c][2 * i + 1];
+                    const float pa = ex2(__fmaf_rn(sa, ROT ? factor : p.score_scale, -m_use)), pb = ex2(__fmaf_rn(sb, ROT ? factor : p.score_scale, -m_use));
                     ls4[i & 3] += pa + pb;
                     const __half2 h = __floats2half2_rn(pa, pb);
                     const float2 hf = __half22float2(h);
@@ -915,12 +925,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
     tc_fence_before();
     __syncthreads();
     if (!aborted) {
+        const int first_token = place[2], rows = place[3], q_start = place[4];
         for (int row = wid; row < kPpCtaRows; row += kPpWarps) {
-            const int trow = row0 + row;
-            if (trow >= rows_used) break;
-            const int q_off = tok0 + trow / p.gqa;
+            const int trow = (int)cluster_rank() * kPpCtaRows + row;
+            if (trow >= rows) break;
+            const int q_off = first_token + trow / p.gqa;
             const int q_head = kv_head * p.gqa + trow % p.gqa;
-            if (p.batch.valid_token_mask != nullptr && p.batch.valid_token_mask[g.q_start + q_off] == 0) continue;
+            if (p.batch.valid_token_mask != nullptr && p.batch.valid_token_mask[q_start + q_off] == 0) continue;
             const float* src = stage + row * kPpOutStride;
             float l = src[256], m = src[257];
             float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -935,7 +946,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
                     for (int i = 0; i < 8; ++i) v[i] *= up;
                 }
             }
-            const size_t out_row = (size_t)(g.q_start + q_off) * p.num_q_heads + q_head;
+            const size_t out_row = (size_t)(q_start + q_off) * p.num_q_heads + q_head;
             if (p.splits > 1) {
                 const size_t part_row = (size_t)blockIdx.z * p.batch.total_tokens * p.num_q_heads + out_row;
                 float4* dst = reinterpret_cast<float4*>(p.parts + part_row * kHeadDim + 8 * lane);
@@ -1036,12 +1047,12 @@ static int launch_prefill_pair(const warp34_exec* ex, const warp34_kv_layer_layo
     if (PpFormat<FMT>::kRotated) {
         pp.q_scale /= kPpLutScale;
     } else if (pp.q_scale != 0.0f) {
-        pp.score_scale = fabsf(pp.q_scale);
+        pp.score_scale = fmaxf(fabsf(pp.q_scale), 1.2e-38f);      // (never 0: masked scores are -infinity)
         pp.q_scale = pp.q_scale < 0.0f ? -1.0f : 1.0f;
     }
     pp.status = status;
     pp.og = og;
-    pp.skip_rows = skip_rows;
+    pp.skip_tokens = skip_rows / pp.gqa;
     const PrefillPairPlan plan = prefill_pair_plan(ex, layout, batch, num_q_heads, sm_count, skip_rows);
     const long long tiles = plan.tiles;
     if (tiles > 0x3fffffffll) return (int)cudaErrorInvalidValue;
