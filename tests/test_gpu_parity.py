@@ -916,3 +916,16 @@ def test_graph_steps_match_eager_ones_at_their_switches(env, hq, q_len, ctx):
         outs.append(res)
     for it, (a, b) in enumerate(zip(*outs)):
         assert torch.equal(a, b), it
+
+
+def test_device_output_of_a_graph_step(env):
+    """DecodeStep.out_dev holds the last step's output on the device whether or not graphs are used."""
+    kv, synth = env["kv"], env["synth"]
+    wl = synth.PagedWorkload([50, 70], [1, 1], 4, seed=73)
+    wl.fill_context(kv.Executor(8 << 20), 73)
+    step = kv.DecodeStep(wl.layer, wl.seqs, 16, scratch_bytes=8 << 20)
+    for it in range(3):
+        k, v = synth.make_kv(2, 4, 950 + it)
+        step.k_host.copy_(k); step.v_host.copy_(v); step.q_host.copy_(synth.make_q(2, 16, 950 + it))
+        out = step.run([1, 1], graph=it != 1)
+        assert torch.equal(step.out_dev.cpu(), out) and bool((out != 0).any())

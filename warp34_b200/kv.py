@@ -611,7 +611,8 @@ class DecodeStep:
         self.k_host, self.v_host, self.q_host = views(self.io.host)
         self.k_dev, self.v_dev, self.q_dev = views(self.io.dev)
         self.out_host = torch.zeros(*shapes[2], dtype=torch.float16).pin_memory()
-        self.out_dev = torch.zeros_like(self.out_host, device=device)
+        self._out_dev = torch.zeros_like(self.out_host, device=device)
+        self._out_dev_stale = False     # a replayed step writes its output to pinned memory only
         self.payload_bytes = self.payload_words * 4
         self.h2d_bytes = self.io.nbytes + self.payload_bytes      # upper bound: a full metadata upload
         self.h2d_bytes_total = 0                                  # bytes actually copied by run() so far
@@ -695,8 +696,10 @@ class DecodeStep:
             self.meta_bytes_last = self.io.upload(tables_only=True) + 4 * self.io.head_words - self.payload_bytes
             self.h2d_bytes_total += self.meta_bytes_last + self.payload_bytes
             g.replay()
+            self._out_dev_stale = True
             self._finish(sync)
             return self.out_host
+        self._out_dev_stale = False
         self.io.pack(self.seqs, q_lens, sm_scale, mask_mode, sliding_window)
         self.meta_bytes_last = self.io.upload() - self.payload_bytes      # K, V and Q with it
         self.h2d_bytes_total += self.meta_bytes_last + self.payload_bytes
@@ -710,6 +713,14 @@ class DecodeStep:
         self.out_host.copy_(self.out_dev, non_blocking=True)
         self._finish(sync)
         return self.out_host
+
+    @property
+    def out_dev(self):
+        """The last step's output on the device (after a replayed step copied there when asked for)."""
+        if self._out_dev_stale:
+            self._out_dev.copy_(self.out_host, non_blocking=True)
+            self._out_dev_stale = False
+        return self._out_dev
 
     def _finish(self, sync):
         if sync:
