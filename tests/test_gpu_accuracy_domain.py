@@ -61,7 +61,8 @@ def _float64_attention(env, wl, ctx, q, hq, hkv, q_len=1):
 @pytest.mark.parametrize("ctx,q_len", [([1, 2, 3, 5, 8, 13, 17, 31, 40], 1), ([100, 150, 299], 1),
                                        ([64, 300], 4), ([90, 260], 70)])
 def test_default_kernels_hold_the_bound_beyond_the_benchmark_distribution(env, ctx, q_len):
-    """Decode (stream kernel), draft tokens (three 8-row items per kv head) and a prefill chunk (128-row kernel)."""
+    """Decode (one-warp stream kernel), draft tokens (24-row items of the tcgen05 stream kernel from 128 keys on) and a prefill
+    chunk (CTA-pair kernel)."""
     ffi, kv, synth = env["ffi"], env["kv"], env["synth"]
     hq, hkv, n = 24, 4, len(ctx)
     worst = {"default": 0.0, "fp32": 0.0}

@@ -34,10 +34,14 @@ def test_rows_of_any_alignment_and_value(native_libs, hkv, n, shift):
 
 
 def test_two_byte_aligned_destinations_and_non_finite_rows(native_libs):
-    """The 16-bit store path writes what the 32-bit one does; a row with NaN or infinity leaves its neighbours alone."""
+    """The 16-bit store path writes what the 32-bit one does; a row with NaN or infinity leaves its neighbours alone: every other
+    (token, head) row, of K and of V, is what it is when those two values are finite."""
     from warp34_b200 import kv, synth
     n, hkv = 20, 2
     k, v = synth.make_kv(n, hkv, 9, device="cuda")
+    clean = synth.PagedWorkload([0], [n], hkv, seed=3, fill=0x3C)
+    kv.kv_cache_write(kv.Executor(1 << 16), clean.layer, clean.step(), k, v)
+    torch.cuda.synchronize()
     k[3, 5], v[7, 300] = float("nan"), float("inf")
     pools = []
     for off in (0, 2):
@@ -49,3 +53,9 @@ def test_two_byte_aligned_destinations_and_non_finite_rows(native_libs):
         pools.append((base[off:off + wl.layer.k.numel()].cpu(), wl.layer.v.cpu()))
     assert torch.equal(pools[0][0], pools[1][0]) and torch.equal(pools[0][1], pools[1][1])
     assert (pools[0][0] != 0x3C).any()
+    pages = clean.seqs[0].pages      # the same seed: the same pages
+    for got, want, token, head in ((pools[0][0], clean.layer.k.cpu(), 3, 0), (pools[0][1], clean.layer.v.cpu(), 7, 1)):
+        differ = (got.view(-1, hkv, 16, 132) != want.view(-1, hkv, 16, 132)).any(-1)
+        poisoned = torch.zeros_like(differ)
+        poisoned[pages[token // 16], head, token % 16] = True
+        assert differ[poisoned].all() and not differ[~poisoned].any(), torch.nonzero(differ & ~poisoned)[:4]

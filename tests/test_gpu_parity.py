@@ -830,9 +830,9 @@ def test_forced_kernel_selector_validates_like_the_reference(env):
 
 @pytest.mark.parametrize("mode", ["default", "short_chunk", "verify", "fast", "fast_short_chunk", "fast_verify", "verify_flag"])
 def test_prefill_dispatch_paths_agree_with_the_oracle(env, mode):
-    """Default: the register-MMA prefill kernel with value + residual operands (also with partly
-    filled 128-row tiles) and 8-row items for a verify batch, held to the plain bound.  With the
-    fast flag: the tcgen05 kernel and the four-warp team kernel, held to the bound of the fast build."""
+    """Default: the CTA-pair prefill kernel with value + residual operands (also with partly filled
+    256-row tiles) and the tcgen05 stream kernel for a verify batch, held to the plain bound.  With the fast flag:
+    the single-operand tcgen05 prefill kernel, and the same stream kernel, held to the bound of the fast build."""
     kv, synth, ffi = env["kv"], env["synth"], env["ffi"]
     hkv = 4
     shape = {"default": (16, 200, 333), "short_chunk": (16, 20, 100), "verify": (24, 4, 1500)}

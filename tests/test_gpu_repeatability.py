@@ -19,7 +19,7 @@ CASES = {
     "decode_fast": ([3000, 17, 811, 4096, 260, 1], 1, "EXEC_FLAG_FAST_ATTENTION", "tq4", (24, 4)),
     "decode_one_long_row": ([40000], 1, None, "tq4", (16, 4)),
     "verify": ([900, 2100, 64], 4, None, "tq4", (24, 4)),
-    "verify_team": ([900, 2100, 64], 4, "EXEC_FLAG_FAST_ATTENTION", "tq4", (24, 4)),
+    "verify_fast": ([900, 2100, 64], 4, "EXEC_FLAG_FAST_ATTENTION", "tq4", (24, 4)),
     "chunk": ([700, 300], 150, None, "tq4", (16, 4)),
     "chunk_tcgen05": ([700, 300], 150, "EXEC_FLAG_FAST_ATTENTION", "tq4", (16, 4)),
     "fp32": ([500, 90], 1, "EXEC_FLAG_PRECISE_ATTENTION", "tq4", (24, 4)),
