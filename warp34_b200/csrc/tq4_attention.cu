@@ -1986,18 +1986,18 @@ static warp34_attention_batch kv8_short_part(const warp34_attention_batch* batch
     b.total_tokens = (int)part_tokens(&b, b.num_reqs);
     return b;
 }
-// Times in microseconds.  Stream: 23 + 1.2 for every thousand (page, kv head, 8 rows); pair: 2.3 a block of its own estimate.  Against
-// FP8 and Q8_0 batches of 1 to 64 requests of 5 to 24 tokens (24 and 16 heads on 4) after 128 to 16384 keys: stream kernel 382 us,
-// pair kernel 611, for 64 requests of 30 rows after 4096 keys; 720 and 641 for 60 rows; 24 and 18 for one of 30 rows after 128;
-// 46 and 57 after 16384.  The choice is the slower one by at most 12 %.  63 decode rows of 16384 keys beside a chunk of 512 tokens:
-// 1831 us with the pair kernel for all, 612 with both (two requests, 16384 keys and a chunk of 64 tokens after 100: 92 and 78).
+// Times in microseconds.  Stream: 23 + 1.2 (Q8_0: 1.4) for every thousand (page, kv head, 8 rows); pair: 2.15 a block of its own estimate.
+// Measured on FP8 batches (24 and 16 heads on 4), stream / pair kernel: 64 requests of 30 rows after 4096 keys 382 / 520, of 60 rows
+// 720 / 577; 64 of 30 rows after 1024 keys 110 / 184, of 72 rows 212 / 192; 16 of 48 rows after 4096 keys 122 / 126 (Q8_0 151 / 125); one of
+// 30 rows after 128 keys 24 / 18, after 16384 44 / 57.  Both kernels for 63 decode rows of 16384 keys beside a chunk of 512 tokens 612,
+// the pair kernel for all 1831 (one decode row and 64 tokens after 100 keys: 78 and 92).
 static Kv8Route kv8_chunk_route(const warp34_exec* ex, const warp34_kv_layer_layout* l, const warp34_attention_batch* b, const void* q_in, int hq,
                                 int io_bf16, int sms) {
     const int gqa = hq / l->local_kv_heads, short_tokens = kKv8ShortRows / gqa;
     if (!kv8_stream_ok(ex, l, b, q_in, io_bf16)) return kKv8Pair;
     const float keys = (float)(b->max_seq_len > 0 ? (long long)b->max_seq_len : (long long)b->max_blocks_per_req * kPageTokens);
-    const float per_item = 1.2e-3f * (float)l->local_kv_heads * (keys / kPageTokens + 1.0f);
-    const float pair_all = 2.3f * prefill_pair_plan(ex, l, b, hq, sms, 0).cost;
+    const float per_item = (l->k_format == WARP34_KV_FORMAT_FP8_E4M3 ? 1.2e-3f : 1.4e-3f) * (float)l->local_kv_heads * (keys / kPageTokens + 1.0f);
+    const float pair_all = 2.15f * prefill_pair_plan(ex, l, b, hq, sms, 0).cost;
     if ((long long)b->max_q_len * gqa <= 3 * kKv8ShortRows) {
         const float items = (float)b->total_tokens * (float)gqa / kRowsPerGroup + 0.5f * (float)b->num_reqs;
         if (23.0f + per_item * items < pair_all && kv8_stream_workers(ex, l, b, hq, b->num_reqs, b->total_tokens) >= (long long)sms * kKv8StreamWarps / 2) return kKv8Stream;
@@ -2010,7 +2010,7 @@ static Kv8Route kv8_chunk_route(const warp34_exec* ex, const warp34_kv_layer_lay
     if (shorts < 1 || !lopsided) return kKv8Pair;
     const warp34_attention_batch rest = kv8_short_part(b, gqa);
     if (kv8_stream_workers(ex, l, &rest, hq, rest.num_reqs, rest.total_tokens) < (long long)sms * kKv8StreamWarps / 2) return kKv8Pair;
-    const float both = 2.3f * prefill_pair_plan(ex, l, b, hq, sms, kKv8ShortRows).cost + 18.0f + per_item * (float)shorts;
+    const float both = 2.15f * prefill_pair_plan(ex, l, b, hq, sms, kKv8ShortRows).cost + 18.0f + per_item * (float)shorts;
     return both < pair_all ? kKv8Both : kKv8Pair;
 }
 
