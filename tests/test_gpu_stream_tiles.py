@@ -90,3 +90,33 @@ def test_row_triples(env):
     out = torch.zeros_like(q)
     env["kv"].paged_attention(env["ex"], wl.layer, b, q, out, 16)
     _check(env, out, want)
+
+
+@pytest.mark.parametrize("hq,hkv,exps", [(24, 4, (-10, -10)), (16, 4, (-13, -13)), (24, 4, (-13, 3)), (24, 4, (6, -9))])
+def test_accuracy_does_not_depend_on_the_magnitude_of_v(env, hq, hkv, exps):
+    """V times 2^b: the stored codes are the same and every scale is the same but for a power of two, so the outputs are those of
+    magnitude 1 times 2^b.  At magnitude 1 about 1 % of them are not the float64 result's nearest fp16 value: at most twice that
+    many differ.  Two exponents: the second one for the tokens from 700 on, and the comparison is with the fp32 kernel."""
+    kv, synth = env["kv"], env["synth"]
+    ctx, new = [2000, 600, 1300], [4, 4, 3]
+    n, outs, ones = sum(new), {}, (0, 0)
+    for e in (ones, exps):
+        wl = synth.PagedWorkload([0] * 3, [c + m for c, m in zip(ctx, new)], hkv, seed=5, fill=0x7F)
+        k, v = synth.make_kv(sum(ctx) + n, hkv, 6, device="cuda")
+        tok = torch.cat([torch.arange(c + m) for c, m in zip(ctx, new)]).cuda()
+        v = (v.float() * 16).round() / 16 * torch.where(tok < 700, 2.0 ** e[0], 2.0 ** e[1])[:, None]
+        kv.kv_cache_write(env["ex"], wl.layer, wl.step(), k, v.half())
+        for s, c in zip(wl.seqs, ctx):
+            s.commit(c)
+        b = wl.step(q_lens=new)
+        q = synth.make_q(n, hq, 6, device="cuda")
+        out, want = torch.zeros_like(q), torch.zeros_like(q)
+        env["ex"].scratch.fill_(0xA5)
+        kv.paged_attention(env["ex"], wl.layer, b, q, out, hq)
+        kv.paged_attention(env["ex"], wl.layer, b, q, want, hq, scalar=True)
+        _check(env, out, want)
+        outs[e] = out.float()
+    if exps[0] == exps[1]:
+        base, got = outs[ones], outs[exps] * 2.0 ** -exps[0]
+        normal = base.abs() >= 2.0 ** (-13 - exps[0])           # fp16 has all its bits on both sides
+        assert float((got != base)[normal].float().mean()) <= 0.02

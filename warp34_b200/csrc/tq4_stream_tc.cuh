@@ -11,7 +11,10 @@
 // scores of both halves and applies its K scales there, and P is multiplied by the V scale of its key and half.
 //
 //   softmax: four warps per eight rows, thread = key.  P goes to shared memory as the B operand; the running maximum is a
-//            reference that moves only when it is exceeded by 2^3, so a block usually needs no reduction over its keys
+//            reference that moves only when it is exceeded by 2^3, so a block usually needs no reduction over its keys.  P d_v is held
+//            times a power of two that moves with it and brings the block's largest V scale to [2^11, 2^12): two fp16 numbers then
+//            hold 22 bits of the weights of small V rows as well (without it 7.9 % of the outputs over V of magnitude 2^-10 were not the
+//            nearest fp16 value, 4.1 % with three 8-row items of the one-warp kernel)
 //   V:       eight warps, thread = fragment position (16x256b stores put channel pairs of four keys in place), half x quadrant;
 //            64 keys at a time, values into one granule, residuals into the next
 //   K:       eight warps, thread = key, 32 channels at a time into a ring of four TMEM granules; values and residuals lie next
@@ -43,6 +46,7 @@ struct XtShared {
     float2 k_scale[2][kXtKeys];
     __align__(16) float m_ref[24], alpha[24], mass[24];
     float red[4][24];                // [warp of the part][row]
+    float red_v[4][3];               // [warp of the part][part]
     int row_min[24], row_max[24];
     uint32_t tmem;
     uint32_t aborted;
@@ -530,6 +534,7 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                     safe_hi = min(safe_hi, row_max[i]);
                 }
             }
+            float v_up = 1.0f;         // power of two by which P d_v is multiplied
             float l[P], m_lag[P];      // this key's mass of every row; the reference maxima plus the lag
 #pragma unroll
             for (int i = 0; i < P; ++i) {
@@ -583,11 +588,29 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                         if (key > last || pos < row_min[i] || pos > row_max[i]) sc[i] = -INFINITY;
                     }
                 }
-                bool ahead = false;
+                bad = bad || !wait_all(bar(kXtRawVFull + (int)(c % STAGES)), (c / STAGES) & 1u);
+                const uint32_t v_row = raw_v((int)(c % STAGES)) + (uint32_t)key * kTq4RowBytes;
+                float2 dv = make_float2(__half2float(__ushort_as_half((unsigned short)(lds32(v_row) & 0xffffu))),
+                                        __half2float(__ushort_as_half((unsigned short)(lds32(v_row + 64) >> 16))));
+                if (!full) {      // a key no row can see may hold never-written bytes: its scale must not meet a zero weight
+                    bool seen = false;
+#pragma unroll
+                    for (int i = 0; i < P; ++i) seen = seen || sc[i] > -INFINITY;
+                    if (!seen) dv = make_float2(0.0f, 0.0f);
+                }
+                const float v_most = fmaxf(fabsf(dv.x), fabsf(dv.y));
+                bool ahead = v_most * v_up > 32768.0f && v_most <= 65504.0f;      // (infinite scales have no power of two)
 #pragma unroll
                 for (int i = 0; i < P; ++i) ahead = ahead || sc[i] > m_lag[i];
                 const bool moved = xt_any(ahead, part);
-                if (moved) {      // the reference maximum of some row moves: take the block's maxima
+                float v_by = 1.0f;
+                if (moved) {      // the reference maximum of some row moves, or V outgrows its power of two: take the block's maxima
+                    {
+                        float t = v_most <= 65504.0f ? v_most : 0.0f;
+#pragma unroll
+                        for (int d = 16; d > 0; d >>= 1) t = fmaxf(t, __shfl_xor_sync(0xffffffffu, t, d));
+                        if (lane == 0) sh.red_v[wid & 3][part] = t;
+                    }
 #pragma unroll
                     for (int i = 0; i < P; ++i) {
                         float t = sc[i];
@@ -609,11 +632,13 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                         l[i] *= alpha[i];
                         m_lag[i] = m_ref[i] + kXtLag;
                     }
+                    const float t = fmaxf(fmaxf(sh.red_v[0][part], sh.red_v[1][part]), fmaxf(sh.red_v[2][part], sh.red_v[3][part]));
+                    if (t > 0.0f) {
+                        v_by = 1.0f / v_up;      // (powers of two throughout)
+                        v_up = __uint_as_float((uint32_t)(127 + 11 + 127 - (int)(__float_as_uint(t) >> 23)) << 23);
+                        v_by *= v_up;
+                    }
                 }
-                bad = bad || !wait_all(bar(kXtRawVFull + (int)(c % STAGES)), (c / STAGES) & 1u);
-                const uint32_t v_row = raw_v((int)(c % STAGES)) + (uint32_t)key * kTq4RowBytes;
-                float2 dv = make_float2(__half2float(__ushort_as_half((unsigned short)(lds32(v_row) & 0xffffu))),
-                                        __half2float(__ushort_as_half((unsigned short)(lds32(v_row + 64) >> 16))));
                 // P and O are in use until the output product of the block before has completed
                 bad = bad || (c > 0 && !wait_all(bar(kXtPvDone), (c - 1) & 1u));
                 if (moved && b > 0) {
@@ -626,19 +651,15 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                             tc_ld4(o, t_o + (uint32_t)(q * R + i0));
                             tc_wait_ld();
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha[i0 + i]);
+                            for (int i = 0; i < 4; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * (alpha[i0 + i] * v_by));
                             tc_st4(t_o + (uint32_t)(q * R + i0), o);
                         }
                     }
                     tc_wait_st();
                     tc_fence_before();
                 }
-                if (!full) {      // a key no row can see may hold never-written bytes: its scale must not meet a zero weight
-                    bool seen = false;
-#pragma unroll
-                    for (int i = 0; i < P; ++i) seen = seen || sc[i] > -INFINITY;
-                    if (!seen) dv = make_float2(0.0f, 0.0f);
-                }
+                dv.x *= v_up;
+                dv.y *= v_up;
                 // 16-byte chunk of the key's column, swizzled by the row
                 const uint32_t at = p_t + (uint32_t)(key >> 6) * (uint32_t)(N * 128) + (uint32_t)row0 * 128u + 2u * (uint32_t)(key & 7) +
                                     (((uint32_t)(key & 63) >> 3) << 4);
@@ -672,6 +693,7 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                 float* dst = partials + (size_t)sg.slot * (R * kHeadDim + 2 * R);
                 // TMEM lane 32 q + 16 T + gid (+ 8): code word 4 q + gid / 2, channels 2 (2 (gid & 1) + T) (+ 1) of it
                 const int T = lane >> 4, gid = lane & 7, odd = (lane >> 3) & 1;
+                const float v_down = 1.0f / v_up;
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int ch = vword_col(h, 4 * (wid & 3) + (gid >> 1), 2 * (2 * (gid & 1) + T) + odd);
@@ -682,7 +704,7 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                         tc_ld4(b4, t_o + (uint32_t)(h * N + R + i0));
                         tc_wait_ld();
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) dst[(row0 + i0 + i) * kHeadDim + ch] = __uint_as_float(a[i]) + __uint_as_float(b4[i]);
+                        for (int i = 0; i < 4; ++i) dst[(row0 + i0 + i) * kHeadDim + ch] = (__uint_as_float(a[i]) + __uint_as_float(b4[i])) * v_down;
                     }
                 }
                 if (key < P) {
