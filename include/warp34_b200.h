@@ -57,7 +57,8 @@ enum {
  * tcgen05 kernel, one 128-row CTA per request and KV head, instead of the split-KV kernel. */
 #define WARP34_B200_EXEC_FLAG_TCGEN05_VERIFY (1ull << 42)
 /* Additive: the tensor-core kernels feed every operand as one fp16 value, as the reference's own
- * tensor-core kernel does (op_paged_attn.cu:357, :47-50, :470).  Faster; a softmax weight is then
+ * tensor-core kernel does (op_paged_attn.cu:357, :47-50, :470), except that steps of 9 to 24 query rows
+ * per request and kv head keep the default kernel, which is the faster one there.  Faster; a softmax weight is then
  * off by a few 1e-4 relative, so an output channel in which large values of V cancel can miss
  * 2e-3 + 1e-2 |b| against dequant-then-attend.  Without the flag the kernels carry the rounding
  * residuals of Q', of the K centroids and of P through extra products and meet that bound. */
@@ -206,12 +207,15 @@ int warp34_fused_k_rmsnorm_rope_kv_cache_write_f16(
  * activations far beyond that (x60 outliers in 32 channels and a query scale of
  * 3: a few outputs per million miss the bound by up to 3.6x) WARP34_B200_EXEC_FLAG_PRECISE_ATTENTION
  * selects the fp32 kernel, which stays below a seventh of the bound on all of these.
- * WARP34_B200_EXEC_FLAG_FAST_ATTENTION trades the residual operands for speed.  Kernels: decode and verify batches
- * (up to 24 query rows per request and kv head) stream split-KV work items of 8 rows; larger
+ * WARP34_B200_EXEC_FLAG_FAST_ATTENTION trades the residual operands for speed.  Kernels: decode batches
+ * (up to 8 query rows per request and kv head) stream split-KV work items of 8 rows; verify batches of 9 to 24 rows
+ * stream items of 16 or 24 rows on a tcgen05 kernel (8-row items below 128 keys or with little scratch); larger
  * chunks, of TQ4 and of 8-bit layers, take a tcgen05 kernel of two CTAs and 256 rows (TQ4 with the fast flag: one
  * CTA, 128 rows, single operands).
- * 8-bit boundary layers (Q8_0, FP8 E4M3) in the canonical packing stream the same way on a
- * tensor-core kernel whose operands are exact (codes convert exactly to fp16); other packings of
+ * 8-bit boundary layers (Q8_0, FP8 E4M3) in the canonical packing stream 8-row items on a
+ * tensor-core kernel whose operands are exact (codes convert exactly to fp16); where a batch has requests of more
+ * than 24 rows, the requests, or the whole batch, go to that kernel or to the one for chunks, whichever an estimate
+ * from the batch's geometry says is faster.  Other packings of
  * them, callers without scratch and WARP34_B200_EXEC_FLAG_PRECISE_ATTENTION take an fp32 kernel.
  */
 int warp34_paged_attention_f16(const warp34_exec* ex, const warp34_kv_layer_layout* layout,
@@ -419,8 +423,8 @@ int warp34_kv_page_copy(const warp34_exec* ex, const warp34_kv_layer_layout* lay
  *    group of 8 query rows and one more per request, for every kv head, plus 8) and 6.25 KiB of
  *    query fragments per group; about 730 (request, kv head) pairs of a decode batch, e.g. 182
  *    requests at 4 kv heads, is the ceiling.  A
- *    prefill chunk (more than 24 query rows per request and kv head) uses only the status word,
- *    whatever its size.  Larger batches are refused with cudaErrorInvalidValue and nothing is
+ *    prefill chunk (more than 24 query rows per request and kv head) needs only the status word,
+ *    whatever its size; a short one uses the rest of the array for the parts of its key ranges.  Larger batches are refused with cudaErrorInvalidValue and nothing is
  *    launched; when `scratch_needed` is not NULL it receives the bytes the batch would have
  *    needed, so the caller can tell "too large" from a malformed argument.
  *  - TQ4 layers in the canonical 132-byte-row packing only: other packings and the 8-bit
@@ -434,7 +438,7 @@ int warp34_kv_page_copy(const warp34_exec* ex, const warp34_kv_layer_layout* lay
  *  - All calls on a device share the one array, and it keeps whatever the previous call left.
  *    Every call rewrites the plan and each partial before reading it, so no clearing is needed,
  *    but two calls whose kernels overlap on the GPU (different streams without an event
- *    between them) race on it.  Serialise them.
+ *    between them), chunks included, race on it.  Serialise them.
  */
 int warp34_paged_attention_f16_static_scratch(uintptr_t stream, const warp34_kv_layer_layout* layout,
                                               const warp34_attention_batch* batch,

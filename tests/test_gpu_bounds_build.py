@@ -44,7 +44,7 @@ CASES = {
     # name: (contexts, q_len, flags name, formats)
     "decode": ([700, 31, 2000, 16], 1, None, None),
     "verify": ([300, 1000], 4, None, None),
-    "verify_team": ([300, 1000], 4, "EXEC_FLAG_FAST_ATTENTION", None),
+    "verify_fast": ([300, 1000], 4, "EXEC_FLAG_FAST_ATTENTION", None),
     "chunk": ([90, 260], 70, None, None),
     "chunk_tcgen05": ([90, 260], 70, "EXEC_FLAG_FAST_ATTENTION", None),
     "fp32": ([500, 40], 1, "EXEC_FLAG_PRECISE_ATTENTION", None),

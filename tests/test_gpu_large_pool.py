@@ -20,7 +20,7 @@ CASES = {
     "tq4_decode_fast": ("tq4", [700, 31, 2000], 1, "EXEC_FLAG_FAST_ATTENTION", (24, 4)),
     "tq4_fp32": ("tq4", [300, 40], 1, "EXEC_FLAG_PRECISE_ATTENTION", (24, 4)),
     "tq4_verify": ("tq4", [300, 1000], 4, None, (24, 4)),
-    "tq4_verify_team": ("tq4", [300, 1000], 4, "EXEC_FLAG_FAST_ATTENTION", (24, 4)),
+    "tq4_verify_fast": ("tq4", [300, 1000], 4, "EXEC_FLAG_FAST_ATTENTION", (24, 4)),
     "tq4_chunk": ("tq4", [200, 400], 100, None, (16, 4)),
     "tq4_chunk_tcgen05": ("tq4", [200, 400], 100, "EXEC_FLAG_FAST_ATTENTION", (16, 4)),
     "fp8_decode": ("fp8", [700, 31], 1, None, (24, 4)),

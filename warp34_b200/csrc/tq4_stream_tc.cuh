@@ -7,7 +7,7 @@
 //   S^T[128 keys x 2R]      per 128-half = Khi [Q'hi | Q'lo]^T + Klo [Q'hi | Q'lo]^T        lane = key
 //   O^T[128 channels x 2R]  per 128-half += (Vhi + Vlo)^T [(P d_v)hi | (P d_v)lo]^T          lane = channel
 // (the centroids' residuals on every block: leaving them out where no key has a large weight takes one more vote of the softmax
-// warps a block, 921 us against 914, and an error several times as large).  Scales stay outside the operands: a thread holds a key's
+// warps a block, then 921 us against 914, and an error several times as large).  Scales stay outside the operands: a thread holds a key's
 // scores of both halves and applies its K scales there, and P is multiplied by the V scale of its key and half.
 //
 //   softmax: four warps per eight rows, thread = key.  P goes to shared memory as the B operand; the running maximum is a
@@ -21,10 +21,11 @@
 //            to each other as the table returns them, and the query operand repeats each pair of columns to match
 //   one warp copies raw pages and query rows, one issues the score products, one the output products
 //
-// Measured on 128 requests of 2048 to 16384 keys, four query tokens, 24 / 4 heads (1.26 GB of pages): 898 us against 1464 with
-// three 8-row items of the one-warp kernel (tq4_stream_exact.cuh), which looks every code up three times.  Bound by the softmax
-// warps' serial chain from scores to P and by the shared-memory data pipe that the look-ups share with them: a block of 128 keys
-// takes about 6700 cycles at 14100 instructions; the pipe is 72 % busy, the issue slots 60 %, the tensor pipe 26 %.  Taking the
+// Measured on 128 requests of 2048 to 16384 keys, four query tokens, 24 / 4 heads (1.26 GB of pages): attention call 870 us against 1458
+// with three 8-row items of the one-warp kernel (tq4_stream_exact.cuh), which looks every code up three times.  Bound by the softmax
+// warps' serial chain from scores to P and by the shared-memory data pipe that the look-ups share with them.  (Counters of the build whose
+// V residuals still had bank conflicts, 877 us: 6700 cycles and 14100 instructions a block of 128 keys, the pipe 72 % busy, the issue
+// slots 60 %, the tensor pipe 26 %.)  Taking the
 // weights before the vote on the reference (one barrier a block fewer) put them behind the wait for the previous output
 // product: 1008 us.
 #pragma once
