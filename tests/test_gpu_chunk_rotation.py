@@ -1,0 +1,58 @@
+"""The chunk kernel rotates its query rows and its outputs in groups of four: groups that end inside a tile, head groups that do not
+divide four, masked tokens inside a group, rows off a 16-byte boundary, with and without the output gate, in both activation types,
+against the fp32 dequant-then-attend path of the same entry point."""
+import pytest
+
+from util import plain_parity
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("hq,hkv,new,off,mode,drop", [
+    (1, 1, [25], 0, 0, ()),                     # 25 rows: the last group has one
+    (3, 1, [43, 9], 0, 1, (0, 2, 50)),          # 129 rows: one row of the second CTA; masked tokens inside groups
+    (6, 1, [5, 64], 0, 2, ()),                  # 30 rows, and 384: the second tile ends at its 128th row
+    (10, 2, [51, 52], 4, 1, (3,)),              # 5 heads, rows 8 bytes off a 16-byte boundary
+    (12, 2, [43], 4, 2, ()),
+])
+def test_row_groups_match_dequant_then_attend(native_libs, hq, hkv, new, off, mode, drop):
+    import numpy as np
+    from warp34_b200 import ffi, kv, synth
+    f, tr = ffi.KV_FORMAT_TQ4, ffi.KV_TRANSFORM_RADEMACHER_WHT256
+    wl = synth.PagedWorkload([70] * len(new), new, hkv, seed=3, formats=(f, f, tr, tr))
+    ex = kv.Executor(64 << 20)
+    wl.fill_context(ex, 3)
+    n = sum(new)
+    k, v = synth.make_kv(n, hkv, 4, device="cuda")
+    kv.kv_cache_write(ex, wl.layer, wl.step(), k, v)
+    vtm = np.ones(n, np.uint8)
+    vtm[list(drop)] = 0
+    b = wl.step(valid_token_mask=vtm)
+
+    def shifted(t):
+        store = torch.zeros(t.numel() + 8, dtype=t.dtype, device="cuda")
+        store[off:off + t.numel()] = t.reshape(-1)
+        return store[off:off + t.numel()].view(n, hq, 256)
+
+    q, gate = shifted(synth.make_q(n, hq, 5, device="cuda")), shifted(synth.make_q(n, hq, 6, device="cuda"))
+    outs = []
+    for flags in (0, ffi.EXEC_FLAG_PRECISE_ATTENTION):
+        ex.ex.flags = flags
+        out = shifted(torch.full((n, hq, 256), -7.0, dtype=torch.float16, device="cuda"))
+        if mode:
+            kv.paged_attention_gated(ex, wl.layer, b, q, gate, out, hq, hadamard64=mode == 2)
+        else:
+            kv.paged_attention(ex, wl.layer, b, q, out, hq)
+        torch.cuda.synchronize()
+        outs.append(out.float().cpu().numpy())
+    keep = vtm.astype(bool)
+    assert (outs[0][~keep] == -7.0).all()
+    got, want = outs[0][keep], outs[1][keep]
+    if mode == 2:      # an output mixes 64 gated values, each within its own bound: compared before the mixing
+        h = torch.ones(1, 1)
+        for _ in range(6):
+            h = torch.cat([torch.cat([h, h], 1), torch.cat([h, -h], 1)], 0)
+        got, want = ((x.reshape(-1, 64) @ (h / 8).numpy()) for x in (got, want))
+    ok, msg = plain_parity(got, want)
+    assert ok, msg

@@ -208,6 +208,75 @@ struct PrefillPairParams {
     float2* parts_ml;
 };
 
+// ---- rotation of a tile's rows, four at a time -------------------------------------------------------
+// Eight lanes hold a row, 32 columns each, so that five of the eight levels of the 256-point transform are register arithmetic; between two
+// such layouts the columns change lanes through shared memory.  (A row over a whole warp takes 40 shuffles; those of a tile's 128 rows kept
+// the SM busy for 16 000 cycles before the first product and for as long again behind the last: 31 of the 46 thousand cycles of a
+// tile of one block.)
+//   chunks: lane j of a row, register 8 i + e: column 8 (j + 8 i) + e         quads: lane l, register 4 j + e: column 8 (j + 8 (l / 2)) + 4 (l % 2) + e
+// Where 16-byte quad u of a row is kept while its columns change lanes: without bank conflicts from either side.
+__device__ __forceinline__ uint32_t quad_place(uint32_t u) { return u ^ ((u >> 3) & 1u) ^ (((u >> 4) & 3u) << 1); }
+// Levels of the transform whose bit of the column is a bit of the register index, for the bits in LEVELS.  Two butterflies at a time (the
+// difference as fma(b, -1, a), the same number): half the instructions, which is what these phases are bound by.
+__device__ __forceinline__ uint64_t pair_of(float a, float b) { return (uint64_t)__float_as_uint(a) | ((uint64_t)__float_as_uint(b) << 32); }
+template <int LEVELS>
+__device__ __forceinline__ void rotate_registers(float (&v)[32]) {
+    if (LEVELS & 1) {
+#pragma unroll
+        for (int k = 0; k < 32; k += 2) {
+            const float a = v[k], b = v[k + 1];
+            v[k] = a + b;
+            v[k + 1] = a - b;
+        }
+    }
+    const uint64_t minus_one = pair_of(-1.0f, -1.0f);
+    uint64_t x[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) x[k] = pair_of(v[2 * k], v[2 * k + 1]);
+#pragma unroll
+    for (int d = 1; d < 16; d <<= 1) {
+        if (!(LEVELS & (2 * d))) continue;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            if (k & d) continue;
+            const uint64_t a = x[k], b = x[k | d];
+            asm("add.rn.f32x2 %0, %1, %2;" : "=l"(x[k]) : "l"(a), "l"(b));
+            asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(x[k | d]) : "l"(b), "l"(minus_one), "l"(a));
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        v[2 * k] = __uint_as_float((uint32_t)x[k]);
+        v[2 * k + 1] = __uint_as_float((uint32_t)(x[k] >> 32));
+    }
+}
+__device__ __forceinline__ void quads_store(uint32_t row, int j, const float (&v)[32]) {      // from chunks
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        sts128(row + (quad_place((uint32_t)(2 * (j + 8 * (k >> 1)) + (k & 1))) << 4), __float_as_uint(v[4 * k]), __float_as_uint(v[4 * k + 1]),
+               __float_as_uint(v[4 * k + 2]), __float_as_uint(v[4 * k + 3]));
+    }
+}
+__device__ __forceinline__ void lds128f(uint32_t addr, float& a, float& b, float& c, float& d) {
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(a), "=f"(b), "=f"(c), "=f"(d) : "r"(addr));
+}
+__device__ __forceinline__ uint32_t quad_of(int l, int j) { return (uint32_t)(2 * (j + 8 * (l >> 1)) + (l & 1)); }
+// Where 16-byte chunk c of a query row is staged: conflict-free for a thread per row and for the lanes of a rotated group.
+template <bool ROT>
+__device__ __forceinline__ uint32_t q_chunk_place(uint32_t c, uint32_t row) { return ROT ? (c & ~7u) | ((c ^ row ^ (2u * (c >> 3))) & 7u) : c ^ (row & 31u); }
+__device__ __forceinline__ void sts64(uint32_t addr, uint32_t a, uint32_t b) {
+    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
+}
+// The sign diagonal's bits of a lane's four chunks, a byte each (from immediates: the constant bank serves one address at a time).
+__device__ __forceinline__ uint32_t chunk_signs(int j) {
+    constexpr uint32_t kMask[8] = W34_TQ4_SIGN_MASK;
+    uint32_t bits = 0u;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) bits |= ((((j & 4) ? kMask[2 * i + 1] : kMask[2 * i]) >> (8 * (j & 3))) & 0xffu) << (8 * i);
+    asm volatile("" : "+r"(bits));      // (kept as one word: expanded into 32 selects it makes the kernel spill)
+    return bits;
+}
+
 // Accumulator of one row (columns [8 lane, + 8)) and its mass -> output row.
 template <bool ROT>
 __device__ __forceinline__ void prefill_finish_row(const PrefillPairParams& p, float (&v)[8], float l, size_t row_base, int lane) {
@@ -218,7 +287,9 @@ __device__ __forceinline__ void prefill_finish_row(const PrefillPairParams& p, f
         butterfly8<5>(v, lane);
         sign8(v, lane);
     }
-    apply_output_gate8(v, p.og, row_base, lane, p.io_bf16);
+    uint32_t gate[4];
+    load_gate8(p.og, row_base, lane, gate);
+    apply_output_gate8(v, p.og, gate, lane, p.io_bf16);
     store8(p.attn_out, row_base, lane, p.io_bf16, v);
 }
 
@@ -501,35 +572,69 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
         for (int i = 0; i < 8; ++i) v[i] = 0.0f;
         if (ok) load8(p.q_in, ((size_t)(g.q_start + q_off) * p.num_q_heads + q_head) * kHeadDim, lane, p.io_bf16, v);
     };
-    float ahead[8];
-    load_row(wid, ahead);
-    for (int row = wid; row < kPpCtaRows; row += kPpWarps) {
-        float v[8];      // columns [8 lane, + 8)
+    if (ROT) {
+        const int r4 = lane >> 3, j = lane & 7;
+        const uint32_t signs = chunk_signs(j);
+        uint32_t raw_q[4][4];
+        auto load_group = [&](int grp) {
+            const int trow = row0 + 4 * grp + r4;
+            const int q_off = tok0 + trow / p.gqa;
+            const int q_head = kv_head * p.gqa + trow % p.gqa;
+            const bool ok = 4 * grp < kPpCtaRows && trow < rows_used &&
+                            (p.batch.valid_token_mask == nullptr || p.batch.valid_token_mask[g.q_start + q_off] != 0);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = ahead[i];
-        load_row(row + kPpWarps, ahead);
-        if (ROT) {
-            sign8(v, lane);
-            butterfly8<5>(v, lane);
+            for (int i = 0; i < 4; ++i) {
+                raw_q[i][0] = raw_q[i][1] = raw_q[i][2] = raw_q[i][3] = 0u;
+                if (ok) load8_raw(p.q_in, ((size_t)(g.q_start + q_off) * p.num_q_heads + q_head) * kHeadDim, j + 8 * i, raw_q[i]);
+            }
+        };
+#pragma unroll 1
+        for (int grp = wid; 4 * grp < kPpCtaRows; grp += kPpWarps) {
+            const int row = 4 * grp + r4;
+            float v[32];
+            load_group(grp);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] *= p.q_scale * 0.0625f;
-        } else {
+            for (int i = 0; i < 4; ++i) {
+                float x[8];
+                widen8(raw_q[i], p.io_bf16, x);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] *= p.q_scale;
+                for (int e = 0; e < 8; ++e) v[8 * i + e] = __uint_as_float(__float_as_uint(x[e]) ^ (((signs >> (8 * i + e)) & 1u) << 31));
+            }
+            rotate_registers<31>(v);
+            // two of the four rows change lanes where the group's values will lie, two in this warp's part of the space behind the staging rows
+            const uint32_t turn = q_stage + (uint32_t)(r4 & 1) * 1024u + 2048u * (uint32_t)(r4 < 2 ? grp : kPpCtaRows / 4 + wid);
+            quads_store(turn, j, v);
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < 8; ++k) lds128f(turn + (quad_place(quad_of(j, k)) << 4), v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+            __syncwarp();
+            rotate_registers<4 + 8 + 16>(v);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {      // chunk k + 8 (j / 2), its half j % 2
+                uint32_t hi[2], lo[2];
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    const float y0 = v[4 * k + 2 * x] * (p.q_scale * 0.0625f), y1 = v[4 * k + 2 * x + 1] * (p.q_scale * 0.0625f);
+                    const __half2 h = __floats2half2_rn(y0, y1);
+                    const float2 hf = __half22float2(h);
+                    hi[x] = *reinterpret_cast<const uint32_t*>(&h);
+                    lo[x] = pack_half2(y0 - hf.x, y1 - hf.y);
+                }
+                const uint32_t half = 8u * (uint32_t)(j & 1);
+                sts64(q_stage + (uint32_t)row * 512u + (q_chunk_place<ROT>((uint32_t)(k + 8 * (j >> 1)), (uint32_t)row) << 4) + half, hi[0], hi[1]);
+                sts64(qlo_t + (uint32_t)(j >> 1) * (kPpCtaRows * 128u) + (uint32_t)row * 128u + (uint32_t)((k ^ (row & 7)) << 4) + half, lo[0], lo[1]);
+            }
         }
-        uint32_t hi[4], lo[4];
+    } else {
+        float ahead[8];
+        load_row(wid, ahead);
+        for (int row = wid; row < kPpCtaRows; row += kPpWarps) {
+            float v[8];      // columns [8 lane, + 8)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const __half2 h = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
-            const float2 hf = __half22float2(h);
-            hi[i] = *reinterpret_cast<const uint32_t*>(&h);
-            lo[i] = pack_half2(v[2 * i] - hf.x, v[2 * i + 1] - hf.y);
-        }
-        // staging row = 512 B; its 16-byte chunks are XOR-swizzled by the row (the reads below are thread-per-row)
-        sts128(q_stage + (uint32_t)row * 512u + (uint32_t)((lane ^ (row & 31)) << 4), hi[0], hi[1], hi[2], hi[3]);
-        if (ROT) {
-            sts128(qlo_t + (uint32_t)(lane >> 3) * (kPpCtaRows * 128u) + (uint32_t)row * 128u + (uint32_t)(((lane & 7) ^ (row & 7)) << 4),
-                   lo[0], lo[1], lo[2], lo[3]);
+            for (int i = 0; i < 8; ++i) v[i] = ahead[i] * p.q_scale;
+            load_row(row + kPpWarps, ahead);
+            const uint32_t at = q_stage + (uint32_t)row * 512u + (q_chunk_place<ROT>((uint32_t)lane, (uint32_t)row) << 4);
+            sts128(at, pack_half2(v[0], v[1]), pack_half2(v[2], v[3]), pack_half2(v[4], v[5]), pack_half2(v[6], v[7]));
         }
     }
     if (wid == 12) {
@@ -550,7 +655,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
                 const uint32_t chunk = (uint32_t)(8 * c4 + c);
-                const uint32_t addr = q_stage + (uint32_t)tid * 512u + ((chunk ^ (uint32_t)(tid & 31)) << 4);
+                const uint32_t addr = q_stage + (uint32_t)tid * 512u + (q_chunk_place<ROT>(chunk, (uint32_t)tid) << 4);
                 asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
                              : "=r"(r[4 * c]), "=r"(r[4 * c + 1]), "=r"(r[4 * c + 2]), "=r"(r[4 * c + 3]) : "r"(addr));
             }
@@ -915,7 +1020,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
                 tc_wait_ld();
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    *reinterpret_cast<uint4*>(mine + 32 * c + 4 * i) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+                    *reinterpret_cast<uint4*>(mine + 4u * (ROT ? quad_place((uint32_t)(8 * c + i)) : (uint32_t)(8 * c + i))) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
                 }
             }
         }
@@ -926,36 +1031,84 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
     __syncthreads();
     if (!aborted) {
         const int first_token = place[2], rows = place[3], q_start = place[4];
-        for (int row = wid; row < kPpCtaRows; row += kPpWarps) {
-            const int trow = (int)cluster_rank() * kPpCtaRows + row;
-            if (trow >= rows) break;
-            const int q_off = first_token + trow / p.gqa;
-            const int q_head = kv_head * p.gqa + trow % p.gqa;
-            if (p.batch.valid_token_mask != nullptr && p.batch.valid_token_mask[q_start + q_off] == 0) continue;
-            const float* src = stage + row * kPpOutStride;
-            float l = src[256], m = src[257];
-            float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            if (!fits) {
-                prefill_row_fp32<FMT>(p, place[0], q_off, q_head, place[1] << 6, ((place[1] + nblocks) << 6) - 1, v, l, m);
-            } else if (PpFormat<FMT>::has_keys(l)) {
-                const float4 a = *reinterpret_cast<const float4*>(src + 8 * lane), b = *reinterpret_cast<const float4*>(src + 8 * lane + 4);
-                v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-                if (v_exp != 0) {
-                    const float up = power_of_two(v_exp);
+        const bool by_rows = !ROT || !fits || p.splits > 1;      // (no rotation here, or the rare tile that is computed in fp32)
+        if (by_rows) {
+            for (int row = wid; row < kPpCtaRows; row += kPpWarps) {
+                const int trow = (int)cluster_rank() * kPpCtaRows + row;
+                if (trow >= rows) break;
+                const int q_off = first_token + trow / p.gqa;
+                const int q_head = kv_head * p.gqa + trow % p.gqa;
+                if (p.batch.valid_token_mask != nullptr && p.batch.valid_token_mask[q_start + q_off] == 0) continue;
+                const float* src = stage + row * kPpOutStride;
+                float l = src[256], m = src[257];
+                float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                if (!fits) {
+                    prefill_row_fp32<FMT>(p, place[0], q_off, q_head, place[1] << 6, ((place[1] + nblocks) << 6) - 1, v, l, m);
+                } else if (PpFormat<FMT>::has_keys(l)) {
+                    const uint32_t qa = ROT ? quad_place(2u * lane) : 2u * lane;      // (the next quad is its neighbour)
+                    const float4 a = *reinterpret_cast<const float4*>(src + 4u * qa), b = *reinterpret_cast<const float4*>(src + 4u * (qa ^ 1u));
+                    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+                    if (v_exp != 0) {
+                        const float up = power_of_two(v_exp);
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) v[i] *= up;
+                        for (int i = 0; i < 8; ++i) v[i] *= up;
+                    }
+                }
+                const size_t out_row = (size_t)(q_start + q_off) * p.num_q_heads + q_head;
+                if (p.splits > 1) {
+                    const size_t part_row = (size_t)blockIdx.z * p.batch.total_tokens * p.num_q_heads + out_row;
+                    float4* dst = reinterpret_cast<float4*>(p.parts + part_row * kHeadDim + 8 * lane);
+                    dst[0] = make_float4(v[0], v[1], v[2], v[3]);
+                    dst[1] = make_float4(v[4], v[5], v[6], v[7]);
+                    if (lane == 0) p.parts_ml[part_row] = make_float2(m, l);
+                    continue;
+                }
+                prefill_finish_row<ROT>(p, v, l, out_row * kHeadDim, lane);
+            }
+        } else {
+            const int r4 = lane >> 3, j = lane & 7;
+#pragma unroll 1
+            for (int grp = wid; 4 * grp < kPpCtaRows; grp += kPpWarps) {
+                const int row = 4 * grp + r4, trow = (int)cluster_rank() * kPpCtaRows + row;
+                if ((int)cluster_rank() * kPpCtaRows + 4 * grp >= rows) break;      // warp-uniform
+                const int q_off = first_token + trow / p.gqa;
+                const size_t out_base = ((size_t)(q_start + q_off) * p.num_q_heads + kv_head * p.gqa + trow % p.gqa) * kHeadDim;
+                const bool ok = trow < rows && (p.batch.valid_token_mask == nullptr || p.batch.valid_token_mask[q_start + q_off] != 0);
+                const bool gated = ok && p.og.mode != 0 && p.og.gate != nullptr;
+                const uint32_t at = smem_u32(smem_raw) + (uint32_t)row * (4u * kPpOutStride);
+                const float l = __uint_as_float(lds32(at + 1024u));
+                float inv = l > 0.0f ? 1.0f / (l * (kPpLutScale * 16.0f)) : 0.0f;
+                const bool keys = PpFormat<FMT>::has_keys(l);
+                if (v_exp != 0) inv *= power_of_two(v_exp);
+                float v[32];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) lds128f(at + (quad_place(quad_of(j, k)) << 4), v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+#pragma unroll
+                for (int k = 0; k < 32; ++k) v[k] = keys ? v[k] * inv : 0.0f;
+                rotate_registers<31>(v);
+                __syncwarp();
+#pragma unroll
+                for (int k = 0; k < 8; ++k) sts128(at + (quad_place(quad_of(j, k)) << 4), __float_as_uint(v[4 * k]), __float_as_uint(v[4 * k + 1]), __float_as_uint(v[4 * k + 2]), __float_as_uint(v[4 * k + 3]));
+                __syncwarp();
+#pragma unroll
+                for (int k = 0; k < 8; ++k) lds128f(at + (quad_place((uint32_t)(2 * (j + 8 * (k >> 1)) + (k & 1))) << 4), v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+                uint32_t gate[2][4] = {{0u, 0u, 0u, 0u}, {0u, 0u, 0u, 0u}};      // two ahead: a store would hold a load behind it back
+                if (gated) {
+                    load8_raw(p.og.gate, out_base, j, gate[0]);
+                    load8_raw(p.og.gate, out_base, j + 8, gate[1]);
+                }
+                rotate_registers<4 + 8 + 16>(v);
+                const uint32_t signs = chunk_signs(j);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    float x[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) x[e] = __uint_as_float(__float_as_uint(v[8 * i + e]) ^ (((signs >> (8 * i + e)) & 1u) << 31));
+                    apply_output_gate8(x, p.og, gate[i & 1], lane, p.io_bf16);
+                    if (i < 2 && gated) load8_raw(p.og.gate, out_base, j + 8 * (i + 2), gate[i & 1]);
+                    if (ok) store8(p.attn_out, out_base, j + 8 * i, p.io_bf16, x);
                 }
             }
-            const size_t out_row = (size_t)(q_start + q_off) * p.num_q_heads + q_head;
-            if (p.splits > 1) {
-                const size_t part_row = (size_t)blockIdx.z * p.batch.total_tokens * p.num_q_heads + out_row;
-                float4* dst = reinterpret_cast<float4*>(p.parts + part_row * kHeadDim + 8 * lane);
-                dst[0] = make_float4(v[0], v[1], v[2], v[3]);
-                dst[1] = make_float4(v[4], v[5], v[6], v[7]);
-                if (lane == 0) p.parts_ml[part_row] = make_float2(m, l);
-                continue;
-            }
-            prefill_finish_row<ROT>(p, v, l, out_row * kHeadDim, lane);
         }
     } else if (tid == 0 && p.status != nullptr) {
         atomicOr(p.status, 1);

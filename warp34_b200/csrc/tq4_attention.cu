@@ -308,9 +308,8 @@ __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
 
 // ---- rows held as 8 consecutive columns per lane ------------------------------------------------------------
 // 16-byte accesses when the matrix starts on a 16-byte boundary (rows are 512 bytes apart).
-__device__ __forceinline__ void load8(const void* base, size_t row_base, int lane, int bf16, float (&v)[8]) {
+__device__ __forceinline__ void load8_raw(const void* base, size_t row_base, int lane, uint32_t (&w)[4]) {
     const uint16_t* src = static_cast<const uint16_t*>(base) + row_base + 8 * lane;
-    uint32_t w[4];
     if (((uintptr_t)base & 15u) == 0u) {
         const uint4 q = *reinterpret_cast<const uint4*>(src);
         w[0] = q.x; w[1] = q.y; w[2] = q.z; w[3] = q.w;
@@ -318,6 +317,8 @@ __device__ __forceinline__ void load8(const void* base, size_t row_base, int lan
 #pragma unroll
         for (int i = 0; i < 4; ++i) w[i] = (uint32_t)src[2 * i] | ((uint32_t)src[2 * i + 1] << 16);
     }
+}
+__device__ __forceinline__ void widen8(const uint32_t (&w)[4], int bf16, float (&v)[8]) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const float2 f = bf16 ? make_float2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u))
@@ -326,9 +327,12 @@ __device__ __forceinline__ void load8(const void* base, size_t row_base, int lan
         v[2 * i + 1] = f.y;
     }
 }
-__device__ __forceinline__ void store8(void* base, size_t row_base, int lane, int bf16, const float (&v)[8]) {
-    uint16_t* dst = static_cast<uint16_t*>(base) + row_base + 8 * lane;
+__device__ __forceinline__ void load8(const void* base, size_t row_base, int lane, int bf16, float (&v)[8]) {
     uint32_t w[4];
+    load8_raw(base, row_base, lane, w);
+    widen8(w, bf16, v);
+}
+__device__ __forceinline__ void narrow8(const float (&v)[8], int bf16, uint32_t (&w)[4]) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         if (bf16) {
@@ -338,12 +342,20 @@ __device__ __forceinline__ void store8(void* base, size_t row_base, int lane, in
             w[i] = pack_half2(v[2 * i], v[2 * i + 1]);
         }
     }
+}
+__device__ __forceinline__ void store8_raw(void* base, size_t row_base, int lane, const uint32_t (&w)[4]) {
+    uint16_t* dst = static_cast<uint16_t*>(base) + row_base + 8 * lane;
     if (((uintptr_t)base & 15u) == 0u) {
         *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
     } else {
 #pragma unroll
         for (int i = 0; i < 4; ++i) { dst[2 * i] = (uint16_t)w[i]; dst[2 * i + 1] = (uint16_t)(w[i] >> 16); }
     }
+}
+__device__ __forceinline__ void store8(void* base, size_t row_base, int lane, int bf16, const float (&v)[8]) {
+    uint32_t w[4];
+    narrow8(v, bf16, w);
+    store8_raw(base, row_base, lane, w);
 }
 // Butterfly over column bits [3, 3 + LEVELS): lanes.  Upper lane o - x, lower x + o, one rounding either way.
 template <int LEVELS>
@@ -373,11 +385,11 @@ __device__ __forceinline__ void sign8(float (&v)[8], int lane) {
 }
 
 // The epilogue of apply_output_gate() on a row held that way.
-__device__ __forceinline__ void apply_output_gate8(float (&v)[8], const OutputGate& og, size_t row_base, int lane, int io_bf16) {
+__device__ __forceinline__ void apply_output_gate8(float (&v)[8], const OutputGate& og, const uint32_t (&gate)[4], int lane, int io_bf16) {
     if (og.mode == 0) return;
     if (og.gate != nullptr) {
         float g[8];
-        load8(og.gate, row_base, lane, io_bf16, g);
+        widen8(gate, io_bf16, g);
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = ((og.mode & 4) ? v[i] : round_act(v[i], io_bf16)) * sigmoid_gate(g[i]);
     }
@@ -387,6 +399,10 @@ __device__ __forceinline__ void apply_output_gate8(float (&v)[8], const OutputGa
     butterfly8<3>(v, lane);
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] *= 0.125f;
+}
+__device__ __forceinline__ void load_gate8(const OutputGate& og, size_t row_base, int lane, uint32_t (&gate)[4]) {
+    gate[0] = gate[1] = gate[2] = gate[3] = 0u;
+    if (og.mode != 0 && og.gate != nullptr) load8_raw(og.gate, row_base, lane, gate);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1528,7 +1544,9 @@ __global__ void __launch_bounds__(MW * 32) tq4_attention_merge_kernel(const Stre
         butterfly8<5>(acc, lane);
         sign8(acc, lane);
     }
-    apply_output_gate8(acc, p.og, out_base, lane, p.io_bf16);
+    uint32_t gate[4];
+    load_gate8(p.og, out_base, lane, gate);
+    apply_output_gate8(acc, p.og, gate, lane, p.io_bf16);
     store8(p.attn_out, out_base, lane, p.io_bf16, acc);
 }
 
