@@ -19,7 +19,8 @@
 // 16-byte loads per lane, the reference's 32-lane butterfly sums are register-only, five of the eight WHT stages as well,
 // and a lane's codes are four packed words in place.  A warp encodes 4 rows at once.  (Columns interleaved over the lanes
 // instead needed 2-byte loads, a halving exchange per sum and a nibble transpose: 449 instructions a row, 158 us for
-// 32 768 tokens x 4 kv heads.)  Bound by issue: parity fixes the order of the operations.
+// 32 768 tokens x 4 kv heads.)  Bound by issue: parity fixes the order of the operations, so that what is left is to do two columns at
+// a time (packed fp32 arithmetic) and to find a code in fewer instructions: 112.8 -> 92.5 us, with the K producer 140.7 -> 122.0.
 //
 // This translation unit is compiled with -use_fast_math like the reference
 // build (crates/warp34-kernels/build.rs:56-59), so rsqrtf() and '/' lower to the
@@ -37,23 +38,20 @@ namespace w34 {
 // below are therefore explicit __fmul_rn / __fadd_rn.
 
 constexpr float kBinScale = 58.75f;
+constexpr int kBins = 128;
 
-// code = #{i : rv > boundary_i} for the 15 ascending, symmetric boundaries (b[7] = 0).  For rv > 0 all of b[0..7] are below
-// rv and the code is 8 + #{k : |rv| > B_k} with B_k = b[8 + k]; for rv <= 0 none of b[7..14] is, rv > -B  <=>  |rv| < B, and
-// the code is 7 - #{k : |rv| >= B_k}.  Positive floats order like their bit patterns and ">= B" is "> B - 1 ulp", so both
-// cases count c = #{k : bits(|rv|) + (rv > 0 ? 0 : 1) > bits(B_k)}; the code is then c ^ 8 or c ^ 7.
-// The count: |rv| falls into one of 16 equal bins (kBinScale a unit, chosen so that no bin holds two boundaries and none
-// lies within a fifth of a bin of an edge); the bin's entry {boundary inside it or 2^32 - 1, boundaries below it} settles it
-// with one comparison.  `bins`: shared-memory address of the table less 8 times the bits of 1.5 x 2^23, to which the bin
-// number is added.  NaN goes to the last bin and gives 0, -0 gives 7, as the comparison chain does.
+// code = #{i : rv > boundary_i} for the 15 ascending boundaries.  rv falls into one of kBins equal bins around 0 (kBinScale a unit,
+// chosen so that no bin holds two boundaries and none lies within a fifth of a bin of an edge; |rv| is at most 0.7072, 42 bins); the
+// bin's entry {boundary inside it or infinity, boundaries below it} settles the code with one comparison.  `bins`: shared-memory
+// address of the table, a multiple of its size.  NaN ends in the last entry, which no number reaches, and gives 0 as the
+// comparison chain does; zeros of either sign give 7.  (With the magnitude's bins and the sign handled apart a code took eleven
+// instructions instead of seven.)
 __device__ __forceinline__ int tq4_bucket(float rv, uint32_t bins) {
-    const bool pos = rv > 0.0f;
-    const uint32_t x = (__float_as_uint(rv) & 0x7fffffffu) + (pos ? 0u : 1u);
-    const float bin = fminf(__fmaf_rn(fabsf(rv), kBinScale, 12582912.0f), 12582912.0f + 15.0f);
-    uint32_t boundary, below;
-    asm("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(boundary), "=r"(below) : "r"((__float_as_uint(bin) << 3) + bins));
-    const int c = (int)below + (x > boundary ? 1 : 0);
-    return c ^ (pos ? 8 : 7);
+    const uint32_t bin = __float_as_uint(__fmaf_rn(rv, kBinScale, 12582912.0f + (float)(kBins / 2)));
+    float boundary;
+    uint32_t below;
+    asm("ld.shared.v2.b32 {%0, %1}, [%2];" : "=f"(boundary), "=r"(below) : "r"(((bin << 3) & (8u * kBins - 8u)) | bins));
+    return (int)below + (rv > boundary ? 1 : 0);
 }
 
 // The rest of a group's butterfly, column bits 2, 1, 0, after its levels over bits 4 and 3.
@@ -68,6 +66,29 @@ __device__ __forceinline__ float half_sum(float t, int lane0) {
     s = __fadd_rn(s, __shfl_sync(0xffffffffu, t, lane0 + 1));
     s = __fadd_rn(s, __shfl_sync(0xffffffffu, t, lane0 + 2));
     return __fadd_rn(s, __shfl_sync(0xffffffffu, t, lane0 + 3));
+}
+
+// ---- two columns at a time ------------------------------------------------------------------------------
+// The packed forms round each half as the scalar instruction does (subnormals flushed, as everywhere in this unit), at half the
+// instructions, which is what the kernel is bound by.  a - b is fma(b, -1, a): the same number, signed zeros included.
+typedef unsigned long long Pair;
+__device__ __forceinline__ Pair pair_of(float a, float b) { return (Pair)__float_as_uint(a) | ((Pair)__float_as_uint(b) << 32); }
+__device__ __forceinline__ float first(Pair p) { return __uint_as_float((uint32_t)p); }
+__device__ __forceinline__ float second(Pair p) { return __uint_as_float((uint32_t)(p >> 32)); }
+__device__ __forceinline__ Pair add2(Pair a, Pair b) {
+    Pair r;
+    asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ Pair mul2(Pair a, Pair b) {
+    Pair r;
+    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
+    Pair r;
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
 }
 
 struct AppendParams {
@@ -94,7 +115,7 @@ extern "C" __device__ float __nv_sinf(float);
 extern "C" __device__ float __nv_cosf(float);
 extern "C" __device__ float __nv_powf(float, float);
 
-constexpr int kAppendBlocksPerSm = 6;
+constexpr int kAppendBlocksPerSm = 7;
 constexpr int kProducerBlocksPerSm = 5;
 
 struct ProducerShared {
@@ -198,16 +219,18 @@ __device__ __forceinline__ void k_producer(uint32_t (&raw)[16], int sub, int row
 template <bool IN_BF16, bool PRODUCER>
 __global__ void __launch_bounds__(128, PRODUCER ? kProducerBlocksPerSm : kAppendBlocksPerSm) tq4_append_kernel(const AppendParams p) {
     __shared__ float s_centroid[16];
-    __shared__ uint2 s_bin[16];
+    __shared__ __align__(8 * kBins) uint2 s_bin[kBins];
     __shared__ AppendShared<PRODUCER> s_prod;
-    if (threadIdx.x < 16) {
-        s_centroid[threadIdx.x] = tq4_centroid(threadIdx.x);
-        uint2 e = make_uint2(0xffffffffu, 0u);
-        for (int k = 0; k < 7; ++k) {
-            const int bin = (int)rintf(tq4_boundary(8 + k) * kBinScale);
+    if (threadIdx.x < 16) s_centroid[threadIdx.x] = tq4_centroid(threadIdx.x);
+    static_assert(kBins == 128, "one entry per thread");
+    {
+        uint2 e = make_uint2(0x7f800000u, 0u);
+        for (int k = 0; k < 15; ++k) {
+            const int bin = kBins / 2 + (int)rintf(tq4_boundary(k) * kBinScale);
             if (bin < (int)threadIdx.x) ++e.y;
-            if (bin == (int)threadIdx.x) e.x = c_boundary_bits[8 + k];
+            if (bin == (int)threadIdx.x) e.x = c_boundary_bits[k];
         }
+        if (threadIdx.x == kBins - 1) e.y = 0u;
         s_bin[threadIdx.x] = e;
     }
     const int lane = threadIdx.x & 31;
@@ -218,8 +241,10 @@ __global__ void __launch_bounds__(128, PRODUCER ? kProducerBlocksPerSm : kAppend
         const uint32_t m = c_sign_mask[sub] >> (2 * i);
         sign[i] = ((m & 1u) << 15) | ((m & 2u) << 30);
     }
-    const uint32_t bins = (uint32_t)__cvta_generic_to_shared(s_bin) - (0x4b400000u << 3);
+    const uint32_t bins = (uint32_t)__cvta_generic_to_shared(s_bin);
     // butterfly direction of the three cross-lane WHT stages: upper lanes compute o - v
+    const float one_f = __uint_as_float(0x3f800000u | (uint32_t)(p.layout.head_dim - kHeadDim));      // 1, see quarter_sums
+    const Pair one = pair_of(one_f, one_f);
     const float dir1 = (sub & 1) ? -1.0f : 1.0f, dir2 = (sub & 2) ? -1.0f : 1.0f, dir4 = (sub & 4) ? -1.0f : 1.0f;
     // This kernel may start while the last blocks of the one before it finish (nothing above touches global memory), and an
     // attention kernel launched behind it may set itself up meanwhile.
@@ -285,72 +310,84 @@ __global__ void __launch_bounds__(128, PRODUCER ? kProducerBlocksPerSm : kAppend
         if constexpr (PRODUCER) {
             if (which == 0) k_producer(raw, sub, lane >> 3, tok, p, s_prod.s);   // warp-uniform: a group is all K or all V
         }
-        float v[32];
+        Pair v[16];      // columns 2 i, 2 i + 1
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             const uint32_t w = raw[i] ^ sign[i];
             const float2 f = IN_BF16 ? make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u))
                                      : __half22float2(*reinterpret_cast<const __half2*>(&w));
-            v[2 * i] = f.x;
-            v[2 * i + 1] = f.y;
+            v[i] = pair_of(__fadd_rn(f.x, f.y), __fsub_rn(f.x, f.y));      // stage 1 of the transform
         }
 
         // ---- WHT-256: stages 1 .. 16 in registers, 32, 64, 128 across lanes --------------------------
+        const Pair minus_one = pair_of(-1.0f, -1.0f);
 #pragma unroll
-        for (int s = 1; s < 32; s <<= 1) {
+        for (int s = 1; s < 16; s <<= 1) {
 #pragma unroll
-            for (int r = 0; r < 32; ++r) {
+            for (int r = 0; r < 16; ++r) {
                 if ((r & s) == 0) {
-                    const float a = v[r], b = v[r | s];
-                    v[r] = __fadd_rn(a, b);
-                    v[r | s] = __fsub_rn(a, b);
+                    const Pair a = v[r], b = v[r | s];
+                    v[r] = add2(a, b);
+                    v[r | s] = fma2(b, minus_one, a);
                 }
             }
         }
         // lower lane: v + o, upper lane: o - v; fma(+-1, v, o) is the same single rounding.
+        auto across = [&](float dir, int d) {
+            const Pair dir2 = pair_of(dir, dir);
 #pragma unroll
-        for (int r = 0; r < 32; ++r) v[r] = __fmaf_rn(dir1, v[r], __shfl_xor_sync(0xffffffffu, v[r], 1));
-#pragma unroll
-        for (int r = 0; r < 32; ++r) v[r] = __fmaf_rn(dir2, v[r], __shfl_xor_sync(0xffffffffu, v[r], 2));
-#pragma unroll
-        for (int r = 0; r < 32; ++r) v[r] = __fmaf_rn(dir4, v[r], __shfl_xor_sync(0xffffffffu, v[r], 4));
+            for (int r = 0; r < 16; ++r) {
+                const Pair o = pair_of(__shfl_xor_sync(0xffffffffu, first(v[r]), d), __shfl_xor_sync(0xffffffffu, second(v[r]), d));
+                v[r] = fma2(dir2, v[r], o);
+            }
+        };
+        across(dir1, 1);
+        across(dir2, 2);
+        across(dir4, 4);
         // The transform's factor 1/16.  Sums of fp16 values are multiples of 2^-24 far below the overflow threshold, so
         // that a power of two commutes with every rounding that follows: it is left out and put back into the scale.
         constexpr float kSq = IN_BF16 ? 1.0f : 256.0f, kBack = IN_BF16 ? 1.0f : 0.0625f;
         if (IN_BF16) {
+            const Pair sixteenth = pair_of(0.0625f, 0.0625f);
 #pragma unroll
-            for (int r = 0; r < 32; ++r) v[r] = __fmul_rn(v[r], 0.0625f);
+            for (int r = 0; r < 16; ++r) v[r] = mul2(v[r], sixteenth);
         }
 
         // ---- scale of the lane's half, codes, centroids, least-squares sums ----------------------------------
+        // (a b of columns c + c of 16 further) + (those 8 and 24 further), for columns 2 r, 2 r + 1.  A sum of products is written
+        // fma(x, one, y): the assembler makes one rounding of a packed product and the add behind it, .rn or not, unless the add is
+        // itself a product that it cannot know (3 of 66 million scales then differ by one unit).
+        auto quarter_sums = [&](const Pair (&x)[16], const Pair (&y)[16], float (&t)[8]) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const Pair near = fma2(mul2(x[r], y[r]), one, mul2(x[r + 8], y[r + 8]));
+                const Pair far = fma2(mul2(x[r + 4], y[r + 4]), one, mul2(x[r + 12], y[r + 12]));
+                const Pair q = add2(near, far);
+                t[2 * r] = first(q);
+                t[2 * r + 1] = second(q);
+            }
+        };
         const int half_lane = lane & ~3;
         float inv;
         {
             float t[8];
-#pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                t[r] = __fadd_rn(__fadd_rn(__fmul_rn(v[r], v[r]), __fmul_rn(v[r + 16], v[r + 16])),
-                                 __fadd_rn(__fmul_rn(v[r + 8], v[r + 8]), __fmul_rn(v[r + 24], v[r + 24])));
-            }
+            quarter_sums(v, v, t);
             const float s = half_sum(group_total(t), half_lane);
             inv = (s > 1e-20f * kSq) ? (0.7071067811865475f * rsqrtf(s)) : 0.0f;
         }
         uint32_t nib[4] = {0u, 0u, 0u, 0u};
-        float vct[8], cct[8];
+        Pair c[16];
+        const Pair inv2 = pair_of(inv, inv);
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            float c[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int q = tq4_bucket(__fmul_rn(v[r + 8 * k], inv), bins);
-                nib[k] += (uint32_t)q * (1u << (4 * r));   // disjoint nibbles: add == or
-                c[k] = s_centroid[q];
-            }
-            vct[r] = __fadd_rn(__fadd_rn(__fmul_rn(v[r], c[0]), __fmul_rn(v[r + 16], c[2])),
-                               __fadd_rn(__fmul_rn(v[r + 8], c[1]), __fmul_rn(v[r + 24], c[3])));
-            cct[r] = __fadd_rn(__fadd_rn(__fmul_rn(c[0], c[0]), __fmul_rn(c[2], c[2])),
-                               __fadd_rn(__fmul_rn(c[1], c[1]), __fmul_rn(c[3], c[3])));
+        for (int r = 0; r < 16; ++r) {
+            const Pair x = mul2(v[r], inv2);
+            const int qa = tq4_bucket(first(x), bins), qb = tq4_bucket(second(x), bins);
+            nib[r >> 2] += (uint32_t)qa * (1u << (8 * (r & 3))) + (uint32_t)qb * (1u << (8 * (r & 3) + 4));   // disjoint nibbles: add == or
+            c[r] = pair_of(s_centroid[qa], s_centroid[qb]);
         }
+        float vct[8], cct[8];
+        quarter_sums(v, c, vct);
+        quarter_sums(c, c, cct);
         const float vc = half_sum(group_total(vct), half_lane);
         const float cc = half_sum(group_total(cct), half_lane);
         const float d = (cc > 1e-10f) ? (vc / cc) * kBack : 0.0f;
