@@ -56,3 +56,30 @@ def test_row_groups_match_dequant_then_attend(native_libs, hq, hkv, new, off, mo
         got, want = ((x.reshape(-1, 64) @ (h / 8).numpy()) for x in (got, want))
     ok, msg = plain_parity(got, want)
     assert ok, msg
+
+
+@pytest.mark.parametrize("reqs", [8, 9, 32, 33, 70])
+def test_pairs_find_their_request_among_many(native_libs, reqs):
+    """Requests of 0 to 90 tokens (0 to 3 tiles of 42): the request of a pair is searched one by one up to 8 requests and 32 at a time
+    from 9 on."""
+    import numpy as np
+    from warp34_b200 import ffi, kv, synth
+    f, tr = ffi.KV_FORMAT_TQ4, ffi.KV_TRANSFORM_RADEMACHER_WHT256
+    new = [(7 * r * r + 5 * r) % 91 if r % 5 else 0 for r in range(reqs)]
+    new[-1] = 90
+    wl = synth.PagedWorkload([0] * reqs, new, 1, seed=3, formats=(f, f, tr, tr))
+    ex = kv.Executor(64 << 20)
+    n = sum(new)
+    k, v = synth.make_kv(n, 1, 4, device="cuda")
+    b = wl.step()
+    kv.kv_cache_write(ex, wl.layer, b, k, v)
+    q = synth.make_q(n, 6, 5, device="cuda")
+    outs = []
+    for flags in (0, ffi.EXEC_FLAG_PRECISE_ATTENTION):
+        ex.ex.flags = flags
+        out = torch.full((n, 6, 256), -7.0, dtype=torch.float16, device="cuda")
+        kv.paged_attention(ex, wl.layer, b, q, out, 6)
+        torch.cuda.synchronize()
+        outs.append(out.float().cpu().numpy())
+    ok, msg = plain_parity(*outs)
+    assert ok, msg

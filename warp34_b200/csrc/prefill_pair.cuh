@@ -474,11 +474,38 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
     int req = -1, tile_in_req = 0;
     {
         int t = (int)(blockIdx.x >> 1);
-        for (int r = 0; r < p.batch.num_reqs; ++r) {
-            const int ql = p.batch.query_start_loc[r + 1] - p.batch.query_start_loc[r];
-            const int nt = min((ql + tpt - 1) / tpt, ql > p.skip_tokens ? 0x7fffffff : 0);
-            if (t < nt) { req = r; tile_in_req = nt - 1 - t; break; }    // the tiles with the most keys first
-            t -= nt;
+        if (p.batch.num_reqs <= 8) {
+            for (int r = 0; r < p.batch.num_reqs; ++r) {
+                const int ql = p.batch.query_start_loc[r + 1] - p.batch.query_start_loc[r];
+                const int nt = min((ql + tpt - 1) / tpt, ql > p.skip_tokens ? 0x7fffffff : 0);
+                if (t < nt) { req = r; tile_in_req = nt - 1 - t; break; }    // the tiles with the most keys first
+                t -= nt;
+            }
+        } else {
+            // a lane per request: one round trip to memory, where the loop above makes one for every few requests ahead of the pair's own
+            // (64 requests of 16 tokens 112.0 -> 92.4 us; with two requests the shuffles cost 0.3 us, with eight or fewer the loop stays)
+            for (int base_r = 0; base_r < p.batch.num_reqs && req < 0; base_r += 32) {
+                const int r = base_r + lane;
+                int nt = 0;
+                if (r < p.batch.num_reqs) {
+                    const int ql = p.batch.query_start_loc[r + 1] - p.batch.query_start_loc[r];
+                    nt = max(min((ql + tpt - 1) / tpt, ql > p.skip_tokens ? 0x7fffffff : 0), 0);
+                }
+                int upto = nt;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int x = __shfl_up_sync(0xffffffffu, upto, d);
+                    if (lane >= d) upto += x;
+                }
+                const uint32_t hit = __ballot_sync(0xffffffffu, t < upto);
+                if (hit != 0u) {
+                    const int src = __ffs((int)hit) - 1;
+                    req = base_r + src;
+                    tile_in_req = __shfl_sync(0xffffffffu, upto, src) - 1 - t;
+                } else {
+                    t -= __shfl_sync(0xffffffffu, upto, 31);
+                }
+            }
         }
     }
     if (req < 0) return;
