@@ -589,19 +589,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
     // ---- Q rows of this CTA: one warp per row.  TQ4: rotated, scaled, split into value (staging) and
     //      residual (swizzled A tile); 8-bit: the fp16 row as it is ------------------------------------
     const uint32_t q_stage = k_t;     // 128 rows x 512 B over the tile stages
-    auto load_row = [&](int row, float (&v)[8]) {
-        const int trow = row0 + row;
-        const int q_off = tok0 + trow / p.gqa;
-        const int q_head = kv_head * p.gqa + trow % p.gqa;
-        const bool ok = row < kPpCtaRows && trow < rows_used &&
-                        (p.batch.valid_token_mask == nullptr || p.batch.valid_token_mask[g.q_start + q_off] != 0);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = 0.0f;
-        if (ok) load8(p.q_in, ((size_t)(g.q_start + q_off) * p.num_q_heads + q_head) * kHeadDim, lane, p.io_bf16, v);
-    };
-    if (ROT) {
+    {
         const int r4 = lane >> 3, j = lane & 7;
-        const uint32_t signs = chunk_signs(j);
+        const uint32_t signs = ROT ? chunk_signs(j) : 0u;
         uint32_t raw_q[4][4];
         auto load_group = [&](int grp) {
             const int trow = row0 + 4 * grp + r4;
@@ -618,8 +608,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
 #pragma unroll 1
         for (int grp = wid; 4 * grp < kPpCtaRows; grp += kPpWarps) {
             const int row = 4 * grp + r4;
-            float v[32];
             load_group(grp);
+            if (!ROT) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    float x[8];
+                    widen8(raw_q[i], p.io_bf16, x);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) x[e] *= p.q_scale;
+                    sts128(q_stage + (uint32_t)row * 512u + (q_chunk_place<ROT>((uint32_t)(j + 8 * i), (uint32_t)row) << 4), pack_half2(x[0], x[1]),
+                           pack_half2(x[2], x[3]), pack_half2(x[4], x[5]), pack_half2(x[6], x[7]));
+                }
+                continue;
+            }
+            float v[32];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 float x[8];
@@ -651,17 +653,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
                 sts64(q_stage + (uint32_t)row * 512u + (q_chunk_place<ROT>((uint32_t)(k + 8 * (j >> 1)), (uint32_t)row) << 4) + half, hi[0], hi[1]);
                 sts64(qlo_t + (uint32_t)(j >> 1) * (kPpCtaRows * 128u) + (uint32_t)row * 128u + (uint32_t)((k ^ (row & 7)) << 4) + half, lo[0], lo[1]);
             }
-        }
-    } else {
-        float ahead[8];
-        load_row(wid, ahead);
-        for (int row = wid; row < kPpCtaRows; row += kPpWarps) {
-            float v[8];      // columns [8 lane, + 8)
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = ahead[i] * p.q_scale;
-            load_row(row + kPpWarps, ahead);
-            const uint32_t at = q_stage + (uint32_t)row * 512u + (q_chunk_place<ROT>((uint32_t)lane, (uint32_t)row) << 4);
-            sts128(at, pack_half2(v[0], v[1]), pack_half2(v[2], v[3]), pack_half2(v[4], v[5]), pack_half2(v[6], v[7]));
         }
     }
     if (wid == 12) {
@@ -1058,7 +1049,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
     __syncthreads();
     if (!aborted) {
         const int first_token = place[2], rows = place[3], q_start = place[4];
-        const bool by_rows = !ROT || !fits || p.splits > 1;      // (no rotation here, or the rare tile that is computed in fp32)
+        const bool by_rows = !fits || p.splits > 1;      // (the rare tile that is computed in fp32; no rotation here)
         if (by_rows) {
             for (int row = wid; row < kPpCtaRows; row += kPpWarps) {
                 const int trow = (int)cluster_rank() * kPpCtaRows + row;
@@ -1104,33 +1095,36 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
                 const bool gated = ok && p.og.mode != 0 && p.og.gate != nullptr;
                 const uint32_t at = smem_u32(smem_raw) + (uint32_t)row * (4u * kPpOutStride);
                 const float l = __uint_as_float(lds32(at + 1024u));
-                float inv = l > 0.0f ? 1.0f / (l * (kPpLutScale * 16.0f)) : 0.0f;
+                float inv = l > 0.0f ? 1.0f / (ROT ? l * (kPpLutScale * 16.0f) : l) : 0.0f;
                 const bool keys = PpFormat<FMT>::has_keys(l);
                 if (v_exp != 0) inv *= power_of_two(v_exp);
                 float v[32];
+                const auto chunk_quad = [&](int k) { return (uint32_t)(2 * (j + 8 * (k >> 1)) + (k & 1)); };
 #pragma unroll
-                for (int k = 0; k < 8; ++k) lds128f(at + (quad_place(quad_of(j, k)) << 4), v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+                for (int k = 0; k < 8; ++k) lds128f(at + ((ROT ? quad_place(quad_of(j, k)) : chunk_quad(k)) << 4), v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
 #pragma unroll
                 for (int k = 0; k < 32; ++k) v[k] = keys ? v[k] * inv : 0.0f;
-                rotate_registers<31>(v);
-                __syncwarp();
+                if (ROT) {
+                    rotate_registers<31>(v);
+                    __syncwarp();
 #pragma unroll
-                for (int k = 0; k < 8; ++k) sts128(at + (quad_place(quad_of(j, k)) << 4), __float_as_uint(v[4 * k]), __float_as_uint(v[4 * k + 1]), __float_as_uint(v[4 * k + 2]), __float_as_uint(v[4 * k + 3]));
-                __syncwarp();
+                    for (int k = 0; k < 8; ++k) sts128(at + (quad_place(quad_of(j, k)) << 4), __float_as_uint(v[4 * k]), __float_as_uint(v[4 * k + 1]), __float_as_uint(v[4 * k + 2]), __float_as_uint(v[4 * k + 3]));
+                    __syncwarp();
 #pragma unroll
-                for (int k = 0; k < 8; ++k) lds128f(at + (quad_place((uint32_t)(2 * (j + 8 * (k >> 1)) + (k & 1))) << 4), v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+                    for (int k = 0; k < 8; ++k) lds128f(at + (quad_place(chunk_quad(k)) << 4), v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+                }
                 uint32_t gate[2][4] = {{0u, 0u, 0u, 0u}, {0u, 0u, 0u, 0u}};      // two ahead: a store would hold a load behind it back
                 if (gated) {
                     load8_raw(p.og.gate, out_base, j, gate[0]);
                     load8_raw(p.og.gate, out_base, j + 8, gate[1]);
                 }
-                rotate_registers<4 + 8 + 16>(v);
-                const uint32_t signs = chunk_signs(j);
+                if (ROT) rotate_registers<4 + 8 + 16>(v);
+                const uint32_t signs = ROT ? chunk_signs(j) : 0u;
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     float x[8];
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) x[e] = __uint_as_float(__float_as_uint(v[8 * i + e]) ^ (((signs >> (8 * i + e)) & 1u) << 31));
+                    for (int e = 0; e < 8; ++e) x[e] = ROT ? __uint_as_float(__float_as_uint(v[8 * i + e]) ^ (((signs >> (8 * i + e)) & 1u) << 31)) : v[8 * i + e];
                     apply_output_gate8(x, p.og, gate[i & 1], lane, p.io_bf16);
                     if (i < 2 && gated) load8_raw(p.og.gate, out_base, j + 8 * (i + 2), gate[i & 1]);
                     if (ok) store8(p.attn_out, out_base, j + 8 * i, p.io_bf16, x);
