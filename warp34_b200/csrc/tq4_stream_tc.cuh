@@ -53,8 +53,8 @@ struct XtShared {
     uint32_t aborted;
     uint64_t bars[48];
 };
-enum { kXtRawKFull = 0, kXtRawKFree = 4, kXtRawVFull = 8, kXtRawVFree = 12, kXtKFull = 16, kXtKEmpty = 20, kXtVFull = 24, kXtVEmpty = 26,
-       kXtQFull = 28, kXtQFree, kXtSReady, kXtSFree, kXtPReady, kXtPvDone, kXtKScale,
+enum { kXtRawKFull = 0, kXtRawKFree = 4, kXtRawVFull = 8, kXtRawVFree = 12, kXtKFull = 16, kXtKEmpty = 20, kXtVFull = 24, kXtVEmpty,
+       kXtQFull, kXtQFree, kXtSReady, kXtSFree, kXtPReady, kXtPvDone = kXtPReady + 2, kXtKScale = kXtPvDone + 2,
        kXtDrain = kXtKScale + 2, kXtBarCount };
 static_assert(kXtBarCount <= 48, "barrier slots");
 
@@ -66,11 +66,11 @@ __device__ __forceinline__ void tc_st4(uint32_t taddr, const uint32_t (&r)[4]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};"
                  :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
 }
-// 16 lanes x 256 bits, four times: registers 4 i + {0, 1} go to lane t / 4, columns 8 i + 2 (t % 4) + {0, 1}; 4 i + {2, 3} eight
+// 16 lanes x 256 bits, twice: registers 4 i + {0, 1} go to lane t / 4, columns 8 i + 2 (t % 4) + {0, 1}; 4 i + {2, 3} eight
 // lanes further (t: thread of the warp).
-__device__ __forceinline__ void tc_st_16x256b_x4(uint32_t taddr, const uint32_t (&r)[16]) {
-    asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-                 :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+__device__ __forceinline__ void tc_st_16x256b_x2(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x2.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 // D (+)= A B with A in tensor memory, all output lanes.
 template <bool ACC>
@@ -194,14 +194,13 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
         return false;
     };
 
-    for (int i = tid; i < 256 * 32; i += xt_threads(R)) {      // per byte: {values, residuals} x 16, {residuals, values} x 16
-        const int byte = i >> 5, ln = i & 31;
+    for (int i = tid; i < 256 * 16; i += xt_threads(R)) {      // per byte: {values, residuals} x 16
+        const int byte = i >> 4, ln = i & 15;
         const float c0 = kLutScale * tq4_centroid(byte & 15), c1 = kLutScale * tq4_centroid(byte >> 4);
         const uint32_t hi = pack_half2(c0, c1);
         const float2 hf = __half22float2(*reinterpret_cast<const __half2*>(&hi));
         const uint32_t lo = pack_half2(c0 - hf.x, c1 - hf.y);
-        sts32(lut_addr + (uint32_t)(byte * 256 + ln * 4), (ln & 1) ? lo : hi);
-        sts32(lut_addr + (uint32_t)(byte * 256 + 128 + ln * 4), (ln & 1) ? hi : lo);
+        asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(lut_addr + (uint32_t)(byte * 256 + ln * 8)), "r"(hi), "r"(lo) : "memory");
     }
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -212,16 +211,18 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
         }
         for (int s = 0; s < kXtKRing; ++s) { mbar_init(bar(kXtKFull + s), 4u); mbar_init(bar(kXtKEmpty + s), 1u); }
         for (int s = 0; s < 2; ++s) {
-            mbar_init(bar(kXtVFull + s), 8u);
-            mbar_init(bar(kXtVEmpty + s), 1u);
             mbar_init(bar(kXtKScale + s), 4u);
         }
+        mbar_init(bar(kXtVFull), 8u);
+        mbar_init(bar(kXtVEmpty), 1u);
         mbar_init(bar(kXtQFull), 1u);
         mbar_init(bar(kXtQFree), 1u);
         mbar_init(bar(kXtSReady), 1u);
         mbar_init(bar(kXtSFree), W0);
-        mbar_init(bar(kXtPReady), W0);
-        mbar_init(bar(kXtPvDone), 1u);
+        for (int kk = 0; kk < 2; ++kk) {      // of each half of the keys
+            mbar_init(bar(kXtPReady + kk), W0 / 2);
+            mbar_init(bar(kXtPvDone + kk), 1u);
+        }
         mbar_init(bar(kXtDrain), 2u);
         sh.aborted = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -349,14 +350,14 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
         bool ok = true;
         while (ok && xt_next(p, walk, sg)) {
             for (int b = 0; ok && kXtPages * b < sg.pages; ++b, ++c) {
-                ok = wait_all(bar(kXtPReady), c & 1u);
 #pragma unroll
                 for (int kk = 0; kk < 2; ++kk) {
+                    ok = ok && wait_all(bar(kXtPReady + kk), c & 1u);
+                    ok = ok && wait_all(bar(kXtVFull), (uint32_t)kk);      // fill 2 c + kk
+                    if (ok && elect_one()) {
+                        tc_fence_after();
 #pragma unroll
-                    for (int res = 0; res < 2; ++res) {      // the centroids' values, then their residuals
-                        ok = ok && wait_all(bar(kXtVFull + res), (uint32_t)kk);      // fills 2 c + kk
-                        if (ok && elect_one()) {
-                            tc_fence_after();
+                        for (int res = 0; res < 2; ++res) {      // the centroids' values, then their residuals
 #pragma unroll
                             for (int h = 0; h < 2; ++h) {
 #pragma unroll
@@ -367,13 +368,12 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                                     else xt_mma<false>(d, a, bp, kIdesc);
                                 }
                             }
-                            tc_commit(bar(kXtVEmpty + res));
                         }
-                        __syncwarp();
+                        tc_commit(bar(kXtVEmpty));
+                        tc_commit(bar(kXtPvDone + kk));
                     }
+                    __syncwarp();
                 }
-                if (ok && elect_one()) tc_commit(bar(kXtPvDone));
-                __syncwarp();
             }
         }
         if (!ok) *aborted = 1u;
@@ -387,8 +387,7 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
         const int vw = 4 * (wid & 3) + (gid >> 1);                           // this thread's code word of the half
         const uint32_t word_off = 4u * ((half ? 17u : 0u) + (uint32_t)vw);
         const bool splice_warp = half == 0 && (wid & 3) == 0;                // virtual word 0: (W0 >> 16) | (W16 << 16)
-        // lanes 0-15 read the first half of a table entry, lanes 16-31 the second: 32 banks for the values and for the residuals
-        const uint32_t lut_v = lut_addr + (uint32_t)(lane >> 4) * 132u + 8u * (uint32_t)(lane & 15), lut_r = lut_v ^ 4u;
+        const uint32_t lut_lane = lut_addr + 8u * (uint32_t)(lane & 15);
         // byte 2 (gid & 1) + T of the paired codes belongs to tile T
         const uint32_t sel[2] = {0x7604u + ((uint32_t)(2 * (gid & 1)) << 4), 0x7604u + ((uint32_t)(2 * (gid & 1) + 1) << 4)};
         bool ok = true;
@@ -425,32 +424,32 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                         x[pg][2] = (w2 & 0x0f0f0f0fu) | ((w3 << 4) & 0xf0f0f0f0u);
                         x[pg][3] = ((w2 >> 4) & 0x0f0f0f0fu) | (w3 & 0xf0f0f0f0u);
                     }
-#pragma unroll 1
-                    for (int res = 0; res < 2; ++res) {
-                        const uint32_t lut = res == 0 ? lut_v : lut_r;
-                        uint32_t a[2][16];
+                    const uint32_t dst = tmem + quad + kXtColV + 64u * (uint32_t)half;
 #pragma unroll
-                        for (int pg = 0; pg < 4; ++pg) {
+                    for (int part = 0; part < 4; ++part) {      // tile, pair of pages
+                        const int T = part & 1, pg0 = part & 2;
+                        uint32_t a[8], r[8];      // values, residuals: one look-up for both
 #pragma unroll
-                            for (int T = 0; T < 2; ++T) {
-#pragma unroll
-                                for (int o = 0; o < 2; ++o) {
-                                    a[T][4 * pg + 2 * o] = lds32_lut(__byte_perm(x[pg][o], lut, sel[T]));
-                                    a[T][4 * pg + 2 * o + 1] = lds32_lut(__byte_perm(x[pg][2 + o], lut, sel[T]));
-                                }
-                            }
+                        for (int i = 0; i < 4; ++i) {
+                            const int pg = pg0 + (i >> 1), o = i & 1;
+                            const uint2 e01 = lds64_lut(__byte_perm(x[pg][o], lut_lane, sel[T])), e23 = lds64_lut(__byte_perm(x[pg][2 + o], lut_lane, sel[T]));
+                            a[2 * i] = e01.x;
+                            r[2 * i] = e01.y;
+                            a[2 * i + 1] = e23.x;
+                            r[2 * i + 1] = e23.y;
                         }
-                        if (!(ok = wait_all(bar(kXtVEmpty + res), (uint32_t)(kk ^ 1)))) break;
-                        tc_fence_after();      // the MMAs that read the granule come before the stores over it
-                        const uint32_t dst = tmem + quad + kXtColV + 64u * (uint32_t)half + 32u * (uint32_t)res;
-                        tc_st_16x256b_x4(dst, a[0]);
-                        tc_st_16x256b_x4(dst + (16u << 16), a[1]);
-                        tc_wait_st();
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(bar(kXtVFull + res));
+                        if (part == 0) {
+                            if (!(ok = wait_all(bar(kXtVEmpty), (uint32_t)(kk ^ 1)))) break;
+                            tc_fence_after();      // the MMAs that read the granule come before the stores over it
+                        }
+                        tc_st_16x256b_x2(dst + ((uint32_t)(16 * T) << 16) + 8u * (uint32_t)pg0, a);
+                        tc_st_16x256b_x2(dst + ((uint32_t)(16 * T) << 16) + 8u * (uint32_t)pg0 + 32u, r);
                     }
                     if (!ok) break;
+                    tc_wait_st();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar(kXtVFull));
                 }
                 __syncwarp();
                 if (ok && lane == 0) mbar_arrive(bar(kXtRawVFree + s));
@@ -505,7 +504,7 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
     } else if (wid < W0) {
         // ======================= softmax: thread = key, a part = eight rows =============================================
         constexpr int P = 8;
-        const int part = wid >> 2, row0 = part * P, key = tid & 127;
+        const int part = wid >> 2, row0 = part * P, key = tid & 127, khalf = (wid & 3) >> 1;
         const uint32_t t_s = tmem + quad + kXtColS + (uint32_t)row0, t_o = tmem + quad + kXtColO + (uint32_t)row0;
         float* m_ref = sh.m_ref + row0;      // this part's rows
         float* alpha = sh.alpha + row0;
@@ -640,9 +639,11 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                         v_by *= v_up;
                     }
                 }
-                // P and O are in use until the output product of the block before has completed
-                bad = bad || (c > 0 && !wait_all(bar(kXtPvDone), (c - 1) & 1u));
+                // This half of the keys' P is in use until its output product of the block before has completed, O until both have.  (The
+                // halves follow each other: one's weights are written while the other is multiplied.)
+                bad = bad || (c > 0 && !wait_all(bar(kXtPvDone + khalf), (c - 1) & 1u));
                 if (moved && b > 0) {
+                    bad = bad || !wait_all(bar(kXtPvDone + (khalf ^ 1)), (c - 1) & 1u);
                     tc_fence_after();
 #pragma unroll 1
                     for (int q = 0; q < 4; ++q) {      // value and residual columns of both halves
@@ -658,6 +659,7 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                     }
                     tc_wait_st();
                     tc_fence_before();
+                    xt_sync(part);      // neither half's product starts before all four warps have rescaled their channels
                 }
                 dv.x *= v_up;
                 dv.y *= v_up;
@@ -682,13 +684,13 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                 fence_proxy_async();
                 __syncwarp();
                 if (lane == 0) {
-                    mbar_arrive(bar(kXtPReady));
+                    mbar_arrive(bar(kXtPReady + khalf));
                     mbar_arrive(bar(kXtRawVFree + (int)(c % STAGES)));
                 }
             }
             // ---- the item's share is done: write the partial (lane = channel) ----------------------
             reduce_mass();
-            if (failed || !wait_all(bar(kXtPvDone), (c - 1) & 1u)) failed = true;
+            if (failed || !wait_all(bar(kXtPvDone), (c - 1) & 1u) || !wait_all(bar(kXtPvDone + 1), (c - 1) & 1u)) failed = true;
             tc_fence_after();
             if (sg.slot < p.max_slots) {
                 float* dst = partials + (size_t)sg.slot * (R * kHeadDim + 2 * R);
