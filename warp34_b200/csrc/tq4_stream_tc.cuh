@@ -16,18 +16,18 @@
 //            hold 22 bits of the weights of small V rows as well (without it 7.9 % of the outputs over V of magnitude 2^-10 were not the
 //            nearest fp16 value, 4.1 % with three 8-row items of the one-warp kernel)
 //   V:       eight warps, thread = fragment position (16x256b stores put channel pairs of four keys in place), half x quadrant;
-//            64 keys at a time, values into one granule, residuals into the next
+//            64 keys at a time, values and residuals (one look-up for both) into neighbouring columns of one granule
 //   K:       eight warps, thread = key, 32 channels at a time into a ring of four TMEM granules; values and residuals lie next
 //            to each other as the table returns them, and the query operand repeats each pair of columns to match
 //   one warp copies raw pages and query rows, one issues the score products, one the output products
 //
-// Measured on 128 requests of 2048 to 16384 keys, four query tokens, 24 / 4 heads (1.26 GB of pages): attention call 870 us against 1458
-// with three 8-row items of the one-warp kernel (tq4_stream_exact.cuh), which looks every code up three times.  Bound by the softmax
-// warps' serial chain from scores to P and by the shared-memory data pipe that the look-ups share with them.  (Counters of the build whose
-// V residuals still had bank conflicts, 877 us: 6700 cycles and 14100 instructions a block of 128 keys, the pipe 72 % busy, the issue
-// slots 60 %, the tensor pipe 26 %.)  Taking the
-// weights before the vote on the reference (one barrier a block fewer) put them behind the wait for the previous output
-// product: 1008 us.
+// Measured on 128 requests of 2048 to 16384 keys, four query tokens, 24 / 4 heads (1.26 GB of pages): attention call 800 us against 1458
+// with three 8-row items of the one-warp kernel (tq4_stream_exact.cuh), which looks every code up three times.  A block of 128 keys takes
+// about 5000 cycles: the V warps' look-ups and stores (3500) and the chain from one block's output product over the next one's weights
+// to its own, which share the issue slots.  (With a look-up each for value and residual the V warps were busy for 5700 of 6170
+// cycles, and with one barrier for all keys the weights waited for the whole product before: 895 us.)  Taking the weights before the
+// vote on the reference (one barrier a block fewer) put them behind the wait for the previous output product: 1008 us.  Weights as
+// fragments of four keys by two rows a thread, stored 8 bytes at a time: 830, but 25 us instead of 26.5 on one short request.
 #pragma once
 
 namespace w34 {
@@ -663,6 +663,7 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                 }
                 dv.x *= v_up;
                 dv.y *= v_up;
+                const uint64_t dv2 = pair_of(dv.x, dv.y), minus_one = pair_of(-1.0f, -1.0f);
                 // 16-byte chunk of the key's column, swizzled by the row
                 const uint32_t at = p_t + (uint32_t)(key >> 6) * (uint32_t)(N * 128) + (uint32_t)row0 * 128u + 2u * (uint32_t)(key & 7) +
                                     (((uint32_t)(key & 63) >> 3) << 4);
@@ -670,10 +671,12 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                 for (int i = 0; i < P; ++i) {
                     const float w = ex2(sc[i] - m_lag[i]);
                     l[i] += w;
-                    const float x0 = w * dv.x, x1 = w * dv.y;
-                    const __half2 h = __floats2half2_rn(x0, x1);
+                    uint64_t x, rest;      // of both halves: w d_v, and what its fp16 values leave
+                    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(x) : "l"(pair_of(w, w)), "l"(dv2));
+                    const __half2 h = __floats2half2_rn(__uint_as_float((uint32_t)x), __uint_as_float((uint32_t)(x >> 32)));
                     const float2 hf = __half22float2(h);
-                    const uint32_t hi = *reinterpret_cast<const uint32_t*>(&h), lo = pack_half2(x0 - hf.x, x1 - hf.y);
+                    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(rest) : "l"(pair_of(hf.x, hf.y)), "l"(minus_one), "l"(x));
+                    const uint32_t hi = *reinterpret_cast<const uint32_t*>(&h), lo = pack_half2(__uint_as_float((uint32_t)rest), __uint_as_float((uint32_t)(rest >> 32)));
                     const uint32_t a = (at ^ (uint32_t)(i << 4)) + (uint32_t)i * 128u;
                     sts16(a, hi);
                     sts16(a + (uint32_t)R * 128u, lo);
