@@ -78,22 +78,41 @@ __device__ __forceinline__ void x_build_tables(uint32_t lut_addr) {
 
 // Query fragments of one work item as qprep_block() lays them out: value, and residual as bytes in units of the row's step,
 // widened here once per item.  `word(i)` reads word i of this lane.
-template <class Word>
-__device__ __forceinline__ void x_load_query(Word word, uint32_t (&qb)[16][2], uint32_t (&ql)[16][2]) {
+// FOUR: `word` reads the words of row gid % 4, and the lanes of rows 4-7 keep its residual in place of a value.
+template <bool FOUR, class Word>
+__device__ __forceinline__ void x_load_query(Word word, uint32_t (&qb)[16][2], uint32_t (&ql)[FOUR ? 1 : 16][2]) {
     const float step = __uint_as_float(word(48));
+    const bool low = FOUR && (threadIdx.x & 16) != 0;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
         qb[i][0] = word(2 * i);
         qb[i][1] = word(2 * i + 1);
         const uint32_t b = word(32 + i);
-        ql[i][0] = pack_half2((float)(b & 0xffu) * step, (float)((b >> 8) & 0xffu) * step);
-        ql[i][1] = pack_half2((float)((b >> 16) & 0xffu) * step, (float)(b >> 24) * step);
+        const uint32_t l0 = pack_half2((float)(b & 0xffu) * step, (float)((b >> 8) & 0xffu) * step);
+        const uint32_t l1 = pack_half2((float)((b >> 16) & 0xffu) * step, (float)(b >> 24) * step);
+        if (FOUR) {
+            qb[i][0] = low ? l0 : qb[i][0];
+            qb[i][1] = low ? l1 : qb[i][1];
+        } else {
+            ql[FOUR ? 0 : i][0] = l0;
+            ql[FOUR ? 0 : i][1] = l1;
+        }
     }
 }
 
 // The un-normalised output of one work item, [8 rows][256] in natural column order, into this warp's idle ring.
-__device__ __forceinline__ void x_stage_output(const XWarp& x, float* stage_o, const float (&o)[16][4]) {
+// FOUR: columns 4-7 hold the products of the weights' residuals; their sum with columns 0-3 is rows 0-3.
+template <bool FOUR>
+__device__ __forceinline__ void x_stage_output(const XWarp& x, float* stage_o, float (&o)[16][4]) {
     const int gid = x.gid, tig = x.tig;
+    if (FOUR) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) o[i][c] += __shfl_xor_sync(0xffffffffu, o[i][c], 2);
+        }
+        if (tig >= 2) return;      // rows 4-7 do not exist (their mass is 0)
+    }
 #pragma unroll
     for (int i4 = 0; i4 < 4; ++i4) {
         const int half = i4 >> 1, vw = 4 * (gid >> 1) + (gid & 1) + 2 * (i4 & 1);
@@ -110,7 +129,7 @@ __device__ __forceinline__ void x_stage_output(const XWarp& x, float* stage_o, c
 
 // Streams units [pg0, pg0 + n_here) of one work item.  `load_query(qb, ql)` runs once, after the first copies are on their way.
 // Leaves the accumulators, running maxima and row masses of this lane's rows (2 tig, 2 tig + 1); x.failed when a wait gave up.
-template <bool SPARSE, class LoadQuery>
+template <bool SPARSE, bool FOUR, class LoadQuery>
 __device__ __forceinline__ void x_stream(const StreamParams& p, XWarp& x, int r, const ReqGeom& g, int kv_head, int group, int pg0,
                                          int n_here, LoadQuery load_query, float (&o)[16][4], float (&m_run)[2], float (&l_row)[2]) {
     const int lane = x.lane, gid = x.gid, tig = x.tig, key_a = x.key_a, kv0 = x.kv0;
@@ -187,7 +206,7 @@ __device__ __forceinline__ void x_stream(const StreamParams& p, XWarp& x, int r,
     bool rvalid[2];
 #pragma unroll
     for (int y = 0; y < 2; ++y) {
-        const int row = group * kRowsPerGroup + 2 * tig + y;
+        const int row = group * kRowsPerGroup + 2 * (FOUR ? tig & 1 : tig) + y;
         const int q_off = row / p.gqa;
         rvalid[y] = row < rows_in_req &&
                     (p.batch.valid_token_mask == nullptr || p.batch.valid_token_mask[g.q_start + q_off] != 0);
@@ -202,7 +221,7 @@ __device__ __forceinline__ void x_stream(const StreamParams& p, XWarp& x, int r,
         safe_hi = min(safe_hi, __shfl_xor_sync(0xffffffffu, safe_hi, d));
         safe_lo = max(safe_lo, __shfl_xor_sync(0xffffffffu, safe_lo, d));
     }
-    uint32_t qb[16][2], ql[16][2];
+    uint32_t qb[16][2], ql[FOUR ? 1 : 16][2];
     load_query(qb, ql);
 #pragma unroll
     for (int i = 0; i < 16; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f; }
@@ -259,8 +278,10 @@ __device__ __forceinline__ void x_stream(const StreamParams& p, XWarp& x, int r,
                         mma16816(sh[half][0], a0.x, a0.y, a1.x, a1.y, qb[ks][0], qb[ks][1]);
                         mma16816(sh[half][1], b0.x, b0.y, b1.x, b1.y, qb[ks][0], qb[ks][1]);
                     }
-                    mma16816(sh[half][0], a0.x, a0.y, a1.x, a1.y, ql[ks][0], ql[ks][1]);
-                    mma16816(sh[half][1], b0.x, b0.y, b1.x, b1.y, ql[ks][0], ql[ks][1]);
+                    if (!FOUR) {
+                        mma16816(sh[half][0], a0.x, a0.y, a1.x, a1.y, ql[FOUR ? 0 : ks][0], ql[FOUR ? 0 : ks][1]);
+                        mma16816(sh[half][1], b0.x, b0.y, b1.x, b1.y, ql[FOUR ? 0 : ks][0], ql[FOUR ? 0 : ks][1]);
+                    }
                 }
             }
             const float dka0 = __half2float(__ushort_as_half((unsigned short)(ka0 & 0xffffu)));
@@ -273,6 +294,10 @@ __device__ __forceinline__ void x_stream(const StreamParams& p, XWarp& x, int r,
                            dka1 * (sh[1][0][c] + sh[1][0][c + 2] * (1.0f / kResidualScale));
                 pr[y][2 + c] = dkb0 * (sh[0][1][c] + sh[0][1][c + 2] * (1.0f / kResidualScale)) +
                                dkb1 * (sh[1][1][c] + sh[1][1][c + 2] * (1.0f / kResidualScale));
+            }
+            if (FOUR) {      // value and residual of the query
+#pragma unroll
+                for (int c = 0; c < 4; ++c) pr[y][c] += __shfl_xor_sync(0xffffffffu, pr[y][c], 2);
             }
             const int kv_base = (pg0 + 2 * st + y) << 4;
             int pos_a = kv_base + key_a, pos_b = pos_a + 4;
@@ -388,8 +413,12 @@ __device__ __forceinline__ void x_stream(const StreamParams& p, XWarp& x, int r,
                     const __half2 hi = __floats2half2_rn(pd[h][2 * z], pd[h][2 * z + 1]);
                     const float2 hf = __half22float2(hi);
                     const __half2 lo = __floats2half2_rn(pd[h][2 * z] - hf.x, pd[h][2 * z + 1] - hf.y);
-                    pb[h][z] = movmatrix_trans(*reinterpret_cast<const uint32_t*>(&hi));
-                    pl[h][z] = movmatrix_trans(*reinterpret_cast<const uint32_t*>(&lo));
+                    if (FOUR) {
+                        pb[h][z] = movmatrix_trans(tig < 2 ? *reinterpret_cast<const uint32_t*>(&hi) : *reinterpret_cast<const uint32_t*>(&lo));
+                    } else {
+                        pb[h][z] = movmatrix_trans(*reinterpret_cast<const uint32_t*>(&hi));
+                        pl[h][z] = movmatrix_trans(*reinterpret_cast<const uint32_t*>(&lo));
+                    }
                 }
             }
             // ---- O^T += V^T P^T.  Step i4: half i4 >> 1, virtual word 4 (gid >> 1) + (gid & 1) + 2 (i4 & 1) -----
@@ -402,7 +431,7 @@ __device__ __forceinline__ void x_stream(const StreamParams& p, XWarp& x, int r,
                 for (int t = 0; t < 4; ++t) {
                     const uint32_t a0 = W34_LUT(ab[0], t), a1 = W34_LUT(ab[1], t), a2 = W34_LUT(cd[0], t), a3 = W34_LUT(cd[1], t);
                     mma16816(o[4 * i4 + t], a0, a1, a2, a3, pb[i4 >> 1][0], pb[i4 >> 1][1]);
-                    mma16816(o[4 * i4 + t], a0, a1, a2, a3, pl[i4 >> 1][0], pl[i4 >> 1][1]);
+                    if (!FOUR) mma16816(o[4 * i4 + t], a0, a1, a2, a3, pl[i4 >> 1][0], pl[i4 >> 1][1]);
                 }
             }
         }
@@ -419,7 +448,7 @@ __device__ __forceinline__ void x_stream(const StreamParams& p, XWarp& x, int r,
 #pragma unroll
                 for (int z = 0; z < 2; ++z) {
                     const __half2 s2 = __floats2half2_rn(pd[h][2 * z] * (1.0f / kResidualScale), pd[h][2 * z + 1] * (1.0f / kResidualScale));
-                    ps[h][z] = movmatrix_trans(*reinterpret_cast<const uint32_t*>(&s2));
+                    ps[h][z] = movmatrix_trans(FOUR && tig >= 2 ? 0u : *reinterpret_cast<const uint32_t*>(&s2));
                 }
             }
 #pragma unroll
@@ -462,7 +491,10 @@ struct XHeld {
     uint32_t ring[kExactWarps];
 };
 
-template <bool SPARSE>
+// FOUR: items of at most four query rows.  The N = 8 columns of an MMA hold their values and, beside them, their rounding residuals (of the
+// query for the scores, of the weights for the output), so that one MMA does what takes two with eight rows: 48 instead of 96 a page
+// with the tensor pipe at 45 % and its issue among the stalls.
+template <bool SPARSE, bool FOUR>
 __global__ void __launch_bounds__(kXThreads, 1) tq4_attention_stream_exact_kernel(const StreamParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -530,17 +562,21 @@ __global__ void __launch_bounds__(kXThreads, 1) tq4_attention_stream_exact_kerne
         const int slot = w_global + item_prefix[r] + item;
         const ReqGeom g = stream_req(p, r);
         float o[16][4], m_run[2], l_row[2];
-        const uint32_t* qf = p.qfrag + ((size_t)(r * p.layout.local_kv_heads + kv_head) * p.q_groups_max + group) * (kQFragWords * 32) + lane;
-        x_stream<SPARSE>(p, x, r, g, kv_head, group, pg0, n_here,
+        const uint32_t* qf = p.qfrag + ((size_t)(r * p.layout.local_kv_heads + kv_head) * p.q_groups_max + group) * (kQFragWords * 32) + (FOUR ? lane & 15 : lane);
+        x_stream<SPARSE, FOUR>(p, x, r, g, kv_head, group, pg0, n_here,
                          // (not __ldg: the plan kernel was still writing these words when this one started)
-                         [&](uint32_t (&qb)[16][2], uint32_t (&ql)[16][2]) { x_load_query([&](int i) { return qf[i * 32]; }, qb, ql); },
+                         [&](uint32_t (&qb)[16][2], uint32_t (&ql)[FOUR ? 1 : 16][2]) { x_load_query<FOUR>([&](int i) { return qf[i * 32]; }, qb, ql); },
                          o, m_run, l_row);
         if (x.failed) {
             x_drain(x);
             if (lane == 0) atomicOr(&hdr->status, 1);
             break;
         }
-        x_stage_output(x, ring_gen, o);
+        x_stage_output<FOUR>(x, ring_gen, o);
+        if (FOUR && x.tig >= 2) {
+            m_run[0] = m_run[1] = -1e30f;
+            l_row[0] = l_row[1] = 0.0f;
+        }
         u += n_here;
         if (u >= u_end && neighbours) {      // the last segment: merged with the neighbours' below
             held = slot - w_global;
