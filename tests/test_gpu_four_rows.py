@@ -95,23 +95,33 @@ def test_four_row_lists_match_the_fp32_kernel(native_libs):
     assert ok, msg
 
 
-@pytest.mark.parametrize("new,status_bit", [([2, 1], 0), ([2, 0], 4)])
-def test_more_tokens_than_declared(native_libs, new, status_bit):
-    """Two tokens on four heads declared as one: where the batch's token count shows it they run as an item of eight rows, as ever; where
-    it does not, the second token's rows are left alone and the status says so."""
+@pytest.mark.parametrize("hq,new,declared,served,status_bit", [
+    (4, [2, 1], 1, [2, 1], 0),
+    (4, [2, 0], 1, [2, 0], 0),
+    (4, [1, 2, 0, 1], 1, [1, 2, 0, 1], 0),
+    (2, [4, 0, 0, 0], 1, [4, 0, 0, 0], 0),
+    (1, [5, 1, 0], 2, [5, 1, 0], 0),
+    (4, [2, 0], 0, [2, 0], 0),              # an undeclared length counts as one token
+    (4, [3, 0, 0], 1, [2, 0, 0], 4),        # twelve rows: an item holds eight, the rest is left alone
+])
+def test_more_tokens_than_declared(native_libs, hq, new, declared, served, status_bit):
+    """Requests of more tokens than the batch declares, up to eight query rows per kv head: answered in full, whatever the other requests
+    of the batch hold."""
+    import numpy as np
     from warp34_b200 import kv, synth
-    wl, ex = _workload(1, [60, 90], new)
+    wl, ex = _workload(1, [60 + 30 * r for r in range(len(new))], new)
     n = sum(new)
-    b = wl.step(max_q_len=1)
-    q = synth.make_q(n, 4, 13, device="cuda")
+    b = wl.step(max_q_len=declared)
+    q = synth.make_q(n, hq, 13, device="cuda")
 
     def call():
-        out = torch.full((n, 4, 256), -7.0, dtype=torch.float16, device="cuda")
-        kv.paged_attention(ex, wl.layer, b, q, out, 4)
+        out = torch.full((n, hq, 256), -7.0, dtype=torch.float16, device="cuda")
+        kv.paged_attention(ex, wl.layer, b, q, out, hq)
         return out
     (got, want), status = _both(ex, call)
     assert status == status_bit
-    rows = n if status_bit == 0 else 1
-    ok, msg = plain_parity(got[:rows].float().cpu().numpy(), want[:rows].float().cpu().numpy())
+    keep = np.concatenate([np.arange(t) < s for t, s in zip(new, served)])
+    got, want = got.float().cpu().numpy(), want.float().cpu().numpy()
+    ok, msg = plain_parity(got[keep], want[keep])
     assert ok, msg
-    assert (got[rows:] == -7.0).all()
+    assert (got[~keep] == -7.0).all()

@@ -554,7 +554,7 @@ struct PlanHeader {
     int32_t units_per_warp;
 };
 // Per request (num_reqs + 1 entries where it is a prefix sum), all int32, after the header:
-//   unit_prefix[r], item_prefix[r], page_lo[r], npages[r], ngroups[r]
+//   unit_prefix[r], item_prefix[r], page_lo[r], npages[r], ngroups[r]; page_lo[num_reqs] is a flag, see kRowsByPlan
 constexpr int kPlanArrays = 5;
 
 __host__ __device__ inline size_t plan_bytes(int num_reqs) {
@@ -589,7 +589,6 @@ struct StreamParams {
     int keep_status = 0;             // plan: OR into the status word instead of clearing it (second and later passes)
     int query_tiles = 0;             // qfrag holds tcgen05 operand tiles of rows_per_group rows instead of fragments
     int min_units = kMinUnitsPerWarp;    // smallest share of a worker
-    int item_rows = 0;                   // a request's rows beyond the first item_rows are dropped (0: none; the kernel for items of four)
     // Requests with more query rows per kv head than max_rows take no part (0: all do), and the merge's grid is tokens_per_req x q
     // heads for every request (0: x q heads for every token).
     int max_rows = 0, tokens_per_req = 0;
@@ -651,6 +650,7 @@ __global__ void __launch_bounds__(kPlanThreads) tq4_attention_plan_kernel(const 
     const int hkv = p.layout.local_kv_heads;
     int unit_carry = 0, item_carry = 0;
     bool clamped = false;
+    bool above_four = false;
     for (int base = 0; base < R; base += 32) {
         const int r = base + lane;
         int npages = 0, ngroups = 0, plo = 0;
@@ -672,7 +672,7 @@ __global__ void __launch_bounds__(kPlanThreads) tq4_attention_plan_kernel(const 
                 ngroups = (g.q_len * p.gqa + p.rows_per_group - 1) / p.rows_per_group;
                 // a request longer than the batch's max_q_len has no room in the fragment store
                 if (p.qfrag != nullptr && ngroups > p.q_groups_max) { ngroups = p.q_groups_max; clamped = true; }
-                if (p.item_rows != 0 && g.q_len * p.gqa > p.item_rows) clamped = true;
+                above_four = above_four || g.q_len * p.gqa > 4;
             }
         }
         const int items = hkv * ngroups;
@@ -694,11 +694,12 @@ __global__ void __launch_bounds__(kPlanThreads) tq4_attention_plan_kernel(const 
         unit_carry += __shfl_sync(0xffffffffu, iu, 31);
         item_carry += __shfl_sync(0xffffffffu, ii, 31);
     }
-    const bool clamped_any = __any_sync(0xffffffffu, clamped);
+    const bool clamped_any = __any_sync(0xffffffffu, clamped), above_four_any = __any_sync(0xffffffffu, above_four);
     if (lane == 0) {
         unit_prefix[R] = unit_carry;
         item_prefix[R] = item_carry;
-        page_lo[R] = 0; npages_a[R] = 0; ngroups_a[R] = 0;
+        page_lo[R] = above_four_any ? 1 : 0;      // some request has more than four query rows per kv head (dense batches)
+        npages_a[R] = 0; ngroups_a[R] = 0;
         PlanHeader* h = reinterpret_cast<PlanHeader*>(p.scratch);
         // bit 2: a request's q_len exceeded batch.max_q_len, rows dropped.  A later part of a batch that runs in
         // several passes keeps what the earlier passes reported.
@@ -1449,7 +1450,7 @@ __global__ void __launch_bounds__(MW * 32) tq4_attention_merge_kernel(const Stre
     const int rpg = p.rows_per_group;
     const int part_floats = rpg * kHeadDim + 2 * rpg;
     const int group = row_in_req / rpg, row8 = row_in_req - group * rpg;
-    if (group >= ngroups_a[r] || (p.item_rows != 0 && row_in_req >= p.item_rows)) { skip_row(); return; }  // rows the plan dropped (q_len above the declared max_q_len)
+    if (group >= ngroups_a[r]) { skip_row(); return; }  // rows the plan dropped (q_len above the declared max_q_len)
     const int item = kv_head * ngroups_a[r] + group;
     const int npages = npages_a[r];
     const int per = hdr->units_per_warp;
@@ -1732,8 +1733,8 @@ static DeviceInfo* device_info(int* rc) {
         *rc = (int)cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         if (*rc != 0) return nullptr;
         if ((size_t)optin < stream_smem_min_bytes()) { *rc = (int)cudaErrorNotSupported; return nullptr; }
-        for (auto* kernel : {tq4_attention_stream_exact_kernel<false, false>, tq4_attention_stream_exact_kernel<false, true>,
-                             tq4_attention_stream_exact_kernel<true, false>, tq4_attention_stream_exact_kernel<true, true>}) {
+        for (auto* kernel : {tq4_attention_stream_exact_kernel<false, kEightRows>, tq4_attention_stream_exact_kernel<false, kRowsByPlan>,
+                             tq4_attention_stream_exact_kernel<true, kEightRows>, tq4_attention_stream_exact_kernel<true, kFourRows>}) {
             *rc = (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
             if (*rc != 0) return nullptr;
         }
@@ -2207,11 +2208,10 @@ static int launch_attention(const warp34_exec* ex, const warp34_kv_layer_layout*
     const bool in_parts = reqs_per_pass < batch->num_reqs;
     cudaStream_t st = (cudaStream_t)ex->stream;
     const size_t smem = (size_t)dev->smem_optin;
-    // Items of at most four rows (a decode token on four heads or fewer) take half the MMAs.  Against the eight-row build, 16 / 4 heads, us a
+    // Items of at most four rows (a decode token on four heads or fewer) take fewer MMAs.  Against the eight-row build, 16 / 4 heads, us a
     // call: 64 sequences of 8192 to 32768 492.8 -> 413.1, 16 of 1024 to 8192 57.8 -> 49.6, 100 of 500 to 2000 90.2 -> 76.3, one of
-    // 262143 123.7 -> 104.7, one of 500 18.5 -> 17.9.  (More tokens than max_q_len allows in all: some request has more rows than it says,
-    // which items of eight hold.)
-    const bool four_rows = !fast && (long long)batch->total_tokens <= (long long)batch->num_reqs * (batch->max_q_len > 0 ? batch->max_q_len : 1) && (long long)(batch->max_q_len > 0 ? batch->max_q_len : 1) * gqa <= 4;
+    // 262143 123.7 -> 104.7, one of 500 18.5 -> 17.9.  Where the batch's declaration allows it the plan looks at the requests themselves.
+    const bool four_rows = !fast && (long long)(batch->max_q_len > 0 ? batch->max_q_len : 1) * gqa <= 4;
     for (int r0 = 0; r0 < batch->num_reqs; r0 += reqs_per_pass) {
         const int reqs = (batch->num_reqs - r0 < reqs_per_pass) ? batch->num_reqs - r0 : reqs_per_pass;
         StreamParams p;
@@ -2238,7 +2238,6 @@ static int launch_attention(const warp34_exec* ex, const warp34_kv_layer_layout*
         p.q_scale = batch->sm_scale * 1.4426950408889634f / kLutScale;
         p.natural = 0;
         p.q_floor = fast ? 0 : 1;
-        p.item_rows = four_rows ? 4 : 0;
         p.og = og;
         p.rows_from_first_token = in_parts ? 1 : 0;
         p.keep_status = r0 > 0 ? 1 : 0;
@@ -2248,7 +2247,7 @@ static int launch_attention(const warp34_exec* ex, const warp34_kv_layer_layout*
         rc = launch_behind(tq4_attention_plan_kernel, 1 + (unsigned)q_items, q_items > 0 ? kPlanThreads : 32, 0, st, p);
         if (rc != 0) return rc;
         if (fast) tq4_attention_stream_kernel<kFastStages, kFastWarps><<<grid, kFastWarps * 32, smem, st>>>(p);
-        else rc = launch_behind(four_rows ? tq4_attention_stream_exact_kernel<false, true> : tq4_attention_stream_exact_kernel<false, false>, (unsigned)grid, kXThreads, smem, st, p);
+        else rc = launch_behind(four_rows ? tq4_attention_stream_exact_kernel<false, kRowsByPlan> : tq4_attention_stream_exact_kernel<false, kEightRows>, (unsigned)grid, kXThreads, smem, st, p);
         // rows of the merge: every token of the batch, or (a part) as many as the part can hold, counted
         // from its first token
         const long long rows = (long long)p.batch.total_tokens * num_q_heads;
@@ -2418,7 +2417,7 @@ static int launch_qsa_stream(const warp34_exec* ex, const QsaParams& q, bool* ta
     cudaStream_t st = (cudaStream_t)ex->stream;
     rc = launch_behind(tq4_attention_plan_kernel, 1 + (unsigned)items, kPlanThreads, 0, st, p);
     if (rc != 0) return rc;
-    rc = launch_behind(gqa <= 4 ? tq4_attention_stream_exact_kernel<true, true> : tq4_attention_stream_exact_kernel<true, false>, (unsigned)grid, kXThreads, p.smem_bytes, st, p);
+    rc = launch_behind(gqa <= 4 ? tq4_attention_stream_exact_kernel<true, kFourRows> : tq4_attention_stream_exact_kernel<true, kEightRows>, (unsigned)grid, kXThreads, p.smem_bytes, st, p);
     const long long rows = (long long)q.num_tokens * q.num_q_heads;
     if (rc != 0) return rc;
     *taken = true;

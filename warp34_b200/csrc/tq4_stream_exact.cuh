@@ -494,42 +494,15 @@ struct XHeld {
     uint32_t ring[kExactWarps];
 };
 
+// One worker's share: units [u, u_end) of the step's list.  Writes the partial of every item but, where neighbours are merged, the last,
+// which stays in the worker's ring: returns it (its place among the slots, less the worker's), or -1.
 // FOUR: items of at most four query rows.  The N = 8 columns of an MMA hold their values and, beside them, their rounding residuals (of the
-// query for the scores, of the weights for the output), so that one MMA does what takes two with eight rows: 48 instead of 96 a page
+// query for the scores, of the weights for the output), so that one MMA does what takes two with eight rows: 48 a page instead of 80,
 // with the tensor pipe at 45 % and its issue among the stalls.
 template <bool SPARSE, bool FOUR>
-__global__ void __launch_bounds__(kXThreads, 1) tq4_attention_stream_exact_kernel(const StreamParams p) {
-    extern __shared__ __align__(1024) uint8_t smem[];
+__device__ __forceinline__ int x_share(const StreamParams& p, XWarp& x, PlanHeader* hdr, int u, int u_end, int w_global, bool neighbours,
+                                       float* ring_gen, XHeld& held_by) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    // The lookup table sits at the first 64 KB-aligned SHARED address inside the dynamic window, so that
-    // (table address | code byte << 8 | lane offset) is one PRMT.  Warp rings fill the space below and above it; the
-    // mbarriers follow the last ring.
-    const uint32_t win_lo = smem_u32(smem);
-    const uint32_t win_hi = win_lo + p.smem_bytes;
-    const uint32_t lut_addr = (win_lo + 0xffffu) & ~0xffffu;
-    constexpr uint32_t kRingBytes = 2u * kXSlot;
-    const uint32_t warps_below = (lut_addr - win_lo) / kRingBytes;
-    const uint32_t ring = ((uint32_t)wid < warps_below) ? (win_lo + (uint32_t)wid * kRingBytes)
-                                                         : (lut_addr + kLutBytes + ((uint32_t)wid - warps_below) * kRingBytes);
-    const uint32_t above = (uint32_t)kExactWarps > warps_below ? (uint32_t)kExactWarps - warps_below : 0u;
-    const uint32_t bars_base = lut_addr + kLutBytes + above * kRingBytes;
-    const uint32_t bars = bars_base + (uint32_t)wid * 16u;
-    PlanHeader* hdr = reinterpret_cast<PlanHeader*>(p.scratch);
-    if (lut_addr + kLutBytes > win_hi || bars_base + (uint32_t)kExactWarps * 16u + (uint32_t)sizeof(XHeld) > win_hi) {
-        grid_dependency_wait();
-        if (threadIdx.x == 0) atomicOr(&hdr->status, 2);  // shared-memory window cannot hold the layout
-        return;
-    }
-    XHeld& held_by = *reinterpret_cast<XHeld*>(smem + (bars_base + (uint32_t)kExactWarps * 16u - win_lo));
-    float* ring_gen = reinterpret_cast<float*>(smem + (ring - win_lo));
-
-    XWarp x;
-    x_init(x, lut_addr, ring, bars);
-    x_build_tables(lut_addr);
-    grid_dependency_wait();      // nothing above touches global memory
-    grid_launch_dependents();
-    __syncthreads();
-
     const int R = p.batch.num_reqs;
     const int32_t* unit_prefix = plan_array(p.scratch, 0, R);
     const int32_t* item_prefix = plan_array(p.scratch, 1, R);
@@ -538,18 +511,8 @@ __global__ void __launch_bounds__(kXThreads, 1) tq4_attention_stream_exact_kerne
     const int32_t* ngroups_a = plan_array(p.scratch, 4, R);
     float* partials = reinterpret_cast<float*>(p.scratch + plan_bytes(R));
 
-    const int per = hdr->units_per_warp;
-    const int total_units = hdr->total_units;
-    // A step with work for every worker: the eight workers of a CTA take neighbouring shares, so that what they hold of one
-    // item can be merged before it is written.  A smaller one: consecutive shares sit on different SMs.
-    const bool neighbours = per > kMinUnitsPerWarp;
-    const int w_global = neighbours ? (int)blockIdx.x * kExactWarps + wid : wid * (int)gridDim.x + (int)blockIdx.x;
-    const long long u_ll = (long long)w_global * per;
-    int u = (int)min(u_ll, (long long)total_units);
-    const int u_end = min(u + per, total_units);
     int r = u < u_end ? last_not_above(unit_prefix, R, u) : 0;
     int held = -1;      // item whose state this warp still holds when its share is done
-
 #pragma unroll 1
     while (u < u_end) {
         while (unit_prefix[r + 1] <= u) ++r;  // skips requests without units
@@ -608,7 +571,64 @@ __global__ void __launch_bounds__(kXThreads, 1) tq4_attention_stream_exact_kerne
         }
         __syncwarp();
     }
+    return held;
+}
+
+// Rows per item: eight, four, or four where the plan found that no request has more (kRowsByPlan: a batch that declares up to four, but a
+// request may hold more than its batch declares, and an item of eight still takes all of its rows then).
+enum ItemRows { kEightRows, kFourRows, kRowsByPlan };
+template <bool SPARSE, ItemRows ROWS>
+__global__ void __launch_bounds__(kXThreads, 1) tq4_attention_stream_exact_kernel(const StreamParams p) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    // The lookup table sits at the first 64 KB-aligned SHARED address inside the dynamic window, so that
+    // (table address | code byte << 8 | lane offset) is one PRMT.  Warp rings fill the space below and above it; the
+    // mbarriers follow the last ring.
+    const uint32_t win_lo = smem_u32(smem);
+    const uint32_t win_hi = win_lo + p.smem_bytes;
+    const uint32_t lut_addr = (win_lo + 0xffffu) & ~0xffffu;
+    constexpr uint32_t kRingBytes = 2u * kXSlot;
+    const uint32_t warps_below = (lut_addr - win_lo) / kRingBytes;
+    const uint32_t ring = ((uint32_t)wid < warps_below) ? (win_lo + (uint32_t)wid * kRingBytes)
+                                                         : (lut_addr + kLutBytes + ((uint32_t)wid - warps_below) * kRingBytes);
+    const uint32_t above = (uint32_t)kExactWarps > warps_below ? (uint32_t)kExactWarps - warps_below : 0u;
+    const uint32_t bars_base = lut_addr + kLutBytes + above * kRingBytes;
+    const uint32_t bars = bars_base + (uint32_t)wid * 16u;
+    PlanHeader* hdr = reinterpret_cast<PlanHeader*>(p.scratch);
+    if (lut_addr + kLutBytes > win_hi || bars_base + (uint32_t)kExactWarps * 16u + (uint32_t)sizeof(XHeld) > win_hi) {
+        grid_dependency_wait();
+        if (threadIdx.x == 0) atomicOr(&hdr->status, 2);  // shared-memory window cannot hold the layout
+        return;
+    }
+    XHeld& held_by = *reinterpret_cast<XHeld*>(smem + (bars_base + (uint32_t)kExactWarps * 16u - win_lo));
+    float* ring_gen = reinterpret_cast<float*>(smem + (ring - win_lo));
+
+    XWarp x;
+    x_init(x, lut_addr, ring, bars);
+    x_build_tables(lut_addr);
+    grid_dependency_wait();      // nothing above touches global memory
+    grid_launch_dependents();
+    __syncthreads();
+
+    const int R = p.batch.num_reqs;
+    const int per = hdr->units_per_warp;
+    const int total_units = hdr->total_units;
+    // A step with work for every worker: the eight workers of a CTA take neighbouring shares, so that what they hold of one
+    // item can be merged before it is written.  A smaller one: consecutive shares sit on different SMs.
+    const bool neighbours = per > kMinUnitsPerWarp;
+    const int w_global = neighbours ? (int)blockIdx.x * kExactWarps + wid : wid * (int)gridDim.x + (int)blockIdx.x;
+    const long long u_ll = (long long)w_global * per;
+    const int u = (int)min(u_ll, (long long)total_units);
+    const int u_end = min(u + per, total_units);
+    int held;
+    if constexpr (ROWS == kRowsByPlan) {
+        held = plan_array(p.scratch, 2, R)[R] == 0 ? x_share<SPARSE, true>(p, x, hdr, u, u_end, w_global, neighbours, ring_gen, held_by)
+                                                   : x_share<SPARSE, false>(p, x, hdr, u, u_end, w_global, neighbours, ring_gen, held_by);
+    } else {
+        held = x_share<SPARSE, ROWS == kFourRows>(p, x, hdr, u, u_end, w_global, neighbours, ring_gen, held_by);
+    }
     if (!neighbours) return;
+    float* partials = reinterpret_cast<float*>(p.scratch + plan_bytes(R));
 
     // ---- merge what the CTA's workers hold of one item: warp w does row w of every run of workers with the same item, the
     //      run's first slot takes the result, the others are left empty (l = 0) ------------------------------------
