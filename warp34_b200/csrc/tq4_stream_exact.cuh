@@ -13,7 +13,11 @@
 // another, every fragment had to be gathered with register moves: about 220 of 965 instructions per unit.)  The query's
 // rounding residual, fp16 as well, meets values only: one MMA takes those of both fragments' keys (its four operands are moved next to
 // each other), 80 MMAs a page instead of 96 with the residuals' half of each fragment along: 64 sequences of 8192 to 32768 on 24 / 4
-// heads 495 -> 473 us, error against float64 unchanged (what falls away is below the accumulators' rounding).
+// heads 495 -> 473 us.  What falls away, query residual by centroid residual, is at most 9.3e-8 of sum |q k| (the centroids lie within 9.5e-5 of
+// fp16 values, the residual is below 2^-10 of q), a twentieth of what the residual's own step of 1/255 leaves; the scores' error against
+// float64 over normal, outlier, sparse and large queries is 1 to 14 % lower than with all three products in one accumulator (2.08e-6 of the
+// scores instead of 2.10e-6 on the benchmark's values), and the same to three digits with the product added to the separate one.
+// Items of at most four rows keep it, at no cost (see x_share).
 #pragma once
 
 namespace w34 {
