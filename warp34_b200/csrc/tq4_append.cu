@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(128, PRODUCER ? kProducerBlocksPerSm : kAppend
         // ---- scale of the lane's half, codes, centroids, least-squares sums ----------------------------------
         // (a b of columns c + c of 16 further) + (those 8 and 24 further), for columns 2 r, 2 r + 1.  A sum of products is written
         // fma(x, one, y): the assembler makes one rounding of a packed product and the add behind it, .rn or not, unless the add is
-        // itself a product that it cannot know (3 of 66 million scales then differ by one unit).
+        // itself a product that it cannot know (22 of a million scales then differ; tests/test_gpu_append_edges.py holds rows that show it).
         auto quarter_sums = [&](const Pair (&x)[16], const Pair (&y)[16], float (&t)[8]) {
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
