@@ -112,6 +112,7 @@ template <int FMT> struct PpSmem {
     static constexpr uint32_t kBytes = kOffBars + 288u;
     static_assert(kPpCtaRows * kPpOutStride * 4 <= (int)kOffLut, "epilogue staging must end before the table");
     static_assert(kPpCtaRows * 512 <= (int)kOffQLo, "Q' staging fits the tile stages");
+    static_assert(!PpFormat<FMT>::kRotated || (kPpCtaRows / 4 + kPpWarps) * 2048 <= (int)kOffQLo, "so do the rows that change lanes behind it");
     static_assert(kBytes <= 227u * 1024u, "shared memory");
 };
 
