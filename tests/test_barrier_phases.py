@@ -1,11 +1,12 @@
-"""Parity waits of the two-CTA chunk kernel on the completion of its output products, checked on the CPU from the kernel's own
-expressions.
+"""Parity waits of the two-CTA chunk kernel and of the 9- to 24-row stream kernel on the completion of their output products, checked on
+the CPU from the kernels' own expressions.
 
 An mbarrier wait names a phase by its parity alone: it returns when the barrier's last completed phase has that parity, so it is
 sound only while at most that one phase can have completed.  A consumer warp may be held up for any time between two
 instructions (a slow instruction fetch, a context switch) while the tensor cores go on; what bounds them is that the output
 product of block i needs this warp's weights of block i."""
 import os
+import re
 
 import pytest
 
@@ -68,3 +69,30 @@ def test_a_delayed_consumer_warp_still_sees_the_phase_it_waits_for(which):
             for done in range(block, delivered + 1):           # products completed when the warp gets to look: at least, at most
                 phases = sum(slot_of(i) == slot for i in range(done + 1))
                 assert (phases - 1) & 1 == parity, f"{name}: j {j} of {n}, products up to {done} completed"
+
+
+# The stream kernel has a barrier for each half of a block's keys; the products of block c are number 2 c and 2 c + 1 and complete in
+# order.  Per wait, in the order of the source: the last product that is known to have completed, and the last that can have.
+XT_SRC = os.path.join(os.path.dirname(SRC), "tq4_stream_tc.cuh")
+XT_WAITS = [("start of block c", lambda c, half: 2 * (c - 2) + half, lambda c, half: 2 * c + half - 1),   # its own weights are still due
+            ("rescale in block c", lambda c, half: 2 * (c - 1) + half, lambda c, half: 2 * c - 1),        # all four warps' weights are due
+            ("end, first half", lambda c, half: 2 * (c - 2) + half, lambda c, half: 2 * c - 1),
+            ("end, second half", lambda c, half: 2 * (c - 1), lambda c, half: 2 * c - 1)]
+
+
+@pytest.mark.parametrize("which", range(4))
+def test_a_delayed_softmax_warp_still_sees_the_phase_it_waits_for(which):
+    with open(XT_SRC) as f:
+        code = "".join(x.split("//")[0] for x in f)
+    waits = re.findall(r"wait_all\(bar\((kXtPvDone[^,]*)\), ([^,;]*?1u)\)", code)
+    commits = re.findall(r"tc_commit\(bar\((kXtPvDone[^;]*)\)\);", code)
+    assert len(waits) == 4 and commits == ["kXtPvDone + kk"], (waits, commits)
+    (bar_expr, parity_expr), (name, known, most) = waits[which], XT_WAITS[which]
+    for c in range(1, 12):
+        for khalf in range(2):
+            env = {"kXtPvDone": 0, "khalf": khalf, "c": c}
+            half, parity = eval(bar_expr, env), eval(parity_expr.replace("1u", "1"), env)
+            for done in range(max(known(c, khalf), -1), most(c, khalf) + 1):
+                phases = sum(i % 2 == half for i in range(done + 1))
+                passes = (phases - 1) & 1 == parity
+                assert passes == (done >= 2 * (c - 1) + half), f"{name}: block {c}, half {khalf}, products up to {done} completed"

@@ -643,6 +643,9 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
                 // halves follow each other: one's weights are written while the other is multiplied.)
                 bad = bad || (c > 0 && !wait_all(bar(kXtPvDone + khalf), (c - 1) & 1u));
                 if (moved && b > 0) {
+                    // (The other half's barrier is not waited for in every block.  Its parity is enough all the same: products complete in
+                    // order, so that its phase before this one is over by the wait above, and this block's cannot be, for the other
+                    // half's weights come behind the barrier below.)
                     bad = bad || !wait_all(bar(kXtPvDone + (khalf ^ 1)), (c - 1) & 1u);
                     tc_fence_after();
 #pragma unroll 1
