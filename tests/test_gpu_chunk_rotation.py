@@ -1,6 +1,8 @@
 """The chunk kernel rotates its query rows and its outputs in groups of four: groups that end inside a tile, head groups that do not
-divide four, masked tokens inside a group, rows off a 16-byte boundary, with and without the output gate, in both activation types,
-against the fp32 dequant-then-attend path of the same entry point."""
+divide four, masked tokens inside a group, rows off a 16-byte boundary, with and without the output gate, and bf16 activations (which
+have no gated entry point), against the fp32 dequant-then-attend path of the same entry point."""
+import ctypes as C
+
 import pytest
 
 from util import plain_parity
@@ -56,6 +58,41 @@ def test_row_groups_match_dequant_then_attend(native_libs, hq, hkv, new, off, mo
         got, want = ((x.reshape(-1, 64) @ (h / 8).numpy()) for x in (got, want))
     ok, msg = plain_parity(got, want)
     assert ok, msg
+
+
+@pytest.mark.parametrize("hq,hkv,new,off,drop", [(3, 1, [43, 9], 0, (0, 2, 50)), (6, 1, [5, 64], 4, ()), (10, 2, [51, 52], 1, (3,))])
+def test_bf16_row_groups_match_dequant_then_attend(native_libs, hq, hkv, new, off, drop):
+    """Both outputs are rounded to bf16: 2^-9 of the value each, on top of the plain bound."""
+    import numpy as np
+    from util import ATOL, RTOL
+    from warp34_b200 import ffi, kv, synth
+    wl = synth.PagedWorkload([70] * len(new), new, hkv, seed=3)
+    ex = kv.Executor(64 << 20)
+    wl.fill_context(ex, 3)
+    n = sum(new)
+    k, v = synth.make_kv(n, hkv, 4, device="cuda")
+    kv.kv_cache_write(ex, wl.layer, wl.step(), k, v)
+    vtm = np.ones(n, np.uint8)
+    vtm[list(drop)] = 0
+    b = wl.step(valid_token_mask=vtm)
+
+    def shifted(t):
+        store = torch.zeros(t.numel() + 8, dtype=torch.bfloat16, device="cuda")
+        store[off:off + t.numel()] = t.reshape(-1).to(torch.bfloat16)
+        return store[off:off + t.numel()].view(n, hq, 256)
+
+    q, outs = shifted(synth.make_q(n, hq, 5, device="cuda")), []
+    for flags in (0, ffi.EXEC_FLAG_PRECISE_ATTENTION):
+        ex.ex.flags = flags
+        out = shifted(torch.full((n, hq, 256), -7.0, device="cuda"))
+        assert native_libs[0].warp34_tq4_paged_attention_bf16(C.byref(ex.ex), C.byref(wl.layer.layout), C.byref(b.desc), q.data_ptr(), out.data_ptr(), hq) == 0
+        torch.cuda.synchronize()
+        outs.append(out.float().cpu().numpy())
+    keep = vtm.astype(bool)
+    assert (outs[0][~keep] == -7.0).all()
+    got, want = outs[0][keep], outs[1][keep]
+    bound = ATOL + (RTOL + 2.0 ** -8) * np.abs(want)
+    assert (np.abs(got - want) <= bound).all(), float((np.abs(got - want) / bound).max())
 
 
 @pytest.mark.parametrize("reqs", [8, 9, 32, 33, 70])

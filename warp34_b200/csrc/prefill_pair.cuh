@@ -587,7 +587,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
         }
     }
 
-    // ---- Q rows of this CTA: one warp per row.  TQ4: rotated, scaled, split into value (staging) and
+    // ---- Q rows of this CTA: four rows a warp, eight lanes each.  TQ4: rotated, scaled, split into value (staging) and
     //      residual (swizzled A tile); 8-bit: the fp16 row as it is ------------------------------------
     const uint32_t q_stage = k_t;     // 128 rows x 512 B over the tile stages
     {
@@ -1050,7 +1050,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPpThreads, 1) atten
     __syncthreads();
     if (!aborted) {
         const int first_token = place[2], rows = place[3], q_start = place[4];
-        const bool by_rows = !fits || p.splits > 1;      // (the rare tile that is computed in fp32; no rotation here)
+        const bool by_rows = !fits || p.splits > 1;      // (tiles that are computed in fp32, and parts of a tile's keys, which are not rotated here)
         if (by_rows) {
             for (int row = wid; row < kPpCtaRows; row += kPpWarps) {
                 const int trow = (int)cluster_rank() * kPpCtaRows + row;

@@ -332,30 +332,24 @@ __device__ __forceinline__ void load8(const void* base, size_t row_base, int lan
     load8_raw(base, row_base, lane, w);
     widen8(w, bf16, v);
 }
-__device__ __forceinline__ void narrow8(const float (&v)[8], int bf16, uint32_t (&w)[4]) {
+__device__ __forceinline__ void store8(void* base, size_t row_base, int lane, int bf16, const float (&v)[8]) {
+    uint16_t* dst = static_cast<uint16_t*>(base) + row_base + 8 * lane;
+    uint32_t w[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         if (bf16) {
-            const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-            w[i] = *reinterpret_cast<const uint32_t*>(&h);
+            const __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+            w[i] = *reinterpret_cast<const uint32_t*>(&b);
         } else {
             w[i] = pack_half2(v[2 * i], v[2 * i + 1]);
         }
     }
-}
-__device__ __forceinline__ void store8_raw(void* base, size_t row_base, int lane, const uint32_t (&w)[4]) {
-    uint16_t* dst = static_cast<uint16_t*>(base) + row_base + 8 * lane;
     if (((uintptr_t)base & 15u) == 0u) {
         *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
     } else {
 #pragma unroll
         for (int i = 0; i < 4; ++i) { dst[2 * i] = (uint16_t)w[i]; dst[2 * i + 1] = (uint16_t)(w[i] >> 16); }
     }
-}
-__device__ __forceinline__ void store8(void* base, size_t row_base, int lane, int bf16, const float (&v)[8]) {
-    uint32_t w[4];
-    narrow8(v, bf16, w);
-    store8_raw(base, row_base, lane, w);
 }
 // Butterfly over column bits [3, 3 + LEVELS): lanes.  Upper lane o - x, lower x + o, one rounding either way.
 template <int LEVELS>
@@ -2208,9 +2202,9 @@ static int launch_attention(const warp34_exec* ex, const warp34_kv_layer_layout*
     const bool in_parts = reqs_per_pass < batch->num_reqs;
     cudaStream_t st = (cudaStream_t)ex->stream;
     const size_t smem = (size_t)dev->smem_optin;
-    // Items of at most four rows (a decode token on four heads or fewer) take fewer MMAs.  Against the eight-row build, 16 / 4 heads, us a
-    // call: 64 sequences of 8192 to 32768 492.8 -> 413.1, 16 of 1024 to 8192 57.8 -> 49.6, 100 of 500 to 2000 90.2 -> 76.3, one of
-    // 262143 123.7 -> 104.7, one of 500 18.5 -> 17.9.  Where the batch's declaration allows it the plan looks at the requests themselves.
+    // Items of at most four rows (a decode token on four heads or fewer) take 48 MMAs a page instead of 80.  Against the eight-row build, 16 / 4
+    // heads, us a call: 64 sequences of 8192 to 32768 469.8 -> 406.4, 16 of 1024 to 8192 56.1 -> 49.3, 100 of 500 to 2000 87.8 -> 75.5, one
+    // of 262143 118.8 -> 103.4, one of 500 18.8 -> 17.7.  Where the batch's declaration allows it the plan looks at the requests themselves.
     const bool four_rows = !fast && (long long)(batch->max_q_len > 0 ? batch->max_q_len : 1) * gqa <= 4;
     for (int r0 = 0; r0 < batch->num_reqs; r0 += reqs_per_pass) {
         const int reqs = (batch->num_reqs - r0 < reqs_per_pass) ? batch->num_reqs - r0 : reqs_per_pass;
