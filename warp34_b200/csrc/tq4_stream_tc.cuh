@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(xt_threads(R), 1) tq4_attention_stream_tc_kern
         return false;
     };
 
-    for (int i = tid; i < 256 * 16; i += xt_threads(R)) {      // per byte: {values, residuals} x 16
+    for (int i = tid; i < 256 * 16; i += xt_threads(R)) {      // per byte: {values, residuals} x 16, 256 bytes apart (an address is one byte_perm; 128 are unused)
         const int byte = i >> 4, ln = i & 15;
         const float c0 = kLutScale * tq4_centroid(byte & 15), c1 = kLutScale * tq4_centroid(byte >> 4);
         const uint32_t hi = pack_half2(c0, c1);
